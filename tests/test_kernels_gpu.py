@@ -100,6 +100,25 @@ def test_gemm_simt(dtype, M, N, K):
     assert (got2 - (acc + R.gemm_ref(a, w))).abs().max() <= 2e-6 * math.sqrt(K) * ref.abs().max() + 1e-6
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K", [(31, 127), (33, 1024), (65, 1031), (130, 2052), (64, 9000)])
+def test_gemm_simt_rows_do_not_depend_on_the_batch(dtype, N, K):
+    """Every count of rows at which another kernel or tile takes over, at sizes around a chunk (128 channels) and a section (1,024):
+    against 64-bit products, and row by row the same bits whatever rows stand beside it.  A sum is a chain of 128 products, at most 8
+    chunks and ceil(K / 1024) sections long: gamma = (128 + 8 + sections + 2) 2^-24 times the sum of the products' sizes."""
+    k = _k()
+    a, w, b = _rand(300, K, dtype=dtype), _rand(N, K, dtype=dtype, seed=1), _rand(N, seed=2)
+    ref = a.double() @ w.double().t() + b.double()
+    bound = (138 + -(-K // 1024)) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t() + b.double().abs())
+    whole = k.gemm_simt(a, w, bias=b)
+    assert bool(((whole.double() - ref).abs() <= bound).all())
+    for M in (1, 2, 3, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129):
+        assert torch.equal(k.gemm_simt(a[:M].contiguous(), w, bias=b), whole[:M]), M
+    acc = _rand(33, N, seed=3)
+    for M in (5, 33):
+        assert torch.equal(k.gemm_simt(a[:M].contiguous(), w, bias=b, out=acc[:M].clone(), accumulate=True), acc[:M] + whole[:M]), M
+
+
 def _paged_case(nh, nkv, hd, ps, lens, dtype, seed=0):
     """Requests of the given lengths scattered over shuffled pages; queries for the last few positions."""
     g = torch.Generator().manual_seed(seed)
