@@ -1,101 +1,466 @@
 // Paged causal grouped-query attention on the CUDA cores, fp32 arithmetic throughout.
 //
-// One warp per (token, query head).  A token of request r at position p attends to the keys of r at
-// positions max(0, p - window + 1) .. p, read from the paged cache through r's block table, in order,
-// with an online softmax:  s_j = (q . k_j) / sqrt(HD);  o = sum_j softmax(s)_j v_j
-// (formulas of src/operators/cuda/cuda_flash_attn.cu:154-248 and :297-439; kv head = q head / (NH/NKV)).
-// Because a token's keys are always walked in the same order, its result does not depend on how the
-// request was cut into steps or on what else is in the batch.  This kernel serves the true 32-bit path
-// and any shape the tensor-core kernel refuses: any HD <= 256, any NH/NKV ratio, any page size.
+// A token of request r at position p attends to the keys of r at positions max(0, p - window + 1) .. p, read from the paged cache
+// through r's block table, with an online softmax:  s_j = (q . k_j) / sqrt(HD);  o = sum_j softmax(s)_j v_j
+// (formulas of src/operators/cuda/cuda_flash_attn.cu:154-248 and :297-439; kv head = q head / (NH/NKV)).  It serves the true 32-bit
+// path and any shape the tensor-core kernels refuse: any HD <= 256, any NH/NKV ratio, any page size, any list of tokens.
+//
+// A row (one query head of one token) walks its keys in blocks of 32 that start at multiples of 32 and segments of 64 that start
+// at multiples of 64: a block's scores are dealt to the lanes (lane j: key j), the block's maximum moves the row's reference, the weights
+// are summed by the butterfly and the values added key by key; a segment starts afresh and joins the row's total when it ends,
+// segments in order.  What a row adds up in which order is thus fixed by its position, not by how its request was cut into steps or by what
+// else is in the batch, although two kernels share the work:
+//   tiles     steps of many tokens: a CTA of eight warps takes 32 rows of one kv head, four rows a warp, keys and values through two
+//             buffers in shared memory (cp.async) that all its rows share.  (One warp per row, key by key, which this replaces, waited for
+//             ten shuffles a key.)
+//   segments  steps of few tokens: a CTA, or a cluster of up to eight, takes up to four heads of one token, a warp a segment, read
+//             straight from global memory; the segments' sums meet in (distributed) shared memory.
+// The line between the two is where the tiles alone fill the 148 SMs.  32 / 4 heads of 64 in 32 bits: prompts of 111 and 222 tokens 210 -> 52 us,
+// one token of each 210 -> 42 us.
+#include <algorithm>
 #include "common.cuh"
 #include "checks.cuh"
 
 namespace {
 
-template <int DPL, typename T>  // DPL = dims per lane = ceil(HD / 32)
-__global__ void __launch_bounds__(128)
-paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ kv_cache,
-                            const int32_t* __restrict__ block_table, const int32_t* __restrict__ tok_req,
-                            const int32_t* __restrict__ positions, T* __restrict__ out, int T_tokens, int NH,
-                            int NKV, int HD, int page_size, int max_pages, int window, float scale) {
+constexpr int kRows = 4, kWarps = 8, kBlock = 32, kSegment = 64, kTileRows = kRows * kWarps, kMaxCluster = 8;
+
+// A block's share of kRows rows in one warp.  q: the rows' scaled queries in shared memory, [kRows][HDP]; k(d): four channels of this lane's key
+// from channel d on; v(j, i): channel lane + 32 i of key j.  lo/hi: the keys (0..31 within the block) that a row sees, hi < lo: none.
+template <int DPL, typename KF, typename VF>
+__device__ __forceinline__ void walk_block(const float* __restrict__ q, int HDP, const int (&lo)[kRows], const int (&hi)[kRows], bool key_ok, float* __restrict__ ps,
+                                           KF k, VF v, float (&m)[kRows], float (&l)[kRows], float (&acc)[kRows][DPL]) {
+    const int lane = threadIdx.x & 31;
+    float4 d4[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) d4[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int d = 0; d < HDP; d += 4) {
+        const float4 kk = k(d);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const float4 qq = *reinterpret_cast<const float4*>(q + r * HDP + d);
+            d4[r].x = fmaf(qq.x, kk.x, d4[r].x);
+            d4[r].y = fmaf(qq.y, kk.y, d4[r].y);
+            d4[r].z = fmaf(qq.z, kk.z, d4[r].z);
+            d4[r].w = fmaf(qq.w, kk.w, d4[r].w);
+        }
+    }
+    float s[kRows], top[kRows], sum[kRows];
+    bool whole = true;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        s[r] = key_ok && lane >= lo[r] && lane <= hi[r] ? (d4[r].x + d4[r].y) + (d4[r].z + d4[r].w) : -INFINITY;
+        top[r] = s[r];
+        whole = whole && lo[r] <= 0 && hi[r] >= kBlock - 1;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], o));
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        const float m_new = fmaxf(m[r], top[r]), ref = m_new == -INFINITY ? 0.f : m_new;       // (a row that has seen nothing yet)
+        const float alpha = expf(m[r] - ref);                                                  // expf(-inf) = 0
+        s[r] = expf(s[r] - ref);
+        sum[r] = s[r];
+        m[r] = m_new;
+        l[r] = l[r] * alpha;
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) acc[r][i] *= alpha;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) l[r] += sum[r];
+    __syncwarp();                                                                              // the weights of the block before have been read
+    *reinterpret_cast<float4*>(ps + lane * kRows) = make_float4(s[0], s[1], s[2], s[3]);
+    __syncwarp();
+    if (whole) {
+#pragma unroll 8
+        for (int j = 0; j < kBlock; ++j) {
+            const float4 p4 = *reinterpret_cast<const float4*>(ps + j * kRows);
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) {
+                const float vv = v(j, i);
+                acc[0][i] = fmaf(p4.x, vv, acc[0][i]);
+                acc[1][i] = fmaf(p4.y, vv, acc[1][i]);
+                acc[2][i] = fmaf(p4.z, vv, acc[2][i]);
+                acc[3][i] = fmaf(p4.w, vv, acc[3][i]);
+            }
+        }
+    } else {
+        // a key that a row does not see takes no part in it, whatever number lies there
+        int first = kBlock, last = -1;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+            if (hi[r] >= lo[r]) { first = min(first, max(lo[r], 0)); last = max(last, min(hi[r], kBlock - 1)); }
+        for (int j = first; j <= last; ++j) {
+            const float4 p4 = *reinterpret_cast<const float4*>(ps + j * kRows);
+            const float pv[kRows] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) {
+                const float vv = v(j, i);
+#pragma unroll
+                for (int r = 0; r < kRows; ++r)
+                    if (j >= lo[r] && j <= hi[r]) acc[r][i] = fmaf(pv[r], vv, acc[r][i]);
+            }
+        }
+    }
+}
+
+// A segment's sums join the total: the same operations wherever it happens.
+__device__ __forceinline__ void join_weights(float mt, float ms, float& m, float& a, float& b) {
+    m = fmaxf(mt, ms);
+    a = mt == -INFINITY ? 0.f : expf(mt - m);
+    b = ms == -INFINITY ? 0.f : expf(ms - m);
+}
+__device__ __forceinline__ float join(float total, float a, float part, float b) { return fmaf(total, a, __fmul_rn(part, b)); }
+
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool ok) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+struct SimtAttention {
+    const void *q, *kv;
+    const int32_t *block_table, *tok_req, *positions;
+    void* out;
+    int T, NH, NKV, HD, page_size, max_pages, window;
+    float scale;
+    int vec;                    // rows of keys and values may be read 16 bytes (four numbers of 16 bits: 8) at a time
+};
+
+template <typename T> __device__ __forceinline__ float4 four(const T* p, int n, bool vec);       // n numbers are there, the rest counts as zero
+template <> __device__ __forceinline__ float4 four<float>(const float* p, int n, bool vec) {
+    if (vec) return *reinterpret_cast<const float4*>(p);
+    return make_float4(p[0], n > 1 ? p[1] : 0.f, n > 2 ? p[2] : 0.f, n > 3 ? p[3] : 0.f);
+}
+template <> __device__ __forceinline__ float4 four<__nv_bfloat16>(const __nv_bfloat16* p, int n, bool vec) {
+    if (vec) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(p);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+    return make_float4(__bfloat162float(p[0]), n > 1 ? __bfloat162float(p[1]) : 0.f, n > 2 ? __bfloat162float(p[2]) : 0.f, n > 3 ? __bfloat162float(p[3]) : 0.f);
+}
+
+__host__ __device__ __forceinline__ int padded(int HD) { return (HD + 3) / 4 * 4; }
+__host__ __device__ __forceinline__ int key_stride(int HD) { return padded(HD) + ((padded(HD) / 4) % 2 == 0 ? 4 : 8); }      // an odd number of 16-byte pieces
+
+// ------------------------------------------------------------------------------------------------ tiles of 32 rows
+template <int DPL, typename T>
+__global__ void __launch_bounds__(32 * kWarps)
+simt_tiles_kernel(const SimtAttention d) {
+    extern __shared__ __align__(16) float sm[];
     forge::pdl_launch_dependents();
     forge::pdl_wait();
-    const int warp_global = blockIdx.x * 4 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (warp_global >= T_tokens * NH) return;
-    const int t = warp_global / NH, h = warp_global % NH;
-    const int kvh = h / (NH / NKV);
-    const int pos = positions[t];
-    const int32_t* table = block_table + (size_t)tok_req[t] * max_pages;
-    if (!FORGE_TOKEN_OK(t)) return;
-
-    float qr[DPL], acc[DPL];
-#pragma unroll
-    for (int i = 0; i < DPL; ++i) {
-        const int d = lane + 32 * i;
-        qr[i] = d < HD ? forge::to_float(q[(size_t)t * NH * HD + h * HD + d]) * scale : 0.f;
-        acc[i] = 0.f;
+    const int HD = d.HD, HDP = padded(HD), KS = key_stride(HD), G = d.NH / d.NKV, kvh = blockIdx.y;
+    float* qs = sm;                                        // [32 rows][HDP]
+    float* kb = qs + kTileRows * HDP;                      // [2][32 keys][KS]
+    float* vb = kb + 2 * kBlock * KS;                      // [2][32 keys][HDP]
+    float* ps = vb + 2 * kBlock * HDP;                     // [8 warps][32 keys][4 rows]
+    __shared__ int s_pos[kTileRows], s_req[kTileRows], s_ok[2][kBlock];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const T* q = (const T*)d.q;
+    const T* kv = (const T*)d.kv;
+    const long long r0 = (long long)blockIdx.x * kTileRows, all = (long long)d.T * G;
+    const int rows = (int)min((long long)kTileRows, all - r0);
+    const int t0 = (int)(r0 / G), nt = (int)((r0 + rows - 1) / G) - t0 + 1;        // the tile's tokens
+    if (tid < nt) {
+        s_pos[tid] = d.positions[t0 + tid];
+        s_req[tid] = FORGE_TOKEN_OK(t0 + tid) ? d.tok_req[t0 + tid] : -1;
     }
-    float m = -INFINITY, l = 0.f;
-    int j = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
-    while (j <= pos) {
-        const int page_idx = j / page_size, off0 = j % page_size;
-        const int page = table[page_idx];
-        const int n_here = min(page_size - off0, pos - j + 1);
-        if (!FORGE_PAGE_OK(page)) { j += n_here; continue; }          // (checks build) a page outside the pool is skipped
-        const T* kp = kv_cache + (((size_t)page * 2 + 0) * NKV + kvh) * page_size * HD;
-        const T* vp = kv_cache + (((size_t)page * 2 + 1) * NKV + kvh) * page_size * HD;
-        for (int o = off0; o < off0 + n_here; ++o) {
-            float part = 0.f;
+    for (int i = tid; i < kTileRows * HDP; i += 32 * kWarps) {
+        const int r = i / HDP, c = i % HDP;
+        const long long row = r0 + r;
+        qs[i] = r < rows && c < HD ? forge::to_float(q[(size_t)(row / G) * d.NH * HD + (size_t)(kvh * G + row % G) * HD + c]) * d.scale : 0.f;
+    }
+    __syncthreads();
+    int pos[kRows], req[kRows];
+    float mt[kRows], lt[kRows], at[kRows][DPL];
 #pragma unroll
-            for (int i = 0; i < DPL; ++i) {
-                const int d = lane + 32 * i;
-                if (d < HD) part = fmaf(qr[i], forge::to_float(kp[(size_t)o * HD + d]), part);
-            }
-            const float s = forge::warp_sum(part);
-            const float m_new = fmaxf(m, s);
-            const float alpha = expf(m - m_new);   // expf(-inf) = 0 on the first key
-            const float p = expf(s - m_new);
-            l = l * alpha + p;
+    for (int r = 0; r < kRows; ++r) {
+        const int rr = warp * kRows + r;
+        const int tt = rr < rows ? (int)((r0 + rr) / G) - t0 : 0;
+        pos[r] = s_pos[tt];
+        req[r] = rr < rows ? s_req[tt] : -1;
+        mt[r] = -INFINITY;
+        lt[r] = 0.f;
 #pragma unroll
-            for (int i = 0; i < DPL; ++i) {
-                const int d = lane + 32 * i;
-                const float v = d < HD ? forge::to_float(vp[(size_t)o * HD + d]) : 0.f;
-                acc[i] = fmaf(p, v, acc[i] * alpha);
-            }
-            m = m_new;
+        for (int i = 0; i < DPL; ++i) at[r][i] = 0.f;
+    }
+    const int pieces = HDP / 4;
+    for (int a = 0; a < nt;) {                             // runs of tokens of one request
+        const int run_req = s_req[a];
+        int b = a, most = -1, least = 0x7fffffff;
+        for (; b < nt && s_req[b] == run_req; ++b) {
+            most = max(most, s_pos[b]);
+            least = min(least, d.window > 0 ? max(0, s_pos[b] - d.window + 1) : 0);
         }
-        j += n_here;
-    }
-    const float inv = 1.0f / l;
+        a = b;
+        if (run_req < 0) continue;
+        const int32_t* table = d.block_table + (size_t)run_req * d.max_pages;
+        auto fetch = [&](int blk, int buf) {
+            for (int i = tid; i < kBlock * pieces; i += 32 * kWarps) {
+                const int r = i / pieces, c = (i % pieces) * 4, j = blk * kBlock + r;
+                const bool seen = j >= least && j <= most;
+                const int page = seen ? table[j / d.page_size] : -1;
+                const bool ok = seen && FORGE_PAGE_OK(page) && page >= 0;      // (checks build) a page outside the pool is skipped
+                const size_t at_k = ok ? (((size_t)page * 2 * d.NKV + kvh) * d.page_size + j % d.page_size) * HD + c : 0;
+                const size_t at_v = ok ? at_k + (size_t)d.NKV * d.page_size * HD : 0;
+                float* kd = kb + (buf * kBlock + r) * KS + c;
+                float* vd = vb + (buf * kBlock + r) * HDP + c;
+                if (sizeof(T) == 4 && d.vec) {
+                    copy16(kd, kv + at_k, ok);
+                    copy16(vd, kv + at_v, ok);
+                } else {
+                    *reinterpret_cast<float4*>(kd) = ok ? four<T>(kv + at_k, HD - c, d.vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<float4*>(vd) = ok ? four<T>(kv + at_v, HD - c, d.vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                if (c == 0) s_ok[buf][r] = ok;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        const int first = least / kBlock, last = most / kBlock;
+        float m[kRows], l[kRows], acc[kRows][DPL];
+        auto afresh = [&]() {
 #pragma unroll
-    for (int i = 0; i < DPL; ++i) {
-        const int d = lane + 32 * i;
-        if (d < HD) out[(size_t)t * NH * HD + h * HD + d] = forge::from_float<T>(acc[i] * inv);
+            for (int r = 0; r < kRows; ++r) {
+                m[r] = -INFINITY;
+                l[r] = 0.f;
+#pragma unroll
+                for (int i = 0; i < DPL; ++i) acc[r][i] = 0.f;
+            }
+        };
+        auto settle = [&]() {
+#pragma unroll
+            for (int r = 0; r < kRows; ++r) {
+                float mm, fa, fb;
+                join_weights(mt[r], m[r], mm, fa, fb);
+                if (m[r] != -INFINITY) {
+                    mt[r] = mm;
+                    lt[r] = join(lt[r], fa, l[r], fb);
+#pragma unroll
+                    for (int i = 0; i < DPL; ++i) at[r][i] = join(at[r][i], fa, acc[r][i], fb);
+                }
+            }
+        };
+        afresh();
+        fetch(first, 0);
+        for (int blk = first; blk <= last; ++blk) {
+            const int buf = (blk - first) & 1;
+            if (blk < last) fetch(blk + 1, buf ^ 1);
+            else asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+            int lo[kRows], hi[kRows];
+            bool any = false;
+#pragma unroll
+            for (int r = 0; r < kRows; ++r) {
+                lo[r] = (d.window > 0 ? max(0, pos[r] - d.window + 1) : 0) - blk * kBlock;
+                hi[r] = req[r] == run_req ? pos[r] - blk * kBlock : -1;
+                if (hi[r] < 0 || lo[r] >= kBlock) { lo[r] = 0; hi[r] = -1; }
+                any = any || hi[r] >= lo[r];
+            }
+            if (any) {
+                const float* kr = kb + (buf * kBlock + lane) * KS;
+                const float* vr = vb + buf * kBlock * HDP;
+                walk_block<DPL>(qs + warp * kRows * HDP, HDP, lo, hi, s_ok[buf][lane] != 0, ps + warp * kBlock * kRows,
+                                   [&](int c) { return *reinterpret_cast<const float4*>(kr + c); },
+                                   [&](int j, int i) { const int c = lane + 32 * i; return c < HDP ? vr[j * HDP + c] : 0.f; }, m, l, acc);
+            }
+            if ((blk + 1) % (kSegment / kBlock) == 0) {
+                settle();
+                afresh();
+            }
+            __syncthreads();                               // before a later copy overwrites this buffer
+        }
+        settle();
     }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        const int rr = warp * kRows + r;
+        if (rr >= rows || req[r] < 0) continue;
+        const long long row = r0 + rr;
+        const float inv = 1.0f / lt[r];
+        T* dst = (T*)d.out + (size_t)(row / G) * d.NH * HD + (size_t)(kvh * G + row % G) * HD;
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) {
+            const int c = lane + 32 * i;
+            if (c < HD) dst[c] = forge::from_float<T>(at[r][i] * inv);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ a token's segments
+__device__ __forceinline__ float peer_load(const float* p, int rank, bool remote_ok) {
+    if (!remote_ok) return *p;
+    uint32_t remote;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+__device__ __forceinline__ void meet(int cluster) {
+    if (cluster > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else __syncthreads();
+}
+
+template <int DPL, typename T>
+__global__ void __launch_bounds__(32 * kWarps)
+simt_segments_kernel(const SimtAttention d, int cluster) {
+    extern __shared__ __align__(16) float sm[];
+    forge::pdl_launch_dependents();
+    forge::pdl_wait();
+    const int HD = d.HD, HDP = padded(HD), G = d.NH / d.NKV, groups = (G + kRows - 1) / kRows;
+    const int rank = blockIdx.x % cluster, item = blockIdx.x / cluster;
+    const int t = item / (d.NKV * groups), kvh = item / groups % d.NKV, g0 = item % groups * kRows, heads = min(kRows, G - g0);
+    float* qs = sm;                                        // [4][HDP]
+    float* ps = qs + kRows * HDP;                          // [8 warps][32 keys][4 rows]
+    float* part = ps + kWarps * kBlock * kRows;            // [8 warps][4 rows][HDP + 2]: sums, reference, sum of weights
+    const int PR = HDP + 2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const T* q = (const T*)d.q + (size_t)t * d.NH * HD + (size_t)(kvh * G + g0) * HD;
+    const T* kv = (const T*)d.kv;
+    const bool live = FORGE_TOKEN_OK(t);
+    const int pos = live ? d.positions[t] : -1, least = d.window > 0 ? max(0, pos - d.window + 1) : 0;
+    const int32_t* table = d.block_table + (size_t)(live ? d.tok_req[t] : 0) * d.max_pages;
+    for (int i = tid; i < kRows * HDP; i += 32 * kWarps) {
+        const int r = i / HDP, c = i % HDP;
+        qs[i] = r < heads && c < HD ? forge::to_float(q[(size_t)r * HD + c]) * d.scale : 0.f;
+    }
+    __syncthreads();
+    const int seg_lo = least / kSegment, seg_hi = pos / kSegment, width = kWarps * cluster;
+    // the totals of this CTA's share of the (row, channel) pairs
+    constexpr int kMine = (kRows * 256 + 32 * kWarps - 1) / (32 * kWarps);
+    float mt[kMine], lt[kMine], at[kMine];
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) { mt[i] = -INFINITY; lt[i] = 0.f; at[i] = 0.f; }
+    for (int s0 = seg_lo; s0 <= seg_hi; s0 += width) {
+        const int seg = s0 + rank * kWarps + warp;
+        float m[kRows], l[kRows], acc[kRows][DPL];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            m[r] = -INFINITY;
+            l[r] = 0.f;
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) acc[r][i] = 0.f;
+        }
+        if (seg <= seg_hi) {
+            const int b_hi = min(pos, seg * kSegment + kSegment - 1) / kBlock;
+            for (int blk = max(least, seg * kSegment) / kBlock; blk <= b_hi; ++blk) {
+                const int j = blk * kBlock + lane;
+                const bool seen = j >= least && j <= pos;
+                const int page = seen ? table[j / d.page_size] : -1;
+                const bool ok = seen && FORGE_PAGE_OK(page) && page >= 0;
+                const long long row = ok ? ((long long)page * 2 * d.NKV + kvh) * d.page_size + j % d.page_size : -1;
+                const T* kr = kv + (ok ? row : 0) * HD;
+                int lo[kRows], hi[kRows];
+#pragma unroll
+                for (int r = 0; r < kRows; ++r) { lo[r] = least - blk * kBlock; hi[r] = pos - blk * kBlock; }
+                walk_block<DPL>(qs, HDP, lo, hi, ok, ps + warp * kBlock * kRows,
+                                   [&](int c) { return ok ? four<T>(kr + c, HD - c, d.vec) : make_float4(0.f, 0.f, 0.f, 0.f); },
+                                   [&](int jj, int i) {
+                                       const long long at_row = __shfl_sync(0xffffffffu, row, jj);
+                                       const int c = lane + 32 * i;
+                                       return at_row >= 0 && c < HD ? forge::to_float(kv[(at_row + (long long)d.NKV * d.page_size) * HD + c]) : 0.f;
+                                   },
+                                   m, l, acc);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            float* p = part + (warp * kRows + r) * PR;
+#pragma unroll
+            for (int i = 0; i < DPL; ++i)
+                if (lane + 32 * i < HDP) p[lane + 32 * i] = acc[r][i];
+            if (lane == 0) { p[HDP] = m[r]; p[HDP + 1] = l[r]; }
+        }
+        meet(cluster);
+        const int here = min(width, seg_hi - s0 + 1);
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+            const int e = (i * cluster + rank) * 32 * kWarps + tid;
+            if (e >= kRows * HDP) break;
+            const int r = e / HDP, c = e % HDP;
+            for (int z = 0; z < here; ++z) {
+                const float* p = part + ((z % kWarps) * kRows + r) * PR;
+                const float ms = peer_load(p + HDP, z / kWarps, cluster > 1), ls = peer_load(p + HDP + 1, z / kWarps, cluster > 1),
+                            as = peer_load(p + c, z / kWarps, cluster > 1);
+                float mm, fa, fb;
+                join_weights(mt[i], ms, mm, fa, fb);
+                if (ms != -INFINITY) {
+                    mt[i] = mm;
+                    lt[i] = join(lt[i], fa, ls, fb);
+                    at[i] = join(at[i], fa, as, fb);
+                }
+            }
+        }
+        meet(cluster);                                     // before the next round's sums overwrite these, or a CTA leaves that is still read
+    }
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) {
+        const int e = (i * cluster + rank) * 32 * kWarps + tid;
+        if (e >= kRows * HDP) break;
+        const int r = e / HDP, c = e % HDP;
+        if (live && r < heads && c < HD) ((T*)d.out)[(size_t)t * d.NH * HD + (size_t)(kvh * G + g0 + r) * HD + c] = forge::from_float<T>(at[i] * (1.0f / lt[i]));
+    }
+}
+
+template <int DPL, typename T>
+int launch_one(const SimtAttention& d, cudaStream_t stream) {
+    const int G = d.NH / d.NKV, HDP = padded(d.HD);
+    const long long tiles = ((long long)d.T * G + kTileRows - 1) / kTileRows;
+    if (tiles * d.NKV >= 148) {
+        const size_t smem = sizeof(float) * (kTileRows * HDP + 2 * kBlock * key_stride(d.HD) + 2 * kBlock * HDP + kWarps * kBlock * kRows);
+        static forge::PerDeviceFlag flag;
+        bool& done = flag.current();
+        if (!done) {
+            const int most = (int)(sizeof(float) * (kTileRows * 32 * DPL + 2 * kBlock * (32 * DPL + 8) + 2 * kBlock * 32 * DPL + kWarps * kBlock * kRows));
+            const cudaError_t e = cudaFuncSetAttribute(simt_tiles_kernel<DPL, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+            if (e != cudaSuccess) return forge::check_launch("paged_attention_simt (shared memory)", e);
+            done = true;
+        }
+        return forge::check_launch("paged_attention_simt", forge::launch(simt_tiles_kernel<DPL, T>, dim3((unsigned)tiles, d.NKV), dim3(32 * kWarps), smem, stream, 1, d));
+    }
+    const int items = d.T * d.NKV * ((G + kRows - 1) / kRows);
+    // a cluster where the tokens leave SMs idle and the tables have room for more segments than a CTA has warps
+    const long long segments = ((long long)d.max_pages * d.page_size + kSegment - 1) / kSegment;
+    int cluster = 1;
+    while (cluster < kMaxCluster && 2 * cluster * items <= 296 && segments > (long long)kWarps * cluster) cluster *= 2;
+    const size_t smem = sizeof(float) * (kRows * HDP + kWarps * kBlock * kRows + kWarps * kRows * (HDP + 2));
+    static forge::PerDeviceFlag flag;
+    bool& done = flag.current();
+    if (!done) {
+        const int most = (int)(sizeof(float) * (kRows * 32 * DPL + kWarps * kBlock * kRows + kWarps * kRows * (32 * DPL + 2)));
+        const cudaError_t e = cudaFuncSetAttribute(simt_segments_kernel<DPL, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return forge::check_launch("paged_attention_simt (shared memory)", e);
+        done = true;
+    }
+    return forge::check_launch("paged_attention_simt", forge::launch(simt_segments_kernel<DPL, T>, dim3((unsigned)items * cluster), dim3(32 * kWarps), smem, stream,
+                                                                     cluster, d, cluster));
 }
 
 template <typename T>
 int launch(const void* q, const void* kv, const int32_t* bt, const int32_t* tok_req, const int32_t* positions,
            void* out, int T_tokens, int NH, int NKV, int HD, int page_size, int max_pages, int window,
            float scale, cudaStream_t stream) {
-    const int warps = T_tokens * NH;
-    const unsigned blocks = (unsigned)((warps + 3) / 4);
-    const int dpl = (HD + 31) / 32;
-    cudaError_t e = cudaSuccess;
-#define FORGE_ATT_CASE(D)                                                                                  \
-    case D:                                                                                                \
-        e = forge::launch(paged_attention_simt_kernel<D, T>, dim3(blocks), dim3(128), 0, stream, 1,        \
-            (const T*)q, (const T*)kv, bt, tok_req, positions, (T*)out, T_tokens, NH, NKV, HD, page_size,  \
-            max_pages, window, scale);                                                                     \
-        break;
-    switch (dpl) {
-        FORGE_ATT_CASE(1) FORGE_ATT_CASE(2) FORGE_ATT_CASE(3) FORGE_ATT_CASE(4)
-        FORGE_ATT_CASE(5) FORGE_ATT_CASE(6) FORGE_ATT_CASE(7) FORGE_ATT_CASE(8)
+    const uintptr_t mask = 4 * sizeof(T) - 1;
+    const SimtAttention d{q, kv, bt, tok_req, positions, out, T_tokens, NH, NKV, HD, page_size, max_pages, window, scale,
+                          HD % 4 == 0 && ((uintptr_t)kv & mask) == 0 ? 1 : 0};
+    switch ((HD + 31) / 32) {
+        case 1: return launch_one<1, T>(d, stream);
+        case 2: return launch_one<2, T>(d, stream);
+        case 3: return launch_one<3, T>(d, stream);
+        case 4: return launch_one<4, T>(d, stream);
+        case 5: return launch_one<5, T>(d, stream);
+        case 6: return launch_one<6, T>(d, stream);
+        case 7: return launch_one<7, T>(d, stream);
+        case 8: return launch_one<8, T>(d, stream);
         default: return forge::fail(FORGE_ERR_UNSUPPORTED, "paged_attention_simt: head_dim %d > 256", HD);
     }
-#undef FORGE_ATT_CASE
-    return forge::check_launch("paged_attention_simt", e);
 }
 
 }  // namespace

@@ -153,6 +153,26 @@ def test_paged_attention_simt(dtype, nh, nkv, hd, ps, window):
     assert (got - ref).abs().max() <= tol * ref.abs().max()
 
 
+@pytest.mark.parametrize("nh,nkv,hd,ps,window", [(8, 2, 64, 16, 0), (7, 1, 128, 64, 0), (6, 2, 20, 8, 70), (4, 4, 33, 16, 0)])
+def test_paged_attention_simt_rows_do_not_depend_on_the_batch(nh, nkv, hd, ps, window):
+    """A step of many tokens (tiles of rows that share keys, of several requests in one tile too) gives every token the bits that a step
+    of that token alone gives it (segments of keys dealt to warps and CTAs), and both follow the oracle."""
+    k = _k()
+    lens = [1, 31, 32, 33, 64, 65, 300, 700]
+    q, cache, table, _, _ = _paged_case(nh, nkv, hd, ps, lens, torch.float32, seed=5)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    req = [r for r, n in enumerate(lens) for _ in range(n)]
+    pos = [p for n in lens for p in range(n)]
+    q = torch.randn(len(pos), nh * hd, generator=torch.Generator().manual_seed(7)).to(DEV)
+    got = k.paged_attention_simt(q, cache, table, i32(req), i32(pos), nh, nkv, hd, ps, window=window)
+    want = R.paged_attention_ref(q, cache, table, i32(req), i32(pos), nh, nkv, hd, ps, window)
+    assert (got - want).abs().max() <= 1e-5 * want.abs().max()
+    few = [0, 1, 31, 32, 33, 95, 96, 97, 130, len(pos) - 1, len(pos) - 2, len(pos) - 130, len(pos) - 700]
+    rows = torch.tensor(few, device=DEV)
+    alone = k.paged_attention_simt(q[rows].contiguous(), cache, table, i32([req[i] for i in few]), i32([pos[i] for i in few]), nh, nkv, hd, ps, window=window)
+    assert torch.equal(alone, got[rows])
+
+
 def test_paged_attention_far_key_stands_out():
     """One key among hundreds, on an early page, carries nearly all the weight: a kernel that skips or
     misplaces that page cannot pass."""
