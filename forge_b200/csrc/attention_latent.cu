@@ -249,6 +249,152 @@ head_linear_mma_kernel(const TI* __restrict__ in, long long in_ld, int in_hs, co
     }
 }
 
+// The same for more than 64 tokens and aligned operands: a CTA of eight warps takes 128 tokens of one head with ALL their input channels
+// (converted once; the kernel above reads and converts them again for every 64 output channels) and walks the output channels in chunks of
+// 64, W_h in pieces of [128 x 64] through a ring of three (cp.async); a warp has 32 tokens x 32 channels, results leave through shared
+// memory as rows of 128 bytes.  Bound by shared memory's bandwidth and by the results' way out (1,536 tokens, 32 heads, 128 -> 512 + 64
+// channels: 38 MB in, 57 MB out).  Where tokens and heads leave SMs idle several CTAs share a tile's output channels.
+constexpr int kHltThreads = 256, kHltTokens = 128, kHltN = 64, kHltRing = 3, kHltMaxK = 512;
+constexpr int kHltPiece = kHlmK * kHlmRow;                                 // elements of a staged piece of W
+size_t hlt_smem(int K) { return sizeof(__nv_bfloat16) * ((size_t)kHltTokens * ((K + 15) / 16 * 16 + 8) + kHltRing * kHltPiece + kHltTokens * kHlmRow); }
+
+template <typename TI>
+__global__ void __launch_bounds__(kHltThreads)
+head_linear_tile_kernel(const TI* __restrict__ in, long long in_ld, int in_hs, const __nv_bfloat16* __restrict__ W, __nv_bfloat16* __restrict__ out,
+                        long long out_ld, int out_hs, const int32_t* __restrict__ positions, const float* __restrict__ freq, float amp,
+                        int T, int K, int N, int R, const float* __restrict__ gate, long long gate_ld, int gate_hs, int gate_cs, int halves) {
+    extern __shared__ __align__(16) __nv_bfloat16 hs_smem[];
+    const int KP = (K + 15) / 16 * 16, KR = KP + 8;
+    __nv_bfloat16* As = hs_smem;                                           // [128][KP + 8]
+    __nv_bfloat16* Bs = As + kHltTokens * KR;                              // ring of [128][64 + 8]
+    __nv_bfloat16* Os = Bs + kHltRing * kHltPiece;                         // [128][64 + 8]
+    forge::pdl_launch_dependents();
+    const int t0 = blockIdx.x * kHltTokens, h = blockIdx.y, nt = min(kHltTokens, T - t0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const __nv_bfloat16* Wh = W + (size_t)h * K * N;
+    const int n_chunks = (N + kHltN - 1) / kHltN, k_pieces = (K + kHlmK - 1) / kHlmK;
+    const int c_lo = (int)((long long)n_chunks * blockIdx.z / gridDim.z), c_hi = (int)((long long)n_chunks * (blockIdx.z + 1) / gridDim.z);
+    const int pieces = (c_hi - c_lo) * k_pieces;
+    auto fetch = [&](int i) {
+        if (i < pieces) {
+            const int n0 = (c_lo + i / k_pieces) * kHltN, k0 = i % k_pieces * kHlmK;
+            __nv_bfloat16* dst = Bs + i % kHltRing * kHltPiece;
+#pragma unroll
+            for (int j = 0; j < kHlmK * kHltN / 8 / kHltThreads; ++j) {
+                const int e = threadIdx.x + j * kHltThreads, r = e / (kHltN / 8), c = e % (kHltN / 8) * 8;
+                const bool ok = k0 + r < K && n0 + c < N;
+                const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + r * kHlmRow + c);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(ok ? Wh + (size_t)(k0 + r) * N + n0 + c : Wh), "r"(ok ? 16 : 0) : "memory");
+            }
+        }
+        mma_sync::cp_async_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < kHltRing - 1; ++i) fetch(i);                       // the weights do not wait for the kernel before this one
+    forge::pdl_wait();
+    for (int i0 = 0; i0 < kHltTokens * KP / 8; i0 += 8 * kHltThreads) {
+        uint4 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int e = i0 + threadIdx.x + j * kHltThreads, r = e / (KP / 8), c = e % (KP / 8) * 8;
+            v[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (r < nt && c < K) v[j] = load8_bf16<TI>(in + (size_t)(t0 + r) * in_ld + (size_t)h * in_hs + c, 8, true);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int e = i0 + threadIdx.x + j * kHltThreads, r = e / (KP / 8), c = e % (KP / 8) * 8;
+            if (r < kHltTokens) *reinterpret_cast<uint4*>(As + r * KR + c) = v[j];
+        }
+    }
+    float acc[2][4][4];
+    for (int i = 0; i < pieces; ++i) {
+        const int n0 = (c_lo + i / k_pieces) * kHltN, kp = i % k_pieces, k0 = kp * kHlmK;
+        mma_sync::cp_async_wait<kHltRing - 2>();
+        __syncthreads();                                                   // piece i is here for every thread, and the one before it is done with
+        fetch(i + kHltRing - 1);
+        if (kp == 0) {
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.f;
+        }
+        const __nv_bfloat16* Bp = Bs + i % kHltRing * kHltPiece;
+        const int ksteps = min(kHlmK, KP - k0) / 16;
+        for (int ks = 0; ks < ksteps; ++ks) {
+            uint32_t a[2][4];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) mma_sync::ldmatrix_x4(a[m], As + (wm + m * 16 + (lane & 15)) * KR + k0 + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+            for (int np = 0; np < 2; ++np) {
+                uint32_t b[4];
+                mma_sync::ldmatrix_x4_trans(b, Bp + (ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * kHlmRow + wn + np * 16 + (lane >> 4) * 8);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    mma_sync::mma_bf16(acc[m][2 * np], a[m], b[0], b[1]);
+                    mma_sync::mma_bf16(acc[m][2 * np + 1], a[m], b[2], b[3]);
+                }
+            }
+        }
+        if (kp + 1 < k_pieces) continue;
+        // (the rows of the chunk before have left Os: a barrier has passed since)
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int r = wm + m * 16 + (lane >> 2) + half * 8, c = wn + nb * 8 + (lane & 3) * 2;
+                    float v0 = acc[m][nb][2 * half], v1 = acc[m][nb][2 * half + 1];
+                    if (gate && r < nt && n0 + c < N) {
+                        const float* gr = gate + (size_t)(t0 + r) * gate_ld + (size_t)h * gate_hs;
+                        v0 *= 1.0f / (1.0f + expf(-gr[(n0 + c) * gate_cs]));
+                        v1 *= 1.0f / (1.0f + expf(-gr[(n0 + c + 1) * gate_cs]));
+                    }
+                    *reinterpret_cast<uint32_t*>(Os + r * kHlmRow + c) = mma_sync::pack_bf16(v0, v1);
+                }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kHltTokens * kHltN / 8 / kHltThreads; ++j) {
+            const int e = threadIdx.x + j * kHltThreads, r = e / (kHltN / 8), c = e % (kHltN / 8) * 8;
+            if (r < nt && n0 + c < N)
+                *reinterpret_cast<uint4*>(out + (size_t)(t0 + r) * out_ld + (size_t)h * out_hs + n0 + c) = *reinterpret_cast<const uint4*>(Os + r * kHlmRow + c);
+        }
+    }
+    if (R > 0 && blockIdx.z == 0) {
+        for (int i = threadIdx.x; i < nt * (R >> 1); i += kHltThreads) {
+            const int tt = i / (R >> 1), p = i % (R >> 1);
+            const TI* src = in + (size_t)(t0 + tt) * in_ld + (size_t)h * in_hs + K;
+            float sn, cs;
+            sincosf((float)positions[t0 + tt] * freq[p], &sn, &cs);
+            sn *= amp;
+            cs *= amp;
+            const int a = pair_first(p, halves), b = pair_second(p, R, halves);
+            const float u = forge::to_float(src[a]), v = forge::to_float(src[b]);
+            __nv_bfloat16* dst = out + (size_t)(t0 + tt) * out_ld + (size_t)h * out_hs + N;
+            dst[a] = __float2bfloat16(u * cs - v * sn);
+            dst[b] = __float2bfloat16(v * cs + u * sn);
+        }
+    }
+}
+
+template <typename TI>
+cudaError_t launch_head_linear_tile(cudaStream_t stream, const TI* in, long long in_ld, int in_hs, const __nv_bfloat16* W, __nv_bfloat16* out, long long out_ld,
+                                    int out_hs, const int32_t* positions, const float* freq, float amp, int T, int H, int K, int N, int R, const float* gate,
+                                    long long gate_ld, int gate_hs, int gate_cs, int halves) {
+    static forge::PerDeviceFlag flag;
+    bool& done = flag.current();
+    if (!done) {
+        const cudaError_t e = cudaFuncSetAttribute(head_linear_tile_kernel<TI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hlt_smem(kHltMaxK));
+        if (e != cudaSuccess) return e;
+        done = true;
+    }
+    const int tiles = (T + kHltTokens - 1) / kHltTokens, chunks = (N + kHltN - 1) / kHltN;
+    int share = 1;                                                         // CTAs a tile: until two an SM have work
+    while (share < chunks && (long long)tiles * H * share < 296) ++share;
+    return forge::launch(head_linear_tile_kernel<TI>, dim3(tiles, H, share), dim3(kHltThreads), hlt_smem(K), stream, 1, in, in_ld, in_hs, W, out, out_ld, out_hs,
+                         positions, freq, amp, T, K, N, R, gate, gate_ld, gate_hs, gate_cs, halves);
+}
+
 constexpr int kAttThreads = 256;
 
 // One CTA per (tile of up to TQ consecutive tokens of one request, group of HG heads); tile_t0 = null: tile i is token i.
@@ -404,6 +550,17 @@ extern "C" int forge_head_linear(const void* in, int in_dtype, long long in_ld, 
     if (T == 0) return FORGE_OK;
     cudaError_t e;
     if (dtype == FORGE_BF16 && (in_dtype == FORGE_F32 || in_dtype == FORGE_BF16) && !simt) {
+        // up to 64 tokens are one tile of the small kernel, whose CTAs are many and short; so is whatever is not aligned
+        const int per16 = in_dtype == FORGE_F32 ? 4 : 8;
+        if (T > kHlmTile && K <= kHltMaxK && K % 8 == 0 && N % 8 == 0 && in_ld % per16 == 0 && in_hs % per16 == 0 && out_ld % 8 == 0 && out_hs % 8 == 0 &&
+            (((uintptr_t)in | (uintptr_t)W | (uintptr_t)out) & 15) == 0) {
+            e = in_dtype == FORGE_F32
+                    ? launch_head_linear_tile<float>(stream, (const float*)in, in_ld, in_hs, (const __nv_bfloat16*)W, (__nv_bfloat16*)out, out_ld, out_hs, positions,
+                                                     freq, amp, T, H, K, N, R, gate, gate_ld, gate_hs, gate_cs, halves)
+                    : launch_head_linear_tile<__nv_bfloat16>(stream, (const __nv_bfloat16*)in, in_ld, in_hs, (const __nv_bfloat16*)W, (__nv_bfloat16*)out, out_ld,
+                                                             out_hs, positions, freq, amp, T, H, K, N, R, gate, gate_ld, gate_hs, gate_cs, halves);
+            return forge::check_launch("head_linear (tiles)", e);
+        }
         const dim3 grid((T + kHlmTile - 1) / kHlmTile, H, (N + kHlmTile - 1) / kHlmTile);
         if (in_dtype == FORGE_F32)
             e = forge::launch(head_linear_mma_kernel<float>, grid, dim3(kHlmThreads), 0, stream, 1, (const float*)in, in_ld, in_hs,

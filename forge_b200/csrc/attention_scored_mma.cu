@@ -382,6 +382,47 @@ scored_combine_kernel(const float* __restrict__ u, const float* __restrict__ par
     }
 }
 
+// The same for two maps in one run each: a lane has four neighbouring channels of every 128 (E a multiple of 4 up to 256, everything
+// 16-byte aligned): both maps' loads are in flight together.  (2,048 tokens, 16 heads of 128: 19.5 us channel by channel.)
+__global__ void __launch_bounds__(128)
+scored_combine_pair_kernel(const float* __restrict__ u, __nv_bfloat16* __restrict__ out_base, int rows, int H, int E, float lambda, float post, float eps,
+                           long long out_ld) {
+    forge::pdl_launch_dependents();
+    forge::pdl_wait();
+    const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (w >= rows) return;
+    const float4* a = reinterpret_cast<const float4*>(u + (size_t)w * 2 * E);
+    const float4* b = reinterpret_cast<const float4*>(u + (size_t)w * 2 * E + E);
+    float4 o[2];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int c = lane + 32 * i;
+        o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (4 * c < E) {
+            const float4 x = a[c], y = b[c];
+            o[i] = make_float4(x.x - lambda * y.x, x.y - lambda * y.y, x.z - lambda * y.z, x.w - lambda * y.w);
+        }
+        ss = fmaf(o[i].x, o[i].x, fmaf(o[i].y, o[i].y, fmaf(o[i].z, o[i].z, fmaf(o[i].w, o[i].w, ss))));
+    }
+    ss = forge::warp_sum(ss);
+    const float inv = 1.0f / sqrtf(ss / (float)E + eps) * post;
+    __nv_bfloat16* orow = out_base + (size_t)(w / H) * out_ld + (size_t)(w % H) * E;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int c = lane + 32 * i;
+        if (4 * c < E) *reinterpret_cast<uint2*>(orow + 4 * c) = make_uint2(pack_bf16(o[i].x * inv, o[i].y * inv), pack_bf16(o[i].z * inv, o[i].w * inv));
+    }
+}
+
+cudaError_t launch_combine(const float* u, const float* part_ml, int nsplit, __nv_bfloat16* out, int T, int H, int M, int E, float lambda, float post,
+                           float eps, long long out_ld, const float* sink, cudaStream_t stream) {
+    const unsigned blocks = (unsigned)(((size_t)T * H + 3) / 4);
+    if (M == 2 && nsplit == 1 && E % 4 == 0 && E <= 256 && out_ld % 4 == 0 && ((uintptr_t)u & 15) == 0 && ((uintptr_t)out & 7) == 0)
+        return forge::launch(scored_combine_pair_kernel, dim3(blocks), dim3(128), 0, stream, 1, u, out, T * H, H, E, lambda, post, eps, out_ld);
+    return forge::launch(scored_combine_kernel, dim3(blocks), dim3(128), 0, stream, 1, u, part_ml, nsplit, out, T * H, H, M, E, lambda, post, eps, out_ld, sink);
+}
+
 forge::PerDeviceFlag g_attr_done[6];
 
 template <int VC, bool SPLIT>
@@ -449,10 +490,15 @@ extern "C" int forge_scored_attention_mma(const void* q, const void* cache, cons
     else rc = VC == 64 ? launch_scored<64, false>(0, FORGE_SCORED_ARGS) : VC == 128 ? launch_scored<128, false>(1, FORGE_SCORED_ARGS) : launch_scored<256, false>(2, FORGE_SCORED_ARGS);
 #undef FORGE_SCORED_ARGS
     if (rc != FORGE_OK || (M == 1 && nsplit == 1)) return rc;
-    const unsigned blocks = (unsigned)(((size_t)T * H + 3) / 4);
-    return forge::check_launch("scored_combine", forge::launch(scored_combine_kernel, dim3(blocks), dim3(128), 0, stream, 1, (const float*)u,
-                                                               (const float*)part_ml, nsplit, ob, T * H, H, M, E, lambda,
-                                                               (M == 1 ? 1.0f : post) * out_scale, eps, out_ld, sink));
+    return forge::check_launch("scored_combine", launch_combine(u, part_ml, nsplit, ob, T, H, M, E, lambda, (M == 1 ? 1.0f : post) * out_scale, eps, out_ld, sink, stream));
+}
+
+// Two maps' outputs u fp32 [T, H, 2, E] put together: (a_1 - lambda a_2) / its root mean square * post * out_scale, bf16 rows of out_ld.
+extern "C" int forge_scored_combine(const float* u, void* out, int T, int H, int E, float lambda, float post, float eps, float out_scale, long long out_ld,
+                                    cudaStream_t stream) {
+    if (T < 0 || H <= 0 || E <= 0 || out_ld < (long long)H * E) return forge::fail(FORGE_ERR_ARG, "scored_combine: bad sizes T=%d H=%d E=%d", T, H, E);
+    if (T == 0) return FORGE_OK;
+    return forge::check_launch("scored_combine", launch_combine(u, nullptr, 1, (__nv_bfloat16*)out, T, H, 2, E, lambda, post * out_scale, eps, out_ld, nullptr, stream));
 }
 
 FORGE_DEFINE_CHECKS_ENTRY(attention_scored_mma)

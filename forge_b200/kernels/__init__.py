@@ -78,6 +78,7 @@ _SIGNATURES = {
         "forge_scored_attention": [_P] * 10 + [_I] * 8 + [_LL, _I] + [_F] * 5 + [_I, _I, _LL, _I, _I, _F, _P, _P],
         "forge_scored_mma_supports": [_I] * 6,
         "forge_scored_attention_mma": [_P] * 11 + [_I, _P] + [_I] * 8 + [_LL, _I] + [_F] * 5 + [_LL, _I, _I, _F, _P, _P],
+        "forge_scored_combine": [_P, _P, _I, _I, _I, _F, _F, _F, _F, _LL, _P],
         "forge_token_shift": [_P, _P, _LL, _LL, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
         "forge_head_finish": [_P, _P, _P, _I, _P, _I, _I, _I, _I, _F, _I, _F, _I, _LL, _P],
         "forge_tanh_rows": [_P, _I, _P, _I, _I, _I, _P],
@@ -99,6 +100,12 @@ _SIGNATURES = {
         "forge_latent_mma_supports": [_I] * 4,
         "forge_latent_mma_heads": [_I],
         "forge_latent_attention_mma": [_P] * 9 + [_I, _P] + [_I] * 7 + [_F, _I, _P, _P],
+    },
+    "attention_shaped": {
+        "forge_latent_sm100_supports": [_I] * 4,
+        "forge_scored_sm100_supports": [_I] * 6,
+        "forge_latent_attention_sm100": [_P] * 9 + [_I] * 8 + [_F, _I, _P, _P],
+        "forge_scored_attention_sm100": [_P] * 12 + [_I] * 9 + [_LL, _I, _F, _F, _LL, _I, _I, _F, _P, _P],
     },
     "moe": {
         "forge_moe_route": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _I, _F, _P],
@@ -129,7 +136,8 @@ _CHECK_ENTRIES = {"core": ["forge_checks_configure_rope", "forge_checks_configur
                   "latent": ["forge_checks_configure_attention_latent", "forge_checks_configure_attention_latent_mma"],
                   "gemm_sm100": ["forge_checks_configure_gemm_sm100"],
                   "attention_mma": ["forge_checks_configure_attention_mma", "forge_checks_configure_attention_decode_stream"],
-                  "attention_sm100": ["forge_checks_configure_attention_sm100"]}
+                  "attention_sm100": ["forge_checks_configure_attention_sm100"],
+                  "attention_shaped": ["forge_checks_configure_attention_shaped_sm100"]}
 _check_bounds = [None]          # (num_pages, page_size, num_tokens, status tensor, first_bad tensor) of the current step
 
 
@@ -936,6 +944,26 @@ def headmix_plan(batch, TQ, device):
     return plan
 
 
+def shaped_plan(batch, TQ, device):
+    """The step's tokens cut into tiles of up to TQ consecutive tokens of one request (first token, count), those that reach furthest
+    first, made once per step: for the tcgen05 kernels of prompt portions, whose CTAs are handed out in that order."""
+    key = ("shaped", TQ)
+    plan = batch.attention_plan.get(key)
+    if plan is None:
+        qs, before = batch.host_q_start, getattr(batch, "host_context_before", None) or [0] * batch.num_requests
+        tiles = [(before[s] + min(a + TQ, qs[s + 1]) - qs[s], a, min(TQ, qs[s + 1] - a))
+                 for s in range(batch.num_requests) for a in range(qs[s], qs[s + 1], TQ)]
+        tiles.sort(key=lambda t: (-t[0], t[1]))
+        with once_per_step():
+            plan = batch.attention_plan[key] = (new_ints([t[1] for t in tiles], device), new_ints([t[2] for t in tiles], device), len(tiles))
+    return plan
+
+
+def _brings_portions(batch):
+    """Whether a step brings more than one token for some request (and is no step that a graph replays)."""
+    return not getattr(batch, "decode_only", False) and batch.num_tokens > batch.num_requests
+
+
 def _page_stride(cache):
     n = 1
     for d in cache.shape[1:]:
@@ -1096,6 +1124,23 @@ def scored_attention(q, cache, group_batch, batch, H, G, M, D, E, page_size, sca
         raise KernelError(f"scored_attention: {sink.numel()} sinks for {H} heads")
     T = q.shape[0]
     out, out_ptr, out_ld = _out_slice(out, H * E, T, q.dtype, q.device)
+    if q.dtype == torch.bfloat16 and _TENSOR_CORE_ATTENTION and scale > 0.0 and _brings_portions(batch):
+        # prompt portions: tcgen05, tiles of 128 rows (half a microsecond a tile of 64 keys against the mma.sync kernel's two for 64 rows)
+        sm = library("attention_shaped")
+        if sm.forge_scored_sm100_supports.fn(H, G, M, D, E, page_size):
+            t0, tn, tiles = shaped_plan(batch, 128 // (H // G), q.device)
+            u = new_tensor((T, H, M, E), torch.float32, q.device) if M == 2 else None
+            _check(sm, sm.forge_scored_attention_sm100(
+                _need(q, "q", torch.bfloat16, 2), _need(cache, "cache", torch.bfloat16), _need(group_batch.block_table, "block_table", torch.int32, 2),
+                _need(batch.tok_req, "tok_req", torch.int32), _need(batch.positions, "positions", torch.int32), _need(t0, "tile_t0", torch.int32),
+                _need(tn, "tile_n", torch.int32), _opt(r1, "r1", torch.float32), _opt(r2, "r2", torch.float32), _opt(u, "u", torch.float32), out_ptr,
+                _need(_gemm_status(q.device), "status", torch.int32), T, tiles, cache.shape[0], H, G, M, D, E, page_size, _page_stride(cache),
+                group_batch.block_table.shape[1], float(scale), float(out_scale), out_ld, window, chunk, softcap, _opt(sink, "sink", torch.float32), _stream()),
+                "scored_attention_sm100")
+            if M == 2:
+                _check(lib, lib.forge_scored_combine(_need(u, "u", torch.float32), out_ptr, T, H, E, float(lam), float(post), float(eps), float(out_scale), out_ld,
+                                                     _stream()), "scored_combine")
+            return out
     if q.dtype == torch.bfloat16 and _TENSOR_CORE_ATTENTION and lib.forge_scored_mma_supports.fn(H, G, M, D, E, page_size):
         # tensor cores: every (head, map) a one-pass attention of its own; two maps meet in a second small kernel
         t0, tn, tiles = headmix_plan(batch, max(1, 64 // (H // G)), q.device)
@@ -1441,6 +1486,19 @@ def latent_attention(q, cache, group_batch, batch, H, C, R, page_size, scale, wi
     T = q.shape[0]
     if cache.dtype != q.dtype:
         raise KernelError("latent_attention: q and cache dtypes differ")
+    if q.dtype == torch.bfloat16 and _TENSOR_CORE_ATTENTION and scale > 0.0 and _brings_portions(batch):
+        # prompt portions: tcgen05, tiles of 128 rows
+        sm = library("attention_shaped")
+        if sm.forge_latent_sm100_supports.fn(H, C, R, page_size):
+            t0, tn, tiles = shaped_plan(batch, 128 // H, q.device)
+            out = new_tensor((T, H * C), q.dtype, q.device)
+            _check(sm, sm.forge_latent_attention_sm100(
+                _need(q, "q", torch.bfloat16, 2), _need(cache, "cache", torch.bfloat16), _need(group_batch.block_table, "block_table", torch.int32, 2),
+                _need(batch.tok_req, "tok_req", torch.int32), _need(batch.positions, "positions", torch.int32), _need(t0, "tile_t0", torch.int32),
+                _need(tn, "tile_n", torch.int32), _need(out, "out", torch.bfloat16), _need(_gemm_status(q.device), "status", torch.int32), T, tiles,
+                cache.shape[0], H, C, R, page_size, group_batch.block_table.shape[1], float(scale), window, _opt(sink, "sink", torch.float32), _stream()),
+                "latent_attention_sm100")
+            return out
     if q.dtype == torch.bfloat16 and _TENSOR_CORE_ATTENTION and lib.forge_latent_mma_supports.fn(H, C, R, page_size):
         # tensor cores: rows of (token, head) over the same tiles of latent rows
         HG = lib.forge_latent_mma_heads.fn(H)

@@ -30,6 +30,8 @@ LIBRARIES = {
     "attention_mma": ["attention_mma.cu", "attention_decode_stream.cu"],
     # bf16 tcgen05/TMEM paged attention for prompt portions, head sizes 64 and 128 (built per head size)
     "attention_sm100": ["attention_sm100.cu"],
+    # bf16 tcgen05/TMEM attention for prompt portions over latent rows and with shaped scores
+    "attention_shaped": ["attention_shaped_sm100.cu"],
     # attention whose heads exchange weights, over a window with kept first tokens; attention with shaped scores (two maps per
     # head, a distance term); mixers with a matrix of state per head
     "mixers": ["attention_headmix.cu", "attention_headmix_mma.cu", "attention_scored.cu", "attention_scored_mma.cu", "recurrent.cu",

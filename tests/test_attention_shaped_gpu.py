@@ -1,0 +1,167 @@
+"""The tcgen05 attention of prompt portions over latent rows and with shaped scores, against the definition in 64 bits: tiles of tokens that
+do not fill 128 rows, portions behind cached tokens, pages shorter and longer than a tile of keys, values in one and two chunks, and numbers
+that are none behind a request's last token.
+
+Inputs are bfloat16 and enter exactly; what the kernel rounds is the result (2^-9 of a value), the weights (two bfloat16 terms: 2^-16) and fp32
+scores (an exponent's error of a few 2^-22 times the score's size).  Allowed: 2^-8 of a value and 1e-3 of the largest."""
+import math
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+REQS = [(0, 1), (70, 37), (0, 130), (200, 5)]          # (cached, new) of the step's requests
+
+
+def _batch(reqs, ps, row_numbers, seed):
+    """A step over shuffled pages; the cache's rows behind every request's last token hold NaN."""
+    g = torch.Generator().manual_seed(seed)
+    n_pages = sum(-(-(c + n) // ps) for c, n in reqs) + 2
+    perm = torch.randperm(n_pages, generator=g).tolist()
+    table = torch.full((len(reqs), max(-(-(c + n) // ps) for c, n in reqs)), -1, dtype=torch.int32)
+    for s, (c, n) in enumerate(reqs):
+        for i in range(-(-(c + n) // ps)):
+            table[s, i] = perm.pop()
+    q_start = [0]
+    for _, n in reqs:
+        q_start.append(q_start[-1] + n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(num_requests=len(reqs), num_tokens=q_start[-1], host_q_start=q_start, host_context_before=[c for c, _ in reqs], attention_plan={},
+                            tok_req=i32([s for s, (_, n) in enumerate(reqs) for _ in range(n)]), positions=i32([c + j for c, n in reqs for j in range(n)]))
+    return batch, table, n_pages, g
+
+
+def _fill(view, table, reqs, ps, g):
+    """view: [pages, ps, ...] of a cache, filled where a request has tokens, NaN elsewhere; returns each request's rows in order."""
+    view.fill_(float("nan"))
+    rows = []
+    for s, (c, n) in enumerate(reqs):
+        pages = torch.tensor([int(table[s, p // ps]) for p in range(c + n)])
+        offs = torch.tensor([p % ps for p in range(c + n)])
+        vals = (torch.randn(c + n, *view.shape[2:], generator=g) * 0.7).to(torch.bfloat16)
+        view[pages, offs] = vals
+        rows.append(vals.double())
+    return rows
+
+
+def _softmax_out(s, v, sink=None):
+    if sink is not None:
+        m = torch.maximum(s.max(dim=-1, keepdim=True).values, torch.as_tensor(sink, dtype=torch.float64))
+        p = torch.exp(s - m)
+        return (p / (p.sum(dim=-1, keepdim=True) + torch.exp(sink - m))) @ v
+    return torch.softmax(s, dim=-1) @ v
+
+
+def _visible(c, n, window, chunk):
+    i, j = torch.arange(c, c + n)[:, None], torch.arange(c + n)[None, :]
+    ok = j <= i
+    if window:
+        ok &= i - j < window
+    if chunk:
+        ok &= i // chunk == j // chunk
+    return ok, (i - j).clamp(min=0)
+
+
+def _close(got, want):
+    assert bool(torch.isfinite(got).all())
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3 * want.abs().max()).all()), float((got - want).abs().max() / want.abs().max())
+
+
+@pytest.mark.parametrize("H,C,R,ps,window", [(32, 256, 32, 64, 0), (32, 512, 64, 64, 0), (32, 512, 64, 16, 90), (5, 64, 16, 8, 0), (128, 128, 0, 128, 0),
+                                             (3, 192, 48, 32, 50), (16, 512, 16, 64, 0)])
+def test_latent(H, C, R, ps, window):
+    from forge_b200 import kernels
+    assert kernels.library("attention_shaped").forge_latent_sm100_supports.fn(H, C, R, ps)
+    KD = C + R
+    batch, table, n_pages, g = _batch(REQS, ps, KD, seed=H + C)
+    cache = torch.empty(n_pages, ps * KD, dtype=torch.bfloat16)
+    rows = _fill(cache.view(n_pages, ps, KD), table, REQS, ps, g)
+    q = torch.randn(batch.num_tokens, H * KD, generator=g).to(torch.bfloat16)
+    sink = torch.randn(H, generator=g) if window else None
+    scale = 2.0 * KD ** -0.5
+    group = SimpleNamespace(block_table=table.to(DEV))
+    launches = kernels.launch_count()
+    got = kernels.latent_attention(q.to(DEV), cache.to(DEV), group, batch, H, C, R, ps, scale, window=window, sink=None if sink is None else sink.to(DEV))
+    assert kernels.launch_count() - launches == 1
+    kernels.check_kernel_status(DEV)
+    got, at = got.double().cpu().view(-1, H, C), 0
+    for (c, n), k in zip(REQS, rows):
+        ok, _ = _visible(c, n, window, 0)
+        for h in range(H):
+            s = (q[at:at + n].view(n, H, KD)[:, h].double() @ k.t() * scale).masked_fill(~ok, -math.inf)
+            _close(got[at:at + n, h], _softmax_out(s, k[:, :C], None if sink is None else sink[h].double()))
+        at += n
+
+
+@pytest.mark.parametrize("H,G,M,D,E,ps,opts", [
+    (16, 2, 2, 64, 128, 64, {}), (32, 4, 1, 64, 64, 64, {"window": 70}), (6, 2, 1, 128, 256, 16, {"distance": True}), (4, 1, 1, 64, 512, 128, {"sink": True}),
+    (14, 2, 1, 128, 128, 8, {"softcap": 5.0, "chunk": 48}), (8, 8, 2, 128, 192, 32, {}), (24, 2, 1, 64, 64, 64, {"chunk": 64, "sink": True})])
+def test_scored(H, G, M, D, E, ps, opts):
+    from forge_b200 import kernels
+    assert kernels.library("attention_shaped").forge_scored_sm100_supports.fn(H, G, M, D, E, ps)
+    MD, window, chunk, cap = M * D, opts.get("window", 0), opts.get("chunk", 0), opts.get("softcap", 0.0)
+    batch, table, n_pages, g = _batch(REQS, ps, MD, seed=H + E)
+    cache = torch.empty(n_pages, G * ps * (MD + E), dtype=torch.bfloat16)
+    keys, values = cache[:, :G * ps * MD].unflatten(1, (G, ps, MD)), cache[:, G * ps * MD:].unflatten(1, (G, ps, E))
+    k_rows, v_rows = _fill(keys.transpose(1, 2), table, REQS, ps, g), _fill(values.transpose(1, 2), table, REQS, ps, g)
+    q = torch.randn(batch.num_tokens, H * MD, generator=g).to(torch.bfloat16)
+    r1, r2 = (torch.rand(H, generator=g), torch.rand(H, generator=g)) if opts.get("distance") else (None, None)
+    sink = torch.randn(H, generator=g) if opts.get("sink") else None
+    scale, lam, post, eps = 2.0 * D ** -0.5, 0.6, 0.5, 1e-5
+    dev = lambda t: None if t is None else t.to(DEV)
+    wide = torch.full((batch.num_tokens, H * E + 6), 3.0, dtype=torch.bfloat16, device=DEV)
+    for out in (None, (wide, 2)):
+        res = kernels.scored_attention(q.to(DEV), cache.to(DEV), SimpleNamespace(block_table=table.to(DEV)), batch, H, G, M, D, E, ps, scale, r1=dev(r1), r2=dev(r2),
+                                       lam=lam, post=post, eps=eps, out_scale=0.8, out=out, window=window, chunk=chunk, softcap=cap, sink=dev(sink))
+        got = (res if out is None else wide[:, 2:2 + H * E]).double().cpu().view(-1, H, E)
+        kernels.check_kernel_status(DEV)
+        at = 0
+        for (c, n), k, v in zip(REQS, k_rows, v_rows):
+            ok, dist = _visible(c, n, window, chunk)
+            for h in range(H):
+                maps = []
+                for m in range(M):
+                    s = q[at:at + n].view(n, H, M, D)[:, h, m].double() @ k[:, h // (H // G), m * D:(m + 1) * D].t() * scale
+                    s = cap * torch.tanh(s / cap) if cap else s
+                    if r1 is not None:
+                        s = s - r1[h].double() * torch.log1p(r2[h].double() * dist)
+                    maps.append(_softmax_out(s.masked_fill(~ok, -math.inf), v[:, h // (H // G)], None if sink is None else sink[h].double()))
+                want = maps[0]
+                if M == 2:
+                    want = maps[0] - lam * maps[1]
+                    want = want / torch.sqrt((want * want).mean(dim=-1, keepdim=True) + eps) * post
+                _close(got[at:at + n, h], want * 0.8)
+            at += n
+    assert bool((wide[:, :2] == 3.0).all()) and bool((wide[:, 2 + H * E:] == 3.0).all())
+
+
+@pytest.mark.parametrize("in_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,H,K,N,R,gate", [(65, 3, 128, 512, 64, None), (300, 5, 512, 128, 0, "channel"), (129, 2, 72, 72, 16, None), (128, 32, 64, 256, 32, None),
+                                            (200, 4, 200, 136, 0, "head"), (2000, 2, 8, 64, 8, None)])
+def test_products_per_head_in_tiles(in_dtype, T, H, K, N, R, gate):
+    """More than 64 aligned tokens: tiles of 128 tokens with all their input channels, output channels in chunks of 64 and shared out among CTAs.
+    Inputs are rounded to bfloat16, sums are fp32 (K 2^-24), the result is rounded once (2^-9)."""
+    from forge_b200 import kernels
+    g = torch.Generator().manual_seed(T + N)
+    x = torch.randn(T, H * (K + R), generator=g).to(in_dtype)
+    w = (torch.randn(H, K, N, generator=g) * 0.2).to(torch.bfloat16)
+    pos, freq = torch.arange(5, 5 + T, dtype=torch.int32), torch.tensor([0.5 ** i for i in range(R // 2)], dtype=torch.float32)
+    args = dict(R=R, positions=pos.to(DEV), freq=freq.to(DEV), amp=1.25) if R else {}
+    z = torch.randn(T, 3 + (H if gate == "head" else H * N), generator=g)
+    if gate:
+        args["gate"] = (z.to(DEV), 3) if gate == "channel" else (z.to(DEV), 3, "head")
+    got = kernels.head_linear(x.to(DEV), w.to(DEV), H, K, N, torch.bfloat16, **args).double().cpu().view(T, H, N + R)
+    xd = x.double().view(T, H, K + R)
+    xr = xd[..., :K].to(torch.bfloat16).double()
+    want, size = torch.einsum("thk,hkn->thn", xr, w.double()), torch.einsum("thk,hkn->thn", xr.abs(), w.double().abs())
+    if gate:
+        s = torch.sigmoid(z[:, 3:].double())
+        want = want * (s.view(T, H, N) if gate == "channel" else s[..., None])
+    assert bool(((got[..., :N] - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -22 * size + 1e-6).all())
+    if R:
+        a = pos.double()[:, None] * freq.double()[None, :]
+        u, v = xd[..., K::2], xd[..., K + 1::2]
+        rot = torch.stack([u * a.cos()[:, None] - v * a.sin()[:, None], v * a.cos()[:, None] + u * a.sin()[:, None]], dim=-1).flatten(-2) * 1.25
+        assert bool(((got[..., N:] - rot).abs() <= 2.0 ** -8 * rot.abs() + 2e-3).all())
