@@ -16,7 +16,9 @@
 // there the 256 channels that meet the value blocks lie in TMEM (128 columns beside S and O: the A operand may come from there), and two
 // tiles fit.  With values of up to 128 channels two CTAs fit an SM.
 //
-// Warps 0-3 run one thread each (copies, P V, Q K^T), warps 4-7 are the rows; registers change hands with setmaxnreg.  Every wait is bounded.
+// Warps 0-3 run one thread each (copies, P V, Q K^T), warps 4-7 are the rows; registers change hands with setmaxnreg.  Where one CTA fills an
+// SM its four warps of rows would leave the SM waiting for their chains (2,900 clocks a tile against 1,500 with a second CTA's beside them): there
+// warps 4-11 are the rows, two threads a row with 32 of a tile's keys each, which meet once a tile over the row's maximum.  Every wait is bounded.
 #include "common.cuh"
 #include "checks.cuh"
 #include "sm100.cuh"
@@ -24,11 +26,11 @@
 namespace {
 using namespace sm100;
 
-constexpr int BQ = 128, BKV = 64, kThreads = 256, kQkWarp = 2;
+constexpr int BQ = 128, BKV = 64, kQkWarp = 2;
 constexpr int kLaunchRegs = 128, kRegsFew = 64, kRegsMany = 192;
 static_assert(kRegsFew + kRegsMany <= 2 * kLaunchRegs, "the two warpgroups cannot hold more registers than the CTA was given");
 constexpr int kQBlock = BQ * 128, kBlock = BKV * 128;          // bytes of 64 channels of the queries / of a tile of keys
-constexpr int kMaxStages = 3, kBarBytes = 512, kSmemLimit = 227 * 1024;
+constexpr int kMaxStages = 3, kBarBytes = 256, kSmemLimit = 227 * 1024 - 1024;      // (1 KB of it is the rows' meeting place)
 constexpr float kRefSlack = 8.0f;     // a row's reference exponent moves only when its maximum has grown by more than 2^8 (see attention_sm100.cu)
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -42,6 +44,7 @@ struct ShapedParams {
     int H, heads, inner, M, D, E, VC; // heads: of a CTA; inner: CTAs of one tile (groups x maps x chunks of values)
     int q_channels;                   // channels of a query row that enter S
     int key_blocks, value_blocks;     // blocks of 64 channels of the two kinds
+    int k_boxed, v_boxed;             // blocks that one copy of a tile of keys (values) brings: all, where a page holds a whole tile, else one
     int latent;                       // the value blocks are key blocks too
     int q_tmem;                       // ... and the query channels that meet them are in TMEM, not in shared memory
     int stages, page_size, box_rows, max_pages, window, chunk, vec_out;
@@ -70,13 +73,26 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
-// D[tmem] (+)= A[tmem] . B[smem]^T: row r of A is lane r, 16 channels are eight columns of two bfloat16 numbers
-__device__ __forceinline__ void umma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// The products' descriptors as a low word that moves and a high word that does not: the one thread that issues them pays for every
+// instruction between two of them (whole 64-bit descriptors worked out per product: 120 to 150 clocks each, where the tensor core needs 32).
+// D[tmem] (+)= A[smem] . B[smem]^T
+__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// D[tmem] (+)= A[tmem] . B[smem]^T: row r of A is lane r, 16 channels are eight columns of two bfloat16 numbers
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -84,6 +100,14 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
           "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+
+// 4D tile load: c0 innermost (elements), then c1, c2, c3.
+__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
 
@@ -97,11 +121,13 @@ __device__ __forceinline__ int first_visible(int pos, int window, int chunk) {
 // score i of the row's 64 (i is a constant after unrolling)
 #define SV(i) ((i) < 32 ? sv_lo[(i) & 31] : sv_hi[(i) & 31])
 
-template <bool SHAPED>
-__global__ void __launch_bounds__(kThreads, 2)
+template <bool SHAPED, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 384 : 256, WIDE ? 1 : 2)
 shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                               const __grid_constant__ CUtensorMap tmap_v, const ShapedParams p) {
     extern __shared__ uint8_t smem_raw[];
+    __shared__ float meet[2][WIDE ? BQ : 1];                        // [half]: what a row's two threads tell each other
+    constexpr int kThreads = WIDE ? 384 : 256, kRowWarps = WIDE ? 8 : 4, NK = WIDE ? BKV / 2 : BKV;      // NK: a thread's keys of a tile
     const int tile = blockIdx.x / p.inner;
     const int t0 = p.tile_t0[tile], nq = p.tile_n[tile];
     if (!FORGE_TOKEN_OK(t0) || !FORGE_TOKEN_OK(t0 + nq - 1)) return;
@@ -132,7 +158,7 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         *abort = 0;
         mbar_init(q_full, 1);
         mbar_init(tail, 1);
-        mbar_init(q_ready, 4);
+        mbar_init(q_ready, kRowWarps);
         for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(&k_full[s], 1);
             mbar_init(&k_empty[s], 1);
@@ -141,7 +167,7 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&s_full[b], 1);
-            mbar_init(&p_ready[b], 4);
+            mbar_init(&p_ready[b], kRowWarps);
             mbar_init(&o_done[b], 1);
         }
         mbar_fence_init();
@@ -174,13 +200,14 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
     forge::pdl_wait();
 
     if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsFew));
+    if (!WIDE) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsFew));
     if (warp == 0) {
         // ------------------------------------------------------------------ copies
         const int32_t* table = p.block_table + (size_t)req * p.max_pages;
         const int ppt = p.page_size >= BKV ? 1 : BKV / p.page_size;       // boxes a tile and block
-        const int k_col0 = p.latent ? 0 : mp * p.D, v_col0 = vc * p.VC, row0 = group * p.page_size;
+        const int row0 = group * p.page_size, k_col0 = p.latent ? 0 : mp * p.D;
         const int skip = p.latent ? vc * p.value_blocks : 1 << 20;        // key block i stands for channel block i, or i + value_blocks from here on
+        const int others = p.latent ? (chunks - 1) * p.value_blocks : 0;  // key blocks that are the other chunk's value blocks: they come like them
         if (lane == 0) {
             mbar_arrive_expect_tx(q_full, q_blocks * q_rows * 128);
             for (int b = 0; b < q_blocks; ++b)
@@ -212,9 +239,15 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) break;
                 __syncwarp();
-                if (page >= 0)
-                    for (int b = 0; b < p.key_blocks; ++b)
-                        tma_load_3d(kd + b * kBlock + lane * box_bytes, &tmap_k, &k_full[st], k_col0 + (b < skip ? b : b + p.value_blocks) * 64, row0 + off, page);
+                if (page >= 0) {
+                    uint8_t* dst = kd + lane * box_bytes;
+                    for (int b = 0; b < others; b += p.v_boxed)
+                        tma_load_4d(dst + b * kBlock, &tmap_v, &k_full[st], 0, row0 + off, b < skip ? b : b + p.value_blocks, page);
+                    for (int b = others; b < p.key_blocks; b += p.k_boxed) {
+                        if (p.latent) tma_load_4d(dst + b * kBlock, &tmap_k, &k_full[st], p.E + (b - others) * 64, row0 + off, 0, page);
+                        else tma_load_4d(dst + b * kBlock, &tmap_k, &k_full[st], 0, row0 + off, mp * p.key_blocks + b, page);
+                    }
+                }
             }
             if (lane == 0) {
                 ok = mbar_wait<true>(&v_empty[st], ph ^ 1, abort, p.status, 2);
@@ -224,8 +257,8 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             if (!ok) break;
             __syncwarp();
             if (page >= 0)
-                for (int b = 0; b < p.value_blocks; ++b)
-                    tma_load_3d(vd + b * kBlock + lane * box_bytes, &tmap_v, last ? tail : &v_full[st], v_col0 + b * 64, row0 + off, page);
+                for (int b = 0; b < p.value_blocks; b += p.v_boxed)
+                    tma_load_4d(vd + b * kBlock + lane * box_bytes, &tmap_v, last ? tail : &v_full[st], 0, row0 + off, vc * p.value_blocks + b, page);
             if (last) {
                 // what lies in the cache behind the last token counts as zeros: a weight of 0 would not silence a NaN there
                 if (lane == 0) ok = mbar_wait<true>(tail, tail_ph, abort, p.status, 3);
@@ -244,7 +277,9 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
     } else if (warp == 1) {
         // ------------------------------------------------------------------ P V
         if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16_f32_bmn(BQ, p.VC);
+            const uint32_t idesc = umma_idesc_bf16_f32_bmn(BQ, p.VC), v_step = p.value_blocks * kBlock >> 4;
+            const uint64_t vdesc = umma_desc_mn_sw128(smem_u32(v_s), kBlock);
+            const uint32_t v_lo0 = (uint32_t)vdesc, hi = (uint32_t)(vdesc >> 32);
             bool ok = true;
             int st = 0, ph = 0;
             for (int it = 0; it < n_iter && ok; ++it) {
@@ -252,13 +287,11 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 if (!(ok = mbar_wait<true>(&v_full[st], ph, abort, p.status, 4))) break;
                 if (!(ok = mbar_wait<true>(&p_ready[b], (it >> 1) & 1, abort, p.status, 5))) break;
                 tc_fence_after_sync();
-                const uint64_t vdesc = umma_desc_mn_sw128(smem_u32(v_s + st * p.value_blocks * kBlock), kBlock);
-                const uint32_t pt = tmem_base + b * BKV;
+                const uint32_t v_lo = v_lo0 + st * v_step, pt = tmem_base + b * BKV;
 #pragma unroll
                 for (int k = 0; k < BKV / 16; ++k) {
-                    const uint64_t vk = umma_desc_advance(vdesc, k * 2048);
-                    umma_bf16_ta(tmem_o, pt + 32 + k * 8, vk, idesc, (it | k) != 0);
-                    umma_bf16_ta(tmem_o, pt + k * 8, vk, idesc, 1);
+                    umma_ts(tmem_o, pt + 32 + k * 8, v_lo + k * (2048 >> 4), hi, idesc, k > 0 ? 1 : (uint32_t)(it > 0));
+                    umma_ts(tmem_o, pt + k * 8, v_lo + k * (2048 >> 4), hi, idesc, 1);
                 }
                 umma_commit(&o_done[b]);
                 umma_commit(&v_empty[st]);
@@ -270,29 +303,37 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         if (lane == 0) {
             const uint32_t idesc = umma_idesc_bf16_f32(BQ, BKV);
             const int skip = p.latent ? vc * p.value_blocks : 1 << 20;
+            const uint64_t qdesc = umma_desc_k_sw128(smem_u32(q_s));
+            const uint32_t q_lo = (uint32_t)qdesc, hi = (uint32_t)(qdesc >> 32);
+            const uint32_t k_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(k_s)), v_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(v_s));
+            const uint32_t k_step = p.key_blocks * kBlock >> 4, v_step = p.value_blocks * kBlock >> 4;
+            const int part_steps = p.q_channels % 64 / 16, part_block = part_steps ? p.q_channels / 64 : -1;
             bool ok = mbar_wait<true>(q_full, 0, abort, p.status, 6);
             int st = 0, ph = 0;
             for (int it = 0; it < n_iter && ok; ++it) {
                 const int b = it & 1;
                 // (the scores' buffer holds the weights of tile it - 2 until its P V is done)
                 if (it >= 2 && !(ok = mbar_wait<true>(&o_done[b], ((it - 2) >> 1) & 1, abort, p.status, 7))) break;
-                const uint64_t qdesc = umma_desc_k_sw128(smem_u32(q_s));
+                const uint32_t ds = tmem_base + b * BKV;
                 uint32_t add = 0;
-                // key block `blk` of a ring stage against the query's channel block in shared memory
-                auto product = [&](const uint8_t* blocks, int blk, int q_block, int channel_block) {
-                    const uint64_t a = umma_desc_advance(qdesc, q_block * kQBlock), w = umma_desc_k_sw128(smem_u32(blocks + blk * kBlock));
-                    const int steps = min(4, (p.q_channels - channel_block * 64) / 16);
-                    for (int k = 0; k < steps; ++k) {
-                        umma_bf16(tmem_base + b * BKV, umma_desc_advance(a, k * 32), umma_desc_advance(w, k * 32), idesc, add);
-                        add = 1;
+                // key block at w_lo against the query's channel block at a_lo
+                auto product = [&](uint32_t a_lo, uint32_t w_lo, int channel_block) {
+                    if (channel_block != part_block) {
+                        umma_ss(ds, a_lo, w_lo, hi, idesc, add);
+#pragma unroll
+                        for (int k = 1; k < 4; ++k) umma_ss(ds, a_lo + k * 2, w_lo + k * 2, hi, idesc, 1);
+                    } else {                                              // the last channels do not fill a block
+                        for (int k = 0; k < part_steps; ++k) umma_ss(ds, a_lo + k * 2, w_lo + k * 2, hi, idesc, add | (uint32_t)(k > 0));
                     }
+                    add = 1;
                 };
                 if (p.key_blocks > 0) {
                     if (!(ok = mbar_wait<true>(&k_full[st], ph, abort, p.status, 8))) break;
                     tc_fence_after_sync();
+                    const uint32_t w_lo = k_lo0 + st * k_step;
                     for (int i = 0; i < p.key_blocks; ++i) {
                         const int channel_block = i < skip ? i : i + p.value_blocks;
-                        product(k_s + st * p.key_blocks * kBlock, i, p.q_tmem ? i : channel_block, channel_block);
+                        product(q_lo + (p.q_tmem ? i : channel_block) * (kQBlock >> 4), w_lo + i * (kBlock >> 4), channel_block);
                     }
                     umma_commit(&k_empty[st]);
                 }
@@ -300,18 +341,15 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                     if (it == 0 && p.q_tmem && !(ok = mbar_wait<true>(q_ready, 0, abort, p.status, 13))) break;
                     if (!(ok = mbar_wait<true>(&v_full[st], ph, abort, p.status, 9))) break;
                     tc_fence_after_sync();
-                    for (int i = 0; i < p.value_blocks; ++i) {
-                        const uint8_t* blocks = v_s + st * p.value_blocks * kBlock;
-                        if (p.q_tmem) {
-                            const uint64_t w = umma_desc_k_sw128(smem_u32(blocks + i * kBlock));
+                    const uint32_t w_lo = v_lo0 + st * v_step;
+                    if (p.q_tmem) {
+                        for (int i = 0; i < p.value_blocks; ++i) {
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                umma_bf16_ta(tmem_base + b * BKV, tmem_o + p.VC + i * 32 + k * 8, umma_desc_advance(w, k * 32), idesc, add);
-                                add = 1;
-                            }
-                        } else {
-                            product(blocks, i, skip + i, skip + i);
+                            for (int k = 0; k < 4; ++k) umma_ts(ds, tmem_o + p.VC + i * 32 + k * 8, w_lo + i * (kBlock >> 4) + k * 2, hi, idesc, k > 0 ? 1 : add);
+                            add = 1;
                         }
+                    } else {
+                        for (int i = 0; i < p.value_blocks; ++i) product(q_lo + (skip + i) * (kQBlock >> 4), w_lo + i * (kBlock >> 4), skip + i);
                     }
                 }
                 umma_commit(&s_full[b]);
@@ -320,8 +358,9 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         }
     }
     } else {
-        // ------------------------------------------------------------------ the rows (warps 4..7)
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsMany));
+        // ------------------------------------------------------------------ the rows (warps 4..7, or 4..11)
+        if (!WIDE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsMany));
+        const int half = WIDE ? (warp - 4) >> 2 : 0;
         const int quarter = warp & 3, r = quarter * 32 + lane;
         const bool valid = r < nq * p.heads;
         const int tok = t0 + (valid ? r / p.heads : 0), head = group * p.heads + (valid ? r % p.heads : 0), pos = pos0 + tok - t0;
@@ -334,7 +373,8 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         bool ok = true;
         if (p.q_tmem) {                       // this row's channels vc * VC .. of the query, two to a column
             const __nv_bfloat16* src = p.q + ((size_t)tok * p.H + head) * p.D + vc * p.VC;
-            for (int c = 0; c < p.VC; c += 64) {
+            const int share = p.VC / (WIDE ? 2 : 1);
+            for (int c = half * share; c < (half + 1) * share; c += 64) {
                 uint32_t w[32];
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
@@ -349,18 +389,21 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             __syncwarp();
             if (lane == 0) mbar_arrive(q_ready);
         }
-        for (int it = 0; it < n_iter && ok; ++it) {
-            const int j0 = (t_begin + it) * BKV, b = it & 1;
-            if (!(ok = mbar_wait<true>(&s_full[b], (it >> 1) & 1, abort, p.status, 10))) break;
+        // (a wait that ran out lets the loop go on without waiting: the two threads of a row have to meet in every round)
+        for (int it = 0; it < n_iter; ++it) {
+            const int j0 = (t_begin + it) * BKV + half * NK, b = it & 1;
+            const uint32_t t_s = t_lane + b * BKV;
+            ok = ok && mbar_wait<true>(&s_full[b], (it >> 1) & 1, abort, p.status, 10);
+            __syncwarp();
             tc_fence_after_sync();
             uint32_t sv_lo[32], sv_hi[32];
-            tmem_ld_32x32b_x32(t_lane + b * BKV, sv_lo);
-            tmem_ld_32x32b_x32(t_lane + b * BKV + 32, sv_hi);
+            tmem_ld_32x32b_x32(t_s + half * NK, sv_lo);
+            if (!WIDE) tmem_ld_32x32b_x32(t_s + 32, sv_hi);
             tmem_ld_wait();
-            const bool need_mask = !valid || j0 + BKV - 1 > pos || j0 < see;
+            const bool need_mask = !valid || j0 + NK - 1 > pos || j0 < see;
             if (SHAPED) {                     // in units of log2 e, shaped, from here on
 #pragma unroll
-                for (int i = 0; i < BKV; ++i) {
+                for (int i = 0; i < NK; ++i) {
                     float s = __uint_as_float(SV(i));
                     s = p.softcap > 0.f ? cap_out * tanh_fast(s * cap_in) : s * sl2;
                     if (p.r1) s -= r1v * __log2f(fmaf(r2v, (float)max(pos - j0 - i, 0), 1.0f));
@@ -369,28 +412,50 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             }
             if (need_mask) {
 #pragma unroll
-                for (int i = 0; i < BKV; ++i) {
+                for (int i = 0; i < NK; ++i) {
                     const int j = j0 + i;
                     if (!(valid && j <= pos && j >= see)) SV(i) = __float_as_uint(-INFINITY);
                 }
             }
             float a0 = -INFINITY, a1 = -INFINITY;
 #pragma unroll
-            for (int i = 0; i < BKV; i += 4) {
+            for (int i = 0; i < NK; i += 4) {
                 a0 = max3(a0, __uint_as_float(SV(i)), __uint_as_float(SV(i + 1)));
                 a1 = max3(a1, __uint_as_float(SV(i + 2)), __uint_as_float(SV(i + 3)));
             }
             const float mult = SHAPED ? 1.0f : sl2;
-            const float top = fmaxf(a0, a1) * mult;
+            float top = fmaxf(a0, a1) * mult;
+            if (WIDE) {
+                // Whether any of the two warps' rows has to move its reference; mostly none has, and the row's maximum is nobody's business.
+                // (Both have read their scores by then: either's weights may overwrite the other's.)
+                int moves;
+                __syncwarp();
+                tc_fence_before_sync();
+                asm volatile(
+                    "{\n\t.reg .pred p, q;\n\t"
+                    "setp.gt.f32 p, %1, %2;\n\t"
+                    "barrier.cta.red.or.pred.aligned q, %3, 64, p;\n\t"
+                    "selp.s32 %0, 1, 0, q;\n\t}"
+                    : "=r"(moves) : "f"(top), "f"(m + kRefSlack), "r"(1 + quarter) : "memory");
+                tc_fence_after_sync();
+                if (moves) {
+                    meet[half][WIDE ? r : 0] = top;
+                    asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
+                    top = fmaxf(top, meet[half ^ 1][WIDE ? r : 0]);
+                    asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
+                }
+            }
             const float m_new = top > m + kRefSlack ? top : m;            // (-inf + slack is -inf: the first visible key sets it)
             const float alpha = m_new == m ? 1.0f : ex2(m - m_new);
             m = m_new;
             const float ref = m == -INFINITY ? 0.f : m;
             // O is rescaled only when some row of the warp moved its reference; P V of the tile before must be complete by then
             if (it > 0 && !__all_sync(0xffffffffu, alpha == 1.0f)) {
-                if (!(ok = mbar_wait<true>(&o_done[b ^ 1], ((it - 1) >> 1) & 1, abort, p.status, 11))) break;
+                ok = ok && mbar_wait<true>(&o_done[b ^ 1], ((it - 1) >> 1) & 1, abort, p.status, 11);
+                __syncwarp();
                 tc_fence_after_sync();
-                for (int c = 0; c < p.VC; c += 32) {
+                const int share = p.VC / (WIDE ? 2 : 1);
+                for (int c = half * share; c < (half + 1) * share; c += 32) {
                     uint32_t ov[32];
                     tmem_ld_32x32b_x32(t_out + c, ov);
                     tmem_ld_wait();
@@ -404,7 +469,7 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             // the weights, their sum, and P in two terms over the scores' columns: roundings in the first 32, the rest in the next
             float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
-            for (int c = 0; c < BKV; c += 32) {
+            for (int c = 0; c < NK; c += 32) {
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
@@ -420,14 +485,19 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                     lo[i / 2] = pack_bf16(p0 - __uint_as_float(h01 << 16), p1 - __uint_as_float(h01 & 0xffff0000u));
                     lo[i / 2 + 1] = pack_bf16(p2 - __uint_as_float(h23 << 16), p3 - __uint_as_float(h23 & 0xffff0000u));
                 }
-                tmem_st_32x32b_x16(t_lane + b * BKV + c / 2, hi);
-                tmem_st_32x32b_x16(t_lane + b * BKV + 32 + c / 2, lo);
+                tmem_st_32x32b_x16(t_s + half * 16 + c / 2, hi);
+                tmem_st_32x32b_x16(t_s + 32 + half * 16 + c / 2, lo);
             }
             l = l * alpha + ((s0 + s1) + (s2 + s3));
             tmem_st_wait();
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_ready[b]);
+        }
+        if (WIDE) {                           // the row's sum of weights
+            meet[half][WIDE ? r : 0] = l;
+            asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
+            l = meet[0][WIDE ? r : 0] + meet[1][WIDE ? r : 0];
         }
         if (ok) ok = mbar_wait<true>(&o_done[(n_iter - 1) & 1], ((n_iter - 1) >> 1) & 1, abort, p.status, 12);
         tc_fence_after_sync();
@@ -441,7 +511,8 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             inv *= p.out_scale;
             const int v0 = vc * p.VC;
             // every lane takes part in the TMEM loads (they are warp-wide instructions); only valid rows store
-            for (int c = 0; c < p.VC; c += 32) {
+            const int share = p.VC / (WIDE ? 2 : 1);
+            for (int c = half * share; c < (half + 1) * share; c += 32) {
                 uint32_t ov[32];
                 __syncwarp();
                 tmem_ld_32x32b_x32(t_out + c, ov);
@@ -480,20 +551,35 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
     }
 }
 
-// A bf16 tensor of three dimensions read in boxes of 64 x b1 x b2 with 128-byte swizzle; strides in elements.
-bool map3(const void* ptr, unsigned long long d0, unsigned long long d1, unsigned long long d2, unsigned long long s1, unsigned long long s2, int b1, int b2,
-          CUtensorMap* out, const char** err) {
+// A bf16 tensor of three or four dimensions read in boxes of 64 x b1 x b2 (x b3) with 128-byte swizzle; strides in elements.
+bool tensor_map(const void* ptr, int rank, const unsigned long long (&d)[4], const unsigned long long (&stride)[3], const int (&b)[4], CUtensorMap* out, const char** err) {
     auto fn = encode_fn();
     if (!fn) { *err = "cuTensorMapEncodeTiled is not available from the driver"; return false; }
-    const cuuint64_t dims[3] = {d0, d1, d2}, strides[2] = {s1 * 2, s2 * 2};
-    const cuuint32_t box[3] = {64u, (cuuint32_t)b1, (cuuint32_t)b2}, estr[3] = {1u, 1u, 1u};
-    if ((reinterpret_cast<uintptr_t>(ptr) & 15) || strides[0] % 16 || strides[1] % 16) { *err = "TMA needs 16-byte aligned rows"; return false; }
-    if (fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    cuuint64_t dims[4], strides[3];
+    cuuint32_t box[4], estr[4] = {1u, 1u, 1u, 1u};
+    for (int i = 0; i < 4; ++i) { dims[i] = d[i]; box[i] = (cuuint32_t)b[i]; }
+    for (int i = 0; i < 3; ++i) strides[i] = stride[i] * 2;
+    bool aligned = (reinterpret_cast<uintptr_t>(ptr) & 15) == 0;
+    for (int i = 0; i + 1 < rank; ++i) aligned = aligned && strides[i] % 16 == 0;
+    if (!aligned) { *err = "TMA needs 16-byte aligned rows"; return false; }
+    if (fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
         *err = "cuTensorMapEncodeTiled failed";
         return false;
     }
     return true;
+}
+// queries [T, heads, channels] in boxes of 64 channels of b1 heads of b2 tokens
+bool query_map(const void* ptr, int channels, int heads, int T, int b1, int b2, CUtensorMap* out, const char** err) {
+    return tensor_map(ptr, 3, {(unsigned long long)channels, (unsigned long long)heads, (unsigned long long)T, 1},
+                      {(unsigned long long)channels, (unsigned long long)heads * channels, 0}, {64, b1, b2, 1}, out, err);
+}
+// rows of `channels` numbers, `pitch` apart, seen as blocks of 64: one box is `rows` rows of `blocks` neighbouring blocks of a page, and lands
+// as `blocks` tiles one after the other.  An SM's copies complete about one per 0.3 us whatever their size, so a tile is one copy where a
+// page holds it (latent of 512 + 64 channels: nine copies of 8 KB a tile took 5,300 clocks).
+bool block_map(const void* ptr, int channels, int pitch, int rows, int pages, long long page_stride, int box_rows, int blocks, CUtensorMap* out, const char** err) {
+    return tensor_map(ptr, 4, {64, (unsigned long long)rows, (unsigned long long)(channels / 64), (unsigned long long)pages},
+                      {(unsigned long long)pitch, 64, (unsigned long long)page_stride}, {64, box_rows, blocks, 1}, out, err);
 }
 
 bool pages_fit(int page_size) { return page_size >= 8 && (page_size & (page_size - 1)) == 0 && page_size <= 65536; }
@@ -503,12 +589,31 @@ size_t smem_bytes(int q_blocks, int blocks, int stages) { return (size_t)q_block
 // value columns of a CTA: all up to 256, else chunks of 256 (0: not taken)
 int value_columns(int E) { return E % 64 ? 0 : E <= 256 ? E : E % 256 ? 0 : 256; }
 
+template <bool SHAPED, bool WIDE>
+int launch_one(const char* what, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const ShapedParams& p, size_t smem, int num_tiles,
+               cudaStream_t stream) {
+    auto* kernel = shaped_attention_sm100_kernel<SHAPED, WIDE>;
+    static forge::PerDeviceFlag configured_on;
+    bool& configured = configured_on.current();
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+        if (e != cudaSuccess) return forge::fail(FORGE_ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(e));
+        // the warpgroups trade registers inside what the CTA was given at launch: a build that gives less is refused
+        cudaFuncAttributes attr;
+        e = cudaFuncGetAttributes(&attr, kernel);
+        if (e != cudaSuccess) return forge::fail(FORGE_ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(e));
+        if (!WIDE && attr.numRegs * 2 < kRegsFew + kRegsMany)
+            return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: built with %d registers per thread, needs %d", what, attr.numRegs, (kRegsFew + kRegsMany + 1) / 2);
+        configured = true;
+    }
+    return forge::check_launch(what, forge::launch(kernel, dim3((unsigned)num_tiles * p.inner), dim3(WIDE ? 384 : 256), smem, stream, 1, tq, tk, tv, p));
+}
+
 template <bool SHAPED>
 int launch(const char* what, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, ShapedParams p, int num_tiles, cudaStream_t stream) {
     int q_blocks = (p.q_channels + 63) / 64;
     const int blocks = p.key_blocks + p.value_blocks;
     // where the queries leave room for one tile of rows, those that meet the value blocks go to TMEM if it has the columns
-    // (latent of 512 + 64 channels: one tile 268 us, two 110 for the portions of 512 and 1,024 tokens behind 700 and none)
     if (p.latent && smem_bytes(q_blocks, blocks, 2) > kSmemLimit && 2 * BKV + p.VC + p.value_blocks * 32 <= 512 && ((uintptr_t)p.q & 15) == 0 && p.D % 8 == 0) {
         p.q_tmem = 1;
         q_blocks -= p.value_blocks;
@@ -519,21 +624,9 @@ int launch(const char* what, const CUtensorMap& tq, const CUtensorMap& tk, const
     if (smem > kSmemLimit) return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: queries of %d channels", what, p.q_channels);
     p.tmem_cols = 2 * BKV + p.VC + (p.q_tmem ? p.value_blocks * 32 : 0) <= 256 ? 256 : 512;
     p.box_rows = p.page_size < BKV ? p.page_size : BKV;
-    static forge::PerDeviceFlag configured_on;
-    bool& configured = configured_on.current();
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(shaped_attention_sm100_kernel<SHAPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-        if (e != cudaSuccess) return forge::fail(FORGE_ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(e));
-        // the warpgroups trade registers inside what the CTA was given at launch: a build that gives less is refused
-        cudaFuncAttributes attr;
-        e = cudaFuncGetAttributes(&attr, shaped_attention_sm100_kernel<SHAPED>);
-        if (e != cudaSuccess) return forge::fail(FORGE_ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(e));
-        if (attr.numRegs * 2 < kRegsFew + kRegsMany)
-            return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: built with %d registers per thread, needs %d", what, attr.numRegs, (kRegsFew + kRegsMany + 1) / 2);
-        configured = true;
-    }
-    return forge::check_launch(what, forge::launch(shaped_attention_sm100_kernel<SHAPED>, dim3((unsigned)num_tiles * p.inner), dim3(kThreads), smem, stream, 1,
-                                                   tq, tk, tv, p));
+    // one CTA an SM, by its tensor memory or its shared memory: two threads a row
+    const bool alone = p.tmem_cols > 256 || smem > 112 * 1024;
+    return alone ? launch_one<SHAPED, true>(what, tq, tk, tv, p, smem, num_tiles, stream) : launch_one<SHAPED, false>(what, tq, tk, tv, p, smem, num_tiles, stream);
 }
 
 }  // namespace
@@ -562,9 +655,12 @@ extern "C" int forge_latent_attention_sm100(const void* q, const void* cache, co
     if (T == 0 || num_tiles == 0) return FORGE_OK;
     const int KD = C + R, VC = value_columns(C), chunks = C / VC;
     const char* err = nullptr;
-    CUtensorMap tq, tk;
-    if (!map3(q, KD, H, T, KD, (unsigned long long)H * KD, H, BQ / H, &tq, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "latent_attention_sm100: q: %s", err);
-    if (!map3(cache, KD, page_size, num_pages, KD, (unsigned long long)page_size * KD, page_size < BKV ? page_size : BKV, 1, &tk, &err))
+    CUtensorMap tq, tk, tv;
+    const int rows = page_size < BKV ? page_size : BKV, v_boxed = rows == BKV ? VC / 64 : 1;
+    if (!query_map(q, KD, H, T, H, BQ / H, &tq, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "latent_attention_sm100: q: %s", err);
+    const unsigned long long pages = (unsigned long long)num_pages, page = (unsigned long long)page_size * KD;
+    if (!block_map(cache, C, KD, page_size, num_pages, (long long)page, rows, v_boxed, &tv, &err) ||
+        !tensor_map(cache, 4, {(unsigned long long)KD, (unsigned long long)page_size, 1, pages}, {(unsigned long long)KD, page, page}, {64, rows, 1, 1}, &tk, &err))
         return forge::fail(FORGE_ERR_UNSUPPORTED, "latent_attention_sm100: cache: %s", err);
     ShapedParams p{};
     p.out = (__nv_bfloat16*)out; p.out_ld = (long long)H * C;
@@ -572,9 +668,10 @@ extern "C" int forge_latent_attention_sm100(const void* q, const void* cache, co
     p.sink = sink; p.q = (const __nv_bfloat16*)q;
     p.H = p.heads = H; p.inner = chunks; p.M = 1; p.D = KD; p.E = C; p.VC = VC;
     p.q_channels = KD; p.value_blocks = VC / 64; p.key_blocks = (KD + 63) / 64 - p.value_blocks; p.latent = 1;
+    p.k_boxed = 1; p.v_boxed = v_boxed;
     p.page_size = page_size; p.max_pages = max_pages; p.window = window;
     p.vec_out = ((uintptr_t)out & 15) == 0; p.scale = scale; p.out_scale = 1.0f; p.status = status;
-    return launch<false>("latent_attention_sm100", tq, tk, tk, p, num_tiles, stream);
+    return launch<false>("latent_attention_sm100", tq, tk, tv, p, num_tiles, stream);
 }
 
 // q bf16 [T, H, M, D]; cache pages of page_stride numbers, [G, page_size, M*D] keys then [G, page_size, E] values; one map: out bf16, rows of
@@ -594,9 +691,10 @@ extern "C" int forge_scored_attention_sm100(const void* q, const void* cache, co
     const int MD = M * D, Gq = H / G, VC = value_columns(E), rows = page_size < BKV ? page_size : BKV;
     const char* err = nullptr;
     CUtensorMap tq, tk, tv;
-    if (!map3(q, MD, H, T, MD, (unsigned long long)H * MD, Gq, BQ / Gq, &tq, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "scored_attention_sm100: q: %s", err);
-    if (!map3(cache, MD, (unsigned long long)G * page_size, num_pages, MD, page_stride, rows, 1, &tk, &err) ||
-        !map3((const __nv_bfloat16*)cache + (size_t)G * page_size * MD, E, (unsigned long long)G * page_size, num_pages, E, page_stride, rows, 1, &tv, &err))
+    if (!query_map(q, MD, H, T, Gq, BQ / Gq, &tq, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "scored_attention_sm100: q: %s", err);
+    const int k_boxed = rows == BKV ? D / 64 : 1, v_boxed = rows == BKV ? VC / 64 : 1;
+    if (!block_map(cache, MD, MD, G * page_size, num_pages, page_stride, rows, k_boxed, &tk, &err) ||
+        !block_map((const __nv_bfloat16*)cache + (size_t)G * page_size * MD, E, E, G * page_size, num_pages, page_stride, rows, v_boxed, &tv, &err))
         return forge::fail(FORGE_ERR_UNSUPPORTED, "scored_attention_sm100: cache: %s", err);
     ShapedParams p{};
     p.out = (__nv_bfloat16*)out; p.out_ld = out_ld; p.u = M == 2 ? u : nullptr;
@@ -604,6 +702,7 @@ extern "C" int forge_scored_attention_sm100(const void* q, const void* cache, co
     p.r1 = r1; p.r2 = r2; p.sink = sink;
     p.H = H; p.heads = Gq; p.inner = G * M * (E / VC); p.M = M; p.D = D; p.E = E; p.VC = VC;
     p.q_channels = D; p.key_blocks = D / 64; p.value_blocks = VC / 64; p.latent = 0;
+    p.k_boxed = k_boxed; p.v_boxed = v_boxed;
     p.page_size = page_size; p.max_pages = max_pages; p.window = window; p.chunk = chunk; p.softcap = softcap;
     p.vec_out = ((uintptr_t)out & 15) == 0 && out_ld % 8 == 0; p.scale = scale; p.out_scale = M == 1 ? out_scale : 1.0f; p.status = status;
     return r1 != nullptr || softcap > 0.f ? launch<true>("scored_attention_sm100", tq, tk, tv, p, num_tiles, stream)
