@@ -49,17 +49,11 @@ struct GemmParams {
     const int32_t* slot_mapping;     // [M] page * page_size + offset of each row's token (negative or null: no cache write)
     __nv_bfloat16* kv_cache;         // [pages, 2, NKV, page_size, head_dim]
     int NH, NKV, head_dim, page_size;
-    // a device word that an earlier kernel wrote: where it holds 0 the whole product is skipped (nothing is read or written); null: none
-    const int* live;
+    // (GROUPED kernels) rows of A packed by expert, counts[e] of them each, against W [groups, N, K]; N is one expert's
+    const int* counts;
+    int groups;
     float act_a, act_b;              // numbers of the activation in the bfloat16 store (builds with -DFORGE_CAST_ACT=2)
 };
-
-// Every thread of every CTA leaves before anything is set up (no barrier, tensor memory or copy exists yet), all the same way.
-#define FORGE_SKIP_IF_NOT_LIVE(p)                       \
-    if ((p).live != nullptr) {                          \
-        forge::pdl_wait();                              \
-        if (*(p).live == 0) return;                     \
-    }
 
 template <int BN> struct Cfg {
     static constexpr int kStageBytes = (BM + BN) * BK * 2;
@@ -105,10 +99,49 @@ __device__ __forceinline__ float gate_act(int epilogue, float g) {
 #endif
 }
 
+// Products of many small matrices, one per expert of a routed feed-forward: expert e's rows of A lie packed behind those of the experts
+// before it, how many they are is a word on the device that a kernel before this one wrote, and W is [groups, N, K].  One launch does
+// what a launch per expert did (16 hand-overs a layer, and a wait of the host for the counts where a step is long): 8 tokens, two of 8 experts
+// of [7168 x 4096] each, both products 268 us in 16 launches, 196 us (6.3 TB/s) in two; 1,501 tokens, experts of [2816 x 2048], 250 us and 140 us.  The whole CTA calls this
+// after the dependency wait; first[e] becomes the first row of expert e, work[e] the sum of unit(rows) over the experts before it.
+__host__ __device__ constexpr int group_bytes(int groups) { return 2 * (groups + 1) * 4; }
+template <typename Unit>
+__device__ __forceinline__ void group_sums(const int* counts, int groups, int* first, int* work, Unit unit) {
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int rows = 0, units = 0;
+        for (int e0 = 0; e0 < groups; e0 += 32) {
+            const int n = e0 + lane < groups ? counts[e0 + lane] : 0;
+            int a = n, b = n > 0 ? unit(n) : 0;
+            const int own_a = a, own_b = b;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+                if (lane >= o) { a += x; b += y; }
+            }
+            if (e0 + lane < groups) { first[e0 + lane] = rows + a - own_a; work[e0 + lane] = units + b - own_b; }
+            rows += __shfl_sync(0xffffffffu, a, 31);
+            units += __shfl_sync(0xffffffffu, b, 31);
+        }
+        if (lane == 0) { first[groups] = rows; work[groups] = units; }
+    }
+    __syncthreads();
+}
+// the expert whose work holds unit u
+__device__ __forceinline__ int group_of(const int* work, int groups, int u) {
+    int lo = 0, hi = groups - 1;                              // the last expert whose work begins at or before u (those without work share a beginning)
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (work[mid] <= u) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
 // Applies the epilogue to 32 consecutive columns (n .. n+31) of output row m held in r (fp32 bits) and stores them.
 template <int BN>
-__device__ __forceinline__ void store_row_chunk(const GemmParams& p, const uint32_t (&r)[32], int m, int n) {
-    if (m < p.M && n < p.N) {
+__device__ __forceinline__ void store_row_chunk(const GemmParams& p, const uint32_t (&r)[32], int m, int n, int m_end) {
+    if (m < m_end && n < p.N) {
         float v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
@@ -232,13 +265,12 @@ __device__ __forceinline__ void qkv_rope_row(const GemmParams& p, uint32_t t_row
     }
 }
 
-template <int BN>
+template <int BN, bool GROUPED = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                   const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
     using C = Cfg<BN>;
     constexpr int kStages = C::kStages;
-    FORGE_SKIP_IF_NOT_LIVE(p);
     extern __shared__ uint8_t smem_raw[];
     // tiles need 1024-byte alignment for the 128-byte swizzle pattern to line up with the descriptors
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -254,7 +286,21 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
-    const int num_tiles = tiles_m * tiles_n;
+    int num_tiles = tiles_m * tiles_n;
+    int* first_row = reinterpret_cast<int*>(out_s);               // (GROUPED: results do not leave through these buffers)
+    int* first_tile = first_row + p.groups + 1;
+    // a tile's rows of A, column of the result, row of W, and the row its results end before
+    struct Place { int m0, n0, w0, m_end; };
+    auto place = [&](int tile) {
+        if constexpr (GROUPED) {
+            const int e = group_of(first_tile, p.groups, tile), rows = first_row[e + 1] - first_row[e], tm = (rows + BM - 1) / BM, t = tile - first_tile[e];
+            const int n0 = t / tm * BN;
+            return Place{first_row[e] + t % tm * BM, n0, e * p.N + n0, first_row[e + 1]};
+        } else {
+            const int n0 = (tile / tiles_m) * BN;
+            return Place{(tile % tiles_m) * BM, n0, n0, p.M};
+        }
+    };
     const int num_kb = (p.K + BK - 1) / BK;
 
     if (threadIdx.x == 0) {
@@ -274,6 +320,11 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     forge::pdl_launch_dependents();
+    if constexpr (GROUPED) {
+        forge::pdl_wait();
+        group_sums(p.counts, p.groups, first_row, first_tile, [&](int rows) { return (rows + BM - 1) / BM * tiles_n; });
+        num_tiles = first_tile[p.groups];
+    }
     // A, bias and C may come from (or still be read by) earlier kernels: the thread that copies and the warps that
     // write wait for them below.  W does not: the first tile's first k-blocks of it are asked for before the wait.
 
@@ -283,7 +334,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             uint32_t it = 0;       // k-blocks issued so far, over all tiles
             bool ok = true;
             uint32_t ahead = 0;    // stages whose W is on its way already
-            if ((int)blockIdx.x < num_tiles) {
+            if (!GROUPED && (int)blockIdx.x < num_tiles) {
                 const int n0 = ((int)blockIdx.x / tiles_m) * BN;
                 ahead = num_kb < kStages ? num_kb : kStages;
                 for (uint32_t s = 0; s < ahead; ++s) {
@@ -293,7 +344,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
             forge::pdl_wait();
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
+                const Place at = place(tile);
+                const int m0 = at.m0, n0 = at.w0;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % kStages;
                     uint8_t* a_dst = tiles + s * C::kStageBytes;
@@ -357,12 +409,13 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
             const int a = local & 1;
             const uint32_t aph = (local >> 1) & 1;
-            const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
+            const Place at = place(tile);
+            const int m0 = at.m0, n0 = at.n0;
             if (!(ok = mbar_wait(&acc_full[a], aph, abort, p.status))) break;
             tc_fence_after_sync();
             const int m = m0 + row_in_tile;
             const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * BN;
-            if constexpr (C::kOutBytes > 0) {
+            if constexpr (C::kOutBytes > 0 && !GROUPED) {
                 if (p.tma_out) {
                     // fp32 results: a chunk of 32 columns of all 128 rows goes to shared memory (the layout of a
                     // 128-byte-swizzled box) and from there to global memory with one TMA instruction, a store
@@ -400,7 +453,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                     continue;
                 }
             }
-            if constexpr (BN % 128 == 0) {
+            if constexpr (BN % 128 == 0 && !GROUPED) {
                 if (p.epilogue == EPI_QKV_ROPE) {
                     if (p.head_dim == 64) qkv_rope_row<BN, 64>(p, t_row, m, n0);
                     else qkv_rope_row<BN, 128>(p, t_row, m, n0);
@@ -421,12 +474,12 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                     for (int i = 0; i < 16; ++i) { r[i] = h[i]; r[i + 16] = 0; }
                 }
                 tmem_ld_wait();
-                store_row_chunk<BN>(p, r, m, n0 + c);
+                store_row_chunk<BN>(p, r, m, n0 + c, at.m_end);
             }
             tc_fence_before_sync();
             mbar_arrive(&acc_empty[a]);
         }
-        if (C::kOutBytes > 0 && p.tma_out && threadIdx.x == 64) bulk_wait_group<0>();   // results are in global memory before the CTA leaves
+        if (!GROUPED && C::kOutBytes > 0 && p.tma_out && threadIdx.x == 64) bulk_wait_group<0>();   // results are in global memory before the CTA leaves
     }
 
     tc_fence_before_sync();
@@ -512,7 +565,6 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     constexpr int g = G > 0 ? G : 1;
     constexpr int kStages = C::kRingBlocks / g, BNH = PBN / 2;
     constexpr int kABytes = g * BM * BK * 2, kStageBytes = g * C::kBlockBytes;
-    FORGE_SKIP_IF_NOT_LIVE(p);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* tiles = smem;                         // [kStages][ g tiles of A | g tiles of this CTA's half of W ]
@@ -690,7 +742,7 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                     uint32_t r[32];
                     tmem_ld_32x32b_x32(t_row + c, r);
                     tmem_ld_wait();
-                    store_row_chunk<PBN>(p, r, m, n0 + c);
+                    store_row_chunk<PBN>(p, r, m, n0 + c, p.M);
                 }
             }
             tc_fence_before_sync();
@@ -752,7 +804,6 @@ gemm_sm100_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     using C = SplitKCfg<G>;
     constexpr int kStages = C::kStages, BN = kSplitBN;
     constexpr int kTileA = BM * BK * 2, kTileW = BN * BK * 2;                            // one k-block of either operand
-    FORGE_SKIP_IF_NOT_LIVE(p);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* tiles = smem;                                                               // slot: G tiles of A, then G tiles of W
@@ -1007,7 +1058,6 @@ gemm_sm100_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     const int w_block = tile_rows * BK * 2;                                 // one k-block of the tile
     const int w_bytes = g * w_block, x_bytes = g * NT * BK * 2;           // one stage of each operand
     const int x_region = kStages * x_bytes;
-    FORGE_SKIP_IF_NOT_LIVE(p);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* w_tiles = smem;                                   // [kStages][g][128 x 64]
@@ -1279,12 +1329,13 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 __device__ __forceinline__ void epilogue_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 constexpr int kStreamKThreads = 224;       // warps 0 and 6 load, 1 issues the MMAs, 2..5 are the epilogue
-template <int NT>
+// GROUPED: the tiles of all experts that have rows, one after the other; how many units a CTA gets follows from the counts on the device.
+// A CTA leaves at most one piece of a tile unfinished (its range's last), so the partial sums and flags are one per CTA.
+template <int NT, bool GROUPED = false>
 __global__ void __launch_bounds__(kStreamKThreads, 1)
 gemm_sm100_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                           const GemmParams p, const StreamKWork wk, const int kStages) {
     using C = StreamKCfg<NT>;
-    FORGE_SKIP_IF_NOT_LIVE(p);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* tiles = smem;
@@ -1299,8 +1350,26 @@ gemm_sm100_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_kb = (p.K + BK - 1) / BK;
     const int tiles_n = (p.N + BM - 1) / BM;
-    const int total = tiles_n * num_kb;
-    const int u_begin = min((int)blockIdx.x * wk.per_cta, total), u_end = min(u_begin + wk.per_cta, total);
+    int total = tiles_n * num_kb, per_cta = wk.per_cta;
+    int* first_row = reinterpret_cast<int*>(smem + kStages * C::kStageBytes + 1024);
+    int* first_tile = first_row + p.groups + 1;
+    if constexpr (GROUPED) {
+        forge::pdl_wait();
+        group_sums(p.counts, p.groups, first_row, first_tile, [&](int rows) { return (rows + NT - 1) / NT * tiles_n; });
+        total = first_tile[p.groups] * num_kb;
+        per_cta = max((total + (int)gridDim.x - 1) / (int)gridDim.x, (num_kb + 63) / 64);      // (128 threads look at the flags of a tile's pieces)
+    }
+    // a tile's row of W, first row of the tokens, column of the result, and how many tokens there are
+    struct Place { int w0, x0, n0, rows; };
+    auto place = [&](int tile) {
+        if constexpr (GROUPED) {
+            const int e = group_of(first_tile, p.groups, tile), t = tile - first_tile[e], n0 = t % tiles_n * BM, x0 = first_row[e] + t / tiles_n * NT;
+            return Place{e * p.N + n0, x0, n0, first_row[e + 1] - x0};
+        } else {
+            return Place{tile * BM, 0, tile * BM, p.M};
+        }
+    };
+    const int u_begin = min((int)blockIdx.x * per_cta, total), u_end = min(u_begin + per_cta, total);
     // Fragments are worked on from the LAST tile of the range to the first.  The last one is the piece this
     // CTA may have to hand to its successor, the first one the piece for which it may need its predecessors:
     // handing on first and collecting last means the partial sums a CTA needs were written long before it
@@ -1347,19 +1416,22 @@ gemm_sm100_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
             for (int i = who; i < first; i += 2) {
                 const int u = unit_at(i);
                 mbar_arrive_expect_tx(&full[i], C::kStageBytes);
-                tma_load_2d(tiles + i * C::kStageBytes, &tmap_w, &full[i], (u % num_kb) * BK, (u / num_kb) * BM);
+                tma_load_2d(tiles + i * C::kStageBytes, &tmap_w, &full[i], (u % num_kb) * BK, place(u / num_kb).w0);
             }
             forge::pdl_wait();
-            for (int i = who; i < first; i += 2)
-                tma_load_2d(tiles + i * C::kStageBytes + BM * BK * 2, &tmap_x, &full[i], (unit_at(i) % num_kb) * BK, 0);
+            for (int i = who; i < first; i += 2) {
+                const int u = unit_at(i);
+                tma_load_2d(tiles + i * C::kStageBytes + BM * BK * 2, &tmap_x, &full[i], (u % num_kb) * BK, place(u / num_kb).x0);
+            }
             bool ok = true;
             for (int i = first + ((first ^ who) & 1); i < n_units && ok; i += 2) {
                 const int s = i % kStages, u = unit_at(i);
                 if (!(ok = mbar_wait(&empty[s], ((i / kStages) - 1) & 1, abort, p.status))) break;
                 mbar_arrive_expect_tx(&full[s], C::kStageBytes);
                 uint8_t* dst = tiles + s * C::kStageBytes;
-                tma_load_2d(dst, &tmap_w, &full[s], (u % num_kb) * BK, (u / num_kb) * BM);
-                tma_load_2d(dst + BM * BK * 2, &tmap_x, &full[s], (u % num_kb) * BK, 0);
+                const Place at = place(u / num_kb);
+                tma_load_2d(dst, &tmap_w, &full[s], (u % num_kb) * BK, at.w0);
+                tma_load_2d(dst + BM * BK * 2, &tmap_x, &full[s], (u % num_kb) * BK, at.x0);
             }
         }
     } else if (warp == 1) {
@@ -1398,8 +1470,9 @@ gemm_sm100_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         // Finishes a tile this CTA owns: adds the `part` earlier fragments' partial sums (if any) in fragment
         // order, applies the epilogue and writes C.  Returns false if the bounded wait ran out.
         auto finish_tile = [&](float (&acc)[NT], int tile, int part) -> bool {
+            const Place at = place(tile);
             if (part > 0) {
-                int* tile_flags = wk.flags + tile * wk.max_parts;
+                int* tile_flags = GROUPED ? wk.flags + ((int)blockIdx.x - part) : wk.flags + tile * wk.max_parts;
                 if (et < part) {
                     const unsigned long long t0 = global_ns();
                     while (ld_acquire(&tile_flags[et]) == 0) {
@@ -1413,21 +1486,22 @@ gemm_sm100_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
                 epilogue_bar();
                 if (*abort) return false;
                 for (int q = 0; q < part; ++q) {
-                    const float* src = wk.partials + ((size_t)tile * wk.max_parts + q) * NT * BM;
+                    const float* src = wk.partials + (GROUPED ? (size_t)((int)blockIdx.x - part + q) : (size_t)tile * wk.max_parts + q) * NT * BM;
 #pragma unroll
                     for (int m = 0; m < NT; ++m)
-                        if (m < p.M) acc[m] += __ldcg(src + m * BM + n_local);
+                        if (m < at.rows) acc[m] += __ldcg(src + m * BM + n_local);
                 }
                 epilogue_bar();
                 if (et < part) tile_flags[et] = 0;
             }
             // a thread holds weight row n for all tokens; per token a warp writes 32 consecutive columns
-            const int n = tile * BM + n_local;
+            const int n = at.n0 + n_local;
             const float b = (p.bias && n < p.N) ? p.bias[n] : 0.f;
 #pragma unroll
-            for (int m = 0; m < NT; ++m) {
-                if (m >= p.M) break;
-                const float v = acc[m] + b;
+            for (int mm = 0; mm < NT; ++mm) {
+                if (mm >= at.rows) break;
+                const int m = at.x0 + mm;
+                const float v = acc[mm] + b;
                 if (is_gated(p.epilogue)) {
                     const float other = __shfl_xor_sync(0xffffffffu, v, 1);
                     if ((lane & 1) == 0 && n + 1 < p.N)
@@ -1465,16 +1539,17 @@ gemm_sm100_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
             tc_fence_before_sync();
             mbar_arrive(&acc_empty[a]);             // the MMA warp may reuse this accumulator now
             // which fragment of its tile is this?  The tile's first unit belongs to CTA c0.
-            const int part = (int)blockIdx.x - (tile * num_kb) / wk.per_cta;
+            const int part = (int)blockIdx.x - (tile * num_kb) / per_cta;
             if (kb1 < num_kb) {
                 // not the owner: park the partial sum and announce it
-                float* my_partial = wk.partials + ((size_t)tile * wk.max_parts + part) * NT * BM;
+                float* my_partial = wk.partials + (GROUPED ? (size_t)blockIdx.x : (size_t)tile * wk.max_parts + part) * NT * BM;
+                const int rows = place(tile).rows;
 #pragma unroll
                 for (int m = 0; m < NT; ++m)
-                    if (m < p.M) my_partial[m * BM + n_local] = acc[m];
+                    if (m < rows) my_partial[m * BM + n_local] = acc[m];
                 __threadfence();
                 epilogue_bar();
-                if (et == 0) st_release(&wk.flags[tile * wk.max_parts + part], 1);
+                if (et == 0) st_release(&wk.flags[GROUPED ? (int)blockIdx.x : tile * wk.max_parts + part], 1);
             } else {
                 ok = finish_tile(acc, tile, kb0 > 0 ? part : 0);
             }
@@ -1785,7 +1860,7 @@ extern "C" int forge_gemm_sm100_set_workspace(void* ptr, long long bytes) {
 // the few-rows kernel with K cut across a cluster of that many CTAs; -100 (M <= 64 only) = the few-rows kernel
 // that deals units of work out evenly to persistent CTAs (the default once a workspace has been set).  status: device int, bit 1 raised if a wait ran out.
 extern "C" int forge_gemm_sm100(const void* A, const void* W, const float* bias, void* C, int* status, int M, int N,
-                                int K, int epilogue, int tile_n, const int* live, float act_a, float act_b, cudaStream_t stream) {
+                                int K, int epilogue, int tile_n, float act_a, float act_b, cudaStream_t stream) {
     if (M < 0 || N <= 0 || K <= 0) return forge::fail(FORGE_ERR_ARG, "gemm_sm100: bad sizes M=%d N=%d K=%d", M, N, K);
     if (M == 0) return FORGE_OK;
     if (K % 8 != 0) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_sm100: K=%d is not a multiple of 8 (TMA row stride)", K);
@@ -1820,7 +1895,7 @@ extern "C" int forge_gemm_sm100(const void* A, const void* W, const float* bias,
             if (!bf16_tile_map(W, N, K, BM, &tw, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_sm100: W: %s", err);
             if (!bf16_tile_map(A, M, K, nt, &tx, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_sm100: A: %s", err);
             GemmParams p{C, bias, M, N, K, epilogue, status};
-            p.live = live; p.act_a = act_a; p.act_b = act_b;
+            p.act_a = act_a; p.act_b = act_b;
             switch (nt) {
                 case 16: return launch_streamk<16>(tw, tx, p, stream);
                 case 32: return launch_streamk<32>(tw, tx, p, stream);
@@ -1872,7 +1947,7 @@ extern "C" int forge_gemm_sm100(const void* A, const void* W, const float* bias,
         // 128-wide tiles is the faster one there (22 against 28-33 us at [11264 x 2048])
         const bool token_major_instead = nt == 128 && tile_n == 0 && ksplit == 1;
         GemmParams p{C, bias, M, N, K, epilogue, status};
-        p.live = live; p.act_a = act_a; p.act_b = act_b;
+        p.act_a = act_a; p.act_b = act_b;
         if (!token_major_instead) switch (nt) {
             case 16: return launch_skinny<16>(W, A, p, ksplit, tile_rows, stream);
             case 32: return launch_skinny<32>(W, A, p, ksplit, tile_rows, stream);
@@ -1895,7 +1970,7 @@ extern "C" int forge_gemm_sm100(const void* A, const void* W, const float* bias,
         }
         if (ks > 0) {
             GemmParams p{C, bias, M, N, K, epilogue, status};
-            p.live = live; p.act_a = act_a; p.act_b = act_b;
+            p.act_a = act_a; p.act_b = act_b;
             return launch_splitk(A, W, p, ks, stream);
         }
     }
@@ -1932,7 +2007,7 @@ extern "C" int forge_gemm_sm100(const void* A, const void* W, const float* bias,
     if (bn == 512 || bn == 1192 || bn == 1128) {
         if (M <= BM) return forge::fail(FORGE_ERR_ARG, "gemm_sm100: the two-CTA tile is for more than %d rows, got %d", BM, M);
         GemmParams p{C, bias, M, N, K, epilogue, status};
-        p.live = live; p.act_a = act_a; p.act_b = act_b;
+        p.act_a = act_a; p.act_b = act_b;
         if (bn == 512) return launch_pair(A, W, p, stream);
         if (K % BK != 0 || K < 2 * BK)
             return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_sm100: two-CTA tiles of %d columns need K %% 64 == 0 and K >= 128, got %d", bn - 1000, K);
@@ -1942,7 +2017,7 @@ extern "C" int forge_gemm_sm100(const void* A, const void* W, const float* bias,
     if (!bf16_tile_map(A, M, K, BM, &ta, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_sm100: A: %s", err);
     if (!bf16_tile_map(W, N, K, bn, &tw, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_sm100: W: %s", err);
     GemmParams p{C, bias, M, N, K, epilogue, status};
-    p.live = live; p.act_a = act_a; p.act_b = act_b;
+    p.act_a = act_a; p.act_b = act_b;
     switch (bn) {
         case 256: return launch<256>(ta, tw, p, stream);
         case 224: return launch<224>(ta, tw, p, stream);
@@ -1954,6 +2029,94 @@ extern "C" int forge_gemm_sm100(const void* A, const void* W, const float* bias,
         case 16: return launch<16>(ta, tw, p, stream);
         default: return forge::fail(FORGE_ERR_ARG, "gemm_sm100: tile_n must be 16, 32, 64, 128, 160, 192, 224, 256, or 512 / 1192 / 1128 (two CTAs on 256 x 256 / 192 / 128), got %d", bn);
     }
+}
+
+namespace {
+constexpr int kMaxGroups = 2048;
+template <int BN>
+int launch_grouped(const void* A, const void* W, const GemmParams& p, cudaStream_t stream) {
+    using C = Cfg<BN>;
+    static_assert(2 * C::kOutBytes >= group_bytes(kMaxGroups), "the experts' sums lie where results would leave");
+    static forge::PerDeviceFlag configured_on;
+    bool& configured = configured_on.current();
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_sm100_kernel<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+        if (e != cudaSuccess) return forge::fail(FORGE_ERR_LAUNCH, "gemm_grouped: cannot set %d bytes of shared memory: %s", C::kSmemBytes, cudaGetErrorString(e));
+        configured = true;
+    }
+    CUtensorMap ta, tw;
+    const char* err = nullptr;
+    if (!bf16_tile_map(A, p.M, p.K, BM, &ta, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_grouped: A: %s", err);
+    if (!bf16_tile_map(W, p.groups * p.N, p.K, BN, &tw, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_grouped: W: %s", err);
+    return forge::check_launch("gemm_grouped", forge::launch(gemm_sm100_kernel<BN, true>, dim3(g_num_sms), dim3(kThreads), C::kSmemBytes, stream, 1, ta, tw, ta, p));
+}
+
+template <int NT>
+int launch_grouped_few(const void* A, const void* W, const GemmParams& p, cudaStream_t stream) {
+    using C = StreamKCfg<NT>;
+    const int room = (kSmemLimit - 2048 - group_bytes(p.groups)) / C::kStageBytes, stages = room < C::kStages ? room : C::kStages;
+    const int smem = C::smem_bytes(stages) + group_bytes(p.groups);
+    static forge::PerDeviceFlag configured_on;
+    bool& configured = configured_on.current();
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_sm100_streamk_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+        if (e != cudaSuccess) return forge::fail(FORGE_ERR_LAUNCH, "gemm_grouped: cannot set %d bytes of shared memory: %s", kSmemLimit, cudaGetErrorString(e));
+        configured = true;
+    }
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int num_kb = (p.K + BK - 1) / BK, tiles_n = (p.N + BM - 1) / BM;
+    const long long most = ((long long)p.groups + p.M / NT) * tiles_n * num_kb;
+    if (most > 0x7fffffffLL) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_grouped: %d experts of [%d x %d]", p.groups, p.N, p.K);
+    const int grid = most < g_num_sms ? (int)most : g_num_sms;
+    if (dev < 0 || dev >= 64 || !g_workspace[dev].ptr || g_workspace[dev].bytes < kFlagBytes + (long long)grid * NT * BM * 4 || grid * 4 > kFlagBytes)
+        return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_grouped: no workspace for the partial sums (call forge_gemm_sm100_set_workspace)");
+    CUtensorMap tw, tx;
+    const char* err = nullptr;
+    if (!bf16_tile_map(W, p.groups * p.N, p.K, BM, &tw, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_grouped: W: %s", err);
+    if (!bf16_tile_map(A, p.M, p.K, NT, &tx, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_grouped: A: %s", err);
+    const StreamKWork wk{reinterpret_cast<float*>(static_cast<char*>(g_workspace[dev].ptr) + kFlagBytes), static_cast<int*>(g_workspace[dev].ptr), 0, 0};
+    return forge::check_launch("gemm_grouped (few rows)", forge::launch(gemm_sm100_streamk_kernel<NT, true>, dim3(grid), dim3(kStreamKThreads), smem, stream, 1,
+                                                                       tw, tx, p, wk, stages));
+}
+}  // namespace
+
+// Products of `groups` experts (at most 2048): A [M, K] bf16, expert e's counts[e] rows behind those of the experts before it (counts int32 [groups]
+// on the device, their sum at most M), W [groups, N, K] bf16; C [M, N] fp32 (epilogue 0), bf16 (2) or bf16 [M, N/2] (3, gated).  most: the most
+// rows that an expert is expected to have (more cost time, nothing else).  K % 8 == 0, 16-byte aligned.
+extern "C" int forge_gemm_grouped(const void* A, const void* W, void* C, int* status, const int* counts, int groups, int M, int most, int N, int K,
+                                  int epilogue, cudaStream_t stream) {
+    if (M < 0 || N <= 0 || K <= 0 || groups <= 0 || most < 0 || !counts) return forge::fail(FORGE_ERR_ARG, "gemm_grouped: bad sizes M=%d N=%d K=%d groups=%d", M, N, K, groups);
+    if (M == 0) return FORGE_OK;
+    if (K % 8 != 0 || groups > kMaxGroups || (long long)groups * N > 0x7fffffffLL)
+        return forge::fail(FORGE_ERR_UNSUPPORTED, "gemm_grouped: K=%d, %d experts of %d rows", K, groups, N);
+    if (epilogue != EPI_STORE_F32 && epilogue != EPI_STORE_BF16 && !(epilogue == EPI_SWIGLU_BF16 && N % 2 == 0))
+        return forge::fail(FORGE_ERR_ARG, "gemm_grouped: epilogue %d with N=%d", epilogue, N);
+    if (g_num_sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+        if (g_num_sms <= 0) g_num_sms = 148;
+    }
+    GemmParams p{C, nullptr, M, N, K, epilogue, status};
+    p.counts = counts;
+    p.groups = groups;
+    // Up to 64 rows an expert, or twice the even share where that is less: as long as the weights take to arrive, dealt out evenly over the SMs
+    // (an expert with more rows has its weights read again, out of the L2 as a rule).  More rows: tiles of 128.
+    const int even = (M + groups - 1) / groups, few = most < 2 * even ? most : 2 * even;
+    if (few <= 16) return launch_grouped_few<16>(A, W, p, stream);
+    if (few <= 32) return launch_grouped_few<32>(A, W, p, stream);
+    if (few <= 64) return launch_grouped_few<64>(A, W, p, stream);
+    // the tile's width as for one matrix (see forge_gemm_sm100), with the rows spread evenly over the experts
+    const long tm = (long)groups * (((M + groups - 1) / groups + BM - 1) / BM), ksteps = (K + UMMA_K - 1) / UMMA_K;
+    long best = -1;
+    int bn = 256;
+    for (int cand : {256, 192, 128}) {
+        const long tiles = tm * ((N + cand - 1) / cand);
+        const long cost = ((tiles + g_num_sms - 1) / g_num_sms) * ksteps * (64 + cand / 2) + 36L * cand;
+        if (best < 0 || cost < best) { best = cost; bn = cand; }
+    }
+    return bn == 256 ? launch_grouped<256>(A, W, p, stream) : bn == 192 ? launch_grouped<192>(A, W, p, stream) : launch_grouped<128>(A, W, p, stream);
 }
 
 // The fused projection of a prompt step: x [M, K] . [Wq; Wk; Wv]^T (+ bias), whose epilogue rotates q and k by the rows'

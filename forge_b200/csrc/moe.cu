@@ -54,7 +54,12 @@ __device__ __forceinline__ float route_dot<__nv_bfloat16>(const __nv_bfloat16* _
 
 constexpr int kRouteThreads = 256;
 
-template <typename TA>
+// FEW (bfloat16 inputs, up to kFewExperts experts, rows of a multiple of 8 channels, all aligned to 16 bytes): a thread takes eight channels against
+// all experts, so a row is read once and every load of a thread is in flight together; the sums meet by the butterfly and then warp by warp.
+// (8 tokens of 4,096 channels, 8 experts: 12 us with a warp an expert, whose rounds of loads wait for one another.)
+constexpr int kFewExperts = 16;
+
+template <typename TA, bool FEW>
 __global__ void __launch_bounds__(kRouteThreads)
 moe_route_kernel(const TA* __restrict__ x, const float* __restrict__ Wr, int32_t* __restrict__ idx, float* __restrict__ wts, int T,
                  int W, int E, int top, int softmax, int renorm, const float* __restrict__ corr, int groups, int keep, int group_top, float factor) {
@@ -64,9 +69,47 @@ moe_route_kernel(const TA* __restrict__ x, const float* __restrict__ Wr, int32_t
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
     float* s = sc;
     const TA* xr = x + (size_t)t * W;
-    for (int e = warp; e < E; e += kRouteThreads / 32) {
-        const float a = forge::warp_sum(route_dot(xr, Wr + (size_t)e * W, W, lane));
-        if (lane == 0) s[e] = a;
+    if constexpr (FEW) {
+        __shared__ float parts[kRouteThreads / 32][kFewExperts];
+        float a[kFewExperts];
+#pragma unroll
+        for (int e = 0; e < kFewExperts; ++e) a[e] = 0.f;
+        for (int c = threadIdx.x * 8; c < W; c += kRouteThreads * 8) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(xr + c);
+            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+            float xv[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 f = __bfloat1622float2(p[i]);
+                xv[2 * i] = f.x;
+                xv[2 * i + 1] = f.y;
+            }
+#pragma unroll
+            for (int e = 0; e < kFewExperts; ++e) {
+                if (e >= E) break;                            // (the same for every thread)
+                const float4 w0 = *reinterpret_cast<const float4*>(Wr + (size_t)e * W + c), w1 = *reinterpret_cast<const float4*>(Wr + (size_t)e * W + c + 4);
+                a[e] = fmaf(xv[0], w0.x, a[e]); a[e] = fmaf(xv[1], w0.y, a[e]); a[e] = fmaf(xv[2], w0.z, a[e]); a[e] = fmaf(xv[3], w0.w, a[e]);
+                a[e] = fmaf(xv[4], w1.x, a[e]); a[e] = fmaf(xv[5], w1.y, a[e]); a[e] = fmaf(xv[6], w1.z, a[e]); a[e] = fmaf(xv[7], w1.w, a[e]);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < kFewExperts; ++e) {
+            if (e >= E) break;
+            a[e] = forge::warp_sum(a[e]);
+            if (lane == 0) parts[warp][e] = a[e];
+        }
+        __syncthreads();
+        if (threadIdx.x < E) {
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < kRouteThreads / 32; ++w) v += parts[w][threadIdx.x];
+            s[threadIdx.x] = softmax ? v : sigmoidf(v);
+        }
+    } else {
+        for (int e = warp; e < E; e += kRouteThreads / 32) {
+            const float a = forge::warp_sum(route_dot(xr, Wr + (size_t)e * W, W, lane));
+            if (lane == 0) s[e] = softmax ? a : sigmoidf(a);
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -75,8 +118,6 @@ moe_route_kernel(const TA* __restrict__ x, const float* __restrict__ Wr, int32_t
             for (int e = 0; e < E; ++e) m = fmaxf(m, s[e]);
             for (int e = 0; e < E; ++e) { s[e] = expf(s[e] - m); sum += s[e]; }
             for (int e = 0; e < E; ++e) s[e] /= sum;
-        } else {
-            for (int e = 0; e < E; ++e) s[e] = sigmoidf(s[e]);
         }
         // ch: what the choice is made by (the scores themselves unless a correction or groups say otherwise)
         float* ch = s;
@@ -385,83 +426,133 @@ moe_expert_rows_kernel(const TA* __restrict__ in, int in_div, const TW* __restri
 }
 
 // One CTA per expert walks all pairs in order: rank[p] = how many earlier pairs chose the same expert; counts[e].
-__global__ void __launch_bounds__(256)
+constexpr int kRankThreads = 1024;
+__global__ void __launch_bounds__(kRankThreads)
 moe_rank_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ rank, int32_t* __restrict__ counts, int P) {
-    __shared__ int warp_tot[8];
-    __shared__ int base;
+    __shared__ int before_warp[kRankThreads / 32 + 1];
     forge::pdl_launch_dependents();
     forge::pdl_wait();
     const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) base = 0;
-    __syncthreads();
-    for (int p0 = 0; p0 < P; p0 += 256) {
+    int base = 0;
+    for (int p0 = 0; p0 < P; p0 += kRankThreads) {
         const int p = p0 + threadIdx.x;
         const bool mine = p < P && idx[p] == e;
         const unsigned m = __ballot_sync(0xffffffffu, mine);
-        if (lane == 0) warp_tot[warp] = __popc(m);
+        if (lane == 0) before_warp[warp] = __popc(m);
         __syncthreads();
-        int before = base;
-        for (int w = 0; w < warp; ++w) before += warp_tot[w];
-        if (mine) rank[p] = before + __popc(m & ((1u << lane) - 1u));
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int tot = 0;
-            for (int w = 0; w < 8; ++w) tot += warp_tot[w];
-            base += tot;
+        if (warp == 0) {                                       // counts of the warps become sums over the warps before
+            const int n = before_warp[lane];
+            int x = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            before_warp[lane] = x - n;
+            if (lane == 31) before_warp[32] = x;
         }
+        __syncthreads();
+        if (mine) rank[p] = base + before_warp[warp] + __popc(m & ((1u << lane) - 1u));
+        base += before_warp[32];
         __syncthreads();
     }
     if (threadIdx.x == 0) counts[e] = base;
 }
 
-// One CTA per pair: its row in the sorted order = (pairs of lower experts) + rank, or with room for `cap` rows per expert
-// (cap > 0) expert * cap + rank; copies the token's input there.
+// Steps of few pairs: ranking and gathering at once.  One CTA per pair looks at all of them for its place, dest = the pairs of lower experts and the
+// earlier ones of its own; CTA e also counts expert e's (the grid has at least E CTAs).
+constexpr int kPlacePairs = 1024;         // pairs up to which that is less than a kernel of its own
+template <typename TA>
+__global__ void __launch_bounds__(128)
+moe_place_kernel(const TA* __restrict__ x, const int32_t* __restrict__ idx, int32_t* __restrict__ counts, int32_t* __restrict__ dest, TA* __restrict__ xg,
+                 int P, int W, int E, int top) {
+    __shared__ int red[2][4];
+    forge::pdl_launch_dependents();
+    forge::pdl_wait();
+    const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int own = b < P ? idx[b] : -1;
+    int before = 0, of_b = 0;                                  // pairs that lie before this CTA's; pairs of expert b
+    for (int p = threadIdx.x; p < P; p += 128) {
+        const int e = idx[p];
+        before += e < own || (e == own && p < b);
+        of_b += e == b;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+        of_b += __shfl_xor_sync(0xffffffffu, of_b, o);
+    }
+    if (lane == 0) { red[0][warp] = before; red[1][warp] = of_b; }
+    __syncthreads();
+    if (threadIdx.x == 0 && b < E) counts[b] = red[1][0] + red[1][1] + red[1][2] + red[1][3];
+    if (b >= P) return;
+    const int row = red[0][0] + red[0][1] + red[0][2] + red[0][3];
+    if (threadIdx.x == 0) dest[b] = row;
+    const TA* src = x + (size_t)(b / top) * W;
+    TA* dst = xg + (size_t)row * W;
+    constexpr int kVec = 16 / sizeof(TA);
+    if (W % kVec == 0 && (((uintptr_t)x | (uintptr_t)xg) & 15) == 0) {
+#pragma unroll 4
+        for (int c = threadIdx.x; c < W / kVec; c += 128) reinterpret_cast<uint4*>(dst)[c] = reinterpret_cast<const uint4*>(src)[c];
+    } else {
+        for (int c = threadIdx.x; c < W; c += 128) dst[c] = src[c];
+    }
+}
+
+// One CTA per pair: its row in the sorted order = (pairs of lower experts) + rank; copies the token's input there.
 template <typename TA>
 __global__ void __launch_bounds__(128)
 moe_gather_kernel(const TA* __restrict__ x, const int32_t* __restrict__ idx, const int32_t* __restrict__ rank,
-                  const int32_t* __restrict__ counts, int32_t* __restrict__ dest, TA* __restrict__ xg, int W, int top, int cap) {
+                  const int32_t* __restrict__ counts, int32_t* __restrict__ dest, TA* __restrict__ xg, int W, int top) {
     __shared__ int s_dest;
     forge::pdl_launch_dependents();
     forge::pdl_wait();
     const int p = blockIdx.x, t = p / top;
     if (threadIdx.x == 0) {
         const int e = idx[p];
-        int off = e * cap;
-        if (cap <= 0)
-            for (int i = 0; i < e; ++i) off += counts[i];
+        int off = 0;
+        for (int i = 0; i < e; ++i) off += counts[i];
         s_dest = off + rank[p];
         dest[p] = s_dest;
     }
     __syncthreads();
     const TA* src = x + (size_t)t * W;
     TA* dst = xg + (size_t)s_dest * W;
-    for (int c = threadIdx.x; c < W; c += 128) dst[c] = src[c];
+    constexpr int kVec = 16 / sizeof(TA);
+    if (W % kVec == 0 && (((uintptr_t)x | (uintptr_t)xg) & 15) == 0) {
+#pragma unroll 2
+        for (int c = threadIdx.x; c < W / kVec; c += 128) reinterpret_cast<uint4*>(dst)[c] = reinterpret_cast<const uint4*>(src)[c];
+    } else {
+        for (int c = threadIdx.x; c < W; c += 128) dst[c] = src[c];
+    }
 }
 
-// y[t, :] = sum_k wts[t, k] * ys[dest[t, k], :], k in order.
+// y[t, :] = sum_k wts[t, k] * ys[dest[t, k], :], k in order (add: added to what y holds).  The CTAs of a token take 512 channels each.
 __global__ void __launch_bounds__(128)
 moe_combine_kernel(const float* __restrict__ ys, const int32_t* __restrict__ dest, const float* __restrict__ wts, float* __restrict__ y,
-                   int W, int top) {
+                   int W, int top, int add) {
     forge::pdl_launch_dependents();
     forge::pdl_wait();
     const int t = blockIdx.x;
     if ((W & 3) == 0 && (((uintptr_t)ys | (uintptr_t)y) & 15) == 0) {          // four channels a load, the experts in the same order
-#pragma unroll 4
-        for (int c = threadIdx.x * 4; c < W; c += 512) {
-            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c = (blockIdx.y * 128 + threadIdx.x) * 4; c < W; c += gridDim.y * 512) {
+            float4* dst = reinterpret_cast<float4*>(y + (size_t)t * W + c);
+            float4 old = make_float4(0.f, 0.f, 0.f, 0.f), sum = old;
+            if (add) old = *dst;
             for (int k = 0; k < top; ++k) {
                 const float w = wts[(size_t)t * top + k];
                 const float4 v = *reinterpret_cast<const float4*>(ys + (size_t)dest[(size_t)t * top + k] * W + c);
                 sum.x = fmaf(w, v.x, sum.x); sum.y = fmaf(w, v.y, sum.y); sum.z = fmaf(w, v.z, sum.z); sum.w = fmaf(w, v.w, sum.w);
             }
-            *reinterpret_cast<float4*>(y + (size_t)t * W + c) = sum;
+            if (add) { sum.x += old.x; sum.y += old.y; sum.z += old.z; sum.w += old.w; }
+            *dst = sum;
         }
         return;
     }
-    for (int c = threadIdx.x; c < W; c += 128) {
+    for (int c = blockIdx.y * 128 + threadIdx.x; c < W; c += gridDim.y * 128) {
         float sum = 0.f;
         for (int k = 0; k < top; ++k) sum = fmaf(wts[(size_t)t * top + k], ys[(size_t)dest[(size_t)t * top + k] * W + c], sum);
-        y[(size_t)t * W + c] = sum;
+        y[(size_t)t * W + c] = add ? y[(size_t)t * W + c] + sum : sum;
     }
 }
 
@@ -478,9 +569,14 @@ extern "C" int forge_moe_route(const void* x, int dtype, const float* Wr, int32_
     if (E > 2048) return forge::fail(FORGE_ERR_UNSUPPORTED, "moe_route: %d experts", E);
     if (T == 0) return FORGE_OK;
     cudaError_t e = cudaSuccess;
-    FORGE_DISPATCH_DTYPE(dtype, TT,
-        e = forge::launch(moe_route_kernel<TT>, dim3(T), dim3(kRouteThreads), sizeof(float) * (2 * E + (groups > 1 ? groups : 0)), stream, 1, (const TT*)x, Wr,
-                          idx, wts, T, W, E, top, softmax, renorm, corr, groups > 1 ? groups : 0, keep, group_top, factor));
+    const size_t smem = sizeof(float) * (2 * E + (groups > 1 ? groups : 0));
+    if (dtype == FORGE_BF16 && E <= kFewExperts && W % 8 == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0) {
+        e = forge::launch(moe_route_kernel<__nv_bfloat16, true>, dim3(T), dim3(kRouteThreads), smem, stream, 1, (const __nv_bfloat16*)x, Wr, idx, wts, T, W, E, top,
+                          softmax, renorm, corr, groups > 1 ? groups : 0, keep, group_top, factor);
+        return forge::check_launch("moe_route", e);
+    }
+    FORGE_DISPATCH_DTYPE(dtype, TT, e = forge::launch(moe_route_kernel<TT, false>, dim3(T), dim3(kRouteThreads), smem, stream, 1, (const TT*)x, Wr, idx, wts, T, W, E, top,
+                                                      softmax, renorm, corr, groups > 1 ? groups : 0, keep, group_top, factor));
     return forge::check_launch("moe_route", e);
 }
 
@@ -564,24 +660,31 @@ extern "C" int forge_moe_expert_rows(const void* x, const void* Wg, const void* 
     return forge::check_launch("moe_expert_rows", e);
 }
 
-// idx int32 [P]; rank, dest int32 [P]; counts int32 [E]; x [T, W]; xg of type dtype: [P, W], or with cap > 0 [E * cap, W], expert e's
-// rows from row e * cap on (cap >= the most pairs one expert can get; the rows beyond an expert's count are not written).
+// idx int32 [P]; rank, dest int32 [P]; counts int32 [E]; x [T, W]; xg of type dtype [P, W].
 extern "C" int forge_moe_sort(const void* x, int dtype, const int32_t* idx, int32_t* rank, int32_t* counts, int32_t* dest, void* xg, int T,
-                              int W, int E, int top, int cap, cudaStream_t stream) {
+                              int W, int E, int top, cudaStream_t stream) {
     if (T < 0 || W <= 0 || E <= 0 || top <= 0) return forge::fail(FORGE_ERR_ARG, "moe_sort: bad sizes T=%d W=%d E=%d top=%d", T, W, E, top);
     if (T == 0) return FORGE_OK;
-    cudaError_t e = forge::launch(moe_rank_kernel, dim3(E), dim3(256), 0, stream, 1, idx, rank, counts, T * top);
+    const int P = T * top;
+    cudaError_t e;
+    if (P <= kPlacePairs) {
+        FORGE_DISPATCH_DTYPE(dtype, TT, e = forge::launch(moe_place_kernel<TT>, dim3(P > E ? P : E), dim3(128), 0, stream, 1, (const TT*)x, idx, counts, dest,
+                                                          (TT*)xg, P, W, E, top));
+        return forge::check_launch("moe_sort", e);
+    }
+    e = forge::launch(moe_rank_kernel, dim3(E), dim3(kRankThreads), 0, stream, 1, idx, rank, counts, P);
     if (e != cudaSuccess) return forge::check_launch("moe_sort (rank)", e);
     FORGE_DISPATCH_DTYPE(dtype, TT,
-        e = forge::launch(moe_gather_kernel<TT>, dim3(T * top), dim3(128), 0, stream, 1, (const TT*)x, idx, rank, counts, dest, (TT*)xg, W, top, cap));
+        e = forge::launch(moe_gather_kernel<TT>, dim3(P), dim3(128), 0, stream, 1, (const TT*)x, idx, rank, counts, dest, (TT*)xg, W, top));
     return forge::check_launch("moe_sort", e);
 }
 
-// ys fp32 [P, W] in sorted order; y fp32 [T, W].
-extern "C" int forge_moe_combine(const float* ys, const int32_t* dest, const float* wts, float* y, int T, int W, int top, cudaStream_t stream) {
+// ys fp32 [P, W] in sorted order; y fp32 [T, W], written or (add) added to.
+extern "C" int forge_moe_combine(const float* ys, const int32_t* dest, const float* wts, float* y, int T, int W, int top, int add, cudaStream_t stream) {
     if (T < 0 || W <= 0 || top <= 0) return forge::fail(FORGE_ERR_ARG, "moe_combine: bad sizes T=%d W=%d top=%d", T, W, top);
     if (T == 0) return FORGE_OK;
-    cudaError_t e = forge::launch(moe_combine_kernel, dim3(T), dim3(128), 0, stream, 1, ys, dest, wts, y, W, top);
+    const int cols = (W + 511) / 512;
+    cudaError_t e = forge::launch(moe_combine_kernel, dim3(T, cols < 1024 ? cols : 1024), dim3(128), 0, stream, 1, ys, dest, wts, y, W, top, add);
     return forge::check_launch("moe_combine", e);
 }
 

@@ -12,11 +12,9 @@ The router's arithmetic is fp32.  Three paths, all with everything but the last 
 
   by pairs      fewer (token, expert) pairs than experts: each pair on its own streams its expert's rows once (32-bit runs: every
                 step below the last path's size, from two tokens on expert by expert with the same numbers to the last bit)
-  with room     16-bit steps of up to 127 tokens, and every larger step that a CUDA graph replays: the pairs are ranked by expert into
-                a buffer with room for a step's tokens per expert (an expert is chosen at most once per token), every expert's rows go
-                through the tensor-core products, and a product whose expert nobody chose is skipped on the device by its row count
-  ranked        steps of many tokens: the pairs lie packed by expert, the row counts come to the host (one wait per layer) and
-                every expert's rows go through the ordinary matrix products
+  grouped       every other 16-bit step: the pairs lie packed by expert, and one tensor-core launch does a product of all experts
+  ranked        32-bit steps of many tokens: the row counts come to the host (one wait per layer) and every expert's rows go
+                through the ordinary matrix products
 A token's experts are added up in the router's order in all three.
 """
 import torch
@@ -101,18 +99,12 @@ class RoutedExperts(Part):
                 off += n
         return kernels.moe_combine(ys, dest, wts)
 
-    def _with_room(self, x, idx, wts):
-        """Nothing waits for the device: expert e's rows lie from row e * T on, and its two products are skipped where counts[e] is 0.
-        The rows beyond an expert's count hold whatever the buffer held; a product's rows do not mix, and nobody reads theirs."""
-        T, W, F, E = x.shape[0], self.hidden_size, self.intermediate_size, self.experts
-        xg, counts, dest = kernels.moe_sort(x, idx, E, cap=T)
-        act = kernels.new_tensor((E * T, F), self.rt.dtype, x.device)
-        ys = kernels.new_tensor((E * T, W), torch.float32, x.device)
-        for e in range(E):
-            rows, live = slice(e * T, (e + 1) * T), counts[e:e + 1]
-            self.gate_up_of[e].forward(xg[rows], epilogue="swiglu", out=act[rows], live=live)
-            self.down_of[e].forward(act[rows], out=ys[rows], live=live)
-        return kernels.moe_combine(ys, dest, wts)
+    def _grouped(self, x, idx, wts, into):
+        """Nothing waits for the device: the products find an expert's rows by the counts that the ranking left there."""
+        T = x.shape[0]
+        xg, counts, dest = kernels.moe_sort(x, idx, self.experts)
+        act = kernels.gemm_grouped(xg, self.gate_up, counts, T, epilogue="swiglu")       # (a token chooses an expert at most once)
+        return kernels.moe_combine(kernels.gemm_grouped(act, self.down, counts, T), dest, wts, accumulate_into=into)
 
     def _pairs_fit(self):
         """Whether the path by pairs holds a token's input and its experts' activations in a CTA's shared memory."""
@@ -123,14 +115,16 @@ class RoutedExperts(Part):
         idx, wts = kernels.moe_route(x, self.router, self.top, softmax=self.score == "softmax", renorm=self.renormalize,
                                      correction=self.bias, groups=self.groups, keep=self.keep, factor=self.route_scale, group_top=self.group_top)
         T = x.shape[0]
+        into = residual if self.shared is None and residual is not None and residual.is_contiguous() else None   # the sum joins the stream in its own kernel
         tensor_core = self.gate_up_of[0].tensor_core and self.down_of[0].tensor_core
-        if T >= self.SORTED_FROM and not torch.cuda.is_current_stream_capturing():
+        grouped = tensor_core and self.experts <= kernels.GROUPED_EXPERTS
+        if grouped and (T * self.top >= self.experts or T >= self.SORTED_FROM or not self._pairs_fit()):
+            y = self._grouped(x, idx, wts, into)
+            if into is not None:
+                return y
+        elif T >= self.SORTED_FROM and not torch.cuda.is_current_stream_capturing():
             y = self._ranked(x, idx, wts)
-        elif tensor_core and (T * self.top >= self.experts or T >= self.SORTED_FROM or not self._pairs_fit()):
-            y = self._with_room(x, idx, wts)
-        elif tensor_core:
-            y = kernels.moe_pairs(x, idx, wts, self.gate_up, self.down)
-        elif x.shape[0] >= self.BY_EXPERT_FROM and kernels.moe_experts_supported(x.shape[0] * self.top, self.hidden_size, self.intermediate_size):
+        elif not tensor_core and T >= self.BY_EXPERT_FROM and kernels.moe_experts_supported(T * self.top, self.hidden_size, self.intermediate_size):
             y = kernels.moe_experts(x, idx, wts, self.gate_up, self.down)
         else:
             y = kernels.moe_pairs(x, idx, wts, self.gate_up, self.down)

@@ -1,0 +1,94 @@
+"""The products of all experts in one launch, and the ranking, the routing of few experts and the weighted sum around them."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+if torch.cuda.is_available():
+    from forge_b200 import kernels
+
+DEV = "cuda"
+
+
+def _counts(kind, E, M, gen):
+    if kind == "even":
+        return [M // E + (e < M % E) for e in range(E)]
+    if kind == "one":                                          # the last expert has every row
+        return [0] * (E - 1) + [M]
+    cuts = torch.sort(torch.randint(0, M + 1, (E - 1,), generator=gen)).values.tolist()
+    return [b - a for a, b in zip([0] + cuts, cuts + [M])]
+
+
+# E, M, most, N, K: the few-rows form at the edges of its tiles of tokens, with more rows than a tile has, and tiles of 128 rows
+SHAPES = [(8, 16, 8, 256, 512), (5, 17, 17, 136, 72), (3, 33, 32, 128, 128), (64, 200, 100, 200, 136), (2, 64, 64, 520, 1024), (4, 260, 65, 264, 200),
+          (8, 1027, 500, 768, 256), (3, 129, 129, 1040, 64), (300, 700, 70, 64, 64), (2, 3, 3, 64, 16384)]
+
+
+@pytest.mark.parametrize("kind", ["even", "one", "any"])
+@pytest.mark.parametrize("E,M,most,N,K", SHAPES)
+def test_products_of_all_experts(E, M, most, N, K, kind):
+    gen = torch.Generator().manual_seed(E * 1000 + M)
+    counts = _counts(kind, E, M, gen)
+    x = torch.randn(M, K, generator=gen).bfloat16()
+    w = torch.randn(E, N, K, generator=gen).bfloat16()
+    row_of = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
+    want, size = torch.empty(M, N), torch.empty(M, N)
+    for e in range(E):
+        rows = row_of == e
+        want[rows] = x[rows].float() @ w[e].float().T
+        size[rows] = x[rows].float().abs() @ w[e].float().abs().T
+    xd, wd, cd = x.to(DEV), w.to(DEV), torch.tensor(counts, dtype=torch.int32, device=DEV)
+    bound = K * 2.0 ** -23 * size                              # both sides round each of the K additions in 32 bits
+    for _ in range(2):                                         # (the flags of the partial sums are zero again)
+        got = kernels.gemm_grouped(xd, wd, cd, most).cpu()
+        assert bool(((got - want).abs() <= bound).all())
+    got = kernels.gemm_grouped(xd, wd, cd, most, epilogue="cast").float().cpu()
+    assert bool(((got - want).abs() <= bound + 2.0 ** -8 * want.abs()).all())
+    got = kernels.gemm_grouped(xd, wd, cd, most, epilogue="swiglu").float().cpu()
+    g, u = want[:, 0::2].double(), want[:, 1::2].double()
+    ref = torch.nn.functional.silu(g) * u
+    # silu's slope is at most 1.1; 2^-8: the store, 2^-18: the device's exponential
+    slack = 1.1 * bound[:, 0::2] * u.abs() + torch.nn.functional.silu(g).abs() * bound[:, 1::2] + (2.0 ** -8 + 2.0 ** -18) * ref.abs() + 1e-6
+    assert bool(((got - ref).abs() <= slack).all())
+
+
+@pytest.mark.parametrize("T,top,E,W", [(1, 2, 8, 64), (7, 3, 5, 40), (512, 2, 8, 72), (513, 2, 8, 72), (300, 4, 200, 12), (1025, 1, 3, 7)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_ranking_gathers_pairs_by_expert_and_token(T, top, E, W, dtype):
+    gen = torch.Generator().manual_seed(T + E)
+    idx = torch.stack([torch.randperm(E, generator=gen)[:top] for _ in range(T)]).int()
+    x = torch.randn(T, W, generator=gen).to(dtype)
+    xg, counts, dest = kernels.moe_sort(x.to(DEV), idx.to(DEV), E)
+    order = torch.argsort(idx.flatten().long(), stable=True)
+    rank = torch.empty(T * top, dtype=torch.int32)
+    rank[order] = torch.arange(T * top, dtype=torch.int32)
+    assert torch.equal(counts.cpu(), torch.bincount(idx.flatten().long(), minlength=E).int())
+    assert torch.equal(dest.cpu().flatten(), rank)
+    assert torch.equal(xg.cpu(), x[order // top])
+
+
+@pytest.mark.parametrize("T,W,E,top", [(3, 8, 2, 1), (9, 264, 16, 3), (5, 4096, 8, 2), (4, 2056, 7, 7), (6, 264, 17, 3)])
+def test_routing_of_few_experts(T, W, E, top):
+    gen = torch.Generator().manual_seed(W + E)
+    x = torch.randn(T, W, generator=gen).bfloat16()
+    wr = torch.randn(E, W, generator=gen) * W ** -0.5
+    idx, wts = kernels.moe_route(x.to(DEV), wr.to(DEV), top, softmax=True, renorm=True)
+    s = torch.softmax(x.double() @ wr.double().T, -1)
+    best = torch.topk(s, top)
+    assert torch.equal(idx.cpu().long(), best.indices)         # (scores of random rows lie further apart than 32 bits blur)
+    assert torch.allclose(wts.cpu().double(), best.values / best.values.sum(-1, keepdim=True), rtol=W * 2.0 ** -22, atol=0)
+
+
+@pytest.mark.parametrize("T,W,top", [(3, 512, 2), (2, 516, 3), (5, 1030, 1), (4, 7, 2)])
+def test_weighted_sum_joins_the_stream(T, W, top):
+    gen = torch.Generator().manual_seed(W)
+    ys, wts, y0 = torch.randn(T * top, W, generator=gen), torch.rand(T, top, generator=gen), torch.randn(T, W, generator=gen)
+    dest = torch.randperm(T * top, generator=gen).int().view(T, top)
+    want = (ys[dest.long()].double() * wts.double()[..., None]).sum(1)
+    got = kernels.moe_combine(ys.to(DEV), dest.to(DEV), wts.to(DEV))
+    slack = (top + 1) * 2.0 ** -24 * ((ys[dest.long()].abs() * wts[..., None]).sum(1) + y0.abs() + 1)
+    assert bool(((got.cpu() - want).abs() <= slack).all())
+    y = y0.to(DEV)
+    assert kernels.moe_combine(ys.to(DEV), dest.to(DEV), wts.to(DEV), accumulate_into=y) is y
+    assert bool(((y.cpu() - (y0 + want)).abs() <= slack).all())
+    assert torch.equal(y.cpu(), y0 + got.cpu())
