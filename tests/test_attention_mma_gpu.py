@@ -130,6 +130,26 @@ def test_decode_step_in_one_kernel(nh, nkv, hd, ps, window, rotary):
             assert (work.float() - cache_ref.float()).abs().max() <= 1e-2 * cache_ref.float().abs().max()   # k, v landed in their slots
 
 
+@pytest.mark.parametrize("hd,ps", [(64, 16), (128, 32)])
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("requests", [80, 128, 129])
+def test_decode_step_of_more_pairs_than_sms_takes_the_longest_first(hd, ps, window, requests):
+    """Every (request, kv head) once, whatever the order of the requests' lengths, with equal ones among them; the order ends at 128 requests."""
+    from forge_b200 import kernels as k
+    nh, nkv = 4, 2
+    ctxs = [(37 * i) % 211 for i in range(requests - 3)] + [1000, 63, 64]
+    q, cache, group, batch, tok_req, positions = make_case(nh, nkv, hd, ps, [(c, 1) for c in ctxs], seed=5)
+    qkv = torch.randn(requests, (nh + 2 * nkv) * hd, generator=torch.Generator().manual_seed(1)).to(q.device)
+    slots = torch.tensor([int(group.block_table[s, c // ps]) * ps + c % ps for s, c in enumerate(ctxs)], dtype=torch.int32, device=q.device)
+    q_ref, cache_ref = R.rope_kv_write_ref(qkv, positions, slots, cache, nh, nkv, hd, ps, 1e4, True)
+    cache_ref = cache_ref.to(torch.bfloat16)
+    ref = R.paged_attention_ref(q_ref.to(torch.bfloat16), cache_ref, group.block_table, tok_req, positions, nh, nkv, hd, ps, window)
+    got = k.decode_attention_stream(qkv, cache, group.block_table, positions, slots, nh, nkv, hd, ps, 1e4, window=window).float()
+    k.check_kernel_status()
+    assert float((got - ref).abs().max()) <= 1e-2 * float(ref.abs().max())
+    assert (cache.float() - cache_ref.float()).abs().max() <= 1e-2 * cache_ref.float().abs().max()
+
+
 @pytest.mark.parametrize("nh,nkv,hd,ps", [(32, 4, 64, 64), (32, 4, 64, 16), (14, 2, 128, 64), (16, 2, 128, 32), (3, 1, 64, 32), (16, 1, 64, 64)])
 @pytest.mark.parametrize("window,rotary", [(0, True), (100, True), (0, False)])
 def test_decode_step_with_the_cache_streamed_through_a_ring(nh, nkv, hd, ps, window, rotary):
