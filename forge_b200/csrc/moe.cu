@@ -54,12 +54,13 @@ __device__ __forceinline__ float route_dot<__nv_bfloat16>(const __nv_bfloat16* _
 
 constexpr int kRouteThreads = 256;
 
-// FEW (bfloat16 inputs, up to kFewExperts experts, rows of a multiple of 8 channels, all aligned to 16 bytes): a thread takes eight channels against
-// all experts, so a row is read once and every load of a thread is in flight together; the sums meet by the butterfly and then warp by warp.
-// (8 tokens of 4,096 channels, 8 experts: 12 us with a warp an expert, whose rounds of loads wait for one another.)
+// FEW (bfloat16 inputs, up to FEW = 8 or 16 experts in no groups, rows of a multiple of 8 channels, all aligned to 16 bytes): a thread takes eight
+// channels against all experts, every load of theirs in flight together, and one warp with an expert a lane makes the scores and the choice.
+// (A warp an expert and one thread's choice out of shared memory: both are chains of memory latencies, 12 us for 8 tokens of
+// 4,096 channels, 5.7 us so.)
 constexpr int kFewExperts = 16;
 
-template <typename TA, bool FEW>
+template <typename TA, int FEW>
 __global__ void __launch_bounds__(kRouteThreads)
 moe_route_kernel(const TA* __restrict__ x, const float* __restrict__ Wr, int32_t* __restrict__ idx, float* __restrict__ wts, int T,
                  int W, int E, int top, int softmax, int renorm, const float* __restrict__ corr, int groups, int keep, int group_top, float factor) {
@@ -69,42 +70,84 @@ moe_route_kernel(const TA* __restrict__ x, const float* __restrict__ Wr, int32_t
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
     float* s = sc;
     const TA* xr = x + (size_t)t * W;
-    if constexpr (FEW) {
-        __shared__ float parts[kRouteThreads / 32][kFewExperts];
-        float a[kFewExperts];
+    if constexpr (FEW > 0) {
+        __shared__ float parts[kRouteThreads / 32][FEW];
+        float a[FEW];
 #pragma unroll
-        for (int e = 0; e < kFewExperts; ++e) a[e] = 0.f;
+        for (int e = 0; e < FEW; ++e) a[e] = 0.f;
         for (int c = threadIdx.x * 8; c < W; c += kRouteThreads * 8) {
             const uint4 raw = *reinterpret_cast<const uint4*>(xr + c);
-            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+            float4 w[8][2];
             float xv[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 f = __bfloat1622float2(p[i]);
-                xv[2 * i] = f.x;
-                xv[2 * i + 1] = f.y;
-            }
+            for (int e0 = 0; e0 < FEW; e0 += 8) {
 #pragma unroll
-            for (int e = 0; e < kFewExperts; ++e) {
-                if (e >= E) break;                            // (the same for every thread)
-                const float4 w0 = *reinterpret_cast<const float4*>(Wr + (size_t)e * W + c), w1 = *reinterpret_cast<const float4*>(Wr + (size_t)e * W + c + 4);
-                a[e] = fmaf(xv[0], w0.x, a[e]); a[e] = fmaf(xv[1], w0.y, a[e]); a[e] = fmaf(xv[2], w0.z, a[e]); a[e] = fmaf(xv[3], w0.w, a[e]);
-                a[e] = fmaf(xv[4], w1.x, a[e]); a[e] = fmaf(xv[5], w1.y, a[e]); a[e] = fmaf(xv[6], w1.z, a[e]); a[e] = fmaf(xv[7], w1.w, a[e]);
+                for (int e = 0; e < 8; ++e) {                 // (beyond the last expert: its row once more, for nobody)
+                    const float4* r = reinterpret_cast<const float4*>(Wr + (size_t)min(e0 + e, E - 1) * W + c);
+                    w[e][0] = r[0];
+                    w[e][1] = r[1];
+                }
+                if (e0 == 0) {
+                    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = __bfloat1622float2(p[i]);
+                        xv[2 * i] = f.x;
+                        xv[2 * i + 1] = f.y;
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    float v = a[e0 + e];
+                    v = fmaf(xv[0], w[e][0].x, v); v = fmaf(xv[1], w[e][0].y, v); v = fmaf(xv[2], w[e][0].z, v); v = fmaf(xv[3], w[e][0].w, v);
+                    v = fmaf(xv[4], w[e][1].x, v); v = fmaf(xv[5], w[e][1].y, v); v = fmaf(xv[6], w[e][1].z, v); v = fmaf(xv[7], w[e][1].w, v);
+                    a[e0 + e] = v;
+                }
             }
         }
 #pragma unroll
-        for (int e = 0; e < kFewExperts; ++e) {
-            if (e >= E) break;
+        for (int e = 0; e < FEW; ++e) {
             a[e] = forge::warp_sum(a[e]);
             if (lane == 0) parts[warp][e] = a[e];
         }
         __syncthreads();
-        if (threadIdx.x < E) {
-            float v = 0.f;
+        if (warp != 0) return;
+        const bool mine = lane < E;
+        float score = 0.f;
 #pragma unroll
-            for (int w = 0; w < kRouteThreads / 32; ++w) v += parts[w][threadIdx.x];
-            s[threadIdx.x] = softmax ? v : sigmoidf(v);
+        for (int w = 0; w < kRouteThreads / 32; ++w) score += parts[w][min(lane, FEW - 1)];
+        if (softmax) {
+            float m = mine ? score : -INFINITY;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            score = mine ? expf(score - m) : 0.f;
+            score /= forge::warp_sum(score);
+        } else {
+            score = sigmoidf(score);
         }
+        float choice = mine ? (corr ? score + corr[lane] : score) : -INFINITY, total = 0.f, weight = 0.f;
+        int chosen = 0;
+        for (int k = 0; k < top; ++k) {                       // the lower index wins a tie; NaN is never picked, and where nothing is, expert 0
+            float v = choice == choice ? choice : -INFINITY;
+            int best = lane;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+                const int ob = __shfl_xor_sync(0xffffffffu, best, o);
+                if (ov > v || (ov == v && ob < best)) { v = ov; best = ob; }
+            }
+            if (v == -INFINITY) best = 0;
+            const float got = __shfl_sync(0xffffffffu, score, best);
+            if (lane == k) { chosen = best; weight = got; }
+            if (lane == best) choice = -INFINITY;
+            total += got;
+        }
+        if (lane < top) {
+            if (renorm) weight /= total;
+            idx[(size_t)t * top + lane] = chosen;
+            wts[(size_t)t * top + lane] = weight * factor;
+        }
+        return;
     } else {
         for (int e = warp; e < E; e += kRouteThreads / 32) {
             const float a = forge::warp_sum(route_dot(xr, Wr + (size_t)e * W, W, lane));
@@ -570,12 +613,13 @@ extern "C" int forge_moe_route(const void* x, int dtype, const float* Wr, int32_
     if (T == 0) return FORGE_OK;
     cudaError_t e = cudaSuccess;
     const size_t smem = sizeof(float) * (2 * E + (groups > 1 ? groups : 0));
-    if (dtype == FORGE_BF16 && E <= kFewExperts && W % 8 == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0) {
-        e = forge::launch(moe_route_kernel<__nv_bfloat16, true>, dim3(T), dim3(kRouteThreads), smem, stream, 1, (const __nv_bfloat16*)x, Wr, idx, wts, T, W, E, top,
-                          softmax, renorm, corr, groups > 1 ? groups : 0, keep, group_top, factor);
+    if (dtype == FORGE_BF16 && E <= kFewExperts && groups <= 1 && W % 8 == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0) {
+        auto few = E <= 8 ? moe_route_kernel<__nv_bfloat16, 8> : moe_route_kernel<__nv_bfloat16, 16>;
+        e = forge::launch(few, dim3(T), dim3(kRouteThreads), smem, stream, 1, (const __nv_bfloat16*)x, Wr, idx, wts, T, W, E, top, softmax, renorm, corr, 0, keep,
+                          group_top, factor);
         return forge::check_launch("moe_route", e);
     }
-    FORGE_DISPATCH_DTYPE(dtype, TT, e = forge::launch(moe_route_kernel<TT, false>, dim3(T), dim3(kRouteThreads), smem, stream, 1, (const TT*)x, Wr, idx, wts, T, W, E, top,
+    FORGE_DISPATCH_DTYPE(dtype, TT, e = forge::launch(moe_route_kernel<TT, 0>, dim3(T), dim3(kRouteThreads), smem, stream, 1, (const TT*)x, Wr, idx, wts, T, W, E, top,
                                                       softmax, renorm, corr, groups > 1 ? groups : 0, keep, group_top, factor));
     return forge::check_launch("moe_route", e);
 }

@@ -67,16 +67,27 @@ def test_ranking_gathers_pairs_by_expert_and_token(T, top, E, W, dtype):
     assert torch.equal(xg.cpu(), x[order // top])
 
 
-@pytest.mark.parametrize("T,W,E,top", [(3, 8, 2, 1), (9, 264, 16, 3), (5, 4096, 8, 2), (4, 2056, 7, 7), (6, 264, 17, 3)])
-def test_routing_of_few_experts(T, W, E, top):
+@pytest.mark.parametrize("softmax,corrected", [(True, False), (False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("T,W,E,top", [(3, 8, 2, 1), (9, 264, 16, 3), (5, 4096, 8, 2), (4, 2056, 7, 7), (6, 264, 17, 3), (5, 520, 9, 9)])
+def test_routing_of_few_experts(T, W, E, top, softmax, corrected):
     gen = torch.Generator().manual_seed(W + E)
     x = torch.randn(T, W, generator=gen).bfloat16()
     wr = torch.randn(E, W, generator=gen) * W ** -0.5
-    idx, wts = kernels.moe_route(x.to(DEV), wr.to(DEV), top, softmax=True, renorm=True)
-    s = torch.softmax(x.double() @ wr.double().T, -1)
-    best = torch.topk(s, top)
-    assert torch.equal(idx.cpu().long(), best.indices)         # (scores of random rows lie further apart than 32 bits blur)
-    assert torch.allclose(wts.cpu().double(), best.values / best.values.sum(-1, keepdim=True), rtol=W * 2.0 ** -22, atol=0)
+    corr = torch.randn(E, generator=gen) if corrected else None
+    idx, wts = kernels.moe_route(x.to(DEV), wr.to(DEV), top, softmax=softmax, renorm=True, correction=None if corr is None else corr.to(DEV), factor=1.5)
+    s = x.double() @ wr.double().T
+    s = torch.softmax(s, -1) if softmax else torch.sigmoid(s)
+    order = torch.topk(s + corr.double() if corrected else s, top).indices
+    assert torch.equal(idx.cpu().long(), order)                # (random rows' scores lie further apart than 32 bits blur)
+    best = torch.gather(s, 1, order)
+    assert torch.allclose(wts.cpu().double(), 1.5 * best / best.sum(-1, keepdim=True), rtol=W * 2.0 ** -22, atol=0)
+
+
+def test_a_tie_goes_to_the_lower_expert_and_no_number_to_the_first():
+    x = torch.ones(2, 8).bfloat16()
+    x[1] = float("nan")
+    idx, _ = kernels.moe_route(x.to(DEV), torch.zeros(6, 8, device=DEV), 3, softmax=True)
+    assert idx.cpu().tolist() == [[0, 1, 2], [0, 0, 0]]
 
 
 @pytest.mark.parametrize("T,W,top", [(3, 512, 2), (2, 516, 3), (5, 1030, 1), (4, 7, 2)])
