@@ -161,7 +161,7 @@ latent_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __re
                 }
             }
             // scale, mask, and the tile's maximum per row.  A tile that every row of the CTA sees whole needs no mask.
-            const bool whole = rows == qrows && qrows == BM && j0 + BN - 1 <= pos0 && j0 >= see_last;
+            const bool whole = rows == qrows && j0 + BN - 1 <= pos0 && j0 >= see_last;
             float tmax[2] = {-INFINITY, -INFINITY};
             if (whole) {
 #pragma unroll
@@ -339,6 +339,9 @@ int launch_latent(int which, dim3 grid, size_t smem, cudaStream_t stream, const 
 }
 
 size_t latent_mma_smem(int qrows, int KD, int nbuf) { return sizeof(__nv_bfloat16) * (size_t)(qrows + nbuf * BN) * (KD + kPad); }
+// Rows of queries that a CTA keeps: a token's heads in a step of single tokens, so that two CTAs fit an SM, else a whole tile.  (16 requests of 125 to
+// 2,000 rows, 32 heads, 256 + 32 channels: one CTA of 64 rows an SM 26.2 us, two of 32 19.5; 64 requests 81.6 and 51.8; 100 requests 150 and 98.)
+int latent_rows(int HG, bool single) { return single && HG <= 32 ? (HG <= 16 ? 16 : 32) : BM; }
 
 }  // namespace
 
@@ -351,6 +354,12 @@ extern "C" int forge_latent_mma_supports(int H, int C, int R, int page_size) {
 
 // Heads a CTA takes (the caller cuts the step into tiles of 64 / this many tokens).
 extern "C" int forge_latent_mma_heads(int H) { return H < BM ? H : BM; }
+
+// CTAs of a step of single tokens that an SM holds, by their shared memory (at most two: more would share its tensor units).
+extern "C" int forge_latent_mma_resident(int H, int C, int R) {
+    const int KD = C + R, qrows = latent_rows(forge_latent_mma_heads(H), true);
+    return latent_mma_smem(qrows, KD, 2) + 1024 <= 227 * 1024 / 2 ? 2 : 1;
+}
 
 // q bf16 [T, H*(C+R)]; out bf16 [T, H*C]; u fp32 [nsplit, T, H, C] and part_ml fp32 [nsplit, T, H, 2] (scratch, nsplit > 1: steps of
 // single tokens only).  tile_t0 / tile_n: tiles of consecutive tokens of one request with tile_n * min(H, 64) <= 64 (both null:
@@ -370,8 +379,7 @@ extern "C" int forge_latent_attention_mma(const void* q, const void* cache, cons
     for (int cand : {128, 256})
         if ((C + cand - 1) / cand * cand <= (C + VC - 1) / VC * VC) VC = cand;
     const int chunks = (C + VC - 1) / VC, HG = forge_latent_mma_heads(H), KD = C + R;
-    // a step of single tokens brings at most HG rows a tile: 16 rows of queries in shared memory leave room for more CTAs on the SM
-    const int qrows = (tile_t0 == nullptr && HG <= 16) ? 16 : BM;
+    const int qrows = latent_rows(HG, tile_t0 == nullptr);
     const int nbuf = latent_mma_smem(qrows, KD, 2) <= (size_t)kSmemLimit ? 2 : 1;
     const size_t smem = latent_mma_smem(qrows, KD, nbuf);
     // prompt portions over a latent of an even number of value chunks: a CTA of eight warps takes two chunks (a step of single

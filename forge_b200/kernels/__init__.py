@@ -100,6 +100,7 @@ _SIGNATURES = {
         "forge_latent_attention": [_P] * 8 + [_I] * 8 + [_F, _I, _I, _I, _P, _P],
         "forge_latent_mma_supports": [_I] * 4,
         "forge_latent_mma_heads": [_I],
+        "forge_latent_mma_resident": [_I, _I, _I],
         "forge_latent_attention_mma": [_P] * 9 + [_I, _P] + [_I] * 7 + [_F, _I, _P, _P],
     },
     "attention_shaped": {
@@ -1507,10 +1508,10 @@ def latent_attention(q, cache, group_batch, batch, H, C, R, page_size, scale, wi
         nsplit = 1
         if getattr(batch, "decode_only", False):
             # a step of single tokens brings T * (head groups) * (value chunks) CTAs: deal a request's tiles out to several, up to
-            # one CTA per SM, as far as the longest context (the graph's bucket) has tiles
+            # as many as the SMs hold, as far as the longest context (the graph's bucket) has tiles
             ctas = T * -(-H // HG) * -(-C // 256)
             reach = min(batch.max_context, window + 63) if window else batch.max_context
-            nsplit = max(1, min(LATENT_SPLITS, -(-reach // 64), _sm_count(q.device) // max(1, ctas)))
+            nsplit = max(1, min(LATENT_SPLITS, -(-reach // 64), lib.forge_latent_mma_resident.fn(H, C, R) * _sm_count(q.device) // max(1, ctas)))
         u = new_tensor((nsplit, T, H, C), torch.float32, q.device) if nsplit > 1 else None
         part_ml = new_tensor((nsplit, T, H, 2), torch.float32, q.device) if nsplit > 1 else None
         out = new_tensor((T, H * C), q.dtype, q.device)
