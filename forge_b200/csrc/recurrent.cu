@@ -584,9 +584,14 @@ extern "C" int forge_state_scan(int mode, const float* r, int ld_r, const float*
 // Retention over the step's tokens: q, k fp32 (row t at p + t * ld, head n's K channels at columns n*K ..) are rotated and
 // scaled IN PLACE, then S <- decay[n] S + k v^T, out = S^T q per head; v and out have N*KV columns, a head's state is [K, KV].
 // freq fp32 [rot_dims / 2] (null with rot_dims 0); decay fp32 [N].
+extern "C" int forge_decay_chunks(const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v, const float* decay, float* s, float* state,
+                                  long long state_stride, const int32_t* q_start, const int32_t* slots, float* out, int T, int S, int N, int K, int KV,
+                                  cudaStream_t stream);                                                     // recurrent_chunk.cu
+
+// chunk_states: null, or scratch for forge_decay_chunks, which then walks the tokens (heads that it takes, rows aligned to 16 bytes).
 extern "C" int forge_retention_scan(float* q, int ld_q, float* k, int ld_k, const float* v, int ld_v, const int32_t* positions,
                                     const float* freq, int rot_dims, float k_scale, const float* decay, float* state,
-                                    long long state_stride, const int32_t* q_start, const int32_t* slots, float* out, int T, int S,
+                                    long long state_stride, const int32_t* q_start, const int32_t* slots, float* out, float* chunk_states, int T, int S,
                                     int N, int K, int KV, cudaStream_t stream) {
     if (T < 0 || S < 0 || N <= 0 || K <= 0 || KV <= 0 || rot_dims < 0 || rot_dims > K || (rot_dims & 1))
         return forge::fail(FORGE_ERR_ARG, "retention_scan: bad sizes S=%d N=%d K=%d V=%d rot=%d", S, N, K, KV, rot_dims);
@@ -598,6 +603,8 @@ extern "C" int forge_retention_scan(float* q, int ld_q, float* k, int ld_k, cons
     cudaError_t e = forge::launch(retention_prepare_kernel, dim3(blocks), dim3(128), 0, stream, 1, q, ld_q, k, ld_k, positions, freq, rot_dims,
                                   k_scale, T, N, K);
     if (e != cudaSuccess) return forge::check_launch("retention_scan (prepare)", e);
+    if (chunk_states)
+        return forge_decay_chunks(q, ld_q, k, ld_k, v, ld_v, decay, chunk_states, state, state_stride, q_start, slots, out, T, S, N, K, KV, stream);
     const int kmax = K <= 128 ? (K + 31) / 32 * 32 : (K <= 192 ? 192 : 256);
     const dim3 grid(S, N, (KV + kCols - 1) / kCols);
     ScanInput Q{q, ld_q}, Kk{k, ld_k}, V{v, ld_v}, D{decay, 0};

@@ -380,15 +380,23 @@ extern "C" int forge_gated_delta_scan(const float* q, int ld_q, const float* k, 
     return run<true>(BlockScan{q, k, v, ld_q, ld_k, ld_v, nullptr, g, beta, state, state_stride, q_start, slots, out, N, M, K, KV, 0}, gram, T, S, stream);
 }
 
+extern "C" int forge_decay_chunks(const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v, const float* decay, float* s, float* state,
+                                  long long state_stride, const int32_t* q_start, const int32_t* slots, float* out, int T, int S, int N, int K, int KV,
+                                  cudaStream_t stream);                                                     // recurrent_chunk.cu
+
 // Lightning attention over the step's tokens: fp32 rows of ld numbers [q: N*K | k: N*K | v: N*KV] from proj on pass silu IN PLACE, then the
-// recurrence with decay fp32 [N]; gram: fp32 scratch, 64 * N * (T / 8 + S) numbers; out fp32 [T, N*KV]; the state as above.
-extern "C" int forge_lightning_scan(float* proj, int ld, const float* decay, float* gram, float* state, long long state_stride,
+// recurrence with decay fp32 [N]; gram: fp32 scratch, 64 * N * (T / 8 + S) numbers, or (chunk_states not null, see forge_decay_chunks) not
+// needed; out fp32 [T, N*KV]; the state as above.
+extern "C" int forge_lightning_scan(float* proj, int ld, const float* decay, float* gram, float* chunk_states, float* state, long long state_stride,
                                     const int32_t* q_start, const int32_t* slots, float* out, int T, int S, int N, int K, int KV, cudaStream_t stream) {
     int rc = check("lightning_scan", T, S, N, N, K, KV, state_stride);
     if (rc == FORGE_OK && ld < N * (2 * K + KV)) rc = forge::fail(FORGE_ERR_ARG, "lightning_scan: rows of %d are too short", ld);
     if (rc != FORGE_OK || S == 0 || T == 0) return rc;
     rc = forge_silu_columns(proj, ld, T, N * (2 * K + KV), stream);
     if (rc != FORGE_OK) return rc;
+    if (chunk_states)
+        return forge_decay_chunks(proj, ld, proj + N * K, ld, proj + 2 * N * K, ld, decay, chunk_states, state, state_stride, q_start, slots, out, T, S, N, K,
+                                  KV, stream);
     return run<false>(BlockScan{proj, proj + N * K, proj + 2 * N * K, ld, ld, ld, nullptr, decay, nullptr, state, state_stride, q_start, slots, out, N, N, K, KV, 0},
                       gram, T, S, stream);
 }

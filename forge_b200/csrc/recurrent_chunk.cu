@@ -1,0 +1,511 @@
+// The recurrences of recurrent_block.cu over long portions, 32 tokens at a time (fp32 throughout), for heads of 64 key channels:
+//
+//     gated delta rule   S <- g_t S;   S <- S + k_t (b_t (v_t - S^T k_t))^T;   o_t = S^T q_t
+//     one fixed decay    S <- g S + k_t v_t^T;   o_t = S^T q_t                        (lightning attention, retention; u_t = v_t)
+//
+// With S the state before a chunk of tokens 0 .. 31, P_j = g_0 .. g_j and R_ij = g_{i+1} .. g_j, the rule over the chunk is
+//     u_j = b_j (v_j - P_j S^T k_j - sum_{i<j} R_ij (k_i . k_j) u_i)
+//     o_j = P_j S^T q_j + sum_{i<=j} R_ij (k_i . q_j) u_i
+//     S  <- P_31 S + sum_i R_i,31 k_i u_i^T
+// and what waits for S is little: the triangle of the u_j is solved for both of its right-hand sides ahead, U from b_j v_j and W from
+// b_j P_j k_j, so that u = U - W S.  Three kernels, of which only the second walks a request's chunks one after the other:
+//     1  per (chunk, head)          W and U                          (fixed decay: Z = sum_i R_i,31 k_i v_i^T, all a chunk does to the state)
+//     2  per (request, head, cols)  u = U - W S, the state before every chunk kept, S moved on        (fixed decay: S <- P_31 S + Z)
+//     3  per (chunk, head)          the outputs, from the kept states
+// The block scan they replace makes a chain of 900 instructions of every eight tokens with two to four warps an SM.  2,001 tokens in three portions, 32 heads:
+// 216 us with its gram matrices, 185 us here (solve 38, walk 103, outputs 44).  Fixed decay, 1,500 tokens in two portions, 64 heads: 252 us token by
+// token, 110 us here.  Every R is a
+// product of its decays (no quotients), so a decay of zero does no harm.  Scratch: W, U [chunks, N, 32, 64 | V] and the states
+// [chunks, N, 64, V], chunks = T / 32 + S.
+#include "common.cuh"
+
+namespace {
+
+constexpr int CH = 32, K = 64, kThreads = 128, LD = K + 4, VB = 64, kColsB = 16;
+
+__device__ __forceinline__ void stage16(float* dst, const float* src, bool ok) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void stages_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void stages_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+struct Chunks {
+    const float *q, *k, *v;
+    int ld_q, ld_k, ld_v;
+    const float* g;                   // DELTA: decays [T, N]; else [N]
+    const float* beta;                // DELTA: [T, N]
+    float *w, *u, *s;
+    float* state;
+    long long stride;
+    const int32_t *q_start, *slots;
+    float* out;
+    int S, N, M, V;
+};
+
+// The first chunk of request s in the row of all requests' chunks (n tokens take at most n/32 + 1 of them).
+__device__ __forceinline__ int first_chunk(const int32_t* __restrict__ q_start, int s) { return q_start[s] / CH + s; }
+
+// The tokens of a chunk: the first one and how many (0: a chunk that its request does not have).
+__device__ __forceinline__ int chunk_tokens(const Chunks& d, int chunk, int& t0) {
+    int lo = 0, hi = d.S - 1;                                 // the last request whose first chunk is not behind this one
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (first_chunk(d.q_start, mid) <= chunk) lo = mid;
+        else hi = mid - 1;
+    }
+    t0 = d.q_start[lo] + (chunk - first_chunk(d.q_start, lo)) * CH;
+    return min(CH, d.q_start[lo + 1] - t0);
+}
+
+// 32 rows of 64 numbers (row t at src + t * ld), zeros from row n on, as rows of LD
+template <int THREADS = kThreads>
+__device__ __forceinline__ void stage_rows(float* dst, const float* src, int ld, int n) {
+    for (int i = threadIdx.x; i < CH * K / 4; i += THREADS) {
+        const int r = i / (K / 4), c = i % (K / 4) * 4;
+        stage16(dst + r * LD + c, r < n ? src + (size_t)r * ld + c : src, r < n);
+    }
+}
+
+__device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
+    return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, acc))));
+}
+
+// r[j][i] = g_{i+1} .. g_j for i <= j (zero above): thread j of the first 32 makes row j.
+__device__ __forceinline__ void decay_triangle(float (*r)[CH + 1], const float* g) {
+    if (threadIdx.x < CH) {
+        const int j = threadIdx.x;
+        float x = 1.f;
+        for (int i = CH - 1; i >= 0; --i) {
+            r[j][i] = i <= j ? x : 0.f;
+            if (i <= j) x *= g[i];
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ 1: before the walk
+// DELTA: thread c solves the triangle for column c of [W | U].
+__global__ void __launch_bounds__(kThreads)
+chunk_solve_kernel(const Chunks d) {
+    __shared__ __align__(16) float ks[CH * LD], A[CH][CH + 4];
+    __shared__ float R[CH][CH + 1], gs[CH], bs[CH], P[CH];
+    // (no early word to the scheduler: the walk's few CTAs would be placed between this kernel's many)
+    forge::pdl_wait();
+    int t0;
+    const int chunk = blockIdx.x, head = blockIdx.y, n = chunk_tokens(d, chunk, t0), tid = threadIdx.x;
+    if (n <= 0) return;
+    stage_rows(ks, d.k + (size_t)t0 * d.ld_k + head / (d.N / d.M) * K, d.ld_k, n);
+    stages_commit();
+    if (tid < CH) {
+        gs[tid] = tid < n ? d.g[(size_t)(t0 + tid) * d.N + head] : 1.0f;
+        bs[tid] = tid < n ? d.beta[(size_t)(t0 + tid) * d.N + head] : 0.f;
+    }
+    __syncthreads();
+    decay_triangle(R, gs);
+    if (tid == CH) {
+        float p = 1.f;
+        for (int i = 0; i < CH; ++i) P[i] = p *= gs[i];
+    }
+    stages_wait<0>();
+    __syncthreads();
+    {
+        const int j = tid >> 2, i0 = tid & 3;                 // entries (j, i0 + 4 m): a warp's rows lie in different banks
+        float acc[CH / 4];
+#pragma unroll
+        for (int m = 0; m < CH / 4; ++m) acc[m] = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < K; c += 4) {
+            const float4 kj = *reinterpret_cast<const float4*>(ks + j * LD + c);
+#pragma unroll
+            for (int m = 0; m < CH / 4; ++m) acc[m] = dot4(kj, *reinterpret_cast<const float4*>(ks + (i0 + 4 * m) * LD + c), acc[m]);
+        }
+#pragma unroll
+        for (int m = 0; m < CH / 4; ++m) A[i0 + 4 * m][j] = bs[j] * R[j][i0 + 4 * m] * acc[m];        // transposed: what row i does to the rows below
+    }
+    __syncthreads();
+    for (int c = tid; c < K + d.V; c += kThreads) {
+        float x[CH];
+        if (c < K) {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) x[j] = bs[j] * P[j] * ks[j * LD + c];
+        } else {
+            const float* v = d.v + (size_t)t0 * d.ld_v + (size_t)head * d.V + c - K;
+#pragma unroll
+            for (int j = 0; j < CH; ++j) x[j] = j < n ? bs[j] * v[(size_t)j * d.ld_v] : 0.f;
+        }
+        // a finished x_i goes to all rows below at once: independent multiply-adds, where a row's own sum would be a chain
+#pragma unroll
+        for (int i = 0; i + 1 < CH; ++i) {
+#pragma unroll
+            for (int j = (i + 1) / 4 * 4; j < CH; j += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(&A[i][j]);
+                if (j > i) x[j] = fmaf(-a.x, x[i], x[j]);
+                if (j + 1 > i) x[j + 1] = fmaf(-a.y, x[i], x[j + 1]);
+                if (j + 2 > i) x[j + 2] = fmaf(-a.z, x[i], x[j + 2]);
+                if (j + 3 > i) x[j + 3] = fmaf(-a.w, x[i], x[j + 3]);
+            }
+        }
+        const size_t at = ((size_t)chunk * d.N + head) * CH;
+        if (c < K) {
+#pragma unroll
+            for (int j = 0; j < CH; j += 4)                        // transposed, as the walk reads it: 32 tokens of a channel side by side
+                *reinterpret_cast<float4*>(d.w + at * K + c * CH + j) = make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) d.u[(at + j) * d.V + c - K] = x[j];
+        }
+    }
+}
+
+// Fixed decay: Z = sum_t g^(n-1-t) k_t v_t^T, 64 x 64 columns a CTA, a thread 8 x 4 of them.
+__global__ void __launch_bounds__(kThreads)
+chunk_update_kernel(const Chunks d) {
+    __shared__ __align__(16) float ks[CH * LD], vs[CH * LD];
+    forge::pdl_wait();
+    int t0;
+    const int chunk = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * VB, n = chunk_tokens(d, chunk, t0), tid = threadIdx.x;
+    if (n <= 0) return;
+    stage_rows(ks, d.k + (size_t)t0 * d.ld_k + head * K, d.ld_k, n);
+    stage_rows(vs, d.v + (size_t)t0 * d.ld_v + (size_t)head * d.V + v0, d.ld_v, n);
+    stages_commit();
+    const float g = d.g[head];
+    float acc[8][4];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.f;
+    stages_wait<0>();
+    __syncthreads();
+    const int kr = tid / 16 * 4, c = tid % 16 * 4;            // rows kr .. kr+3 and 32 + kr ..
+    float w = 1.f;
+    for (int t = n - 1; t >= 0; --t, w *= g) {
+        const float4 v = *reinterpret_cast<const float4*>(vs + t * LD + c);
+        const float4 k0 = *reinterpret_cast<const float4*>(ks + t * LD + kr), k1 = *reinterpret_cast<const float4*>(ks + t * LD + 32 + kr);
+        const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w}, vw[4] = {w * v.x, w * v.y, w * v.z, w * v.w};
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(kk[a], vw[b], acc[a][b]);
+    }
+    float* z = d.s + ((size_t)chunk * d.N + head) * K * d.V + v0 + c;
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+        *reinterpret_cast<float4*>(z + (size_t)(kr + (a & 3) + (a >> 2) * 32) * d.V) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+}
+
+// ------------------------------------------------------------------------------------------------ 2: the walk
+// DELTA: 16 columns of one head's S a CTA; the next chunk's W, K, U and decays are on their way while the present one is worked on.  A chunk is
+// two small products, one after the other: u = U - W S (32 x 16 numbers over 64 channels) and S + K^T u (64 x 16 over 32 tokens).  What
+// bounds them is how often shared memory is asked, so a thread has 4 x 4 numbers of a product and the warps share the sum: eight channels a
+// warp, eight tokens two warps, the parts added up out of shared memory (a whole sum of 1 x 4 numbers a thread asked twice as often, and three
+// portions of 2,001 tokens in all, 32 heads, took 146 us; 103 us so).
+constexpr int kWalkThreads = 256, kPartLd = kColsB + 4;
+constexpr int kStageB = 2 * CH * K + CH * kColsB + CH;        // floats of a chunk's W, K, U, decays
+constexpr int kPartB = 8 * CH * kPartLd;                      // eight parts of u or four of S
+static_assert(kPartB == 4 * K * kPartLd, "both fill it");
+constexpr size_t kWalkSmem = sizeof(float) * (2 * kStageB + kPartB + K * kColsB + CH * kColsB + CH + 4);
+
+__global__ void __launch_bounds__(kWalkThreads, 3)
+chunk_walk_kernel(const Chunks d) {
+    extern __shared__ __align__(16) float sm[];
+    float* part = sm + 2 * kStageB;                           // [8][32][16 + 4] or [4][64][16 + 4]
+    float* S = part + kPartB;                                 // [64][16]
+    float* us = S + K * kColsB;                               // [32][16]: u_t times the decays behind it
+    float* wt = us + CH * kColsB;                             // [32]: the decays behind a token, then the chunk's whole decay
+    forge::pdl_launch_dependents();
+    forge::pdl_wait();
+    const int s = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * kColsB, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int t_lo = d.q_start[s], t_hi = d.q_start[s + 1];
+    if (t_lo >= t_hi) return;
+    const int chunks = (t_hi - t_lo + CH - 1) / CH, at0 = first_chunk(d.q_start, s);
+    const float* k = d.k + (size_t)head / (d.N / d.M) * K;
+    auto fetch = [&](int i) {
+        if (i < chunks) {
+            float* w = sm + (i & 1) * kStageB;
+            const int t0 = t_lo + i * CH, n = min(CH, t_hi - t0);
+            const size_t at = ((size_t)(at0 + i) * d.N + head) * CH;
+#pragma unroll
+            for (int h = 0; h < CH * K / 4; h += kWalkThreads) {
+                const int e = h + tid, r = e / (K / 4), c = e % (K / 4) * 4;
+                stage16(w + e * 4, d.w + at * K + e * 4, true);
+                stage16(w + CH * K + e * 4, k + (size_t)(r < n ? t0 + r : t0) * d.ld_k + c, r < n);
+            }
+            if (tid < CH * kColsB / 4) stage16(w + 2 * CH * K + tid * 4, d.u + (at + tid / 4) * d.V + c0 + tid % 4 * 4, true);
+            else if (tid < CH * kColsB / 4 + CH) {
+                const int t = tid - CH * kColsB / 4;
+                float* dst = w + 2 * CH * K + CH * kColsB + t;
+                if (t < n) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(d.g + (size_t)(t0 + t) * d.N + head) : "memory");
+                else *dst = 1.0f;
+            }
+        }
+        stages_commit();
+    };
+    fetch(0);
+    // four numbers of S stay with a thread: row tid / 4, columns tid % 4 * 4 ..
+    const int row = tid / 4, col = tid % 4 * 4;
+    float* S_g = d.state + (size_t)d.slots[s] * d.stride + (size_t)head * K * d.V + (size_t)row * d.V + c0 + col;
+    float4 own = *reinterpret_cast<const float4*>(S_g);
+    *reinterpret_cast<float4*>(S + row * kColsB + col) = own;
+    const int tg = lane / 4 * 4, cg = lane % 4 * 4;           // a thread's 4 x 4 numbers: tokens tg .. (or rows) and columns cg ..
+    for (int i = 0; i < chunks; ++i) {
+        fetch(i + 1);
+        stages_wait<1>();
+        __syncthreads();                                      // chunk i is here and S stands
+        const float* w = sm + (i & 1) * kStageB;
+        const float* ks = w + CH * K;
+        if (tid < CH) {                                       // the decays behind token t, and the chunk's
+            float x = w[2 * CH * K + CH * kColsB + tid];      // becomes g_t .. g_31
+#pragma unroll
+            for (int o = 1; o < CH; o <<= 1) {
+                const float y = __shfl_down_sync(0xffffffffu, x, o);
+                if (tid + o < CH) x *= y;
+            }
+            const float next = __shfl_down_sync(0xffffffffu, x, 1);
+            wt[tid] = tid + 1 < CH ? next : 1.0f;
+            if (tid == 0) wt[CH] = x;
+        }
+        *reinterpret_cast<float4*>(d.s + (((size_t)(at0 + i) * d.N + head) * K + row) * d.V + c0 + col) = own;
+        float a[4][4];
+        auto product = [&](const float* l, int ld_l, const float* r) {      // eight steps of a (+)= l[k][4] r[k][4]
+#pragma unroll
+            for (int x = 0; x < 4; ++x) a[x][0] = a[x][1] = a[x][2] = a[x][3] = 0.f;
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk) {
+                const float4 x = *reinterpret_cast<const float4*>(l + kk * ld_l), y = *reinterpret_cast<const float4*>(r + kk * kColsB);
+                const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    a[e][0] = fmaf(xv[e], y.x, a[e][0]);
+                    a[e][1] = fmaf(xv[e], y.y, a[e][1]);
+                    a[e][2] = fmaf(xv[e], y.z, a[e][2]);
+                    a[e][3] = fmaf(xv[e], y.w, a[e][3]);
+                }
+            }
+        };
+        auto leave = [&](float* dst) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) *reinterpret_cast<float4*>(dst + e * kPartLd) = make_float4(a[e][0], a[e][1], a[e][2], a[e][3]);
+        };
+        product(w + warp * 8 * CH + tg, CH, S + warp * 8 * kColsB + cg);
+        leave(part + (warp * CH + tg) * kPartLd + cg);
+        __syncthreads();
+        {
+            const int t = tid / 8, c = tid % 8 * 2;
+            float2 u = *reinterpret_cast<const float2*>(w + 2 * CH * K + t * kColsB + c);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float2 x = *reinterpret_cast<const float2*>(part + (q * CH + t) * kPartLd + c);
+                u.x -= x.x;
+                u.y -= x.y;
+            }
+            const float r = wt[t];
+            *reinterpret_cast<float2*>(us + t * kColsB + c) = make_float2(u.x * r, u.y * r);
+            *reinterpret_cast<float2*>(d.u + (((size_t)(at0 + i) * d.N + head) * CH + t) * d.V + c0 + c) = u;
+        }
+        __syncthreads();
+        const int half = (warp & 1) * 32, t8 = (warp >> 1) * 8;             // rows half + tg .., tokens t8 .. t8 + 7
+        product(ks + t8 * K + half + tg, K, us + t8 * kColsB + cg);
+        leave(part + ((warp >> 1) * K + half + tg) * kPartLd + cg);
+        __syncthreads();
+        const float p = wt[CH];
+        own.x *= p; own.y *= p; own.z *= p; own.w *= p;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 x = *reinterpret_cast<const float4*>(part + (q * K + row) * kPartLd + col);
+            own.x += x.x; own.y += x.y; own.z += x.z; own.w += x.w;
+        }
+        *reinterpret_cast<float4*>(S + row * kColsB + col) = own;
+        // (chunk i's buffer was last read before the last barrier, and part, us and wt are not written before the next one)
+    }
+    *reinterpret_cast<float4*>(S_g) = own;
+}
+
+// Fixed decay: four neighbouring numbers of the state a thread; where Z of a chunk lay the state before it stays.
+__global__ void __launch_bounds__(kThreads)
+chunk_sum_kernel(const Chunks d) {
+    forge::pdl_launch_dependents();
+    forge::pdl_wait();
+    const int s = blockIdx.x, head = blockIdx.y, e = (blockIdx.z * kThreads + threadIdx.x) * 4;
+    const int t_lo = d.q_start[s], t_hi = d.q_start[s + 1], size = K * d.V;
+    if (t_lo >= t_hi || e >= size) return;
+    const int chunks = (t_hi - t_lo + CH - 1) / CH, last = t_hi - t_lo - (chunks - 1) * CH;
+    const float g = d.g[head];
+    float p = 1.f, p_last = 1.f;
+    for (int i = 0; i < CH; ++i) {
+        p *= g;
+        if (i < last) p_last = p;
+    }
+    float* S_g = d.state + (size_t)d.slots[s] * d.stride + (size_t)head * size + e;
+    float* z = d.s + ((size_t)first_chunk(d.q_start, s) * d.N + head) * size + e;
+    const size_t step = (size_t)d.N * size;
+    float4 x = *reinterpret_cast<const float4*>(S_g);
+    constexpr int kAhead = 8;                                 // chunks whose Z is asked for before the first is used
+    for (int i0 = 0; i0 < chunks; i0 += kAhead) {
+        float4 y[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+            if (i0 + i < chunks) y[i] = *reinterpret_cast<const float4*>(z + (size_t)(i0 + i) * step);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+            if (i0 + i < chunks) {
+                *reinterpret_cast<float4*>(z + (size_t)(i0 + i) * step) = x;
+                const float f = i0 + i + 1 < chunks ? p : p_last;
+                x = make_float4(fmaf(f, x.x, y[i].x), fmaf(f, x.y, y[i].y), fmaf(f, x.z, y[i].z), fmaf(f, x.w, y[i].w));
+            }
+    }
+    *reinterpret_cast<float4*>(S_g) = x;
+}
+
+// ------------------------------------------------------------------------------------------------ 3: the outputs
+// A CTA has 64 of a head's value columns, a thread eight tokens x four columns (bound by shared memory: a wider tile reads less of it).
+constexpr int kOutThreads = 64, TJ = CH * VB / 4 / kOutThreads;
+template <bool DELTA>
+__global__ void __launch_bounds__(kOutThreads)
+chunk_output_kernel(const Chunks d) {
+    __shared__ __align__(16) float qs[CH * LD], S[K * VB], us[CH * VB], Mx[CH][CH + 4];
+    __shared__ float R[CH][CH + 1], gs[CH], P[CH];
+    float* ks = S;                                            // the keys until the products stand, then the state
+    static_assert(CH * LD <= K * VB, "the keys fit where the state will lie");
+    forge::pdl_launch_dependents();
+    forge::pdl_wait();
+    int t0;
+    const int chunk = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * VB, n = chunk_tokens(d, chunk, t0), tid = threadIdx.x;
+    if (n <= 0) return;
+    const int hk = head / (d.N / d.M);
+    stage_rows<kOutThreads>(qs, d.q + (size_t)t0 * d.ld_q + hk * K, d.ld_q, n);
+    stage_rows<kOutThreads>(ks, d.k + (size_t)t0 * d.ld_k + hk * K, d.ld_k, n);
+    stages_commit();
+    const float* u = DELTA ? d.u + ((size_t)chunk * d.N + head) * CH * d.V + v0 : d.v + (size_t)t0 * d.ld_v + (size_t)head * d.V + v0;
+    const int ld_u = DELTA ? d.V : d.ld_v;
+    for (int i = tid; i < CH * VB / 4; i += kOutThreads) {
+        const int r = i / (VB / 4), c = i % (VB / 4) * 4;
+        stage16(us + r * VB + c, r < n ? u + (size_t)r * ld_u + c : u, r < n);
+    }
+    stages_commit();
+    if (tid < CH) gs[tid] = tid >= n ? 1.0f : DELTA ? d.g[(size_t)(t0 + tid) * d.N + head] : d.g[head];
+    __syncthreads();
+    decay_triangle(R, gs);
+    if (tid == CH) {
+        float p = 1.f;
+        for (int i = 0; i < CH; ++i) P[i] = p *= gs[i];
+    }
+    stages_wait<1>();
+    __syncthreads();
+    {
+        const int j = tid >> 1, i0 = tid & 1;
+        float acc[CH / 2];
+#pragma unroll
+        for (int m = 0; m < CH / 2; ++m) acc[m] = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < K; c += 4) {
+            const float4 qj = *reinterpret_cast<const float4*>(qs + j * LD + c);
+#pragma unroll
+            for (int m = 0; m < CH / 2; ++m) acc[m] = dot4(qj, *reinterpret_cast<const float4*>(ks + (i0 + 2 * m) * LD + c), acc[m]);
+        }
+#pragma unroll
+        for (int m = 0; m < CH / 2; ++m) Mx[j][i0 + 2 * m] = R[j][i0 + 2 * m] * acc[m];
+    }
+    __syncthreads();                                          // the keys have been read
+    const float* kept = d.s + ((size_t)chunk * d.N + head) * K * d.V + v0;
+    for (int i = tid; i < K * VB / 4; i += kOutThreads) stage16(S + i * 4, kept + (size_t)(i / (VB / 4)) * d.V + i % (VB / 4) * 4, true);
+    stages_commit();
+    const int j0 = tid / 16 * TJ, c = tid % 16 * 4;
+    float acc[TJ][4];
+#pragma unroll
+    for (int a = 0; a < TJ; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.f;
+    stages_wait<0>();
+    __syncthreads();
+#pragma unroll 2
+    for (int kk = 0; kk < K; kk += 4) {
+        float qv[TJ][4];
+#pragma unroll
+        for (int a = 0; a < TJ; ++a) *reinterpret_cast<float4*>(qv[a]) = *reinterpret_cast<const float4*>(qs + (j0 + a) * LD + kk);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float4 x = *reinterpret_cast<const float4*>(S + (kk + e) * VB + c);
+#pragma unroll
+            for (int a = 0; a < TJ; ++a) {
+                acc[a][0] = fmaf(qv[a][e], x.x, acc[a][0]);
+                acc[a][1] = fmaf(qv[a][e], x.y, acc[a][1]);
+                acc[a][2] = fmaf(qv[a][e], x.z, acc[a][2]);
+                acc[a][3] = fmaf(qv[a][e], x.w, acc[a][3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < TJ; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] *= P[j0 + a];
+    for (int i = 0; i < j0 + TJ; i += 4) {                     // (the triangle's zeros take part up to the block on the diagonal)
+        float mv[TJ][4];
+#pragma unroll
+        for (int a = 0; a < TJ; ++a) *reinterpret_cast<float4*>(mv[a]) = *reinterpret_cast<const float4*>(&Mx[j0 + a][i]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float4 x = *reinterpret_cast<const float4*>(us + (i + e) * VB + c);
+#pragma unroll
+            for (int a = 0; a < TJ; ++a) {
+                if (i + e > j0 + a) continue;                 // a later token takes no part, whatever its numbers
+                acc[a][0] = fmaf(mv[a][e], x.x, acc[a][0]);
+                acc[a][1] = fmaf(mv[a][e], x.y, acc[a][1]);
+                acc[a][2] = fmaf(mv[a][e], x.z, acc[a][2]);
+                acc[a][3] = fmaf(mv[a][e], x.w, acc[a][3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < TJ; ++a)
+        if (j0 + a < n)
+            *reinterpret_cast<float4*>(d.out + (size_t)(t0 + j0 + a) * d.N * d.V + (size_t)head * d.V + v0 + c) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+}
+
+bool aligned(const float* p, long long ld) { return ((uintptr_t)p & 15) == 0 && ld % 4 == 0; }
+
+int check(const char* what, const Chunks& d, int T, int Kc) {
+    if (T < 0 || d.S < 0 || d.N <= 0 || d.M <= 0 || d.N % d.M != 0 || d.V <= 0) return forge::fail(FORGE_ERR_ARG, "%s: bad sizes S=%d N=%d M=%d V=%d", what, d.S, d.N, d.M, d.V);
+    if (Kc != K || d.V % VB != 0 || d.V > 65535 * kColsB || d.N > 65535) return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: heads of %d and %d channels", what, Kc, d.V);
+    if (d.stride < (long long)d.N * K * d.V) return forge::fail(FORGE_ERR_ARG, "%s: state rows are too short", what);
+    if (!aligned(d.q, d.ld_q) || !aligned(d.k, d.ld_k) || !aligned(d.v, d.ld_v) || !aligned(d.state, d.stride) || !aligned(d.out, 4) || !aligned(d.s, 4))
+        return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: rows that are not aligned to 16 bytes", what);
+    return FORGE_OK;
+}
+
+}  // namespace
+
+// 1 if the kernels take heads of these sizes (rows must be aligned to 16 bytes).
+extern "C" int forge_chunk_scan_supports(int key_channels, int value_channels) { return key_channels == K && value_channels % VB == 0 ? 1 : 0; }
+
+// The gated delta rule as forge_gated_delta_scan defines it; w, u, s fp32 scratch of C * N * 32 * 64, C * N * 32 * V and C * N * 64 * V
+// numbers, C = T / 32 + S.
+extern "C" int forge_gated_delta_chunks(const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v, const float* g, const float* beta,
+                                        float* w, float* u, float* s, float* state, long long state_stride, const int32_t* q_start, const int32_t* slots,
+                                        float* out, int T, int S, int N, int M, int Kc, int V, cudaStream_t stream) {
+    const Chunks d{q, k, v, ld_q, ld_k, ld_v, g, beta, w, u, s, state, state_stride, q_start, slots, out, S, N, M, V};
+    const int rc = check("gated_delta_chunks", d, T, Kc);
+    if (rc != FORGE_OK || S == 0 || T == 0) return rc;
+    if (!aligned(w, 4) || !aligned(u, 4)) return forge::fail(FORGE_ERR_ARG, "gated_delta_chunks: scratch that is not aligned");
+    static forge::PerDeviceFlag flag;
+    bool& done = flag.current();
+    if (!done) {
+        const cudaError_t e = cudaFuncSetAttribute(chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem);
+        if (e != cudaSuccess) return forge::check_launch("gated_delta_chunks (shared memory)", e);
+        done = true;
+    }
+    const unsigned chunks = T / CH + S;
+    cudaError_t e = forge::launch(chunk_solve_kernel, dim3(chunks, N), dim3(kThreads), 0, stream, 1, d);
+    if (e == cudaSuccess) e = forge::launch(chunk_walk_kernel, dim3(S, N, V / kColsB), dim3(kWalkThreads), kWalkSmem, stream, 1, d);
+    if (e == cudaSuccess) e = forge::launch(chunk_output_kernel<true>, dim3(chunks, N, V / VB), dim3(kOutThreads), 0, stream, 1, d);
+    return forge::check_launch("gated_delta_chunks", e);
+}
+
+// S <- decay[n] S + k v^T, out = S^T q per head over the step's tokens (q and k of every head); s as above.
+extern "C" int forge_decay_chunks(const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v, const float* decay, float* s, float* state,
+                                  long long state_stride, const int32_t* q_start, const int32_t* slots, float* out, int T, int S, int N, int Kc, int V,
+                                  cudaStream_t stream) {
+    const Chunks d{q, k, v, ld_q, ld_k, ld_v, decay, nullptr, nullptr, nullptr, s, state, state_stride, q_start, slots, out, S, N, N, V};
+    const int rc = check("decay_chunks", d, T, Kc);
+    if (rc != FORGE_OK || S == 0 || T == 0) return rc;
+    const unsigned chunks = T / CH + S;
+    cudaError_t e = forge::launch(chunk_update_kernel, dim3(chunks, N, V / VB), dim3(kThreads), 0, stream, 1, d);
+    if (e == cudaSuccess) e = forge::launch(chunk_sum_kernel, dim3(S, N, (K * V / 4 + kThreads - 1) / kThreads), dim3(kThreads), 0, stream, 1, d);
+    if (e == cudaSuccess) e = forge::launch(chunk_output_kernel<false>, dim3(chunks, N, V / VB), dim3(kOutThreads), 0, stream, 1, d);
+    return forge::check_launch("decay_chunks", e);
+}

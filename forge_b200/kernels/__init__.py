@@ -85,14 +85,16 @@ _SIGNATURES = {
         "forge_tanh_rows": [_P, _I, _P, _I, _I, _I, _P],
         "forge_gla_scan": [_P, _I] * 4 + [_I, _P, _P, _F, _F, _P, _P, _LL, _P, _P, _P, _I, _I, _I, _I, _I, _P],
         "forge_gla_token": [_P, _I] * 5 + [_I, _P, _P, _F, _F, _P, _LL, _P, _P, _P, _F, _P, _I, _LL, _I, _I, _I, _I, _P],
-        "forge_lightning_scan": [_P, _I, _P, _P, _P, _LL, _P, _P, _P] + [_I] * 5 + [_P],
+        "forge_lightning_scan": [_P, _I, _P, _P, _P, _P, _LL, _P, _P, _P] + [_I] * 5 + [_P],
+        "forge_chunk_scan_supports": [_I, _I],
+        "forge_gated_delta_chunks": [_P, _I] * 3 + [_P] * 6 + [_LL, _P, _P, _P] + [_I] * 6 + [_P],
         "forge_lightning_token": [_P, _I, _P, _P, _LL, _P, _P, _P] + [_I] * 4 + [_P],
         "forge_gated_delta_scan": [_P, _I] * 3 + [_P, _P, _P, _P, _LL, _P, _P, _P] + [_I] * 6 + [_P],
         "forge_delta_prepare": [_P, _I, _I, _I, _P, _I, _P, _LL, _LL] + [_P] * 9 + [_I] * 6 + [_P],
         "forge_gated_delta_token": [_P, _I, _I, _I, _I, _P, _I, _P, _LL, _LL] + [_P] * 6 + [_F, _P, _I, _LL] + [_I] * 5 + [_P],
         "forge_token_state_supports": [_I] * 3,
         "forge_gated_rows": [_P, _P, _P, _I, _P, _I, _LL, _I, _I, _F, _P],
-        "forge_retention_scan": [_P, _I, _P, _I, _P, _I, _P, _P, _I, _F, _P, _P, _LL, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+        "forge_retention_scan": [_P, _I, _P, _I, _P, _I, _P, _P, _I, _F, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     },
     "latent": {
         "forge_latent_prepare": [_P, _I, _P, _P, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
@@ -1226,12 +1228,13 @@ def retention_scan(q, k, v, batch, freq, k_scale, decay, state, N, K, KV):
     out = new_tensor((T, N * KV), torch.float32, q[0].device)
     (qp, ql), (kp, kl), (vp, vl) = _cols(*q), _cols(*k), _cols(*v)
     rot = 0 if freq is None else 2 * freq.numel()
+    chunks = _chunk_states(batch, T, N, K, KV, (qp, ql), (kp, kl), (vp, vl), state)
     _check(lib, lib.forge_retention_scan(
         qp, ql, kp, kl, vp, vl, _need(batch.positions, "positions", torch.int32), _opt(freq, "freq", torch.float32) if rot else None, rot,
         float(k_scale), _need(decay, "decay", torch.float32), _need(state, "state", torch.float32, 2), state.shape[1],
-        _need(batch.q_start, "q_start", torch.int32), _need(batch.slots, "slots", torch.int32), _need(out, "out", torch.float32), T,
-        batch.num_requests, N, K, KV, _stream()), "retention_scan")
-    count_launches(1)              # the kernel that rotates and scales q and k, in place
+        _need(batch.q_start, "q_start", torch.int32), _need(batch.slots, "slots", torch.int32), _need(out, "out", torch.float32),
+        _opt(chunks, "chunks", torch.float32), T, batch.num_requests, N, K, KV, _stream()), "retention_scan")
+    count_launches(1 if chunks is None else 3)              # the kernel that rotates and scales q and k, in place (and two more chunk by chunk)
     return out
 
 
@@ -1289,6 +1292,24 @@ def _gram(batch, T, heads, device):
     return new_tensor(((T // 8 + batch.num_requests) * heads * 64,), torch.float32, device)
 
 
+CHUNK_TOKENS = 32                  # of the recurrences that go chunk by chunk (csrc/recurrent_chunk.cu)
+CHUNKS_FROM = 64                   # tokens a request from which they do: below, eight tokens at a time are as fast and need no scratch
+CHUNK_SCRATCH_LIMIT = 1 << 30      # bytes of states that a step may keep
+
+
+def _chunk_states(batch, T, N, K, V, q, k, v, state):
+    """Room for the state before every chunk of every request, if the step's portions are long enough, the heads of a size that the
+    kernels take and all rows ((pointer, row length) q, k, v; state) aligned to 16 bytes; else None."""
+    if T < CHUNKS_FROM * batch.num_requests or not library("mixers").forge_chunk_scan_supports.fn(int(K), int(V)):
+        return None
+    if any(p % 16 or ld % 4 for p, ld in (q, k, v, (state.data_ptr(), state.shape[1]))):
+        return None
+    shape = (T // CHUNK_TOKENS + batch.num_requests, N, K, V)
+    if 4 * shape[0] * N * K * V > CHUNK_SCRATCH_LIMIT:
+        return None
+    return new_tensor(shape, torch.float32, state.device)
+
+
 def token_state_supports(batch, K, V, delta):
     """A step in which every request brings one token, and heads of K x V numbers that the kernel of single tokens takes."""
     return batch.num_tokens == batch.num_requests and bool(library("mixers").forge_token_state_supports.fn(int(K), int(V), 1 if delta else 0))
@@ -1301,10 +1322,12 @@ def lightning_scan(proj, col, decay, batch, state, N, K, V):
     T = proj.shape[0]
     out = new_tensor((T, N * V), torch.float32, proj.device)
     p, ld = _cols(proj, col)
-    _check(lib, lib.forge_lightning_scan(p, ld, _need(decay, "decay", torch.float32), _need(_gram(batch, T, N, proj.device), "gram"), _need(state, "state", torch.float32, 2), state.shape[1],
+    chunks = _chunk_states(batch, T, N, K, V, (p, ld), (p, ld), (p, ld), state)
+    gram = _gram(batch, T, N, proj.device) if chunks is None else None
+    _check(lib, lib.forge_lightning_scan(p, ld, _need(decay, "decay", torch.float32), _opt(gram, "gram"), _opt(chunks, "chunks"), _need(state, "state", torch.float32, 2), state.shape[1],
                                          _need(batch.q_start, "q_start", torch.int32), _need(batch.slots, "slots", torch.int32),
                                          _need(out, "out", torch.float32), T, batch.num_requests, N, K, V, _stream()), "lightning_scan")
-    count_launches(2)              # the kernels that apply silu and take the blocks' products
+    count_launches(2 if chunks is None else 3)              # the kernels that apply silu and take the blocks' products (or those of the chunks)
     return out
 
 
@@ -1373,6 +1396,16 @@ def gated_delta_scan(qkv, g, beta, batch, state, N, M, K, V):
     T = qkv.shape[0]
     out = new_tensor((T, N * V), torch.float32, qkv.device)
     (qp, ld), (kp, _), (vp, _) = _cols(qkv, 0), _cols(qkv, M * K), _cols(qkv, 2 * M * K)
+    chunks = _chunk_states(batch, T, N, K, V, (qp, ld), (kp, ld), (vp, ld), state)
+    if chunks is not None:
+        rows = (T // CHUNK_TOKENS + batch.num_requests) * N * CHUNK_TOKENS
+        w, u = new_tensor((rows, K), torch.float32, qkv.device), new_tensor((rows, V), torch.float32, qkv.device)
+        _check(lib, lib.forge_gated_delta_chunks(
+            qp, ld, kp, ld, vp, ld, _need(g, "g", torch.float32, 2), _need(beta, "beta", torch.float32, 2), _need(w, "w"), _need(u, "u"), _need(chunks, "chunks"),
+            _need(state, "state", torch.float32, 2), state.shape[1], _need(batch.q_start, "q_start", torch.int32), _need(batch.slots, "slots", torch.int32),
+            _need(out, "out", torch.float32), T, batch.num_requests, N, M, K, V, _stream()), "gated_delta_chunks")
+        count_launches(2)          # the walk over the chunks, and the outputs
+        return out
     _check(lib, lib.forge_gated_delta_scan(
         qp, ld, kp, ld, vp, ld, _need(g, "g", torch.float32, 2), _need(beta, "beta", torch.float32, 2), _need(_gram(batch, T, M, qkv.device), "gram"),
         _need(state, "state", torch.float32, 2), state.shape[1], _need(batch.q_start, "q_start", torch.int32), _need(batch.slots, "slots", torch.int32), _need(out, "out", torch.float32),

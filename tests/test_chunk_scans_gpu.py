@@ -1,0 +1,90 @@
+"""The recurrences with one decay per head and token, 32 tokens at a time, against the same in 64 bits token by token: requests whose
+portions end at, before and behind a chunk's edge in one step, decays from 0 to 1, shared query/key heads, states that are not zero.
+
+Sums are fp32 over up to 64 channels and a chunk's triangle of 32, the state's over all tokens: 1e-5 of the largest number, as the scans of eight
+tokens are held to."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+LENS = [300, 1, 31, 32, 33, 64, 95, 5]
+
+
+def _case(seed, N, M, V, lens=LENS):
+    g = torch.Generator().manual_seed(seed)
+    T, starts = sum(lens), [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    slots = list(range(len(lens)))[::-1]
+    r = lambda *shape: torch.randn(*shape, generator=g)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(num_requests=len(lens), num_tokens=T, q_start=i32(starts), slots=i32(slots), positions=i32([j for n in lens for j in range(n)]))
+    return r, T, starts, slots, batch, r(len(lens) + 1, N * 64 * V + 8)
+
+
+def _close(got, want):
+    assert float((got.double().cpu() - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+def _check(got, state, state0, starts, slots, N, V, walk):
+    for s, (lo, hi) in enumerate(zip(starts, starts[1:])):
+        S = state0[slots[s]][:N * 64 * V].double().view(N, 64, V).clone()
+        want = []
+        for t in range(lo, hi):
+            S, o = walk(t, S)
+            want.append(o.reshape(-1))
+        _close(got[lo:hi], torch.stack(want))
+        _close(state[slots[s]][:N * 64 * V], S.reshape(-1))
+    assert torch.equal(state[:, N * 64 * V:].cpu(), state0[:, N * 64 * V:]) and torch.equal(state[-1].cpu(), state0[-1])
+
+
+@pytest.mark.parametrize("N,M,V,decay", [(4, 2, 64, "mild"), (3, 1, 128, "mild"), (2, 2, 64, "strong"), (2, 1, 64, "edges")])
+def test_gated_delta(N, M, V, decay):
+    from forge_b200 import kernels
+    r, T, starts, slots, batch, state0 = _case(N + V, N, M, V)
+    qkv = r(T, 2 * M * 64 + N * V)
+    for m in range(2 * M):
+        x = qkv[:, m * 64:(m + 1) * 64]
+        x /= x.norm(dim=1, keepdim=True) * (8.0 if m < M else 1.0)
+    g = torch.exp(-torch.nn.functional.softplus(r(T, N) + (3.0 if decay == "strong" else -4.0)))
+    if decay == "edges":
+        g[::7], g[3::7] = 0.0, 1.0
+    beta = torch.sigmoid(r(T, N))
+    state, launches = state0.to(DEV), kernels.launch_count()
+    got = kernels.gated_delta_scan(qkv.to(DEV), g.to(DEV), beta.to(DEV), batch, state, N, M, 64, V)
+    assert kernels.launch_count() - launches == 3
+    q, k = (qkv[:, i * M * 64:(i + 1) * M * 64].double().view(T, M, 64).repeat_interleave(N // M, dim=1) for i in range(2))
+    v = qkv[:, 2 * M * 64:].double().view(T, N, V)
+
+    def walk(t, S):
+        S = g[t].double()[:, None, None] * S
+        u = beta[t].double()[:, None] * (v[t] - torch.einsum("nkv,nk->nv", S, k[t]))
+        S = S + k[t][:, :, None] * u[:, None, :]
+        return S, torch.einsum("nkv,nk->nv", S, q[t])
+    _check(got, state, state0, starts, slots, N, V, walk)
+
+
+@pytest.mark.parametrize("kind", ["retention", "lightning"])
+@pytest.mark.parametrize("N,V", [(4, 64), (3, 128)])
+def test_fixed_decay(kind, N, V):
+    from forge_b200 import kernels
+    r, T, starts, slots, batch, state0 = _case(N + V, N, N, V)
+    decay = torch.tensor([0.0, 0.3, 0.97, 1.0])[:N].contiguous()
+    p = r(T, N * (128 + V) + 4) * 0.3
+    q, k, v = p[:, :N * 64].double().view(T, N, 64), p[:, N * 64:N * 128].double().view(T, N, 64), p[:, N * 128:N * (128 + V)].double().view(T, N, V)
+    state, pd, launches = state0.to(DEV), p.to(DEV), kernels.launch_count()
+    if kind == "lightning":
+        got = kernels.lightning_scan(pd, 0, decay.to(DEV), batch, state, N, 64, V)
+        q, k, v = (z * torch.sigmoid(z) for z in (q, k, v))
+    else:
+        got = kernels.retention_scan((pd, 0), (pd, N * 64), (pd, N * 128), batch, None, 0.125, decay.to(DEV), state, N, 64, V)
+        k = k * 0.125
+    assert kernels.launch_count() - launches == 4
+
+    def walk(t, S):
+        S = decay.double()[:, None, None] * S + k[t][:, :, None] * v[t][:, None, :]
+        return S, torch.einsum("nkv,nk->nv", S, q[t])
+    _check(got, state, state0, starts, slots, N, V, walk)
