@@ -326,6 +326,149 @@ head_finish_kernel(const float* __restrict__ o, const float* __restrict__ weight
     }
 }
 
+// Retention for a step in which every request brings one token: a CTA per (request, head) asks for its state first, rotates q and k meanwhile,
+// and norms, gates and stores the head itself.  A row of the state is V / 4 packs of four value channels; thread t holds pack t % CG (CG = V / 4)
+// of the rows t / CG, t / CG + RG, ...; the RG partial sums of an output are added in their order.  Bound by the state's way in and out (64 requests,
+// 64 heads of 64 x 64: 134 MB; the scan of portions with the rotation before and the norm behind it 57 us, 33 us so, 4.1 TB/s).
+constexpr int kRetThreads = 256, kRetHeld = 16;
+bool retention_token_fits(int K, int V) {
+    const int cg = V / 4;
+    return V % 4 == 0 && V > 0 && cg <= 64 && K > 0 && K <= 256 && (K + kRetThreads / cg - 1) / (kRetThreads / cg) <= kRetHeld;
+}
+
+template <int HELD, typename TA>
+__global__ void __launch_bounds__(kRetThreads)
+retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const int32_t* __restrict__ positions, const float* __restrict__ freq, int rot_dims,
+                       float k_scale, const float* __restrict__ decay, float* __restrict__ state, long long state_stride, const int32_t* __restrict__ q_start,
+                       const int32_t* __restrict__ slots, const float* __restrict__ weight, float eps, TA* __restrict__ out, long long out_ld, int N, int K, int V) {
+    __shared__ float qs[256], ks[256], red[8];
+    __shared__ __align__(16) float4 part[kRetThreads];
+    forge::pdl_launch_dependents();
+    forge::pdl_wait();
+    const int s = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, t = q_start[s];
+    const int CG = V / 4, RG = kRetThreads / CG, rg = tid / CG, cp = tid % CG;
+    const bool live = rg < RG;
+    float4* S = reinterpret_cast<float4*>(state + (size_t)slots[s] * state_stride + (size_t)head * K * V);
+    float4 held[HELD];
+#pragma unroll
+    for (int m = 0; m < HELD; ++m) {
+        const int row = rg + m * RG;
+        held[m] = live && row < K ? S[(size_t)row * CG + cp] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float dec = decay[head];
+    float4 vv = make_float4(0.f, 0.f, 0.f, 0.f), gate = vv, w = vv;
+    if (live) {
+        const float* vp = v.p + (size_t)t * v.ld + (size_t)head * V + cp * 4;
+        vv = make_float4(vp[0], vp[1], vp[2], vp[3]);
+    }
+    if (rg == 0) {                                             // what the end needs is asked for now
+        const float* gp = g.p + (size_t)t * g.ld + (size_t)head * V + cp * 4;
+        const float* wp = weight + cp * 4;
+        gate = make_float4(gp[0], gp[1], gp[2], gp[3]);
+        w = make_float4(wp[0], wp[1], wp[2], wp[3]);
+    }
+    const float* qp = q.p + (size_t)t * q.ld + (size_t)head * K;
+    const float* kp = k.p + (size_t)t * k.ld + (size_t)head * K;
+    const int half = rot_dims >> 1;
+    for (int i = tid; i < half; i += kRetThreads) {
+        float sn, cs;
+        sincosf((float)positions[t] * freq[i], &sn, &cs);
+        const float q0 = qp[i], q1 = qp[i + half], k0 = kp[i], k1 = kp[i + half];
+        qs[i] = q0 * cs - q1 * sn;
+        qs[i + half] = q1 * cs + q0 * sn;
+        ks[i] = (k0 * cs - k1 * sn) * k_scale;
+        ks[i + half] = (k1 * cs + k0 * sn) * k_scale;
+    }
+    for (int i = rot_dims + tid; i < K; i += kRetThreads) {
+        qs[i] = qp[i];
+        ks[i] = kp[i] * k_scale;
+    }
+    __syncthreads();
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int m = 0; m < HELD; ++m) {
+        const int row = rg + m * RG;
+        if (!live || row >= K) continue;
+        const float kk = ks[row], qq = qs[row];
+        float4 x = held[m];
+        x.x = fmaf(dec, x.x, kk * vv.x); x.y = fmaf(dec, x.y, kk * vv.y); x.z = fmaf(dec, x.z, kk * vv.z); x.w = fmaf(dec, x.w, kk * vv.w);
+        S[(size_t)row * CG + cp] = x;
+        acc.x = fmaf(qq, x.x, acc.x); acc.y = fmaf(qq, x.y, acc.y); acc.z = fmaf(qq, x.z, acc.z); acc.w = fmaf(qq, x.w, acc.w);
+    }
+    part[tid] = acc;
+    __syncthreads();
+    // the partial sums of a pack, by thread cp of the first CG, in their order
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    float ss = 0.f;
+    if (rg == 0) {
+        o = part[cp];
+        for (int r = 1; r < RG; ++r) {
+            const float4 y = part[r * CG + cp];
+            o.x += y.x; o.y += y.y; o.z += y.z; o.w += y.w;
+        }
+        ss = fmaf(o.x, o.x, fmaf(o.y, o.y, fmaf(o.z, o.z, o.w * o.w)));
+    }
+    ss = forge::warp_sum(ss);                                  // (packs lie in the first 64 threads; the other warps add zeros)
+    if ((tid & 31) == 0) red[tid >> 5] = ss;
+    __syncthreads();
+    if (rg != 0) return;
+    const float inv = 1.0f / sqrtf((red[0] + red[1]) / (float)V + eps);
+    TA* dst = out + (size_t)t * out_ld + (size_t)head * V + cp * 4;
+    dst[0] = forge::from_float<TA>(o.x * inv * w.x * (gate.x * sigmoidf(gate.x)));
+    dst[1] = forge::from_float<TA>(o.y * inv * w.y * (gate.y * sigmoidf(gate.y)));
+    dst[2] = forge::from_float<TA>(o.z * inv * w.z * (gate.z * sigmoidf(gate.z)));
+    dst[3] = forge::from_float<TA>(o.w * inv * w.w * (gate.w * sigmoidf(gate.w)));
+}
+
+// The same for heads of 32, 64 or 128 channels and aligned rows: K / 4 neighbouring lanes a head with four channels each, so that a warp has 4, 2
+// or 1 heads in one load of every operand, and kFinishDeep of them asked for before the first is used.  (2,001 tokens of 2,048 channels: 24 us a
+// channel a load, 14 us so.)
+constexpr int kFinishDeep = 2;
+template <typename TA, int K>
+__global__ void __launch_bounds__(128)
+head_finish_vec_kernel(const float* __restrict__ o, const float* __restrict__ weight, ScanInput g, TA* __restrict__ out, long long heads,
+                       int N, float eps, int act, float scale, int share_w, long long out_ld) {
+    constexpr int kLanes = K / 4, kHeads = 32 / kLanes;
+    forge::pdl_launch_dependents();
+    forge::pdl_wait();
+    const int lane = threadIdx.x & 31, c = lane % kLanes * 4;
+    const long long first = ((long long)blockIdx.x * 4 + (threadIdx.x >> 5)) * (kHeads * kFinishDeep) + lane / kLanes;
+    float4 x[kFinishDeep], gate[kFinishDeep], w[kFinishDeep];
+#pragma unroll
+    for (int i = 0; i < kFinishDeep; ++i) {
+        const long long at = first + i * kHeads;
+        x[i] = gate[i] = w[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (at < heads) {
+            const long long t = at / N;
+            const int head = (int)(at % N);
+            x[i] = *reinterpret_cast<const float4*>(o + at * K + c);
+            w[i] = *reinterpret_cast<const float4*>(weight + (share_w ? c : head * K + c));
+            if (act != 2) gate[i] = *reinterpret_cast<const float4*>(g.p + (size_t)t * g.ld + head * K + c);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kFinishDeep; ++i) {
+        const long long at = first + i * kHeads;
+        float ss = fmaf(x[i].x, x[i].x, fmaf(x[i].y, x[i].y, fmaf(x[i].z, x[i].z, x[i].w * x[i].w)));
+#pragma unroll
+        for (int d = kLanes / 2; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+        if (at >= heads) continue;
+        const float inv = 1.0f / sqrtf(ss / (float)K + eps);
+        auto one = [&](float v, float wv, float gv) {
+            const float f = act == 2 ? scale : scale * (act == 1 ? gv * sigmoidf(gv) : sigmoidf(gv));
+            return v * inv * wv * f;
+        };
+        const float y0 = one(x[i].x, w[i].x, gate[i].x), y1 = one(x[i].y, w[i].y, gate[i].y), y2 = one(x[i].z, w[i].z, gate[i].z), y3 = one(x[i].w, w[i].w, gate[i].w);
+        TA* dst = out + (at / N) * out_ld + (at % N) * K + c;
+        if (sizeof(TA) == 4) {
+            *reinterpret_cast<float4*>(dst) = make_float4(y0, y1, y2, y3);
+        } else {
+            __nv_bfloat162 a = __floats2bfloat162_rn(y0, y1), b = __floats2bfloat162_rn(y2, y3);
+            *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+        }
+    }
+}
+
 // out[t][c] = tanh(in[t][c]) in the activation type (the hidden layer of a low-rank projection).
 template <typename TA>
 __global__ void tanh_rows_kernel(ScanInput in, TA* __restrict__ out, int T, int n) {
@@ -615,6 +758,29 @@ extern "C" int forge_retention_scan(float* q, int ld_q, float* k, int ld_k, cons
     return forge::check_launch("retention_scan", e);
 }
 
+// 1 if forge_retention_token takes heads of these sizes.
+extern "C" int forge_retention_token_supports(int K, int V) { return retention_token_fits(K, V) ? 1 : 0; }
+
+// The same for a step in which every request brings one token (request s's is token q_start[s]), q and k left as they are, with the head's norm (weight fp32
+// [KV], eps) and silu of the gate g (N*KV columns) multiplied on; out rows of out_ld elements.  State rows aligned to 16 bytes.
+extern "C" int forge_retention_token(const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v, const float* g, int ld_g,
+                                     const int32_t* positions, const float* freq, int rot_dims, float k_scale, const float* decay, float* state,
+                                     long long state_stride, const int32_t* q_start, const int32_t* slots, const float* weight, float eps, void* out, int dtype,
+                                     long long out_ld, int S, int N, int K, int V, cudaStream_t stream) {
+    if (S < 0 || N <= 0 || rot_dims < 0 || rot_dims > K || (rot_dims & 1) || (rot_dims > 0 && !freq) || out_ld < (long long)N * V || state_stride < (long long)N * K * V)
+        return forge::fail(FORGE_ERR_ARG, "retention_token: bad sizes S=%d N=%d K=%d V=%d rot=%d", S, N, K, V, rot_dims);
+    if (!retention_token_fits(K, V) || ((uintptr_t)state & 15) || state_stride % 4 || N > 65535)
+        return forge::fail(FORGE_ERR_UNSUPPORTED, "retention_token: heads of %d and %d channels", K, V);
+    if (S == 0) return FORGE_OK;
+    const int rg = kRetThreads / (V / 4), held = (K + rg - 1) / rg;
+    cudaError_t e = cudaSuccess;
+#define FORGE_RET(HELD) FORGE_DISPATCH_DTYPE(dtype, TT, e = forge::launch(retention_token_kernel<HELD, TT>, dim3(S, N), dim3(kRetThreads), 0, stream, 1, ScanInput{q, ld_q}, \
+        ScanInput{k, ld_k}, ScanInput{v, ld_v}, ScanInput{g, ld_g}, positions, freq, rot_dims, k_scale, decay, state, state_stride, q_start, slots, weight, eps, (TT*)out, out_ld, N, K, V))
+    if (held <= 4) FORGE_RET(4); else if (held <= 8) FORGE_RET(8); else FORGE_RET(kRetHeld);
+#undef FORGE_RET
+    return forge::check_launch("retention_token", e);
+}
+
 // Gated linear attention over the step's tokens: decays a = sigmoid(u . w2 + b)^(1/tau) per key channel into `decay` (fp32 [T, N*K]
 // scratch), then S <- diag(a) S + k v^T, out = q_scale S^T q per head.  q, k, v fp32 (row t at p + t * ld, head n's channels at
 // columns n*K .. or n*KV ..); u fp32 rows of ld_u with r hidden numbers; w2t fp32 [r, N*K], b fp32 [N*K]; out fp32 [T, N*KV]; a
@@ -693,8 +859,18 @@ extern "C" int forge_head_finish(const float* o, const float* weight, const floa
     if (T < 0 || N <= 0 || K <= 0 || act < 0 || act > 2 || (act != 2 && !g)) return forge::fail(FORGE_ERR_ARG, "head_finish: bad sizes T=%d N=%d K=%d", T, N, K);
     if (T == 0) return FORGE_OK;
     if ((long long)T * N > 0x7fffffffLL / 2) return forge::fail(FORGE_ERR_UNSUPPORTED, "head_finish: too many rows");
-    const unsigned blocks = (unsigned)(((long long)T * N + 3) / 4);
     cudaError_t e = cudaSuccess;
+    const uintptr_t out_mask = dtype == FORGE_F32 ? 15 : 7;
+    if ((K == 32 || K == 64 || K == 128) && (((uintptr_t)o | (uintptr_t)weight | (uintptr_t)g) & 15) == 0 && (act == 2 || ld_g % 4 == 0) && out_ld % 4 == 0 &&
+        ((uintptr_t)out & out_mask) == 0) {
+        const long long heads = (long long)T * N, per_cta = 4 * (128 / K) * kFinishDeep;
+        const dim3 grid((unsigned)((heads + per_cta - 1) / per_cta));
+#define FORGE_FINISH(KK) FORGE_DISPATCH_DTYPE(dtype, TT, e = forge::launch(head_finish_vec_kernel<TT, KK>, grid, dim3(128), 0, stream, 1, o, weight, ScanInput{g, ld_g}, (TT*)out, heads, N, eps, act, scale, share_w, out_ld))
+        if (K == 32) FORGE_FINISH(32); else if (K == 64) FORGE_FINISH(64); else FORGE_FINISH(128);
+#undef FORGE_FINISH
+        return forge::check_launch("head_finish", e);
+    }
+    const unsigned blocks = (unsigned)(((long long)T * N + 3) / 4);
     FORGE_DISPATCH_DTYPE(dtype, TT,
         e = forge::launch(head_finish_kernel<TT>, dim3(blocks), dim3(128), 0, stream, 1, o, weight, ScanInput{g, ld_g}, (TT*)out, T, N, K,
                           eps, act, scale, share_w, out_ld));

@@ -94,6 +94,8 @@ _SIGNATURES = {
         "forge_gated_delta_token": [_P, _I, _I, _I, _I, _P, _I, _P, _LL, _LL] + [_P] * 6 + [_F, _P, _I, _LL] + [_I] * 5 + [_P],
         "forge_token_state_supports": [_I] * 3,
         "forge_gated_rows": [_P, _P, _P, _I, _P, _I, _LL, _I, _I, _F, _P],
+        "forge_retention_token_supports": [_I, _I],
+        "forge_retention_token": [_P, _I] * 4 + [_P, _P, _I, _F, _P, _P, _LL, _P, _P, _P, _F, _P, _I, _LL, _I, _I, _I, _I, _P],
         "forge_retention_scan": [_P, _I, _P, _I, _P, _I, _P, _P, _I, _F, _P, _P, _LL, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     },
     "latent": {
@@ -1235,6 +1237,29 @@ def retention_scan(q, k, v, batch, freq, k_scale, decay, state, N, K, KV):
         _need(batch.q_start, "q_start", torch.int32), _need(batch.slots, "slots", torch.int32), _need(out, "out", torch.float32),
         _opt(chunks, "chunks", torch.float32), T, batch.num_requests, N, K, KV, _stream()), "retention_scan")
     count_launches(1 if chunks is None else 3)              # the kernel that rotates and scales q and k, in place (and two more chunk by chunk)
+    return out
+
+
+def retention_token_supports(batch, state, K, V):
+    """A step in which every request brings one token, and heads and state rows that the kernel of single tokens takes."""
+    return batch.num_tokens == batch.num_requests and state.shape[1] % 4 == 0 and state.data_ptr() % 16 == 0 and \
+        bool(library("mixers").forge_retention_token_supports.fn(int(K), int(V)))
+
+
+def retention_token(q, k, v, g, batch, freq, k_scale, decay, state, N, K, V, weight, eps, out_dtype):
+    """``retention_scan`` for a step in which every request brings one token, with the heads' norm (``weight`` fp32 [V], eps) and silu of the gate
+    ``g`` ((fp32 matrix, first column), N*V columns) multiplied on; q and k are left as they are.  Returns [T, N*V] in ``out_dtype``."""
+    lib = library("mixers")
+    T = q[0].shape[0]
+    if T != batch.num_requests or weight.numel() != V:
+        raise KernelError(f"retention_token: {T} tokens of {batch.num_requests} requests, {weight.numel()} norm weights for {V} channels")
+    out = new_tensor((T, N * V), out_dtype, q[0].device)
+    rot = 0 if freq is None else 2 * freq.numel()
+    _check(lib, lib.forge_retention_token(
+        *_cols(*q), *_cols(*k), *_cols(*v), *_cols(*g), _need(batch.positions, "positions", torch.int32), _opt(freq, "freq", torch.float32) if rot else None, rot,
+        float(k_scale), _need(decay, "decay", torch.float32), _need(state, "state", torch.float32, 2), state.shape[1],
+        _need(batch.q_start, "q_start", torch.int32), _need(batch.slots, "slots", torch.int32), _need(weight, "weight", torch.float32), float(eps),
+        _need(out, "out", out_dtype), dtype_code(out_dtype), N * V, T, N, K, V, _stream()), "retention_token")
     return out
 
 

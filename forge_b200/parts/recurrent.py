@@ -239,9 +239,12 @@ class RetentionMixer(Part):
         N, K, V = self.num_heads, self.head_dim, self.v_head_dim
         NK, NV = N * K, N * V
         p = self.proj.forward(x)                                     # fp32 [T, 2*N*K + 2*N*V]: q | k | v | g
-        freq = self.position.inv_freq
-        o = kernels.retention_scan((p, 0), (p, NK), (p, 2 * NK), batch, freq if freq.numel() else None, K ** -0.5, self.decay,
-                                   cache.state, N, K, V)
+        freq = self.position.inv_freq if self.position.inv_freq.numel() else None
+        if kernels.retention_token_supports(batch, cache.state, K, V):       # a step of single tokens: one kernel
+            y = kernels.retention_token((p, 0), (p, NK), (p, 2 * NK), (p, 2 * NK + NV), batch, freq, K ** -0.5, self.decay, cache.state, N, K, V, self.ones, self.eps,
+                                        self.rt.dtype)
+            return self.o.forward(y, accumulate_into=residual)
+        o = kernels.retention_scan((p, 0), (p, NK), (p, 2 * NK), batch, freq, K ** -0.5, self.decay, cache.state, N, K, V)
         y = kernels.head_finish(o, self.ones, (p, 2 * NK + NV), N, V, self.eps, "silu", self.rt.dtype)
         return self.o.forward(y, accumulate_into=residual)
 

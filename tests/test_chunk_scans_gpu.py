@@ -88,3 +88,39 @@ def test_fixed_decay(kind, N, V):
         S = decay.double()[:, None, None] * S + k[t][:, :, None] * v[t][:, None, :]
         return S, torch.einsum("nkv,nk->nv", S, q[t])
     _check(got, state, state0, starts, slots, N, V, walk)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K,V,rot", [(3, 64, 64, 64), (2, 10, 20, 4), (2, 256, 64, 128), (1, 64, 256, 0), (5, 33, 4, 32)])
+def test_one_token_of_every_request_in_one_retention_kernel(dtype, N, K, V, rot):
+    """Outputs (normed, weighted, gated) and states of a step of single tokens at unequal positions, slots in any order, inputs that are columns of a
+    wider matrix whose rows no vector load fits: fp32 to 1e-5 of the largest number, bfloat16 to its rounding (2^-9) of it."""
+    from forge_b200 import kernels
+    g = torch.Generator().manual_seed(N + K + V)
+    B, pos, slots = 4, [0, 7, 2, 3001], [4, 0, 5, 2]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(num_requests=B, num_tokens=B, q_start=i32(list(range(B + 1))), slots=i32(slots), positions=i32(pos))
+    p = torch.randn(B, 1 + N * (2 * K + 2 * V), generator=g)
+    state0 = torch.randn(6, -(-N * K * V // 4) * 4, generator=g)
+    decay, weight = torch.rand(N, generator=g), 1.0 + 0.3 * torch.randn(V, generator=g)
+    freq = 10000.0 ** (-torch.arange(rot // 2, dtype=torch.float32) * 2 / max(rot, 1))
+    state = state0.to(DEV)
+    assert kernels.retention_token_supports(batch, state, K, V)
+    cols = [1, 1 + N * K, 1 + 2 * N * K, 1 + N * (2 * K + V)]
+    pd = p.to(DEV)
+    got = kernels.retention_token(*[(pd, c) for c in cols], batch, freq.to(DEV) if rot else None, K ** -0.5, decay.to(DEV), state, N, K, V, weight.to(DEV), 1e-4, dtype)
+    assert torch.equal(pd.cpu(), p)
+    for s in range(B):
+        q, k = (p[s, c:c + N * K].double().view(N, K) for c in cols[:2])
+        v, z = (p[s, c:c + N * V].double().view(N, V) for c in cols[2:])
+        a = pos[s] * freq.double()
+        turn = lambda x: torch.cat([x[:, :rot // 2] * a.cos() - x[:, rot // 2:rot] * a.sin(), x[:, rot // 2:rot] * a.cos() + x[:, :rot // 2] * a.sin(), x[:, rot:]], dim=1)
+        q, k = turn(q), turn(k) * K ** -0.5
+        S = decay.double()[:, None, None] * state0[slots[s], :N * K * V].double().view(N, K, V) + k[:, :, None] * v[:, None, :]
+        o = torch.einsum("nkv,nk->nv", S, q)
+        want = o / torch.sqrt((o * o).mean(dim=1, keepdim=True) + 1e-4) * weight.double() * z * torch.sigmoid(z)
+        tol = 2e-4 if pos[s] > 1000 else 1e-5                    # (an fp32 angle of some thousand errs by 2^-13 of a turn's unit)
+        assert float((got[s].double().cpu() - want.reshape(-1)).abs().max()) <= (tol if dtype == torch.float32 else 2.0 ** -8) * float(want.abs().max())
+        assert float((state[slots[s], :N * K * V].double().cpu() - S.reshape(-1)).abs().max()) <= tol * float(S.abs().max())
+    for s in (1, 3):
+        assert torch.equal(state[s].cpu(), state0[s])
