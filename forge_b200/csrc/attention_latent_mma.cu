@@ -277,47 +277,43 @@ latent_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __re
     }
 }
 
-// A warp per (token, head): run s counts with 2^(m_s - m); the sums of all runs over the sum of their weights' sums.
+// A warp per (token, head) and 128 channels: run s counts with 2^(m_s - m); the sums of all runs over the sum of their weights' sums.  A lane has a
+// run's maximum and sum and every lane four channels of all runs, asked for at once (one memory latency instead of the runs' one after the other:
+// 16 runs, 16 x 32 heads of 256 channels 7.6 us).
 __global__ void __launch_bounds__(128)
 latent_combine_kernel(const float* __restrict__ u, const float* __restrict__ part_ml, int nsplit, __nv_bfloat16* __restrict__ out, int rows, int C,
                       const float* __restrict__ sink, int H) {
     constexpr int kMaxSplit = 16;
     forge::pdl_launch_dependents();
     forge::pdl_wait();
-    const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, c = (blockIdx.y * 32 + lane) * 4;
     if (w >= rows) return;
-    float wt[kMaxSplit];
-    float m = -INFINITY;
-    for (int s = 0; s < nsplit; ++s) m = fmaxf(m, part_ml[((size_t)s * rows + w) * 2]);
-    float l = 0.f;
+    float4 part[kMaxSplit];
 #pragma unroll
-    for (int s = 0; s < kMaxSplit; ++s) {
-        wt[s] = 0.f;
-        if (s < nsplit) {
-            const float ms = part_ml[((size_t)s * rows + w) * 2];
-            wt[s] = ms == -INFINITY ? 0.f : ex2(ms - m);
-            l += wt[s] * part_ml[((size_t)s * rows + w) * 2 + 1];
-        }
-    }
+    for (int s = 0; s < kMaxSplit; ++s)
+        if (s < nsplit && c < C) part[s] = *reinterpret_cast<const float4*>(u + ((size_t)s * rows + w) * C + c);
+    float2 ml = make_float2(-INFINITY, 0.f);
+    if (lane < nsplit) ml = *reinterpret_cast<const float2*>(part_ml + ((size_t)lane * rows + w) * 2);
+    float m = ml.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float weight = ml.x == -INFINITY ? 0.f : ex2(ml.x - m);
+    float l = forge::warp_sum(weight * ml.y);
     if (sink != nullptr && l > 0.f) l += ex2(sink[w % H] * 1.4426950408889634f - m);      // the sink's weight in the denominator
     const float inv = l > 0.f ? 1.0f / l : 0.f;
-    // four channels a load (C is a multiple of 16), all runs' loads of a channel group in flight together
-    for (int c = lane * 4; c < C; c += 128) {
-        float4 part[kMaxSplit];
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int s = 0; s < kMaxSplit; ++s)
-            if (s < nsplit && wt[s] != 0.f) part[s] = *reinterpret_cast<const float4*>(u + ((size_t)s * rows + w) * C + c);
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int s = 0; s < kMaxSplit; ++s)
-            if (s < nsplit && wt[s] != 0.f) {
-                a.x = fmaf(wt[s], part[s].x, a.x); a.y = fmaf(wt[s], part[s].y, a.y);
-                a.z = fmaf(wt[s], part[s].z, a.z); a.w = fmaf(wt[s], part[s].w, a.w);
-            }
-        __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out + (size_t)w * C + c);
-        o[0] = __floats2bfloat162_rn(a.x * inv, a.y * inv);
-        o[1] = __floats2bfloat162_rn(a.z * inv, a.w * inv);
+    for (int s = 0; s < kMaxSplit; ++s) {
+        const float x = __shfl_sync(0xffffffffu, weight, s);
+        if (s < nsplit && x != 0.f) {
+            a.x = fmaf(x, part[s].x, a.x); a.y = fmaf(x, part[s].y, a.y);
+            a.z = fmaf(x, part[s].z, a.z); a.w = fmaf(x, part[s].w, a.w);
+        }
     }
+    if (c >= C) return;
+    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out + (size_t)w * C + c);
+    o[0] = __floats2bfloat162_rn(a.x * inv, a.y * inv);
+    o[1] = __floats2bfloat162_rn(a.z * inv, a.w * inv);
 }
 
 forge::PerDeviceFlag g_attr_done[6];
@@ -396,7 +392,7 @@ extern "C" int forge_latent_attention_mma(const void* q, const void* cache, cons
 #undef FORGE_LATENT_ARGS
     if (rc != FORGE_OK || nsplit == 1) return rc;
     const unsigned blocks = (unsigned)(((size_t)T * H + 3) / 4);
-    return forge::check_launch("latent_combine", forge::launch(latent_combine_kernel, dim3(blocks), dim3(128), 0, stream, 1, (const float*)u,
+    return forge::check_launch("latent_combine", forge::launch(latent_combine_kernel, dim3(blocks, (C + 127) / 128), dim3(128), 0, stream, 1, (const float*)u,
                                                                (const float*)part_ml, nsplit, ob, T * H, C, sink, H));
 }
 
