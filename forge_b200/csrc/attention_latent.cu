@@ -253,7 +253,9 @@ head_linear_mma_kernel(const TI* __restrict__ in, long long in_ld, int in_hs, co
 // (converted once; the kernel above reads and converts them again for every 64 output channels) and walks the output channels in chunks of
 // 64, W_h in pieces of [128 x 64] through a ring of three (cp.async); a warp has 32 tokens x 32 channels, results leave through shared
 // memory as rows of 128 bytes.  Bound by shared memory's bandwidth and by the results' way out (1,536 tokens, 32 heads, 128 -> 512 + 64
-// channels: 38 MB in, 57 MB out).  Where tokens and heads leave SMs idle several CTAs share a tile's output channels.
+// channels: 38 MB in, 57 MB out; 74 us, with the rotated channels' loads four at a
+// time 66, with the CTAs dealt out by rounds 56).  Several CTAs share a tile's output channels where that
+// fills the SMs better.
 constexpr int kHltThreads = 256, kHltTokens = 128, kHltN = 64, kHltRing = 3, kHltMaxK = 512;
 constexpr int kHltPiece = kHlmK * kHlmRow;                                 // elements of a staged piece of W
 size_t hlt_smem(int K) { return sizeof(__nv_bfloat16) * ((size_t)kHltTokens * ((K + 15) / 16 * 16 + 8) + kHltRing * kHltPiece + kHltTokens * kHlmRow); }
@@ -361,18 +363,30 @@ head_linear_tile_kernel(const TI* __restrict__ in, long long in_ld, int in_hs, c
         }
     }
     if (R > 0 && blockIdx.z == 0) {
-        for (int i = threadIdx.x; i < nt * (R >> 1); i += kHltThreads) {
-            const int tt = i / (R >> 1), p = i % (R >> 1);
-            const TI* src = in + (size_t)(t0 + tt) * in_ld + (size_t)h * in_hs + K;
-            float sn, cs;
-            sincosf((float)positions[t0 + tt] * freq[p], &sn, &cs);
-            sn *= amp;
-            cs *= amp;
-            const int a = pair_first(p, halves), b = pair_second(p, R, halves);
-            const float u = forge::to_float(src[a]), v = forge::to_float(src[b]);
-            __nv_bfloat16* dst = out + (size_t)(t0 + tt) * out_ld + (size_t)h * out_hs + N;
-            dst[a] = __float2bfloat16(u * cs - v * sn);
-            dst[b] = __float2bfloat16(v * cs + u * sn);
+        constexpr int kAhead = 4;                                          // pairs of channels whose loads are in flight together
+        const int pairs = nt * (R >> 1);
+        for (int i0 = threadIdx.x; i0 < pairs; i0 += kAhead * kHltThreads) {
+            float u[kAhead], v[kAhead], angle[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const int i = min(i0 + j * kHltThreads, pairs - 1), tt = i / (R >> 1), p = i % (R >> 1);
+                const TI* src = in + (size_t)(t0 + tt) * in_ld + (size_t)h * in_hs + K;
+                u[j] = forge::to_float(src[pair_first(p, halves)]);
+                v[j] = forge::to_float(src[pair_second(p, R, halves)]);
+                angle[j] = (float)positions[t0 + tt] * freq[p];
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const int i = i0 + j * kHltThreads, tt = i / (R >> 1), p = i % (R >> 1);
+                if (i >= pairs) break;
+                float sn, cs;
+                sincosf(angle[j], &sn, &cs);
+                sn *= amp;
+                cs *= amp;
+                __nv_bfloat16* dst = out + (size_t)(t0 + tt) * out_ld + (size_t)h * out_hs + N;
+                dst[pair_first(p, halves)] = __float2bfloat16(u[j] * cs - v[j] * sn);
+                dst[pair_second(p, R, halves)] = __float2bfloat16(v[j] * cs + u[j] * sn);
+            }
         }
     }
 }
@@ -388,10 +402,17 @@ cudaError_t launch_head_linear_tile(cudaStream_t stream, const TI* in, long long
         if (e != cudaSuccess) return e;
         done = true;
     }
-    const int tiles = (T + kHltTokens - 1) / kHltTokens, chunks = (N + kHltN - 1) / kHltN;
-    int share = 1;                                                         // CTAs a tile: until two an SM have work
-    while (share < chunks && (long long)tiles * H * share < 296) ++share;
-    return forge::launch(head_linear_tile_kernel<TI>, dim3(tiles, H, share), dim3(kHltThreads), hlt_smem(K), stream, 1, in, in_ld, in_hs, W, out, out_ld, out_hs,
+    // CTAs a tile: the fewest rounds of output chunks on the busiest SM, where every CTA brings its tile's tokens first (as long as a chunk and a
+    // half of 128 channels takes)
+    const long long tiles = (long long)((T + kHltTokens - 1) / kHltTokens) * H;
+    const int chunks = (N + kHltN - 1) / kHltN, slots = 148 * (hlt_smem(K) + 1024 <= 114 * 1024 ? 2 : 1);
+    int share = 1;
+    long long best = -1;
+    for (int c = 1; c <= chunks && c <= 16; ++c) {
+        const long long cost = (tiles * c + slots - 1) / slots * (2 * ((chunks + c - 1) / c) + 3);
+        if (best < 0 || cost < best) { best = cost; share = c; }
+    }
+    return forge::launch(head_linear_tile_kernel<TI>, dim3((T + kHltTokens - 1) / kHltTokens, H, share), dim3(kHltThreads), hlt_smem(K), stream, 1, in, in_ld, in_hs, W, out, out_ld, out_hs,
                          positions, freq, amp, T, K, N, R, gate, gate_ld, gate_hs, gate_cs, halves);
 }
 
