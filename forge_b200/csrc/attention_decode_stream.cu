@@ -534,9 +534,12 @@ extern "C" int forge_decode_attention_stream(const float* qkv, void* kv, void* o
     }
     if (p.ksplit > 1) return launch_stream<kFew, kFew, true>(tkv, p, S, NKV, stream);
     if (few) return launch_stream<kFew, kFew, false>(tkv, p, S, NKV, stream);
-    p.longest_first = S <= kSortRequests ? 1 : 0;
-    // (heads of 128: a ring of four tiles is 128 KB, one CTA an SM like the ring of six)
-    return HD == 128 ? launch_stream<kFew, kFew, false>(tkv, p, S, NKV, stream) : launch_stream<4, 4, false>(tkv, p, S, NKV, stream);
+    // The order matters where more CTAs wait than run at once (three an SM, with heads of 128 one) and requests may be many tiles long; looking it up
+    // takes a CTA about a microsecond, which a step of short contexts (35 us and less for a whole layer) would only lose.
+    // (heads of 128: a ring of four tiles is 128 KB, one CTA an SM like the ring of six, which short contexts do not fill)
+    const bool may_be_long = max_context <= 0 || max_context >= 1024;
+    p.longest_first = may_be_long && S <= kSortRequests && (long)S * NKV > (long)sms * (HD == 128 ? 1 : 3) ? 1 : 0;
+    return HD == 128 && may_be_long ? launch_stream<kFew, kFew, false>(tkv, p, S, NKV, stream) : launch_stream<4, 4, false>(tkv, p, S, NKV, stream);
 }
 
 // (checks build) the bounds that this file's kernel tests page ids and slots against

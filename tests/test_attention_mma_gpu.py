@@ -130,13 +130,13 @@ def test_decode_step_in_one_kernel(nh, nkv, hd, ps, window, rotary):
             assert (work.float() - cache_ref.float()).abs().max() <= 1e-2 * cache_ref.float().abs().max()   # k, v landed in their slots
 
 
-@pytest.mark.parametrize("hd,ps", [(64, 16), (128, 32)])
+@pytest.mark.parametrize("hd,ps,nkv", [(64, 16, 4), (128, 32, 2)])
 @pytest.mark.parametrize("window", [0, 70])
 @pytest.mark.parametrize("requests", [80, 128, 129])
-def test_decode_step_of_more_pairs_than_sms_takes_the_longest_first(hd, ps, window, requests):
+def test_decode_step_of_more_pairs_than_run_takes_the_longest_first(hd, ps, nkv, window, requests):
     """Every (request, kv head) once, whatever the order of the requests' lengths, with equal ones among them; the order ends at 128 requests."""
     from forge_b200 import kernels as k
-    nh, nkv = 4, 2
+    nh = 4
     ctxs = [(37 * i) % 211 for i in range(requests - 3)] + [1000, 63, 64]
     q, cache, group, batch, tok_req, positions = make_case(nh, nkv, hd, ps, [(c, 1) for c in ctxs], seed=5)
     qkv = torch.randn(requests, (nh + 2 * nkv) * hd, generator=torch.Generator().manual_seed(1)).to(q.device)
@@ -144,9 +144,10 @@ def test_decode_step_of_more_pairs_than_sms_takes_the_longest_first(hd, ps, wind
     q_ref, cache_ref = R.rope_kv_write_ref(qkv, positions, slots, cache, nh, nkv, hd, ps, 1e4, True)
     cache_ref = cache_ref.to(torch.bfloat16)
     ref = R.paged_attention_ref(q_ref.to(torch.bfloat16), cache_ref, group.block_table, tok_req, positions, nh, nkv, hd, ps, window)
-    got = k.decode_attention_stream(qkv, cache, group.block_table, positions, slots, nh, nkv, hd, ps, 1e4, window=window).float()
-    k.check_kernel_status()
-    assert float((got - ref).abs().max()) <= 1e-2 * float(ref.abs().max())
+    for max_context in (0, 512):                               # 512: short contexts, the order of the requests and the small ring
+        got = k.decode_attention_stream(qkv, cache, group.block_table, positions, slots, nh, nkv, hd, ps, 1e4, window=window, max_context=max_context).float()
+        k.check_kernel_status()
+        assert float((got - ref).abs().max()) <= 1e-2 * float(ref.abs().max())
     assert (cache.float() - cache_ref.float()).abs().max() <= 1e-2 * cache_ref.float().abs().max()
 
 
