@@ -90,21 +90,18 @@ scored_prepare_kernel(const float* __restrict__ proj, int ld, const int32_t* __r
             vbase[((size_t)(idx / E) * page_size + off) * E + idx % E] = forge::from_float<TC>(row[QW + KW + idx]);
 }
 
-// The same four channels at a time, for sizes and rows of a multiple of four that are aligned to 16 bytes: the token's sines and cosines once for all
+// The same four channels at a time, for prompts in bfloat16 with sizes and rows of a multiple of four that are aligned to 16 bytes: the token's sines and cosines once for all
 // its units (one of each for every channel, above, was most of the kernel: 2,048 tokens of 2,048 + 256 + 256 channels 24.6 us, 12.6 us so).
 constexpr int kPrepAngles = 128;
-template <typename TC> __device__ __forceinline__ void store4(TC* p, const float (&v)[4]);
-template <> __device__ __forceinline__ void store4<float>(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
-template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, const float (&v)[4]) {
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
     const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
-template <typename TC>
 __global__ void __launch_bounds__(kPrepThreads)
 scored_prepare_vec_kernel(const float* __restrict__ proj, int ld, const int32_t* __restrict__ positions,
                           const int32_t* __restrict__ slot_mapping, const float* __restrict__ inv_freq,
-                          const float* __restrict__ q_norm, const float* __restrict__ k_norm, TC* __restrict__ q_out,
-                          TC* __restrict__ cache, int QU, int KU, int G, int D, int E, int rot_dims, float eps, float temp_coef,
+                          const float* __restrict__ q_norm, const float* __restrict__ k_norm, __nv_bfloat16* __restrict__ q_out,
+                          __nv_bfloat16* __restrict__ cache, int QU, int KU, int G, int D, int E, int rot_dims, float eps, float temp_coef,
                           float temp_every, int page_size, long long page_stride) {
     __shared__ float red[32];
     __shared__ __align__(16) float sn[kPrepAngles], cs[kPrepAngles];
@@ -117,8 +114,8 @@ scored_prepare_vec_kernel(const float* __restrict__ proj, int ld, const int32_t*
     const bool store = slot >= 0 && FORGE_SLOT_OK(slot);
     const int page = store ? slot / page_size : 0, off = store ? slot % page_size : 0;
     const int QW = QU * D, KW = KU * D, KD = KW / G, half = rot_dims >> 1;
-    TC* kbase = cache + (size_t)page * page_stride;
-    TC* vbase = kbase + (size_t)G * page_size * KD;
+    __nv_bfloat16* kbase = cache + (size_t)page * page_stride;
+    __nv_bfloat16* vbase = kbase + (size_t)G * page_size * KD;
     for (int i = threadIdx.x; i < half; i += kPrepThreads) sincosf(pos * inv_freq[i], &sn[i], &cs[i]);
     auto inverse = [&](const float* x, int n) {
         float ss = 0.f;
@@ -141,7 +138,7 @@ scored_prepare_vec_kernel(const float* __restrict__ proj, int ld, const int32_t*
             v[0] = v[0] * inv * y.x; v[1] = v[1] * inv * y.y; v[2] = v[2] * inv * y.z; v[3] = v[3] * inv * y.w;
         }
     };
-    const int first = (blockIdx.y * kPrepThreads + threadIdx.x) * 4, step = gridDim.y * kPrepThreads * 4;
+    const int first = threadIdx.x * 4, step = kPrepThreads * 4;
 #pragma unroll 2
     for (int idx = first; idx < QW + KW; idx += step) {
         const int d = idx % D;
@@ -159,17 +156,17 @@ scored_prepare_vec_kernel(const float* __restrict__ proj, int ld, const int32_t*
         if (idx < QW) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) x[i] *= temp;
-            store4<TC>(q_out + (size_t)t * QW + idx, x);
+            store4(q_out + (size_t)t * QW + idx, x);
         } else if (store) {
             const int c = idx - QW;
-            store4<TC>(kbase + ((size_t)(c / KD) * page_size + off) * KD + c % KD, x);
+            store4(kbase + ((size_t)(c / KD) * page_size + off) * KD + c % KD, x);
         }
     }
     if (store)
         for (int idx = first; idx < G * E; idx += step) {
             const float4 v = *reinterpret_cast<const float4*>(row + QW + KW + idx);
             const float x[4] = {v.x, v.y, v.z, v.w};
-            store4<TC>(vbase + ((size_t)(idx / E) * page_size + off) * E + idx % E, x);
+            store4(vbase + ((size_t)(idx / E) * page_size + off) * E + idx % E, x);
         }
 }
 
@@ -434,14 +431,14 @@ extern "C" int forge_scored_prepare(const float* proj, int ld, const int32_t* po
         return forge::fail(FORGE_ERR_ARG, "scored_prepare: pages are too small");
     if (T == 0) return FORGE_OK;
     cudaError_t e = cudaSuccess;
-    // (a norm's sum takes another order there: sizes and alignment decide, never the step)
+    // Four channels at a time for prompts in bfloat16.  A step of few tokens is faster with one channel a thread of several CTAs a token (2 requests of 16
+    // heads, two maps of 64: the layer 29.8 us, with four channels 30.7), and in 32 bits a token's numbers may not depend on its step: a norm's
+    // sum takes another order here.
     const uintptr_t at = (uintptr_t)proj | (uintptr_t)q_norm | (uintptr_t)k_norm, to = (uintptr_t)q_out | (uintptr_t)cache;
-    if (D % 4 == 0 && E % 4 == 0 && rot_dims % 8 == 0 && rot_dims / 2 <= kPrepAngles && ld % 4 == 0 && page_stride % 4 == 0 && (at & 15) == 0 &&
-        (to & (dtype == FORGE_F32 ? 15 : 7)) == 0) {
-        FORGE_DISPATCH_DTYPE(dtype, TT,
-            e = forge::launch(scored_prepare_vec_kernel<TT>, dim3(T, T >= 256 ? 1 : min(4, ((QU + KU) * D + 2047) / 2048)), dim3(kPrepThreads), 0, stream, 1, proj, ld,
-                              positions, slot_mapping, inv_freq, q_norm, k_norm, (TT*)q_out, (TT*)cache, QU, KU, G, D, E, rot_dims, eps, temp_coef,
-                              temp_every, page_size, page_stride));
+    if (dtype == FORGE_BF16 && T >= 256 && D % 4 == 0 && E % 4 == 0 && rot_dims % 8 == 0 && rot_dims / 2 <= kPrepAngles && ld % 4 == 0 && page_stride % 4 == 0 &&
+        (at & 15) == 0 && (to & 7) == 0) {
+        e = forge::launch(scored_prepare_vec_kernel, dim3(T), dim3(kPrepThreads), 0, stream, 1, proj, ld, positions, slot_mapping, inv_freq, q_norm, k_norm,
+                          (__nv_bfloat16*)q_out, (__nv_bfloat16*)cache, QU, KU, G, D, E, rot_dims, eps, temp_coef, temp_every, page_size, page_stride);
         return forge::check_launch("scored_prepare", e);
     }
     FORGE_DISPATCH_DTYPE(dtype, TT,

@@ -8,7 +8,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("T", [1, 9, 300])
+@pytest.mark.parametrize("T", [1, 255, 256, 300])
 @pytest.mark.parametrize("H,G,M,D,E,rot,norm,temp", [(4, 2, 2, 64, 64, 64, True, 0.0), (16, 2, 2, 64, 128, 16, False, 0.1), (2, 1, 1, 4, 4, 0, True, 0.0),
                                                      (3, 3, 1, 256, 12, 256, True, 0.2), (1, 1, 2, 20, 8, 8, False, 0.0)])
 def test_four_channels_at_a_time(H, G, M, D, E, rot, norm, temp, T, dtype):
