@@ -71,6 +71,97 @@ latent_prepare_kernel(const float* __restrict__ proj, int ld, const int32_t* __r
     }
 }
 
+// What the attention over spelled-out keys and values reads beside them, in one launch: the queries of a step (fp32 [T, ld], a head's D unrotated
+// and R rotated channels side by side) rounded to bfloat16, their last R channels rotated, a CTA a token; and the step's latent rows out of
+// their pages, packed request behind request (request s from row row_start[s] on), c [rows, C] and kr [rows, R], a warp a row.  Bound by memory:
+// 1,536 tokens of 32 heads of 128 + 64 and 2,236 rows of 512 + 64 are 62 MB.
+constexpr int kExpandThreads = 256;
+__global__ void __launch_bounds__(kExpandThreads)
+latent_expand_kernel(const float* __restrict__ q, long long ld, const int32_t* __restrict__ positions, const float* __restrict__ freq, float amp, int halves,
+                     __nv_bfloat16* __restrict__ q_out, int T, int H, int D, int R, const __nv_bfloat16* __restrict__ cache,
+                     const int32_t* __restrict__ block_table, int max_pages, int page_size, const int32_t* __restrict__ row_start, int S, int rows, int C,
+                     __nv_bfloat16* __restrict__ c_out, __nv_bfloat16* __restrict__ kr_out) {
+    __shared__ float2 turn[64];                                 // (cos, sin) of the token's position, R <= 128
+    forge::pdl_launch_dependents();
+    if ((int)blockIdx.x < T) {
+        const int t = blockIdx.x;
+        if ((int)threadIdx.x < (R >> 1)) {                      // (positions and frequencies were there before the step's first kernel)
+            float sn, cs;
+            sincosf((float)positions[t] * freq[threadIdx.x], &sn, &cs);
+            turn[threadIdx.x] = make_float2(cs * amp, sn * amp);
+        }
+        __syncthreads();
+        forge::pdl_wait();
+        const int width = D + R, pieces = width >> 3;           // (D and R are multiples of 16)
+        const float* src = q + (size_t)t * ld;
+        __nv_bfloat16* dst = q_out + (size_t)t * H * width;
+        const bool vec = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+        auto load4 = [&](const float* p, float* v) {
+            if (vec) {
+                const float4 x = *reinterpret_cast<const float4*>(p);
+                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = p[i];
+            }
+        };
+        for (int i = threadIdx.x; i < H * pieces; i += kExpandThreads) {
+            const int h = i / pieces, c = (i - h * pieces) << 3;
+            const float* s = src + (size_t)h * width + c;
+            float v[8];
+            load4(s, v);
+            load4(s + 4, v + 4);
+            if (c >= D) {
+                const int r = c - D, half = R >> 1;
+                if (!halves) {
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) {
+                        const float2 w = turn[(r + e) >> 1];
+                        const float a = v[e], b = v[e + 1];
+                        v[e] = a * w.x - b * w.y;
+                        v[e + 1] = b * w.x + a * w.y;
+                    }
+                } else {                                        // (R a multiple of 16: a piece of eight lies in one half)
+                    const bool first = r < half;
+                    const float* other = first ? s + half : s - half;
+                    float o[8];
+                    load4(other, o);
+                    load4(other + 4, o + 4);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float2 w = turn[first ? r + e : r + e - half];
+                        v[e] = first ? v[e] * w.x - o[e] * w.y : v[e] * w.x + o[e] * w.y;
+                    }
+                }
+            }
+            *reinterpret_cast<uint4*>(dst + (size_t)h * width + c) =
+                make_uint4(mma_sync::pack_bf16(v[0], v[1]), mma_sync::pack_bf16(v[2], v[3]), mma_sync::pack_bf16(v[4], v[5]), mma_sync::pack_bf16(v[6], v[7]));
+        }
+        return;
+    }
+    forge::pdl_wait();
+    const int lane = threadIdx.x & 31, n = ((int)blockIdx.x - T) * (kExpandThreads / 32) + (threadIdx.x >> 5);
+    if (n >= rows) return;
+    int lo = 0, hi = S - 1;                                     // the last request that begins at or before row n
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (row_start[mid] <= n) lo = mid;
+        else hi = mid - 1;
+    }
+    const int j = n - row_start[lo], idx = j / page_size;
+    int page = idx < max_pages ? block_table[(size_t)lo * max_pages + idx] : -1;
+    if (page >= 0 && !FORGE_PAGE_OK(page)) page = -1;
+    const uint4* src = page < 0 ? nullptr : reinterpret_cast<const uint4*>(cache + ((size_t)page * page_size + j % page_size) * (C + R));
+    uint4* c_dst = reinterpret_cast<uint4*>(c_out + (size_t)n * C);
+    uint4* r_dst = reinterpret_cast<uint4*>(kr_out + (size_t)n * R);
+    const int c_pieces = C >> 3, all = (C + R) >> 3;
+    for (int i = lane; i < all; i += 32) {
+        const uint4 v = src ? src[i] : make_uint4(0, 0, 0, 0);
+        if (i < c_pieces) c_dst[i] = v;
+        else r_dst[i - c_pieces] = v;
+    }
+}
+
 constexpr int kLinThreads = 128, kLinTokens = 8;
 
 // One CTA per (8 tokens, head, 128 output channels).  in: row t, head h at in + t * in_ld + h * in_hs (K channels, then R
@@ -558,6 +649,23 @@ extern "C" int forge_latent_prepare(const float* proj, int ld, const int32_t* po
         e = forge::launch(latent_prepare_kernel<TT>, dim3(T), dim3(kPrepThreads), 0, stream, 1, proj, ld, positions, slot_mapping, freq, amp, wq,
                           wc, (TT*)cq_out, (TT*)cache, Cq, C, R, eps, halves));
     return forge::check_launch("latent_prepare", e);
+}
+
+// q fp32, row t at q + t * ld, a head's D + R channels side by side; q_out bf16 [T, H, D+R]; cache bf16 pages of page_size rows of C + R;
+// row_start int32 [S]; c_out bf16 [rows, C], kr_out bf16 [rows, R].  D, C multiples of 8, R of 16 up to 128, 16-byte aligned cache and outputs.
+extern "C" int forge_latent_expand(const float* q, long long ld, const int32_t* positions, const float* freq, float amp, int halves, void* q_out, int T, int H,
+                                   int D, int R, const void* cache, const int32_t* block_table, int max_pages, int page_size, const int32_t* row_start, int S,
+                                   int rows, int C, void* c_out, void* kr_out, cudaStream_t stream) {
+    if (T < 0 || H <= 0 || D <= 0 || D % 8 || R <= 0 || R % 16 || R > 128 || C <= 0 || C % 8 || ld < (long long)H * (D + R) || S <= 0 || rows <= 0 || page_size <= 0 ||
+        max_pages <= 0 || !positions || !freq || !row_start || !block_table)
+        return forge::fail(FORGE_ERR_ARG, "latent_expand: bad arguments");
+    if ((((uintptr_t)cache | (uintptr_t)q_out | (uintptr_t)c_out | (uintptr_t)kr_out) & 15) || ((uintptr_t)q & 3))
+        return forge::fail(FORGE_ERR_ARG, "latent_expand: 16-byte aligned rows are wanted");
+    if (T == 0) return FORGE_OK;
+    const long long ctas = T + ((long long)rows + kExpandThreads / 32 - 1) / (kExpandThreads / 32);
+    return forge::check_launch("latent_expand", forge::launch(latent_expand_kernel, dim3((unsigned)ctas), dim3(kExpandThreads), 0, stream, 1, q, ld, positions, freq, amp,
+                                                              halves, (__nv_bfloat16*)q_out, T, H, D, R, (const __nv_bfloat16*)cache, block_table, max_pages,
+                                                              page_size, row_start, S, rows, C, (__nv_bfloat16*)c_out, (__nv_bfloat16*)kr_out));
 }
 
 // out[t, h, 0:N] = sum_k in[t, h, k] W[h, k, n], and (R > 0) out[t, h, N:N+R] = in[t, h, K:K+R] rotated by positions[t].

@@ -16,6 +16,10 @@
 // there the 256 channels that meet the value blocks lie in TMEM (128 columns beside S and O: the A operand may come from there), and two
 // tiles fit.  With values of up to 128 channels two CTAs fit an SM.
 //
+// A third reading of the operands serves latent rows whose keys and values a product has spelled out for every head (forge_expanded_attention_sm100):
+// they lie packed, request behind request, [rows, H, D + E], beside the rotated part [rows, R] that all heads share; a tile is 128 tokens of
+// one head, the scores take D + R channels instead of C + R and the outputs E instead of C.
+//
 // Warps 0-3 run one thread each (copies, P V, Q K^T), warps 4-7 are the rows; registers change hands with setmaxnreg.  Where one CTA fills an
 // SM its four warps of rows would leave the SM waiting for their chains (a tile's softmax is one, and no second CTA's runs beside it): there
 // warps 4-11 are the rows, two threads a row with 32 of a tile's keys each, which meet once a tile over the row's maximum.  Every wait is bounded.
@@ -47,6 +51,7 @@ struct ShapedParams {
     int key_blocks, value_blocks;     // blocks of 64 channels of the two kinds
     int k_boxed, v_boxed;             // blocks that one copy of a tile of keys (values) brings: all, where a page holds a whole tile, else one
     int latent;                       // the value blocks are key blocks too
+    const int32_t* row_start;         // (packed keys and values) a request's first row, else null
     int q_tmem;                       // ... and the query channels that meet them are in TMEM, not in shared memory
     int stages, page_size, box_rows, max_pages, window, chunk, vec_out;
     float scale, softcap, out_scale;
@@ -208,7 +213,10 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         const int ppt = p.page_size >= BKV ? 1 : BKV / p.page_size;       // boxes a tile and block
         const int row0 = group * p.page_size, k_col0 = p.latent ? 0 : mp * p.D;
         const int skip = p.latent ? vc * p.value_blocks : 1 << 20;        // key block i stands for channel block i, or i + value_blocks from here on
-        const int others = p.latent ? (chunks - 1) * p.value_blocks : 0;  // key blocks that are the other chunk's value blocks: they come like them
+        const bool packed = p.row_start != nullptr;
+        // key blocks that are the other chunk's value blocks (packed: the head's own blocks of keys): they come like them
+        const int others = p.latent ? (chunks - 1) * p.value_blocks : packed ? p.D / 64 : 0;
+        const int head_blocks = packed ? group * ((p.D + p.E) / 64) : 0, packed_row0 = packed ? p.row_start[req] : 0;
         if (lane == 0) {
             mbar_arrive_expect_tx(q_full, q_blocks * q_rows * 128);
             for (int b = 0; b < q_blocks; ++b)
@@ -223,11 +231,12 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             if (lane < ppt) {
                 const int j = j0 + lane * p.box_rows;
                 const int idx = j / p.page_size;
-                if (j <= pos_last && j + p.box_rows > seen_from && idx < p.max_pages) page = table[idx];
-                if (page >= 0 && !FORGE_PAGE_OK(page)) page = -1;
+                if (packed) page = 0;                                     // (rows behind the request's are another's, or fill: masked, and cleared below)
+                else if (j <= pos_last && j + p.box_rows > seen_from && idx < p.max_pages) page = table[idx];
+                if (page >= 0 && !packed && !FORGE_PAGE_OK(page)) page = -1;
             }
             const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0));
-            const int off = p.page_size > BKV ? j0 % p.page_size : 0;
+            const int row = packed ? packed_row0 + j0 : row0 + (p.page_size > BKV ? j0 % p.page_size : 0);
             const bool last = j0 + BKV - 1 > pos_last;                    // rows behind the last token: cleared below
             uint8_t* kd = k_s + st * p.key_blocks * kBlock;
             uint8_t* vd = v_s + st * p.value_blocks * kBlock;
@@ -243,10 +252,10 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 if (page >= 0) {
                     uint8_t* dst = kd + lane * box_bytes;
                     for (int b = 0; b < others; b += p.v_boxed)
-                        tma_load_4d(dst + b * kBlock, &tmap_v, &k_full[st], 0, row0 + off, b < skip ? b : b + p.value_blocks, page);
+                        tma_load_4d(dst + b * kBlock, &tmap_v, &k_full[st], 0, row, head_blocks + (b < skip ? b : b + p.value_blocks), page);
                     for (int b = others; b < p.key_blocks; b += p.k_boxed) {
-                        if (p.latent) tma_load_4d(dst + b * kBlock, &tmap_k, &k_full[st], p.E + (b - others) * 64, row0 + off, 0, page);
-                        else tma_load_4d(dst + b * kBlock, &tmap_k, &k_full[st], 0, row0 + off, mp * p.key_blocks + b, page);
+                        if (p.latent || packed) tma_load_4d(dst + b * kBlock, &tmap_k, &k_full[st], (p.latent ? p.E : 0) + (b - others) * 64, row, 0, page);
+                        else tma_load_4d(dst + b * kBlock, &tmap_k, &k_full[st], 0, row, mp * p.key_blocks + b, page);
                     }
                 }
             }
@@ -259,7 +268,7 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             __syncwarp();
             if (page >= 0)
                 for (int b = 0; b < p.value_blocks; b += p.v_boxed)
-                    tma_load_4d(vd + b * kBlock + lane * box_bytes, &tmap_v, last ? tail : &v_full[st], 0, row0 + off, vc * p.value_blocks + b, page);
+                    tma_load_4d(vd + b * kBlock + lane * box_bytes, &tmap_v, last ? tail : &v_full[st], 0, row, head_blocks + (packed ? others : 0) + vc * p.value_blocks + b, page);
             if (last) {
                 // what lies in the cache behind the last token counts as zeros: a weight of 0 would not silence a NaN there
                 if (lane == 0) ok = mbar_wait<true>(tail, tail_ph, abort, p.status, 3);
@@ -621,6 +630,9 @@ int launch(const char* what, const CUtensorMap& tq, const CUtensorMap& tk, const
     }
     p.stages = kMaxStages;
     while (p.stages > 1 && smem_bytes(q_blocks, blocks, p.stages) > kSmemLimit) --p.stages;
+    // (heads of 128 + 64 channels, keys and values packed: one tile of keys a CTA and two CTAs an SM 49.2 us, three and one CTA 59.0)
+    if (p.row_start && 2 * BKV + p.VC <= 256 && smem_bytes(q_blocks, blocks, 1) <= 112 * 1024)
+        while (smem_bytes(q_blocks, blocks, p.stages) > 112 * 1024) --p.stages;
     const size_t smem = smem_bytes(q_blocks, blocks, p.stages);
     if (smem > kSmemLimit) return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: queries of %d channels", what, p.q_channels);
     p.tmem_cols = 2 * BKV + p.VC + (p.q_tmem ? p.value_blocks * 32 : 0) <= 256 ? 256 : 512;
@@ -673,6 +685,45 @@ extern "C" int forge_latent_attention_sm100(const void* q, const void* cache, co
     p.page_size = page_size; p.max_pages = max_pages; p.window = window;
     p.vec_out = ((uintptr_t)out & 15) == 0; p.scale = scale; p.out_scale = 1.0f; p.status = status;
     return launch<false>("latent_attention_sm100", tq, tk, tv, p, num_tiles, stream);
+}
+
+// 1 if the kernel takes keys and values of H heads spelled out: D unrotated channels and E values a head (multiples of 64, D up to 256, E up
+// to 256), R rotated ones (a multiple of 16).
+extern "C" int forge_expanded_sm100_supports(int H, int D, int R, int E) {
+    const int q_blocks = (D + R + 63) / 64;
+    return (H > 0 && D > 0 && D % 64 == 0 && D <= 256 && R > 0 && R % 16 == 0 && R <= 128 && E > 0 && E % 64 == 0 && E <= 256 &&
+            smem_bytes(q_blocks, q_blocks + E / 64, 1) <= kSmemLimit) ? 1 : 0;
+}
+
+// q bf16 [T, H, D+R]; kv bf16 [rows, H, D+E]: keys and values of every request of the step, position by position, request s from row row_start[s]
+// on; kr bf16 [rows, R]; out bf16, rows of out_ld, head h's E values from h * E on.  Tiles of up to 128 tokens; the rest as above.
+extern "C" int forge_expanded_attention_sm100(const void* q, const void* kv, const void* kr, const int32_t* row_start, const int32_t* tok_req,
+                                              const int32_t* positions, const int32_t* tile_t0, const int32_t* tile_n, void* out, int* status, int T,
+                                              int num_tiles, int rows, int H, int D, int R, int E, float scale, const float* sink, long long out_ld,
+                                              cudaStream_t stream) {
+    if (!forge_expanded_sm100_supports(H, D, R, E)) return forge::fail(FORGE_ERR_UNSUPPORTED, "expanded_attention_sm100: H=%d D=%d R=%d E=%d", H, D, R, E);
+    if (T < 0 || num_tiles < 0 || rows <= 0 || !row_start || !tile_t0 || !tile_n || !(scale > 0.f) || out_ld < (long long)H * E || (out_ld & 1) ||
+        ((uintptr_t)out & 3))
+        return forge::fail(FORGE_ERR_ARG, "expanded_attention_sm100: bad arguments");
+    if (T == 0 || num_tiles == 0) return FORGE_OK;
+    const int width = H * (D + E), boxed = D == E ? E / 64 : 1;
+    const char* err = nullptr;
+    CUtensorMap tq, tk, tv;
+    if (!query_map(q, D + R, H, T, 1, BQ, &tq, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "expanded_attention_sm100: q: %s", err);
+    const unsigned long long n = (unsigned long long)rows;
+    if (!block_map(kv, width, width, rows, 1, (long long)n * width, BKV, boxed, &tv, &err) ||
+        !tensor_map(kr, 4, {(unsigned long long)R, n, 1, 1}, {(unsigned long long)R, n * R, n * R}, {64, BKV, 1, 1}, &tk, &err))
+        return forge::fail(FORGE_ERR_UNSUPPORTED, "expanded_attention_sm100: keys and values: %s", err);
+    ShapedParams p{};
+    p.out = (__nv_bfloat16*)out; p.out_ld = out_ld;
+    p.tok_req = tok_req; p.positions = positions; p.tile_t0 = tile_t0; p.tile_n = tile_n; p.row_start = row_start;
+    p.sink = sink;
+    p.H = H; p.heads = 1; p.inner = H; p.M = 1; p.D = D; p.E = E; p.VC = E;
+    p.q_channels = D + R; p.key_blocks = (D + R + 63) / 64; p.value_blocks = E / 64; p.latent = 0;
+    p.k_boxed = 1; p.v_boxed = boxed;
+    p.page_size = BKV; p.max_pages = 1;
+    p.vec_out = ((uintptr_t)out & 15) == 0 && out_ld % 8 == 0; p.scale = scale; p.out_scale = 1.0f; p.status = status;
+    return launch<false>("expanded_attention_sm100", tq, tk, tv, p, num_tiles, stream);
 }
 
 // q bf16 [T, H, M, D]; cache pages of page_stride numbers, [G, page_size, M*D] keys then [G, page_size, E] values; one map: out bf16, rows of

@@ -100,6 +100,7 @@ _SIGNATURES = {
     "latent": {
         "forge_latent_prepare": [_P, _I, _P, _P, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
         "forge_head_linear": [_P, _I, _LL, _I, _P, _P, _I, _LL, _I, _P, _P, _F, _I, _I, _I, _I, _I, _I, _P, _LL, _I, _I, _I, _I, _P],
+        "forge_latent_expand": [_P, _LL, _P, _P, _F, _I, _P] + [_I] * 4 + [_P, _P, _I, _I, _P] + [_I] * 3 + [_P] * 3,
         "forge_latent_attention": [_P] * 8 + [_I] * 8 + [_F, _I, _I, _I, _P, _P],
         "forge_latent_mma_supports": [_I] * 4,
         "forge_latent_mma_heads": [_I],
@@ -110,6 +111,8 @@ _SIGNATURES = {
         "forge_latent_sm100_supports": [_I] * 4,
         "forge_scored_sm100_supports": [_I] * 6,
         "forge_latent_attention_sm100": [_P] * 9 + [_I] * 8 + [_F, _I, _P, _P],
+        "forge_expanded_sm100_supports": [_I] * 4,
+        "forge_expanded_attention_sm100": [_P] * 10 + [_I] * 7 + [_F, _P, _LL, _P],
         "forge_scored_attention_sm100": [_P] * 12 + [_I] * 9 + [_LL, _I] + [_F] * 5 + [_LL, _I, _I, _F, _P, _P],
     },
     "moe": {
@@ -1650,6 +1653,93 @@ def latent_attention(q, cache, group_batch, batch, H, C, R, page_size, scale, wi
         _opt(tn, "tile_n", torch.int32), _need(out, "out", q.dtype), dtype_code(q.dtype), tiles, H, HG, C, R, page_size,
         group_batch.block_table.shape[1], float(scale), TQ, LATENT_KEYS_PER_CHUNK, window, _opt(sink, "sink", torch.float32), _stream()),
         "latent_attention")
+    return out
+
+
+EXPANDED_SCRATCH = 1 << 30          # bytes of keys and values that a layer may spell out
+
+
+def latent_expand_supports(H, D, R, E, C, dtype, scale):
+    """Whether a layer's keys and values can be spelled out for the tcgen05 kernel (asked once per layer)."""
+    return (dtype == torch.bfloat16 and _TENSOR_CORE_ATTENTION and _TENSOR_CORE_GEMM and scale > 0.0 and C % 8 == 0 and
+            bool(library("attention_shaped").forge_expanded_sm100_supports.fn(H, D, R, E)))
+
+
+def latent_expand_pays(batch, H, D, R, E, C):
+    """Whether a step's latent attention is faster with every request's keys and values spelled out per head (a product over all rows that the
+    step sees, then D + R and E channels a score and an output) than with the matrices moved to the query and the output (C + R and C
+    channels, and two per-head products over the step's tokens).  Estimated once per step and set of sizes, in microseconds: a tile of
+    queries against a tile of keys holds its CTA for 0.8 + C / 230 (absorbed; a CTA a chunk of 256 values) or 0.9 + (D + R + E) / 450, the attention lasts
+    as long as its longest row of tiles or the SMs' share of all, the product runs at 0.7 and the per-head ones at 0.13 PFLOP/s.  Measured
+    (device, a layer of 32 heads of 128, 4,096 wide): 24 tokens 78 -> 61, 1,600 tokens 522 -> 272, 24 behind 1,000 cached 111 -> 94, four requests of 25 behind
+    1,000 133 -> 134; many cached rows that few tokens see, as in a step of mostly single tokens, stay absorbed."""
+    key = ("expand", H, D, R, E, C)
+    pays = batch.attention_plan.get(key)
+    if pays is None:
+        pays = False
+        if _brings_portions(batch):
+            qs, before = batch.host_q_start, getattr(batch, "host_context_before", None) or [0] * batch.num_requests
+            rows = before[-1] + qs[-1] + sum(before[:-1])
+            if 2 * rows * H * (D + E) <= EXPANDED_SCRATCH:
+                def tiles(TQ):                                  # (of keys: the longest row of tiles, all)
+                    longest = total = 0
+                    for c, a, b in zip(before, qs, qs[1:]):
+                        k = -(-(b - a) // TQ)
+                        ends = -(-(c + b - a) // 64)
+                        longest, total = max(longest, ends), total + k * ((c + min(TQ, b - a) + 63) // 64 + ends) / 2
+                    return longest, total
+                sms, T = _sm_count(batch.positions.device), batch.num_tokens
+                far, work = tiles(max(1, 128 // H))
+                far_x, work_x = tiles(128)
+                absorbed = max(far, work * max(1, C // 256) / sms) * (0.8 + C / 230) + 2 * H * T * C * (D + E) / 130e6 + 10
+                expanded = max(far_x, work_x * H / sms) * (0.9 + (D + R + E) / 450) + 2 * H * rows * C * (D + E) / 700e6 + 12
+                pays = expanded < absorbed
+        batch.attention_plan[key] = pays
+    return pays
+
+
+def latent_expand(q, cache, group_batch, batch, H, C, D, R, page_size, freq, amp=1.0, halves=False):
+    """What the attention over spelled-out keys and values reads, in one launch: the step's queries q (fp32 [T, H*(D+R)], or (matrix, first
+    column)) in bfloat16, every head's last R channels rotated, and all rows of ``cache`` that the step's requests see, packed request behind request:
+    c [rows, C], kr [rows, R]; with them each request's first row (int32 [S])."""
+    q, col = q if isinstance(q, tuple) else (q, 0)
+    T, dev, S = q.shape[0], q.device, batch.num_requests
+    plan = batch.attention_plan.get("rows")
+    if plan is None:
+        qs, before, starts = batch.host_q_start, getattr(batch, "host_context_before", None) or [0] * S, [0]
+        for s in range(S):
+            starts.append(starts[-1] + before[s] + qs[s + 1] - qs[s])
+        with once_per_step():
+            plan = batch.attention_plan["rows"] = (new_ints(starts[:S], dev), starts[S])
+    row_start, rows = plan
+    q_ptr, ld = _cols(q, col)
+    if ld < col + H * (D + R):
+        raise KernelError(f"latent_expand: rows of {ld} numbers from column {col} do not hold {H} heads of {D} + {R}")
+    qr, c, kr = (new_tensor(shape, torch.bfloat16, dev) for shape in ((T, H * (D + R)), (rows, C), (rows, R)))
+    lib, table = library("latent"), group_batch.block_table
+    _check(lib, lib.forge_latent_expand(
+        q_ptr, ld, _need(batch.positions, "positions", torch.int32), _need(freq, "freq", torch.float32), float(amp), 1 if halves else 0, qr.data_ptr(), T, H, D, R,
+        _need(cache, "cache", torch.bfloat16), _need(table, "block_table", torch.int32, 2), table.shape[1], page_size, _need(row_start, "row_start", torch.int32),
+        S, rows, C, c.data_ptr(), kr.data_ptr(), _stream()), "latent_expand")
+    return qr, c, kr, row_start
+
+
+def expanded_attention(q, kv, kr, row_start, batch, H, D, R, E, scale, sink=None, out=None):
+    """Causal softmax attention of q bf16 [T, H*(D+R)] with keys and values of each head, packed request behind request: kv bf16 [rows, H*(D+E)] (a
+    head's D key channels, then its E value channels), kr bf16 [rows, R] the key channels that all heads share, request s from row row_start[s]
+    on.  Returns bf16 [T, H*E] (or writes it into ``out`` = (matrix, first column))."""
+    T, dev, lib = q.shape[0], q.device, library("attention_shaped")
+    if sink is not None and sink.numel() != H:
+        raise KernelError(f"expanded_attention: {sink.numel()} sinks for {H} heads")
+    if q.shape[1] != H * (D + R) or kv.shape[1] != H * (D + E) or kr.shape[1] != R or kv.shape[0] != kr.shape[0]:
+        raise KernelError(f"expanded_attention: q {tuple(q.shape)}, kv {tuple(kv.shape)}, kr {tuple(kr.shape)} do not fit {H} heads of {D} + {R} and {E}")
+    t0, tn, tiles = shaped_plan(batch, 128, dev)
+    out, out_ptr, out_ld = _out_slice(out, H * E, T, torch.bfloat16, dev)
+    _check(lib, lib.forge_expanded_attention_sm100(
+        _need(q, "q", torch.bfloat16, 2), _need(kv, "kv", torch.bfloat16, 2), _need(kr, "kr", torch.bfloat16, 2), _need(row_start, "row_start", torch.int32),
+        _need(batch.tok_req, "tok_req", torch.int32), _need(batch.positions, "positions", torch.int32), _need(t0, "tile_t0", torch.int32),
+        _need(tn, "tile_n", torch.int32), out_ptr, _need(_gemm_status(dev), "status", torch.int32), T, tiles, kv.shape[0], H, D, R, E, float(scale),
+        _opt(sink, "sink", torch.float32), out_ld, _stream()), "expanded_attention_sm100")
     return out
 
 

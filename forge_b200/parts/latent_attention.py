@@ -10,7 +10,9 @@ latent's width and Cq the query latent's:
 
 A token leaves the row [c | kr] in the cache and nothing else.  The per-head matrices move to the query and the output
 (qa_h = [Wuk_h^T qf_h | qr_h] attends over the rows themselves, Wuv_h is applied to the weighted sum of latents), so keys
-and values per head are never formed: one path for prompt portions and single tokens.  A layer with ``cache_from`` has no
+and values per head are not formed, for single tokens and short portions.  A long portion sees each row many times: there one product makes the keys
+and values of all rows that the step sees, and a score takes D + R channels instead of C + R (``kernels.latent_expand_pays``; 16-bit
+layers without a window or a gate).  A layer with ``cache_from`` has no
 Wdkv: it reads the rows that the named layer wrote, with matrices of its own.
 
 The rotation's pairs (channel 2i with 2i+1, or i with i + R/2), its frequencies and the factor on cos and sin come from the
@@ -91,6 +93,10 @@ class LatentAttention(Part):
         # per head [inputs, outputs]: Wuk_h as stored ([D, C]: it is applied transposed, to the query), Wuv_h transposed ([C, E])
         self.uk = self._matrix(tensors[self._n("uk")].reshape(H, D, C))
         self.uv = self._matrix(tensors[self._n("uv")].reshape(H, E, C).transpose(1, 2))
+        # ... and for portions that spell keys and values out: per head the rows that make its key, then those that make its value
+        self.w_kv = None
+        if self.window is None and not self.out_gate and kernels.latent_expand_supports(H, D, self.rot_dim, E, C, self.rt.dtype, self.scale):
+            self.w_kv = self._matrix(torch.cat([tensors[self._n("uk")].reshape(H, D, C), tensors[self._n("uv")].reshape(H, E, C)], dim=1).reshape(H * (D + E), C))
         self.o = Linear(self._matrix(tensors[self._n("o")]), None, self.rt)
 
     def _q_cols(self):
@@ -117,6 +123,10 @@ class LatentAttention(Part):
         cq = kernels.latent_prepare((p, col if Cq else after_q), batch, g.slot_mapping if store else None, cache.kv if store else None, freq, amp,
                                     self.wq, self.wc, Cq or 0, C if self.own_latent else 0, R, self.eps, self.rt.dtype, halves=halves)
         q = self.uq.forward(cq) if Cq else (p, col)                                    # fp32 [T, H*(D+R)]
+        if self.w_kv is not None and kernels.latent_expand_pays(batch, H, D, R, E, C) and (out is None or (out[1] | out[0].shape[1]) % 2 == 0):
+            qr, c, kr, row_start = kernels.latent_expand(q, cache.kv, g, batch, H, C, D, R, cache.page_size, freq, amp, halves)
+            return kernels.expanded_attention(qr, kernels.gemm_sm100(c, self.w_kv, epilogue="cast"), kr, row_start, batch, H, D, R, E, self.scale,
+                                              sink=self.sinks, out=out)
         qa = kernels.head_linear(q, self.uk, H, D, C, self.rt.dtype, R=R, positions=batch.positions, freq=freq, amp=amp, halves=halves, w_at_rest=True)
         lat = kernels.latent_attention(qa, cache.kv, g, batch, H, C, R, cache.page_size, self.scale, window=self.window or 0, sink=self.sinks)
         gate = (p, after_q + (C + R if self.own_latent else 0), self.out_gate) if self.out_gate else None

@@ -1,0 +1,80 @@
+"""Latent attention with keys and values spelled out per head (kernels.latent_expand, kernels.expanded_attention), against the definition in 64 bits.
+Portions shorter and longer than a tile of 128 tokens, behind cached tokens, pages shorter and longer than a tile of keys, shared key channels that do not
+fill a block of 64, keys and values of different widths; numbers that are none behind a request's last token.
+
+The attention's inputs are bfloat16 and enter exactly; allowed as for the other prompt attentions: 2^-8 of a value and 1e-3 of the largest.  The queries'
+rounding moves a number by 2^-9 of itself, their rotation by a few 2^-24 of the pair: 2^-8 of a value and 1e-6 of the pair are allowed."""
+import math
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from test_attention_shaped_gpu import DEV, _batch, _close, _fill, _softmax_out, _visible
+
+pytestmark = pytest.mark.gpu
+REQS = [(0, 1), (70, 37), (0, 130), (200, 5), (0, 257)]          # (cached, new) of the step's requests
+
+
+@pytest.mark.parametrize("H,C,D,R,E,ps,halves,col", [(4, 512, 128, 64, 128, 64, False, 0), (3, 256, 64, 32, 64, 16, True, 3), (2, 64, 64, 16, 192, 8, False, 4),
+                                                     (1, 128, 128, 128, 64, 128, True, 0), (5, 64, 192, 48, 256, 64, False, 1)])
+def test_expanded(H, C, D, R, E, ps, halves, col):
+    from forge_b200 import kernels
+    assert kernels.library("attention_shaped").forge_expanded_sm100_supports.fn(H, D, R, E)
+    KD = C + R
+    batch, table, n_pages, g = _batch(REQS, ps, KD, seed=H + C)
+    cache = torch.empty(n_pages, ps * KD, dtype=torch.bfloat16)
+    rows = _fill(cache.view(n_pages, ps, KD), table, REQS, ps, g)
+    T, W = batch.num_tokens, D + R
+    p = torch.randn(T, col + H * W + 2, generator=g)
+    freq = 10000.0 ** (-2.0 * torch.arange(R // 2) / R)
+    sink = torch.randn(H, generator=g) if halves else None
+    scale, group = 2.0 * W ** -0.5, SimpleNamespace(block_table=table.to(DEV))
+    qr, c, kr, row_start = kernels.latent_expand((p.to(DEV), col), cache.to(DEV), group, batch, H, C, D, R, ps, freq.to(DEV), 1.5, halves)
+    # rows, packed request behind request, bit for bit
+    want = torch.cat(rows)
+    assert row_start.tolist() == [sum(a + b for a, b in REQS[:s]) for s in range(len(REQS))]
+    assert torch.equal(c.double().cpu(), want[:, :C]) and torch.equal(kr.double().cpu(), want[:, C:])
+    # queries
+    q = p[:, col:col + H * W].double().view(T, H, W)
+    # (the angle is a product in 32 bits, as everywhere in the engine)
+    a = (batch.positions.cpu().float()[:, None] * freq.float()).double()[:, None, :]
+    cs, sn = torch.cos(a) * 1.5, torch.sin(a) * 1.5
+    u, v = (q[..., D:D + R // 2], q[..., D + R // 2:]) if halves else (q[..., D::2], q[..., D + 1::2])
+    turned = torch.cat([u * cs - v * sn, v * cs + u * sn], -1) if halves else torch.stack([u * cs - v * sn, v * cs + u * sn], -1).flatten(-2)
+    ref = torch.cat([q[..., :D], turned], -1)
+    got = qr.double().cpu().view(T, H, W)
+    assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all())
+    # attention, over keys and values of any values
+    kv = torch.randn(len(want), H * (D + E), generator=g).to(torch.bfloat16)
+    wide = torch.full((T, H * E + 6), 3.0, dtype=torch.bfloat16, device=DEV)
+    for out in (None, (wide, 2)):
+        launches = kernels.launch_count()
+        res = kernels.expanded_attention(qr, kv.to(DEV), kr, row_start, batch, H, D, R, E, scale, sink=None if sink is None else sink.to(DEV), out=out)
+        assert kernels.launch_count() - launches == 1
+        kernels.check_kernel_status(DEV)
+        o = (res if out is None else wide[:, 2:2 + H * E]).double().cpu().view(T, H, E)
+        at = base = 0
+        for c0, n in REQS:
+            ok, _ = _visible(c0, n, 0, 0)
+            seen = slice(base, base + c0 + n)
+            for h in range(H):
+                k = torch.cat([kv[seen, h * (D + E):h * (D + E) + D].double(), kr[seen].double().cpu()], -1)
+                s = (got[at:at + n, h] @ k.t() * scale).masked_fill(~ok, -math.inf)
+                _close(o[at:at + n, h], _softmax_out(s, kv[seen, h * (D + E) + D:(h + 1) * (D + E)].double(), None if sink is None else sink[h].double()))
+            at, base = at + n, base + c0 + n
+    assert bool((wide[:, :2] == 3.0).all()) and bool((wide[:, 2 + H * E:] == 3.0).all())
+
+
+def test_rows_behind_a_request_are_never_seen():
+    """A request's last tile of keys reaches into the rows of the next one: numbers that are none there change nothing."""
+    from forge_b200 import kernels
+    H, D, R, E, reqs = 2, 64, 32, 64, [(0, 70), (0, 70)]
+    batch, _, _, g = _batch(reqs, 64, 64, seed=1)
+    q = torch.randn(140, H * (D + R), generator=g).to(torch.bfloat16).to(DEV)
+    kv, kr = torch.randn(140, H * (D + E), generator=g).to(torch.bfloat16).to(DEV), torch.randn(140, R, generator=g).to(torch.bfloat16).to(DEV)
+    starts = torch.tensor([0, 70], dtype=torch.int32, device=DEV)
+    whole = kernels.expanded_attention(q, kv, kr, starts, batch, H, D, R, E, 0.1)[:70].clone()
+    kv[70:] = float("nan")
+    kr[70:] = float("nan")
+    assert torch.equal(kernels.expanded_attention(q, kv, kr, starts, batch, H, D, R, E, 0.1)[:70], whole)
