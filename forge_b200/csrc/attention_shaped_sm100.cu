@@ -20,9 +20,8 @@
 // they lie packed, request behind request, [rows, H, D + E], beside the rotated part [rows, R] that all heads share; a tile is 128 tokens of
 // one head, the scores take D + R channels instead of C + R and the outputs E instead of C.
 //
-// Warps 0-3 run one thread each (copies, P V, Q K^T), warps 4-7 are the rows; registers change hands with setmaxnreg.  Where one CTA fills an
-// SM its four warps of rows would leave the SM waiting for their chains (a tile's softmax is one, and no second CTA's runs beside it): there
-// warps 4-11 are the rows, two threads a row with 32 of a tile's keys each, which meet once a tile over the row's maximum.  Every wait is bounded.
+// Warps 0-3 copy keys, multiply P V, multiply Q K^T and copy values, warps 4-11 are the rows, two threads a row with 32 of a tile's keys each,
+// which meet once a tile over the row's maximum; registers change hands with setmaxnreg where two CTAs share an SM.  Every wait is bounded.
 #include "common.cuh"
 #include "checks.cuh"
 #include "scored_combine.cuh"
@@ -31,11 +30,19 @@
 namespace {
 using namespace sm100;
 
-constexpr int BQ = 128, BKV = 64, kQkWarp = 2;
-constexpr int kLaunchRegs = 128, kRegsFew = 64, kRegsMany = 192;
-static_assert(kRegsFew + kRegsMany <= 2 * kLaunchRegs, "the two warpgroups cannot hold more registers than the CTA was given");
+constexpr int BQ = 128, BKV = 64, kQkWarp = 2, kValueWarp = 3;
+constexpr int kThreads = 384, kRowWarps = 8, NK = BKV / 2;      // four warps that run the copies and products, eight of rows; NK: a thread's keys of a tile
+// two CTAs an SM: 65,536 / (2 x 384) registers a thread, dealt out anew between the three warpgroups
+constexpr int kLaunchRegs = 80, kRegsFew = 48, kRegsMany = 96;
+static_assert(kRegsFew + 2 * kRegsMany <= 3 * kLaunchRegs, "the warpgroups cannot hold more registers than the CTA was given");
+#if FORGE_CHECKS
+constexpr bool kPagesMayBeSkipped = true;                      // (a checks build skips a page id that is none)
+#else
+constexpr bool kPagesMayBeSkipped = false;
+#endif
 constexpr int kQBlock = BQ * 128, kBlock = BKV * 128;          // bytes of 64 channels of the queries / of a tile of keys
 constexpr int kMaxStages = 3, kBarBytes = 256, kSmemLimit = 227 * 1024 - 1024;      // (1 KB of it is the rows' meeting place)
+constexpr int kSmemTwo = (228 * 1024 - 2 * 2048) / 2;          // of two CTAs an SM (1 KB of each is the system's, 1 KB the meeting place)
 constexpr float kRefSlack = 8.0f;     // a row's reference exponent moves only when its maximum has grown by more than 2^8 (see attention_sm100.cu)
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -44,7 +51,8 @@ struct ShapedParams {
     float* u;                         // fp32 [T, H, M, E], normalised (two maps)
     long long out_ld;
     const __nv_bfloat16* q;           // (q_tmem) [T, H, D]
-    const int32_t *block_table, *tok_req, *positions, *tile_t0, *tile_n;
+    const int32_t* block_table;
+    const int4* tiles;                // (first token, tokens, request, the first token's position)
     const float *r1, *r2, *sink;
     int H, heads, inner, M, D, E, VC; // heads: of a CTA; inner: CTAs of one tile (groups x maps x chunks of values)
     int q_channels;                   // channels of a query row that enter S
@@ -81,24 +89,27 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 // The products' descriptors as a low word that moves and a high word that does not: the one thread that issues them pays for every
 // instruction between two of them (whole 64-bit descriptors worked out per product: 120 to 150 clocks each, where the tensor core needs 32).
+// The whole warp walks the loop around them, with every operand the same in all lanes, and the instruction itself runs in the elected one
+// (`leader`): operands that the compiler knows to be uniform come from uniform registers, while in a branch of one lane each has to be moved there
+// first (160 clocks a product of the scores, 75 of the outputs).
 // D[tmem] (+)= A[smem] . B[smem]^T
-__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_ss(uint32_t leader, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 e, %6, 0;\n\t"
         "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
-        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(leader)
         : "memory");
 }
 // D[tmem] (+)= A[tmem] . B[smem]^T: row r of A is lane r, 16 channels are eight columns of two bfloat16 numbers
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_ts(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 e, %6, 0;\n\t"
         "mov.b64 b, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(leader)
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -124,18 +135,35 @@ __device__ __forceinline__ int first_visible(int pos, int window, int chunk) {
     return lo;
 }
 
-// score i of the row's 64 (i is a constant after unrolling)
-#define SV(i) ((i) < 32 ? sv_lo[(i) & 31] : sv_hi[(i) & 31])
+typedef unsigned long long u64;
+// two fp32 multiply-adds (or sums) in one instruction, each rounded as fmaf (or +) rounds
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 pair2(uint32_t lo, uint32_t hi) {
+    u64 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+    return d;
+}
+__device__ __forceinline__ float low2(u64 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float high2(u64 v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
-template <bool SHAPED, bool WIDE>
-__global__ void __launch_bounds__(WIDE ? 384 : 256, WIDE ? 1 : 2)
+template <bool SHAPED, int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM)
 shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                               const __grid_constant__ CUtensorMap tmap_v, const ShapedParams p) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ float meet[2][WIDE ? BQ : 1];                        // [half]: what a row's two threads tell each other
-    constexpr int kThreads = WIDE ? 384 : 256, kRowWarps = WIDE ? 8 : 4, NK = WIDE ? BKV / 2 : BKV;      // NK: a thread's keys of a tile
+    __shared__ float meet[2][BQ];                                   // [half]: what a row's two threads tell each other
     const int tile = blockIdx.x / p.inner;
-    const int t0 = p.tile_t0[tile], nq = p.tile_n[tile];
+    const int4 what = p.tiles[tile];
+    const int t0 = what.x, nq = what.y;
     if (!FORGE_TOKEN_OK(t0) || !FORGE_TOKEN_OK(t0 + nq - 1)) return;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int q_blocks = (p.q_channels + 63) / 64 - (p.q_tmem ? p.value_blocks : 0);
@@ -181,11 +209,11 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         prefetch_tensormap(&tmap_k);
         prefetch_tensormap(&tmap_v);
     }
-    // the stages start as zeros: pages that are skipped (behind the window, beyond the request) leave their rows as they are, and those
-    // rows must hold finite numbers (their weights are 0); so do the query rows that a tile of fewer than 128 leaves unwritten
-    {
-        uint4* z = reinterpret_cast<uint4*>(q_rows < BQ ? q_s : k_s);
-        const int n = (int)(reinterpret_cast<uint8_t*>(q_full) - reinterpret_cast<uint8_t*>(z)) / 16;
+    // Where a tile of keys comes as several pages the stages start as zeros: pages that are skipped (behind the window, beyond the request) leave their
+    // rows as they are, and those rows must hold finite numbers (their weights are 0).  (A tile out of one page always lands whole.)
+    if (p.box_rows < BKV || kPagesMayBeSkipped) {
+        uint4* z = reinterpret_cast<uint4*>(k_s);
+        const int n = (int)(reinterpret_cast<uint8_t*>(q_full) - k_s) / 16;
         for (int i = threadIdx.x; i < n; i += kThreads) z[i] = make_uint4(0, 0, 0, 0);
     }
     fence_proxy_async();
@@ -199,58 +227,60 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
     const uint32_t tmem_base = *tmem_slot, tmem_o = tmem_base + 2 * BKV;
     forge::pdl_launch_dependents();
 
-    // (the step's tile lists, positions and tables were written before its first kernel started)
-    const int req = p.tok_req[t0], pos0 = p.positions[t0], pos_last = pos0 + nq - 1;
+    // (the step's tiles and tables were written before its first kernel started)
+    const int req = what.z, pos0 = what.w, pos_last = pos0 + nq - 1;
     const int t_begin = first_visible(pos0, p.window, p.chunk) / BKV, t_end = pos_last / BKV + 1, n_iter = t_end - t_begin;
     const int seen_from = first_visible(pos0, p.window, p.chunk);
     forge::pdl_wait();
 
     if (warp < 4) {
-    if (!WIDE) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsFew));
-    if (warp == 0) {
-        // ------------------------------------------------------------------ copies
+    if (PER_SM > 1) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsFew));
+    if (warp == 0 || warp == kValueWarp) {
+        // ------------------------------------------------------------------ copies: keys (and the queries), values
+        // (a warp each, and nothing between two copies that could be worked out ahead: these warps get an instruction in every ten clocks or so
+        // beside the rows, and a round of 150 instructions for both kinds was longer than the products and weights of a tile)
         const int32_t* table = p.block_table + (size_t)req * p.max_pages;
         const int ppt = p.page_size >= BKV ? 1 : BKV / p.page_size;       // boxes a tile and block
-        const int row0 = group * p.page_size, k_col0 = p.latent ? 0 : mp * p.D;
+        const int page_shift = 31 - __clz(p.page_size), page_mask = p.page_size > BKV ? p.page_size - 1 : 0;     // (a power of two)
+        const int k_col0 = p.latent ? 0 : mp * p.D;
         const int skip = p.latent ? vc * p.value_blocks : 1 << 20;        // key block i stands for channel block i, or i + value_blocks from here on
         const bool packed = p.row_start != nullptr;
         // key blocks that are the other chunk's value blocks (packed: the head's own blocks of keys): they come like them
         const int others = p.latent ? (chunks - 1) * p.value_blocks : packed ? p.D / 64 : 0;
-        const int head_blocks = packed ? group * ((p.D + p.E) / 64) : 0, packed_row0 = packed ? p.row_start[req] : 0;
-        if (lane == 0) {
-            mbar_arrive_expect_tx(q_full, q_blocks * q_rows * 128);
-            for (int b = 0; b < q_blocks; ++b)
-                tma_load_3d(q_s + b * kQBlock, &tmap_q, q_full, k_col0 + (p.q_tmem && b >= skip ? b + p.value_blocks : b) * 64, group * p.heads, t0);
-        }
-        bool ok = true;
-        int st = 0, ph = 0, tail_ph = 0;
-        for (int it = 0; it < n_iter && ok; ++it) {
-            const int j0 = (t_begin + it) * BKV;
-            // one lane a box of rows: its page, or -1 where no token of the tile sees a key
+        const int head_blocks = packed ? group * ((p.D + p.E) / 64) : 0, row0 = packed ? p.row_start[req] : group * p.page_size;
+        const int rounds = __shfl_sync(0xffffffffu, n_iter, 0);
+        // one lane a box of rows: its page, or -1 where no token of the tile sees a key.  Asked for a tile ahead: a trip to the table takes longer than
+        // the products of a small tile
+        auto page_of = [&](int it) {
             int page = -1;
-            if (lane < ppt) {
-                const int j = j0 + lane * p.box_rows;
-                const int idx = j / p.page_size;
+            if (lane < ppt && it < rounds) {
+                const int j = (t_begin + it) * BKV + lane * p.box_rows, idx = j >> page_shift;
                 if (packed) page = 0;                                     // (rows behind the request's are another's, or fill: masked, and cleared below)
                 else if (j <= pos_last && j + p.box_rows > seen_from && idx < p.max_pages) page = table[idx];
-                if (page >= 0 && !packed && !FORGE_PAGE_OK(page)) page = -1;
             }
-            const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0));
-            const int row = packed ? packed_row0 + j0 : row0 + (p.page_size > BKV ? j0 % p.page_size : 0);
-            const bool last = j0 + BKV - 1 > pos_last;                    // rows behind the last token: cleared below
-            uint8_t* kd = k_s + st * p.key_blocks * kBlock;
-            uint8_t* vd = v_s + st * p.value_blocks * kBlock;
-            const uint32_t box_bytes = p.box_rows * 128;
-            if (p.key_blocks > 0) {
-                if (lane == 0) {
-                    ok = mbar_wait<true>(&k_empty[st], ph ^ 1, abort, p.status, 1);
-                    if (ok) mbar_arrive_expect_tx(&k_full[st], p.key_blocks * n_valid * box_bytes);
-                }
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) break;
+            return page;
+        };
+        const uint32_t box_bytes = p.box_rows * 128;
+        int st = 0, ph = 0, next_page = -1;
+        if (warp == 0) {
+            if (lane == 0) {
+                mbar_arrive_expect_tx(q_full, q_blocks * q_rows * 128);
+                for (int b = 0; b < q_blocks; ++b)
+                    tma_load_3d(q_s + b * kQBlock, &tmap_q, q_full, k_col0 + (p.q_tmem && b >= skip ? b + p.value_blocks : b) * 64, group * p.heads, t0);
+            }
+            next_page = page_of(0);
+            if (p.key_blocks > 0)
+            for (int it = 0; it < rounds; ++it) {
+                const int j0 = (t_begin + it) * BKV;
+                int page = next_page;
+                next_page = page_of(it + 1);
+                if (page >= 0 && !packed && !FORGE_PAGE_OK(page)) page = -1;
+                const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0)), row = packed ? row0 + j0 : row0 + (j0 & page_mask);
+                if (!warp_wait<true>(&k_empty[st], ph ^ 1, abort, p.status, 1)) break;
+                if (lane == 0) mbar_arrive_expect_tx(&k_full[st], p.key_blocks * n_valid * box_bytes);
                 __syncwarp();
                 if (page >= 0) {
-                    uint8_t* dst = kd + lane * box_bytes;
+                    uint8_t* dst = k_s + st * p.key_blocks * kBlock + lane * box_bytes;
                     for (int b = 0; b < others; b += p.v_boxed)
                         tma_load_4d(dst + b * kBlock, &tmap_v, &k_full[st], 0, row, head_blocks + (b < skip ? b : b + p.value_blocks), page);
                     for (int b = others; b < p.key_blocks; b += p.k_boxed) {
@@ -258,119 +288,127 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                         else tma_load_4d(dst + b * kBlock, &tmap_k, &k_full[st], 0, row, mp * p.key_blocks + b, page);
                     }
                 }
+                if (++st == p.stages) { st = 0; ph ^= 1; }
             }
-            if (lane == 0) {
-                ok = mbar_wait<true>(&v_empty[st], ph ^ 1, abort, p.status, 2);
-                if (ok) mbar_arrive_expect_tx(last ? tail : &v_full[st], p.value_blocks * n_valid * box_bytes);
-            }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) break;
-            __syncwarp();
-            if (page >= 0)
-                for (int b = 0; b < p.value_blocks; b += p.v_boxed)
-                    tma_load_4d(vd + b * kBlock + lane * box_bytes, &tmap_v, last ? tail : &v_full[st], 0, row, head_blocks + (packed ? others : 0) + vc * p.value_blocks + b, page);
-            if (last) {
-                // what lies in the cache behind the last token counts as zeros: a weight of 0 would not silence a NaN there
-                if (lane == 0) ok = mbar_wait<true>(tail, tail_ph, abort, p.status, 3);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) break;
-                tail_ph ^= 1;
-                const int from = pos_last + 1 - j0, pieces = (BKV - from) * 8;
-                for (int b = 0; b < p.value_blocks; ++b)
-                    for (int i = lane; i < pieces; i += 32) reinterpret_cast<uint4*>(vd + b * kBlock + from * 128)[i] = make_uint4(0, 0, 0, 0);
-                fence_proxy_async();
+        } else {
+            const int block0 = head_blocks + (packed ? others : 0) + vc * p.value_blocks;
+            int tail_ph = 0;
+            next_page = page_of(0);
+            for (int it = 0; it < rounds; ++it) {
+                const int j0 = (t_begin + it) * BKV;
+                int page = next_page;
+                next_page = page_of(it + 1);
+                if (page >= 0 && !packed && !FORGE_PAGE_OK(page)) page = -1;
+                const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0)), row = packed ? row0 + j0 : row0 + (j0 & page_mask);
+                const bool last = j0 + BKV - 1 > pos_last;                // rows behind the last token: cleared below
+                uint64_t* landed = last ? tail : &v_full[st];
+                uint8_t* vd = v_s + st * p.value_blocks * kBlock;
+                if (!warp_wait<true>(&v_empty[st], ph ^ 1, abort, p.status, 2)) break;
+                if (lane == 0) mbar_arrive_expect_tx(landed, p.value_blocks * n_valid * box_bytes);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&v_full[st]);
+                if (page >= 0)
+                    for (int b = 0; b < p.value_blocks; b += p.v_boxed)
+                        tma_load_4d(vd + b * kBlock + lane * box_bytes, &tmap_v, landed, 0, row, block0 + b, page);
+                if (last) {
+                    // what lies in the cache behind the last token counts as zeros: a weight of 0 would not silence a NaN there
+                    if (!warp_wait<true>(tail, tail_ph, abort, p.status, 3)) break;
+                    tail_ph ^= 1;
+                    const int from = pos_last + 1 - j0, pieces = (BKV - from) * 8;
+                    for (int b = 0; b < p.value_blocks; ++b)
+                        for (int i = lane; i < pieces; i += 32) reinterpret_cast<uint4*>(vd + b * kBlock + from * 128)[i] = make_uint4(0, 0, 0, 0);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&v_full[st]);
+                }
+                if (++st == p.stages) { st = 0; ph ^= 1; }
             }
-            if (++st == p.stages) { st = 0; ph ^= 1; }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ P V
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16_f32_bmn(BQ, p.VC), v_step = p.value_blocks * kBlock >> 4;
-            const uint64_t vdesc = umma_desc_mn_sw128(smem_u32(v_s), kBlock);
-            const uint32_t v_lo0 = (uint32_t)vdesc, hi = (uint32_t)(vdesc >> 32);
-            bool ok = true;
-            int st = 0, ph = 0;
-            for (int it = 0; it < n_iter && ok; ++it) {
-                const int b = it & 1;
-                if (!(ok = mbar_wait<true>(&v_full[st], ph, abort, p.status, 4))) break;
-                if (!(ok = mbar_wait<true>(&p_ready[b], (it >> 1) & 1, abort, p.status, 5))) break;
-                tc_fence_after_sync();
-                const uint32_t v_lo = v_lo0 + st * v_step, pt = tmem_base + b * BKV;
+        const uint32_t leader = elect_one(), idesc = umma_idesc_bf16_f32_bmn(BQ, p.VC), v_step = p.value_blocks * kBlock >> 4;
+        const uint64_t vdesc = umma_desc_mn_sw128(smem_u32(v_s), kBlock);
+        const uint32_t v_lo0 = (uint32_t)vdesc, hi = (uint32_t)(vdesc >> 32), o_at = __shfl_sync(0xffffffffu, tmem_o, 0);
+        const int rounds = __shfl_sync(0xffffffffu, n_iter, 0);
+        int st = 0, ph = 0;
+        for (int it = 0; it < rounds; ++it) {
+            const int b = it & 1;
+            if (!warp_wait<true>(&v_full[st], ph, abort, p.status, 4)) break;
+            if (!warp_wait<true>(&p_ready[b], (it >> 1) & 1, abort, p.status, 5)) break;
+            tc_fence_after_sync();
+            const uint32_t v_lo = v_lo0 + st * v_step, pt = o_at - 2 * BKV + b * BKV;
 #pragma unroll
-                for (int k = 0; k < BKV / 16; ++k) {
-                    umma_ts(tmem_o, pt + 32 + k * 8, v_lo + k * (2048 >> 4), hi, idesc, k > 0 ? 1 : (uint32_t)(it > 0));
-                    umma_ts(tmem_o, pt + k * 8, v_lo + k * (2048 >> 4), hi, idesc, 1);
-                }
-                umma_commit(&o_done[b]);
-                umma_commit(&v_empty[st]);
-                if (++st == p.stages) { st = 0; ph ^= 1; }
+            for (int k = 0; k < BKV / 16; ++k) {
+                umma_ts(leader, o_at, pt + 32 + k * 8, v_lo + k * (2048 >> 4), hi, idesc, k > 0 ? 1 : (uint32_t)(it > 0));
+                umma_ts(leader, o_at, pt + k * 8, v_lo + k * (2048 >> 4), hi, idesc, 1);
             }
+            umma_commit_by(leader, &o_done[b]);
+            umma_commit_by(leader, &v_empty[st]);
+            if (++st == p.stages) { st = 0; ph ^= 1; }
         }
     } else if (warp == kQkWarp) {
         // ------------------------------------------------------------------ Q K^T
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16_f32(BQ, BKV);
-            const int skip = p.latent ? vc * p.value_blocks : 1 << 20;
-            const uint64_t qdesc = umma_desc_k_sw128(smem_u32(q_s));
-            const uint32_t q_lo = (uint32_t)qdesc, hi = (uint32_t)(qdesc >> 32);
-            const uint32_t k_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(k_s)), v_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(v_s));
-            const uint32_t k_step = p.key_blocks * kBlock >> 4, v_step = p.value_blocks * kBlock >> 4;
-            const int part_steps = p.q_channels % 64 / 16, part_block = part_steps ? p.q_channels / 64 : -1;
-            bool ok = mbar_wait<true>(q_full, 0, abort, p.status, 6);
-            int st = 0, ph = 0;
-            for (int it = 0; it < n_iter && ok; ++it) {
-                const int b = it & 1;
-                // (the scores' buffer holds the weights of tile it - 2 until its P V is done)
-                if (it >= 2 && !(ok = mbar_wait<true>(&o_done[b], ((it - 2) >> 1) & 1, abort, p.status, 7))) break;
-                const uint32_t ds = tmem_base + b * BKV;
-                uint32_t add = 0;
-                // key block at w_lo against the query's channel block at a_lo
-                auto product = [&](uint32_t a_lo, uint32_t w_lo, int channel_block) {
-                    if (channel_block != part_block) {
-                        umma_ss(ds, a_lo, w_lo, hi, idesc, add);
+        const uint32_t leader = elect_one(), idesc = umma_idesc_bf16_f32(BQ, BKV);
+        const int skip = p.latent ? vc * p.value_blocks : 1 << 20;
+        const uint64_t qdesc = umma_desc_k_sw128(smem_u32(q_s));
+        const uint32_t q_lo = (uint32_t)qdesc, hi = (uint32_t)(qdesc >> 32);
+        const uint32_t k_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(k_s)), v_lo0 = (uint32_t)umma_desc_k_sw128(smem_u32(v_s));
+        const uint32_t k_step = p.key_blocks * kBlock >> 4, v_step = p.value_blocks * kBlock >> 4;
+        const int part_steps = p.q_channels % 64 / 16, part_block = part_steps ? p.q_channels / 64 : -1;
+        const uint32_t s_at = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const int rounds = __shfl_sync(0xffffffffu, n_iter, 0);
+        int st = 0, ph = 0;
+        if (warp_wait<true>(q_full, 0, abort, p.status, 6))
+        for (int it = 0; it < rounds; ++it) {
+            const int b = it & 1;
+            // (the scores' buffer holds the weights of tile it - 2 until its P V is done)
+            if (it >= 2 && !warp_wait<true>(&o_done[b], ((it - 2) >> 1) & 1, abort, p.status, 7)) break;
+            const uint32_t ds = s_at + b * BKV;
+            uint32_t add = 0;
+            // key block at w_lo against the query's channel block at a_lo
+            auto product = [&](uint32_t a_lo, uint32_t w_lo, int channel_block) {
+                if (channel_block != part_block) {
+                    umma_ss(leader, ds, a_lo, w_lo, hi, idesc, add);
 #pragma unroll
-                        for (int k = 1; k < 4; ++k) umma_ss(ds, a_lo + k * 2, w_lo + k * 2, hi, idesc, 1);
-                    } else {                                              // the last channels do not fill a block
-                        for (int k = 0; k < part_steps; ++k) umma_ss(ds, a_lo + k * 2, w_lo + k * 2, hi, idesc, add | (uint32_t)(k > 0));
-                    }
-                    add = 1;
-                };
-                if (p.key_blocks > 0) {
-                    if (!(ok = mbar_wait<true>(&k_full[st], ph, abort, p.status, 8))) break;
-                    tc_fence_after_sync();
-                    const uint32_t w_lo = k_lo0 + st * k_step;
-                    for (int i = 0; i < p.key_blocks; ++i) {
-                        const int channel_block = i < skip ? i : i + p.value_blocks;
-                        product(q_lo + (p.q_tmem ? i : channel_block) * (kQBlock >> 4), w_lo + i * (kBlock >> 4), channel_block);
-                    }
-                    umma_commit(&k_empty[st]);
+                    for (int k = 1; k < 4; ++k) umma_ss(leader, ds, a_lo + k * 2, w_lo + k * 2, hi, idesc, 1);
+                } else {                                              // the last channels do not fill a block
+                    for (int k = 0; k < part_steps; ++k) umma_ss(leader, ds, a_lo + k * 2, w_lo + k * 2, hi, idesc, add | (uint32_t)(k > 0));
                 }
-                if (p.latent) {
-                    if (it == 0 && p.q_tmem && !(ok = mbar_wait<true>(q_ready, 0, abort, p.status, 13))) break;
-                    if (!(ok = mbar_wait<true>(&v_full[st], ph, abort, p.status, 9))) break;
-                    tc_fence_after_sync();
-                    const uint32_t w_lo = v_lo0 + st * v_step;
-                    if (p.q_tmem) {
-                        for (int i = 0; i < p.value_blocks; ++i) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) umma_ts(ds, tmem_o + p.VC + i * 32 + k * 8, w_lo + i * (kBlock >> 4) + k * 2, hi, idesc, k > 0 ? 1 : add);
-                            add = 1;
-                        }
-                    } else {
-                        for (int i = 0; i < p.value_blocks; ++i) product(q_lo + (skip + i) * (kQBlock >> 4), w_lo + i * (kBlock >> 4), skip + i);
-                    }
+                add = 1;
+            };
+            if (p.key_blocks > 0) {
+                if (!warp_wait<true>(&k_full[st], ph, abort, p.status, 8)) break;
+                tc_fence_after_sync();
+                const uint32_t w_lo = k_lo0 + st * k_step;
+                for (int i = 0; i < p.key_blocks; ++i) {
+                    const int channel_block = i < skip ? i : i + p.value_blocks;
+                    product(q_lo + (p.q_tmem ? i : channel_block) * (kQBlock >> 4), w_lo + i * (kBlock >> 4), channel_block);
                 }
-                umma_commit(&s_full[b]);
-                if (++st == p.stages) { st = 0; ph ^= 1; }
+                umma_commit_by(leader, &k_empty[st]);
             }
+            if (p.latent) {
+                if (it == 0 && p.q_tmem && !warp_wait<true>(q_ready, 0, abort, p.status, 13)) break;
+                if (!warp_wait<true>(&v_full[st], ph, abort, p.status, 9)) break;
+                tc_fence_after_sync();
+                const uint32_t w_lo = v_lo0 + st * v_step;
+                if (p.q_tmem) {
+                    for (int i = 0; i < p.value_blocks; ++i) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            umma_ts(leader, ds, s_at + 2 * BKV + p.VC + i * 32 + k * 8, w_lo + i * (kBlock >> 4) + k * 2, hi, idesc, k > 0 ? 1 : add);
+                        add = 1;
+                    }
+                } else {
+                    for (int i = 0; i < p.value_blocks; ++i) product(q_lo + (skip + i) * (kQBlock >> 4), w_lo + i * (kBlock >> 4), skip + i);
+                }
+            }
+            umma_commit_by(leader, &s_full[b]);
+            if (++st == p.stages) { st = 0; ph ^= 1; }
         }
     }
     } else {
-        // ------------------------------------------------------------------ the rows (warps 4..7, or 4..11)
-        if (!WIDE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsMany));
-        const int half = WIDE ? (warp - 4) >> 2 : 0;
+        // ------------------------------------------------------------------ the rows (warps 4..11)
+        if (PER_SM > 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsMany));
+        const int half = (warp - 4) >> 2;
         const int quarter = warp & 3, r = quarter * 32 + lane;
         const bool valid = r < nq * p.heads;
         const int tok = t0 + (valid ? r / p.heads : 0), head = group * p.heads + (valid ? r % p.heads : 0), pos = pos0 + tok - t0;
@@ -383,7 +421,7 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         bool ok = true;
         if (p.q_tmem) {                       // this row's channels vc * VC .. of the query, two to a column
             const __nv_bfloat16* src = p.q + ((size_t)tok * p.H + head) * p.D + vc * p.VC;
-            const int share = p.VC / (WIDE ? 2 : 1);
+            const int share = p.VC / 2;
             for (int c = half * share; c < (half + 1) * share; c += 64) {
                 uint32_t w[32];
 #pragma unroll
@@ -406,54 +444,52 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             ok = ok && mbar_wait<true>(&s_full[b], (it >> 1) & 1, abort, p.status, 10);
             __syncwarp();
             tc_fence_after_sync();
-            uint32_t sv_lo[32], sv_hi[32];
-            tmem_ld_32x32b_x32(t_s + half * NK, sv_lo);
-            if (!WIDE) tmem_ld_32x32b_x32(t_s + 32, sv_hi);
+            uint32_t sv[NK];
+            tmem_ld_32x32b_x32(t_s + half * NK, sv);
             tmem_ld_wait();
-            const bool need_mask = !valid || j0 + NK - 1 > pos || j0 < see;
+            // (a row that stands for no token may hold any number: nobody reads what comes of it)
+            const bool need_mask = valid && (j0 + NK - 1 > pos || j0 < see);
             if (SHAPED) {                     // in units of log2 e, shaped, from here on
 #pragma unroll
                 for (int i = 0; i < NK; ++i) {
-                    float s = __uint_as_float(SV(i));
+                    float s = __uint_as_float(sv[i]);
                     s = p.softcap > 0.f ? cap_out * tanh_fast(s * cap_in) : s * sl2;
                     if (p.r1) s -= r1v * __log2f(fmaf(r2v, (float)max(pos - j0 - i, 0), 1.0f));
-                    SV(i) = __float_as_uint(s);
+                    sv[i] = __float_as_uint(s);
                 }
             }
             if (need_mask) {
 #pragma unroll
                 for (int i = 0; i < NK; ++i) {
                     const int j = j0 + i;
-                    if (!(valid && j <= pos && j >= see)) SV(i) = __float_as_uint(-INFINITY);
+                    if (!(j <= pos && j >= see)) sv[i] = __float_as_uint(-INFINITY);
                 }
             }
             float a0 = -INFINITY, a1 = -INFINITY;
 #pragma unroll
             for (int i = 0; i < NK; i += 4) {
-                a0 = max3(a0, __uint_as_float(SV(i)), __uint_as_float(SV(i + 1)));
-                a1 = max3(a1, __uint_as_float(SV(i + 2)), __uint_as_float(SV(i + 3)));
+                a0 = max3(a0, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
+                a1 = max3(a1, __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]));
             }
             const float mult = SHAPED ? 1.0f : sl2;
             float top = fmaxf(a0, a1) * mult;
-            if (WIDE) {
-                // Whether any of the two warps' rows has to move its reference; mostly none has, and the row's maximum is nobody's business.
-                // (Both have read their scores by then: either's weights may overwrite the other's.)
-                int moves;
-                __syncwarp();
-                tc_fence_before_sync();
-                asm volatile(
-                    "{\n\t.reg .pred p, q;\n\t"
-                    "setp.gt.f32 p, %1, %2;\n\t"
-                    "barrier.cta.red.or.pred.aligned q, %3, 64, p;\n\t"
-                    "selp.s32 %0, 1, 0, q;\n\t}"
-                    : "=r"(moves) : "f"(top), "f"(m + kRefSlack), "r"(1 + quarter) : "memory");
-                tc_fence_after_sync();
-                if (moves) {
-                    meet[half][WIDE ? r : 0] = top;
-                    asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
-                    top = fmaxf(top, meet[half ^ 1][WIDE ? r : 0]);
-                    asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
-                }
+            // Whether any of the two warps' rows has to move its reference; mostly none has, and the row's maximum is nobody's business.
+            // (Both have read their scores by then: either's weights may overwrite the other's.)
+            int moves;
+            __syncwarp();
+            tc_fence_before_sync();
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t"
+                "setp.gt.f32 p, %1, %2;\n\t"
+                "barrier.cta.red.or.pred.aligned q, %3, 64, p;\n\t"
+                "selp.s32 %0, 1, 0, q;\n\t}"
+                : "=r"(moves) : "f"(top), "f"(m + kRefSlack), "r"(1 + quarter) : "memory");
+            tc_fence_after_sync();
+            if (moves) {
+                meet[half][r] = top;
+                asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
+                top = fmaxf(top, meet[half ^ 1][r]);
+                asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
             }
             const float m_new = top > m + kRefSlack ? top : m;            // (-inf + slack is -inf: the first visible key sets it)
             const float alpha = m_new == m ? 1.0f : ex2(m - m_new);
@@ -464,7 +500,7 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 ok = ok && mbar_wait<true>(&o_done[b ^ 1], ((it - 1) >> 1) & 1, abort, p.status, 11);
                 __syncwarp();
                 tc_fence_after_sync();
-                const int share = p.VC / (WIDE ? 2 : 1);
+                const int share = p.VC / 2;
                 for (int c = half * share; c < (half + 1) * share; c += 32) {
                     uint32_t ov[32];
                     tmem_ld_32x32b_x32(t_out + c, ov);
@@ -477,38 +513,37 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             }
             __syncwarp();                     // (the lanes may have parted over the mask; what follows is warp-wide)
             // the weights, their sum, and P in two terms over the scores' columns: roundings in the first 32, the rest in the next
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-            for (int c = 0; c < NK; c += 32) {
+            u64 s01 = 0, s23 = 0;
+            const u64 mult2 = pair2(__float_as_uint(mult), __float_as_uint(mult)), ref2 = pair2(__float_as_uint(-ref), __float_as_uint(-ref));
+            const u64 minus2 = pair2(0xbf800000u, 0xbf800000u);
+            {
                 uint32_t hi[16], lo[16];
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    const float p0 = ex2(fmaf(__uint_as_float(SV(c + i)), mult, -ref)), p1 = ex2(fmaf(__uint_as_float(SV(c + i + 1)), mult, -ref));
-                    const float p2 = ex2(fmaf(__uint_as_float(SV(c + i + 2)), mult, -ref)), p3 = ex2(fmaf(__uint_as_float(SV(c + i + 3)), mult, -ref));
-                    s0 += p0;
-                    s1 += p1;
-                    s2 += p2;
-                    s3 += p3;
+                for (int i = 0; i < NK; i += 4) {
+                    const u64 x01 = fma2(pair2(sv[i], sv[i + 1]), mult2, ref2), x23 = fma2(pair2(sv[i + 2], sv[i + 3]), mult2, ref2);
+                    const float p0 = ex2(low2(x01)), p1 = ex2(high2(x01)), p2 = ex2(low2(x23)), p3 = ex2(high2(x23));
+                    const u64 p01 = pair2(__float_as_uint(p0), __float_as_uint(p1)), p23 = pair2(__float_as_uint(p2), __float_as_uint(p3));
+                    s01 = add2(s01, p01);
+                    s23 = add2(s23, p23);
                     const uint32_t h01 = pack_bf16(p0, p1), h23 = pack_bf16(p2, p3);
                     hi[i / 2] = h01;
                     hi[i / 2 + 1] = h23;
-                    lo[i / 2] = pack_bf16(p0 - __uint_as_float(h01 << 16), p1 - __uint_as_float(h01 & 0xffff0000u));
-                    lo[i / 2 + 1] = pack_bf16(p2 - __uint_as_float(h23 << 16), p3 - __uint_as_float(h23 & 0xffff0000u));
+                    const u64 l01 = fma2(pair2(h01 << 16, h01 & 0xffff0000u), minus2, p01), l23 = fma2(pair2(h23 << 16, h23 & 0xffff0000u), minus2, p23);
+                    lo[i / 2] = pack_bf16(low2(l01), high2(l01));
+                    lo[i / 2 + 1] = pack_bf16(low2(l23), high2(l23));
                 }
-                tmem_st_32x32b_x16(t_s + half * 16 + c / 2, hi);
-                tmem_st_32x32b_x16(t_s + 32 + half * 16 + c / 2, lo);
+                tmem_st_32x32b_x16(t_s + half * 16, hi);
+                tmem_st_32x32b_x16(t_s + 32 + half * 16, lo);
             }
-            l = l * alpha + ((s0 + s1) + (s2 + s3));
+            l = l * alpha + ((low2(s01) + high2(s01)) + (low2(s23) + high2(s23)));
             tmem_st_wait();
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_ready[b]);
         }
-        if (WIDE) {                           // the row's sum of weights
-            meet[half][WIDE ? r : 0] = l;
-            asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
-            l = meet[0][WIDE ? r : 0] + meet[1][WIDE ? r : 0];
-        }
+        meet[half][r] = l;                    // the row's sum of weights
+        asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
+        l = meet[0][r] + meet[1][r];
         if (ok) ok = mbar_wait<true>(&o_done[(n_iter - 1) & 1], ((n_iter - 1) >> 1) & 1, abort, p.status, 12);
         tc_fence_after_sync();
         ok = __all_sync(0xffffffffu, ok);
@@ -520,32 +555,52 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             }
             inv *= p.out_scale;
             const int v0 = vc * p.VC;
-            // every lane takes part in the TMEM loads (they are warp-wide instructions); only valid rows store
-            const int share = p.VC / (WIDE ? 2 : 1);
+            // 32 columns at a time go through 4 KB of shared memory of the warp's own (the queries and stages are done with), so that a store writes whole
+            // rows' pieces of 128 (64) bytes: a row a thread, straight from the registers, took 2.9 to 4.3 us a CTA.  Every lane takes part; only valid
+            // rows store.
+            uint8_t* stage = smem + (warp - 4) * 4096;
+            const long long own = !valid ? -1 : v0 + (p.u != nullptr ? (((long long)tok * p.H + head) * p.M + mp) * p.E : (long long)tok * p.out_ld + (long long)head * p.E);
+            const int share = p.VC / 2;
             for (int c = half * share; c < (half + 1) * share; c += 32) {
                 uint32_t ov[32];
                 __syncwarp();
                 tmem_ld_32x32b_x32(t_out + c, ov);
                 tmem_ld_wait();
-                if (!valid) {
-                } else if (p.u != nullptr) {
-                    float* dst = p.u + (((size_t)tok * p.H + head) * p.M + mp) * p.E + v0 + c;
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(ov[i]) * inv, __uint_as_float(ov[i + 1]) * inv,
-                                                                          __uint_as_float(ov[i + 2]) * inv, __uint_as_float(ov[i + 3]) * inv);
+                for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * inv);
+                if (p.u != nullptr) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        *reinterpret_cast<uint4*>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(ov[4 * j], ov[4 * j + 1], ov[4 * j + 2], ov[4 * j + 3]);
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int row = i * 4 + (lane >> 3), j = lane & 7;
+                        const long long at = __shfl_sync(0xffffffffu, own, row);
+                        const float4 v = *reinterpret_cast<const float4*>(stage + row * 128 + ((j ^ (row & 7)) << 4));
+                        if (at >= 0) *reinterpret_cast<float4*>(p.u + at + c + 4 * j) = v;
+                    }
                 } else {
-                    __nv_bfloat16* dst = p.out + (size_t)tok * p.out_ld + (size_t)head * p.E + v0 + c;
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
+                    for (int j = 0; j < 4; ++j) {
                         uint32_t w[4];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) w[e] = pack_bf16(__uint_as_float(ov[i + 2 * e]) * inv, __uint_as_float(ov[i + 2 * e + 1]) * inv);
-                        if (p.vec_out) {
-                            *reinterpret_cast<uint4*>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);
-                        } else {
+                        for (int e = 0; e < 4; ++e) w[e] = pack_bf16(__uint_as_float(ov[8 * j + 2 * e]), __uint_as_float(ov[8 * j + 2 * e + 1]));
+                        *reinterpret_cast<uint4*>(stage + lane * 64 + ((j ^ (lane >> 1 & 3)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                    __syncwarp();
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) reinterpret_cast<uint32_t*>(dst + i)[e] = w[e];
+                    for (int i = 0; i < 4; ++i) {
+                        const int row = i * 8 + (lane >> 2), j = lane & 3;
+                        const long long at = __shfl_sync(0xffffffffu, own, row);
+                        const uint4 v = *reinterpret_cast<const uint4*>(stage + row * 64 + ((j ^ (row >> 1 & 3)) << 4));
+                        if (at < 0) continue;
+                        __nv_bfloat16* dst = p.out + at + c + 8 * j;
+                        if (p.vec_out) {
+                            *reinterpret_cast<uint4*>(dst) = v;
+                        } else {
+                            uint32_t* d = reinterpret_cast<uint32_t*>(dst);
+                            d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
                         }
                     }
                 }
@@ -599,10 +654,10 @@ size_t smem_bytes(int q_blocks, int blocks, int stages) { return (size_t)q_block
 // value columns of a CTA: all up to 256, else chunks of 256 (0: not taken)
 int value_columns(int E) { return E % 64 ? 0 : E <= 256 ? E : E % 256 ? 0 : 256; }
 
-template <bool SHAPED, bool WIDE>
+template <bool SHAPED, int PER_SM>
 int launch_one(const char* what, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const ShapedParams& p, size_t smem, int num_tiles,
                cudaStream_t stream) {
-    auto* kernel = shaped_attention_sm100_kernel<SHAPED, WIDE>;
+    auto* kernel = shaped_attention_sm100_kernel<SHAPED, PER_SM>;
     static forge::PerDeviceFlag configured_on;
     bool& configured = configured_on.current();
     if (!configured) {
@@ -612,11 +667,11 @@ int launch_one(const char* what, const CUtensorMap& tq, const CUtensorMap& tk, c
         cudaFuncAttributes attr;
         e = cudaFuncGetAttributes(&attr, kernel);
         if (e != cudaSuccess) return forge::fail(FORGE_ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(e));
-        if (!WIDE && attr.numRegs * 2 < kRegsFew + kRegsMany)
-            return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: built with %d registers per thread, needs %d", what, attr.numRegs, (kRegsFew + kRegsMany + 1) / 2);
+        if (PER_SM > 1 && attr.numRegs * 3 < kRegsFew + 2 * kRegsMany)
+            return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: built with %d registers per thread, needs %d", what, attr.numRegs, (kRegsFew + 2 * kRegsMany + 2) / 3);
         configured = true;
     }
-    return forge::check_launch(what, forge::launch(kernel, dim3((unsigned)num_tiles * p.inner), dim3(WIDE ? 384 : 256), smem, stream, 1, tq, tk, tv, p));
+    return forge::check_launch(what, forge::launch(kernel, dim3((unsigned)num_tiles * p.inner), dim3(kThreads), smem, stream, 1, tq, tk, tv, p));
 }
 
 template <bool SHAPED>
@@ -630,16 +685,18 @@ int launch(const char* what, const CUtensorMap& tq, const CUtensorMap& tk, const
     }
     p.stages = kMaxStages;
     while (p.stages > 1 && smem_bytes(q_blocks, blocks, p.stages) > kSmemLimit) --p.stages;
-    // (heads of 128 + 64 channels, keys and values packed: one tile of keys a CTA and two CTAs an SM 49.2 us, three and one CTA 59.0)
-    if (p.row_start && 2 * BKV + p.VC <= 256 && smem_bytes(q_blocks, blocks, 1) <= 112 * 1024)
-        while (smem_bytes(q_blocks, blocks, p.stages) > 112 * 1024) --p.stages;
+    // Two CTAs an SM with fewer stages beat one with more where there are CTAs for both (one map, heads of 128 and values of 128, 2,048 tokens: 80.9 ->
+    // 58.9 us; 128 + 64 channels packed, which leaves one stage each, 1,536 tokens: 52.7 -> 39.5); where every CTA has an SM of its own the stages win
+    // (100 tokens behind 1,000: 24.8 us against 31.1).
+    if ((long long)num_tiles * p.inner > forge::sm_count() && 2 * BKV + p.VC <= 256 && smem_bytes(q_blocks, blocks, 1) <= kSmemTwo)
+        while (smem_bytes(q_blocks, blocks, p.stages) > kSmemTwo) --p.stages;
     const size_t smem = smem_bytes(q_blocks, blocks, p.stages);
     if (smem > kSmemLimit) return forge::fail(FORGE_ERR_UNSUPPORTED, "%s: queries of %d channels", what, p.q_channels);
     p.tmem_cols = 2 * BKV + p.VC + (p.q_tmem ? p.value_blocks * 32 : 0) <= 256 ? 256 : 512;
     p.box_rows = p.page_size < BKV ? p.page_size : BKV;
-    // one CTA an SM, by its tensor memory or its shared memory: two threads a row
-    const bool alone = p.tmem_cols > 256 || smem > 112 * 1024;
-    return alone ? launch_one<SHAPED, true>(what, tq, tk, tv, p, smem, num_tiles, stream) : launch_one<SHAPED, false>(what, tq, tk, tv, p, smem, num_tiles, stream);
+    // one CTA an SM, by its tensor memory or its shared memory, or two
+    const bool alone = p.tmem_cols > 256 || smem > kSmemTwo;
+    return alone ? launch_one<SHAPED, 1>(what, tq, tk, tv, p, smem, num_tiles, stream) : launch_one<SHAPED, 2>(what, tq, tk, tv, p, smem, num_tiles, stream);
 }
 
 }  // namespace
@@ -656,14 +713,13 @@ extern "C" int forge_scored_sm100_supports(int H, int G, int M, int D, int E, in
     return (pages_fit(page_size) && H > 0 && G > 0 && H % G == 0 && H / G <= BQ && (M == 1 || M == 2) && (D == 64 || D == 128) && value_columns(E) > 0) ? 1 : 0;
 }
 
-// q bf16 [T, H, C+R]; cache: pages of page_size rows of C+R; out bf16 [T, H, C].  tile_t0 / tile_n: tiles of up to 128 / H tokens of one
-// request, the first to run first.  window, sink as for forge_latent_attention_mma.  status: bit 1 is raised where a wait ran out.
-extern "C" int forge_latent_attention_sm100(const void* q, const void* cache, const int32_t* block_table, const int32_t* tok_req,
-                                            const int32_t* positions, const int32_t* tile_t0, const int32_t* tile_n, void* out, int* status, int T,
+// q bf16 [T, H, C+R]; cache: pages of page_size rows of C+R; out bf16 [T, H, C].  tiles int32 [num_tiles, 4]: up to 128 / H tokens of one
+// request each (first token, tokens, request, the first token's position), the first to run first.  window, sink as for forge_latent_attention_mma.  status: bit 1 is raised where a wait ran out.
+extern "C" int forge_latent_attention_sm100(const void* q, const void* cache, const int32_t* block_table, const int32_t* tiles, void* out, int* status, int T,
                                             int num_tiles, int num_pages, int H, int C, int R, int page_size, int max_pages, float scale, int window,
                                             const float* sink, cudaStream_t stream) {
     if (!forge_latent_sm100_supports(H, C, R, page_size)) return forge::fail(FORGE_ERR_UNSUPPORTED, "latent_attention_sm100: H=%d C=%d R=%d page=%d", H, C, R, page_size);
-    if (T < 0 || num_tiles < 0 || num_pages <= 0 || max_pages <= 0 || !tile_t0 || !tile_n || !(scale > 0.f))
+    if (T < 0 || num_tiles < 0 || num_pages <= 0 || max_pages <= 0 || !tiles || ((uintptr_t)tiles & 15) || !(scale > 0.f))
         return forge::fail(FORGE_ERR_ARG, "latent_attention_sm100: bad arguments");
     if (T == 0 || num_tiles == 0) return FORGE_OK;
     const int KD = C + R, VC = value_columns(C), chunks = C / VC;
@@ -677,7 +733,7 @@ extern "C" int forge_latent_attention_sm100(const void* q, const void* cache, co
         return forge::fail(FORGE_ERR_UNSUPPORTED, "latent_attention_sm100: cache: %s", err);
     ShapedParams p{};
     p.out = (__nv_bfloat16*)out; p.out_ld = (long long)H * C;
-    p.block_table = block_table; p.tok_req = tok_req; p.positions = positions; p.tile_t0 = tile_t0; p.tile_n = tile_n;
+    p.block_table = block_table; p.tiles = reinterpret_cast<const int4*>(tiles);
     p.sink = sink; p.q = (const __nv_bfloat16*)q;
     p.H = p.heads = H; p.inner = chunks; p.M = 1; p.D = KD; p.E = C; p.VC = VC;
     p.q_channels = KD; p.value_blocks = VC / 64; p.key_blocks = (KD + 63) / 64 - p.value_blocks; p.latent = 1;
@@ -697,12 +753,11 @@ extern "C" int forge_expanded_sm100_supports(int H, int D, int R, int E) {
 
 // q bf16 [T, H, D+R]; kv bf16 [rows, H, D+E]: keys and values of every request of the step, position by position, request s from row row_start[s]
 // on; kr bf16 [rows, R]; out bf16, rows of out_ld, head h's E values from h * E on.  Tiles of up to 128 tokens; the rest as above.
-extern "C" int forge_expanded_attention_sm100(const void* q, const void* kv, const void* kr, const int32_t* row_start, const int32_t* tok_req,
-                                              const int32_t* positions, const int32_t* tile_t0, const int32_t* tile_n, void* out, int* status, int T,
+extern "C" int forge_expanded_attention_sm100(const void* q, const void* kv, const void* kr, const int32_t* row_start, const int32_t* tiles, void* out, int* status, int T,
                                               int num_tiles, int rows, int H, int D, int R, int E, float scale, const float* sink, long long out_ld,
                                               cudaStream_t stream) {
     if (!forge_expanded_sm100_supports(H, D, R, E)) return forge::fail(FORGE_ERR_UNSUPPORTED, "expanded_attention_sm100: H=%d D=%d R=%d E=%d", H, D, R, E);
-    if (T < 0 || num_tiles < 0 || rows <= 0 || !row_start || !tile_t0 || !tile_n || !(scale > 0.f) || out_ld < (long long)H * E || (out_ld & 1) ||
+    if (T < 0 || num_tiles < 0 || rows <= 0 || !row_start || !tiles || ((uintptr_t)tiles & 15) || !(scale > 0.f) || out_ld < (long long)H * E || (out_ld & 1) ||
         ((uintptr_t)out & 3))
         return forge::fail(FORGE_ERR_ARG, "expanded_attention_sm100: bad arguments");
     if (T == 0 || num_tiles == 0) return FORGE_OK;
@@ -716,7 +771,7 @@ extern "C" int forge_expanded_attention_sm100(const void* q, const void* kv, con
         return forge::fail(FORGE_ERR_UNSUPPORTED, "expanded_attention_sm100: keys and values: %s", err);
     ShapedParams p{};
     p.out = (__nv_bfloat16*)out; p.out_ld = out_ld;
-    p.tok_req = tok_req; p.positions = positions; p.tile_t0 = tile_t0; p.tile_n = tile_n; p.row_start = row_start;
+    p.tiles = reinterpret_cast<const int4*>(tiles); p.row_start = row_start;
     p.sink = sink;
     p.H = H; p.heads = 1; p.inner = H; p.M = 1; p.D = D; p.E = E; p.VC = E;
     p.q_channels = D + R; p.key_blocks = (D + R + 63) / 64; p.value_blocks = E / 64; p.latent = 0;
@@ -729,14 +784,13 @@ extern "C" int forge_expanded_attention_sm100(const void* q, const void* kv, con
 // q bf16 [T, H, M, D]; cache pages of page_stride numbers, [G, page_size, M*D] keys then [G, page_size, E] values; one map: out bf16, rows of
 // out_ld, times out_scale; two: the maps' outputs go through u fp32 [T, H, 2, E], and a second kernel makes (a_1 - lambda a_2) / its root mean square
 // * post * out_scale of them.  The rest as for forge_scored_attention_mma; tiles of up to 128 / (H/G) tokens.
-extern "C" int forge_scored_attention_sm100(const void* q, const void* cache, const int32_t* block_table, const int32_t* tok_req,
-                                            const int32_t* positions, const int32_t* tile_t0, const int32_t* tile_n, const float* r1, const float* r2,
+extern "C" int forge_scored_attention_sm100(const void* q, const void* cache, const int32_t* block_table, const int32_t* tiles, const float* r1, const float* r2,
                                             float* u, void* out, int* status, int T, int num_tiles, int num_pages, int H, int G, int M, int D, int E,
                                             int page_size, long long page_stride, int max_pages, float scale, float lambda, float post, float eps, float out_scale,
                                             long long out_ld, int window, int chunk, float softcap, const float* sink, cudaStream_t stream) {
     if (!forge_scored_sm100_supports(H, G, M, D, E, page_size))
         return forge::fail(FORGE_ERR_UNSUPPORTED, "scored_attention_sm100: H=%d G=%d M=%d D=%d E=%d page=%d", H, G, M, D, E, page_size);
-    if (T < 0 || num_tiles < 0 || num_pages <= 0 || max_pages <= 0 || !tile_t0 || !tile_n || !(scale > 0.f) || (r1 == nullptr) != (r2 == nullptr) ||
+    if (T < 0 || num_tiles < 0 || num_pages <= 0 || max_pages <= 0 || !tiles || ((uintptr_t)tiles & 15) || !(scale > 0.f) || (r1 == nullptr) != (r2 == nullptr) ||
         (M == 2 && !u) || !out || (sink && M != 1) || window < 0 || chunk < 0 || softcap < 0.f ||
         out_ld < (long long)H * E || (out_ld & 1) || page_stride < (long long)G * page_size * (M * D + E))
         return forge::fail(FORGE_ERR_ARG, "scored_attention_sm100: bad arguments");
@@ -751,7 +805,7 @@ extern "C" int forge_scored_attention_sm100(const void* q, const void* cache, co
         return forge::fail(FORGE_ERR_UNSUPPORTED, "scored_attention_sm100: cache: %s", err);
     ShapedParams p{};
     p.out = (__nv_bfloat16*)out; p.out_ld = out_ld; p.u = M == 2 ? u : nullptr;
-    p.block_table = block_table; p.tok_req = tok_req; p.positions = positions; p.tile_t0 = tile_t0; p.tile_n = tile_n;
+    p.block_table = block_table; p.tiles = reinterpret_cast<const int4*>(tiles);
     p.r1 = r1; p.r2 = r2; p.sink = sink;
     p.H = H; p.heads = Gq; p.inner = G * M * (E / VC); p.M = M; p.D = D; p.E = E; p.VC = VC;
     p.q_channels = D; p.key_blocks = D / 64; p.value_blocks = VC / 64; p.latent = 0;

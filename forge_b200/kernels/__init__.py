@@ -110,10 +110,10 @@ _SIGNATURES = {
     "attention_shaped": {
         "forge_latent_sm100_supports": [_I] * 4,
         "forge_scored_sm100_supports": [_I] * 6,
-        "forge_latent_attention_sm100": [_P] * 9 + [_I] * 8 + [_F, _I, _P, _P],
+        "forge_latent_attention_sm100": [_P] * 6 + [_I] * 8 + [_F, _I, _P, _P],
         "forge_expanded_sm100_supports": [_I] * 4,
-        "forge_expanded_attention_sm100": [_P] * 10 + [_I] * 7 + [_F, _P, _LL, _P],
-        "forge_scored_attention_sm100": [_P] * 12 + [_I] * 9 + [_LL, _I] + [_F] * 5 + [_LL, _I, _I, _F, _P, _P],
+        "forge_expanded_attention_sm100": [_P] * 7 + [_I] * 7 + [_F, _P, _LL, _P],
+        "forge_scored_attention_sm100": [_P] * 9 + [_I] * 9 + [_LL, _I] + [_F] * 5 + [_LL, _I, _I, _F, _P, _P],
     },
     "moe": {
         "forge_moe_route": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _I, _F, _P],
@@ -965,18 +965,26 @@ def headmix_plan(batch, TQ, device):
     return plan
 
 
+def _tokens_before(batch):
+    """How many tokens each of the step's requests had in the cache before it."""
+    before = getattr(batch, "host_context_before", None)
+    if not before:                     # (a batch that was not laid out by the engine)
+        before = batch.host_context_before = batch.positions[torch.tensor(batch.host_q_start[:-1], device=batch.positions.device)].tolist()
+    return before
+
+
 def shaped_plan(batch, TQ, device):
-    """The step's tokens cut into tiles of up to TQ consecutive tokens of one request (first token, count), those that reach furthest
-    first, made once per step: for the tcgen05 kernels of prompt portions, whose CTAs are handed out in that order."""
+    """The step's tokens cut into tiles of up to TQ consecutive tokens of one request, int32 [tiles, 4]: (first token, tokens, request, the first
+    token's position), those that reach furthest first, made once per step: for the tcgen05 kernels of prompt portions, whose CTAs are handed out in that
+    order."""
     key = ("shaped", TQ)
     plan = batch.attention_plan.get(key)
     if plan is None:
-        qs, before = batch.host_q_start, getattr(batch, "host_context_before", None) or [0] * batch.num_requests
-        tiles = [(before[s] + min(a + TQ, qs[s + 1]) - qs[s], a, min(TQ, qs[s + 1] - a))
-                 for s in range(batch.num_requests) for a in range(qs[s], qs[s + 1], TQ)]
-        tiles.sort(key=lambda t: (-t[0], t[1]))
+        qs, before = batch.host_q_start, _tokens_before(batch)
+        tiles = [(a, min(TQ, qs[s + 1] - a), s, before[s] + a - qs[s]) for s in range(batch.num_requests) for a in range(qs[s], qs[s + 1], TQ)]
+        tiles.sort(key=lambda t: (-t[3] - t[1], t[0]))
         with once_per_step():
-            plan = batch.attention_plan[key] = (new_ints([t[1] for t in tiles], device), new_ints([t[2] for t in tiles], device), len(tiles))
+            plan = batch.attention_plan[key] = new_ints(tiles, device)
     return plan
 
 
@@ -1150,13 +1158,12 @@ def scored_attention(q, cache, group_batch, batch, H, G, M, D, E, page_size, sca
         # device time is 0.34 to 0.88 of that kernel's from 24 to 1,536 tokens of 1 to 4 requests, with single tokens beside them too
         sm = library("attention_shaped")
         if sm.forge_scored_sm100_supports.fn(H, G, M, D, E, page_size):
-            t0, tn, tiles = shaped_plan(batch, 128 // (H // G), q.device)
+            tiles = shaped_plan(batch, 128 // (H // G), q.device)
             u = new_tensor((T, H, M, E), torch.float32, q.device) if M == 2 else None
             _check(sm, sm.forge_scored_attention_sm100(
                 _need(q, "q", torch.bfloat16, 2), _need(cache, "cache", torch.bfloat16), _need(group_batch.block_table, "block_table", torch.int32, 2),
-                _need(batch.tok_req, "tok_req", torch.int32), _need(batch.positions, "positions", torch.int32), _need(t0, "tile_t0", torch.int32),
-                _need(tn, "tile_n", torch.int32), _opt(r1, "r1", torch.float32), _opt(r2, "r2", torch.float32), _opt(u, "u", torch.float32), out_ptr,
-                _need(_gemm_status(q.device), "status", torch.int32), T, tiles, cache.shape[0], H, G, M, D, E, page_size, _page_stride(cache),
+                _need(tiles, "tiles", torch.int32, 2), _opt(r1, "r1", torch.float32), _opt(r2, "r2", torch.float32), _opt(u, "u", torch.float32), out_ptr,
+                _need(_gemm_status(q.device), "status", torch.int32), T, tiles.shape[0], cache.shape[0], H, G, M, D, E, page_size, _page_stride(cache),
                 group_batch.block_table.shape[1], float(scale), float(lam), float(post), float(eps), float(out_scale), out_ld, window, chunk, softcap,
                 _opt(sink, "sink", torch.float32), _stream()), "scored_attention_sm100")
             if M == 2:
@@ -1611,12 +1618,11 @@ def latent_attention(q, cache, group_batch, batch, H, C, R, page_size, scale, wi
         # prompt portions: tcgen05, tiles of 128 rows (a layer's device time is 0.35 to 0.90 of the mma.sync kernel's over the same steps as above)
         sm = library("attention_shaped")
         if sm.forge_latent_sm100_supports.fn(H, C, R, page_size):
-            t0, tn, tiles = shaped_plan(batch, 128 // H, q.device)
+            tiles = shaped_plan(batch, 128 // H, q.device)
             out = new_tensor((T, H * C), q.dtype, q.device)
             _check(sm, sm.forge_latent_attention_sm100(
                 _need(q, "q", torch.bfloat16, 2), _need(cache, "cache", torch.bfloat16), _need(group_batch.block_table, "block_table", torch.int32, 2),
-                _need(batch.tok_req, "tok_req", torch.int32), _need(batch.positions, "positions", torch.int32), _need(t0, "tile_t0", torch.int32),
-                _need(tn, "tile_n", torch.int32), _need(out, "out", torch.bfloat16), _need(_gemm_status(q.device), "status", torch.int32), T, tiles,
+                _need(tiles, "tiles", torch.int32, 2), _need(out, "out", torch.bfloat16), _need(_gemm_status(q.device), "status", torch.int32), T, tiles.shape[0],
                 cache.shape[0], H, C, R, page_size, group_batch.block_table.shape[1], float(scale), window, _opt(sink, "sink", torch.float32), _stream()),
                 "latent_attention_sm100")
             return out
@@ -1678,7 +1684,7 @@ def latent_expand_pays(batch, H, D, R, E, C):
     if pays is None:
         pays = False
         if _brings_portions(batch):
-            qs, before = batch.host_q_start, getattr(batch, "host_context_before", None) or [0] * batch.num_requests
+            qs, before = batch.host_q_start, _tokens_before(batch)
             rows = before[-1] + qs[-1] + sum(before[:-1])
             if 2 * rows * H * (D + E) <= EXPANDED_SCRATCH:
                 def tiles(TQ):                                  # (of keys: the longest row of tiles, all)
@@ -1706,7 +1712,7 @@ def latent_expand(q, cache, group_batch, batch, H, C, D, R, page_size, freq, amp
     T, dev, S = q.shape[0], q.device, batch.num_requests
     plan = batch.attention_plan.get("rows")
     if plan is None:
-        qs, before, starts = batch.host_q_start, getattr(batch, "host_context_before", None) or [0] * S, [0]
+        qs, before, starts = batch.host_q_start, _tokens_before(batch), [0]
         for s in range(S):
             starts.append(starts[-1] + before[s] + qs[s + 1] - qs[s])
         with once_per_step():
@@ -1733,12 +1739,11 @@ def expanded_attention(q, kv, kr, row_start, batch, H, D, R, E, scale, sink=None
         raise KernelError(f"expanded_attention: {sink.numel()} sinks for {H} heads")
     if q.shape[1] != H * (D + R) or kv.shape[1] != H * (D + E) or kr.shape[1] != R or kv.shape[0] != kr.shape[0]:
         raise KernelError(f"expanded_attention: q {tuple(q.shape)}, kv {tuple(kv.shape)}, kr {tuple(kr.shape)} do not fit {H} heads of {D} + {R} and {E}")
-    t0, tn, tiles = shaped_plan(batch, 128, dev)
+    tiles = shaped_plan(batch, 128, dev)
     out, out_ptr, out_ld = _out_slice(out, H * E, T, torch.bfloat16, dev)
     _check(lib, lib.forge_expanded_attention_sm100(
         _need(q, "q", torch.bfloat16, 2), _need(kv, "kv", torch.bfloat16, 2), _need(kr, "kr", torch.bfloat16, 2), _need(row_start, "row_start", torch.int32),
-        _need(batch.tok_req, "tok_req", torch.int32), _need(batch.positions, "positions", torch.int32), _need(t0, "tile_t0", torch.int32),
-        _need(tn, "tile_n", torch.int32), out_ptr, _need(_gemm_status(dev), "status", torch.int32), T, tiles, kv.shape[0], H, D, R, E, float(scale),
+        _need(tiles, "tiles", torch.int32, 2), out_ptr, _need(_gemm_status(dev), "status", torch.int32), T, tiles.shape[0], kv.shape[0], H, D, R, E, float(scale),
         _opt(sink, "sink", torch.float32), out_ld, _stream()), "expanded_attention_sm100")
     return out
 
