@@ -381,7 +381,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const uint32_t leader = elect_one();
+            if (GROUPED) num_tiles = __shfl_sync(0xffffffffu, num_tiles, 0);
             constexpr uint32_t idesc = umma_idesc_bf16_f32(BM, BN);
             uint32_t it = 0;
             bool ok = true;
@@ -389,24 +391,24 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
                 const int a = local & 1;
                 const uint32_t aph = (local >> 1) & 1;
-                if (!(ok = mbar_wait(&acc_empty[a], aph ^ 1, abort, p.status))) break;
+                if (!(ok = warp_wait(&acc_empty[a], aph ^ 1, abort, p.status))) break;
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + a * BN;
+                const uint32_t d_tmem = __shfl_sync(0xffffffffu, tmem_base, 0) + a * BN;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % kStages;
                     const uint32_t ph = (it / kStages) & 1;
-                    if (!(ok = mbar_wait(&full[s], ph, abort, p.status))) break;
+                    if (!(ok = warp_wait(&full[s], ph, abort, p.status))) break;
                     tc_fence_after_sync();
                     const uint32_t a_addr = smem_u32(tiles + s * C::kStageBytes);
                     const uint64_t a_desc = umma_desc_k_sw128(a_addr), w_desc = umma_desc_k_sw128(a_addr + BM * BK * 2);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
-                        umma_bf16(d_tmem, umma_desc_advance(a_desc, k * UMMA_K * 2), umma_desc_advance(w_desc, k * UMMA_K * 2),
+                        umma_bf16_by(leader, d_tmem, umma_desc_advance(a_desc, k * UMMA_K * 2), umma_desc_advance(w_desc, k * UMMA_K * 2),
                                   idesc, k != 0 || kb != 0);
                     }
-                    umma_commit(&empty[s]);       // stage is free once these MMAs have read it
+                    umma_commit_by(leader, &empty[s]);       // stage is free once these MMAs have read it
                 }
-                if (ok) umma_commit(&acc_full[a]);
+                if (ok) umma_commit_by(leader, &acc_full[a]);
             }
         }
     } else {
@@ -551,17 +553,18 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorM
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
         ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_bf16_pair(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
 // One arrival on the barrier at this offset in BOTH CTAs of the pair once all MMAs issued so far have completed.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3)) : "memory");
+__device__ __forceinline__ void umma_commit_pair(uint32_t leader, uint64_t* bar) {
+    asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
+                 "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+                 ::"r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3)), "r"(leader) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
@@ -662,7 +665,8 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (the even CTA's)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const uint32_t leader = elect_one();
             constexpr uint32_t idesc = umma_idesc_bf16_f32(2 * BM, PBN);
             uint32_t it = 0;
             bool ok = true;
@@ -670,13 +674,13 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
             for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
                 const int a = local & 1;
                 const uint32_t aph = (local >> 1) & 1;
-                if (!(ok = mbar_wait(&acc_empty[a], aph ^ 1, abort, p.status))) break;
+                if (!(ok = warp_wait(&acc_empty[a], aph ^ 1, abort, p.status))) break;
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + a * PBN;
+                const uint32_t d_tmem = __shfl_sync(0xffffffffu, tmem_base, 0) + a * PBN;
                 for (int gi = 0; gi < num_groups; ++gi, ++it) {
                     const int s = it % kStages;
                     const uint32_t ph = (it / kStages) & 1;
-                    if (!(ok = mbar_wait(&full[s], ph, abort, p.status))) break;
+                    if (!(ok = warp_wait(&full[s], ph, abort, p.status))) break;
                     tc_fence_after_sync();
                     const uint32_t a_addr = smem_u32(tiles + s * kStageBytes);
                     const uint64_t a_desc = umma_desc_k_sw128(a_addr), w_desc = umma_desc_k_sw128(a_addr + kABytes);
@@ -686,13 +690,13 @@ gemm_sm100_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                         if (j >= here) break;
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; ++k)
-                            umma_bf16_pair(d_tmem, umma_desc_advance(a_desc, j * (BM * BK * 2) + k * UMMA_K * 2),
+                            umma_bf16_pair(leader, d_tmem, umma_desc_advance(a_desc, j * (BM * BK * 2) + k * UMMA_K * 2),
                                            umma_desc_advance(w_desc, j * (BNH * BK * 2) + k * UMMA_K * 2), idesc,
                                            (j | k) != 0 || gi != 0);
                     }
-                    umma_commit_pair(&empty[s]);
+                    umma_commit_pair(leader, &empty[s]);
                 }
-                if (ok) umma_commit_pair(&acc_full[a]);
+                if (ok) umma_commit_pair(leader, &acc_full[a]);
             }
         }
     } else {
@@ -888,12 +892,13 @@ gemm_sm100_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const uint32_t leader = elect_one(), d_tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
             constexpr uint32_t idesc = umma_idesc_bf16_f32(BM, BN);
             bool ok = true;
             for (int i = 0; i < my_groups && ok; ++i) {
                 const int s = i % kStages;
-                if (!(ok = mbar_wait(&full[s], (i / kStages) & 1, abort, p.status))) break;
+                if (!(ok = warp_wait(&full[s], (i / kStages) & 1, abort, p.status))) break;
                 tc_fence_after_sync();
                 const uint32_t slot = smem_u32(tiles + s * C::kStageBytes);
                 const int n_here = min(G, my_kb - i * G);
@@ -903,12 +908,12 @@ gemm_sm100_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                     const uint64_t a_desc = umma_desc_k_sw128(slot + g * kTileA), w_desc = umma_desc_k_sw128(slot + G * kTileA + g * kTileW);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        umma_bf16(tmem_base, umma_desc_advance(a_desc, k * UMMA_K * 2), umma_desc_advance(w_desc, k * UMMA_K * 2),
+                        umma_bf16_by(leader, d_tmem, umma_desc_advance(a_desc, k * UMMA_K * 2), umma_desc_advance(w_desc, k * UMMA_K * 2),
                                   idesc, k != 0 || g != 0 || i != 0);
                 }
-                umma_commit(&empty[s]);
+                umma_commit_by(leader, &empty[s]);
             }
-            if (ok && my_kb > 0) umma_commit(acc_full);
+            if (ok && my_kb > 0) umma_commit_by(leader, acc_full);
         }
     } else {
         // warps 2..5: this CTA's partial sums out of tensor memory, a row per thread
@@ -1150,15 +1155,18 @@ gemm_sm100_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
             }
         }
     } else if (warp == 1 || warp == 6) {
-        if (lane == 0) {
-            // issuer 0 (warp 1) takes k-blocks 0 and 2 of every group, issuer 1 (warp 6) k-blocks 1 and 3
-            const int who = warp == 1 ? 0 : 1;
-            const uint32_t d_tmem = tmem_base + who * NT;
+        {
+            const uint32_t leader = elect_one();
+            // issuer 0 (warp 1) takes k-blocks 0 and 2 of every group, issuer 1 (warp 6) k-blocks 1 and 3.  (The whole warp walks this loop, as in every
+            // kernel of this file: issued from a branch of one lane the products of the last stage were what a CTA ended on.  [2048 x 5632] at 8 rows
+            // 8.87 -> 7.9 us, a decode step of 22 layers 0.80 -> 0.77 ms.)
+            const int who = __shfl_sync(0xffffffffu, warp == 1 ? 0 : 1, 0);
+            const uint32_t d_tmem = __shfl_sync(0xffffffffu, tmem_base, 0) + who * NT;
             constexpr uint32_t idesc = umma_idesc_bf16_f32(BM, NT);
             bool ok = true, fresh = true;
             for (int i = 0; i < my_groups && ok; ++i) {
                 const int s = i % kStages;
-                if (!(ok = mbar_wait(&full[s], (i / kStages) & 1, abort, p.status))) break;
+                if (!(ok = warp_wait(&full[s], (i / kStages) & 1, abort, p.status))) break;
                 tc_fence_after_sync();
                 const uint64_t w_desc = umma_desc_k_sw128(smem_u32(w_tiles + s * w_bytes));
                 const uint64_t x_desc = umma_desc_k_sw128(smem_u32(x_tiles + s * x_bytes));
@@ -1169,13 +1177,13 @@ gemm_sm100_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
                     if (j >= here) break;
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        umma_bf16(d_tmem, umma_desc_advance(w_desc, j * w_block + k * UMMA_K * 2),
+                        umma_bf16_by(leader, d_tmem, umma_desc_advance(w_desc, j * w_block + k * UMMA_K * 2),
                                   umma_desc_advance(x_desc, j * (NT * BK * 2) + k * UMMA_K * 2), idesc, !(fresh && k == 0));
                     fresh = false;
                 }
-                umma_commit(&reuse[s]);           // one of the two arrivals that free the stage
+                umma_commit_by(leader, &reuse[s]);           // one of the two arrivals that free the stage
             }
-            if (ok && my_kb > 0) umma_commit(acc_full);
+            if (ok && my_kb > 0) umma_commit_by(leader, acc_full);
         }
     } else {
         const int quarter = warp & 3;
@@ -1450,29 +1458,32 @@ gemm_sm100_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const uint32_t leader = elect_one(), acc0 = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const int last = __shfl_sync(0xffffffffu, tile_last, 0), first_tile = __shfl_sync(0xffffffffu, tile_first, 0);
+            const int from = __shfl_sync(0xffffffffu, u_begin, 0), to = __shfl_sync(0xffffffffu, u_end, 0);
             constexpr uint32_t idesc = umma_idesc_bf16_f32(BM, NT);
             bool ok = true;
             int frag = 0, i = 0;
-            for (int tile = tile_last; tile >= tile_first && ok; --tile, ++frag) {
-                const int f_begin = max(u_begin, tile * num_kb), f_end = min(u_end, (tile + 1) * num_kb);
+            for (int tile = last; tile >= first_tile && ok; --tile, ++frag) {
+                const int f_begin = max(from, tile * num_kb), f_end = min(to, (tile + 1) * num_kb);
                 const int a = frag & 1;
-                if (!(ok = mbar_wait(&acc_empty[a], ((frag >> 1) & 1) ^ 1, abort, p.status))) break;
+                if (!(ok = warp_wait(&acc_empty[a], ((frag >> 1) & 1) ^ 1, abort, p.status))) break;
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + a * NT;
+                const uint32_t d_tmem = acc0 + a * NT;
                 for (int u = f_begin; u < f_end; ++u, ++i) {
                     const int s = i % kStages;
-                    if (!(ok = mbar_wait(&full[s], (i / kStages) & 1, abort, p.status))) break;
+                    if (!(ok = warp_wait(&full[s], (i / kStages) & 1, abort, p.status))) break;
                     tc_fence_after_sync();
                     const uint32_t w_addr = smem_u32(tiles + s * C::kStageBytes);
                     const uint64_t w_desc = umma_desc_k_sw128(w_addr), x_desc = umma_desc_k_sw128(w_addr + BM * BK * 2);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        umma_bf16(d_tmem, umma_desc_advance(w_desc, k * UMMA_K * 2), umma_desc_advance(x_desc, k * UMMA_K * 2),
+                        umma_bf16_by(leader, d_tmem, umma_desc_advance(w_desc, k * UMMA_K * 2), umma_desc_advance(x_desc, k * UMMA_K * 2),
                                   idesc, k != 0 || u != f_begin);
-                    umma_commit(&empty[s]);
+                    umma_commit_by(leader, &empty[s]);
                 }
-                if (ok) umma_commit(&acc_full[a]);
+                if (ok) umma_commit_by(leader, &acc_full[a]);
             }
         }
     } else {
