@@ -5,19 +5,19 @@
 // group) pair, row r <-> token r / G, head r % G, so a tile is 128 / G tokens (rounded down: with a group that
 // does not divide 128 the last rows of the tile stay empty) and the G heads share every key/value tile.  Per tile
 // of 64 keys (HD = head size):
-//   S = Q K^T      tcgen05.mma M=128 N=64 K=HD, Q and K in shared memory (TMA, 128-byte swizzle), S in TMEM
-//                  (two buffers: the scores of tile it + 2 are computed while the rows work on tile it)
-//   softmax        128 threads, one row each, hold the row's 64 scores in registers, online max/sum in fp32
-//                  (exp2 domain, packed fp32 arithmetic), write P as bf16 into shared memory in the MMA's
-//                  layout (two buffers); the output accumulator in TMEM is rescaled only when a row's
-//                  reference exponent has to move (a maximum that grew by more than 2^8)
-//   O += P V       tcgen05.mma M=128 N=64 K=64 per 64 columns of the head, P K-major, V MN-major (keys are rows of
-//                  128 bytes), O in TMEM
-// Warps 0-3 run one thread each: warp 0 feeds keys and values page by page through the request's block table
-// (one TMA box per page and operand; key and value tiles have rings of three slots each, keys run ahead),
-// warp 1 issues P V, warp 2 issues Q K^T; warps 4-7 are the softmax rows.  The first warpgroup hands most of
-// its registers to the second (setmaxnreg).  With head size 64 two such CTAs fit an SM (99 KB of shared memory,
-// 256 TMEM columns each); with 128 one does (163 KB).  Tiles are listed longest first and the kv heads of a tile are neighbouring CTAs, so the
+//   S = Q K^T      tcgen05.mma M=128 N=64 K=HD, Q and K in shared memory (TMA, 128-byte swizzle), S in TMEM (two or three buffers)
+//   softmax        256 threads, two a row with 32 of the tile's scores each in registers, online max/sum in fp32
+//                  (exp2 domain, packed fp32 arithmetic), P as bf16 into TMEM over the scores it came from; the output
+//                  accumulator in TMEM is rescaled only when a row's reference exponent has to move (a maximum that grew by more than 2^8)
+//   O += P V       tcgen05.mma M=128 N=HD K=64, P from TMEM, V MN-major (keys are rows of 128 bytes), O in TMEM
+// Warps 0 and 3 copy keys and values page by page through the request's block table (a ring of its own for either; the page is looked up a
+// tile ahead), warp 1 multiplies P V, warp 2 Q K^T: the whole warp walks the loop and the elected lane issues, so that operands come from
+// uniform registers.  Warps 4-11 are the softmax rows.  The first warpgroup hands most of its registers to the others (setmaxnreg).  Two such
+// CTAs fit an SM.  Before (one thread a row, P through shared memory, products and copies issued from branches of one lane, heads of 128 with one CTA
+// an SM) and now, in us: heads of 128, 32/8 of them, 1,500 tokens of three requests behind up to 1,000: 47.5, 29.4; 2,048 tokens 74, 48; heads of 64,
+// 32/4: 1,021 tokens of eight requests 10.7, 8.4; 300 tokens of three behind up to 500 15.3, 11.6; 2,048 tokens 42.4, 42.3 (there the
+// special-function unit is busy five sixths of the time: 64 weights of a tile and row at four a clock and scheduler).
+// Tiles are listed longest first and the kv heads of a tile are neighbouring CTAs, so the
 // long tiles of all heads start in the first wave.
 // A step with fewer tiles than the GPU has places for CTAs (a short portion on a long context) may list a tile several
 // times, each entry with a share of the tile's key tiles (``tile_cut``): such a CTA leaves its sums unnormalised in
@@ -40,22 +40,29 @@ using namespace sm100;
 
 constexpr int HD = FORGE_ATT_HD, BQ = 128, BKV = 64, UMMA_K = 16;
 static_assert(HD == 64 || HD == 128, "head size 64 or 128");
+#if FORGE_CHECKS
+constexpr bool kPagesMayBeSkipped = true;         // (a checks build skips a page id that is none)
+#else
+constexpr bool kPagesMayBeSkipped = false;
+#endif
 constexpr int KB = HD / 64;                       // 64-wide blocks of the head: Q, K and V tiles are KB swizzled blocks
-constexpr int kThreads = 256;                     // warps 0-3: copies, P V, Q K^T, (idle); warps 4-7: the softmax rows
-constexpr int kQkWarp = 2;
-constexpr int kCtasPerSm = 2;                     // what the register budget is made for (head size 128: one fits, by shared memory)
+constexpr int kThreads = 384;                     // warps 0-3: keys, P V, Q K^T, values; warps 4-11: the softmax rows
+constexpr int kQkWarp = 2, kValueWarp = 3, kRowWarps = 8, NK = BKV / 2;  // NK: a thread's keys of a tile
+constexpr int kCtasPerSm = 2;
 constexpr int kLaunchRegs = 65536 / (kThreads * kCtasPerSm) / 8 * 8;     // what the compiler gives every thread at launch
-constexpr int kRegsFew = 64, kRegsMany = 192;      // registers per thread of the two warpgroups after they trade
+constexpr int kRegsFew = 48, kRegsMany = 96;       // registers per thread of the three warpgroups after they trade
 // setmaxnreg only moves registers inside the CTA's allocation: asking for more than it holds waits for ever
-static_assert(kRegsFew + kRegsMany <= 2 * kLaunchRegs, "the two warpgroups cannot hold more registers than the CTA was given");
-constexpr int kTileBytes = BQ * 128;              // P, or one block of Q: 128 rows of 128 bytes
+static_assert(kRegsFew + 2 * kRegsMany <= 3 * kLaunchRegs, "the warpgroups cannot hold more registers than the CTA was given");
+constexpr int kTileBytes = BQ * 128;              // one block of Q: 128 rows of 128 bytes
 constexpr int kQBytes = KB * kTileBytes;
 constexpr int kKVBlock = BKV * 128;               // one block of a K or V tile: 64 keys of 128 bytes
 constexpr int kKVBytes = KB * kKVBlock;
-constexpr int kStages = 3;                        // ring slots for key tiles, and as many for value tiles
-constexpr int kPageWindow = 256;                  // block-table entries staged in shared memory at a time
-constexpr int kSmemBytes = kQBytes + 2 * kTileBytes + 2 * kStages * kKVBytes + 1024 + 1024 + kPageWindow * 4;
-constexpr int kTmemCols = 256;                    // S of even / odd tiles: columns 0..63 / 64..127, O: 128..128+HD-1
+constexpr int kStages = HD == 64 ? 4 : 2;         // ring slots for key tiles, and as many for value tiles: what two CTAs an SM leave
+constexpr int kSmemBytes = kQBytes + 2 * kStages * kKVBytes + 1024 + 512;
+static_assert(kSmemBytes <= 112 * 1024, "two CTAs an SM");
+constexpr int kBufs = HD == 64 ? 3 : 2;           // tiles whose scores or weights are in TMEM at a time: what 256 columns leave beside O
+constexpr int kTmemCols = 256, kTmemO = kBufs * BKV;                     // S of tile it: columns it % kBufs * 64 .. (P: the first 32 of them), then O
+static_assert(kTmemO + HD <= kTmemCols, "scores and outputs");
 
 struct AttnTcParams {
     __nv_bfloat16* out;           // [T, NH*HD]
@@ -110,17 +117,31 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // with the same references, makes the result independent of when the reference moved.
 constexpr float kRefSlack = 8.0f;
 
-// score i of the row's 64 (i is a constant after unrolling)
-#define SV(i) ((i) < 32 ? sv_lo[(i) & 31] : sv_hi[(i) & 31])
+// D[tmem] (+)= A[tmem] . B[smem]^T from the elected lane: row r of A is lane r, 16 keys are eight columns of two bfloat16 numbers
+__device__ __forceinline__ void umma_ts_by(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+          "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv,
                              const AttnTcParams p) {
     extern __shared__ uint8_t smem_raw[];
+    __shared__ float meet[2][BQ];                                   // [half]: what a row's two threads tell each other
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* q_s = smem;                                            // [KB][128][64] bf16, K-major, swizzled
-    uint8_t* p_s = smem + kQBytes;                                  // [2][128][64 keys] bf16, K-major, swizzled
-    uint8_t* k_s = p_s + 2 * kTileBytes;                            // [kStages][KB][64 keys][64]
+    uint8_t* k_s = smem + kQBytes;                                  // [kStages][KB][64 keys][64]
     uint8_t* v_s = k_s + kStages * kKVBytes;                        // [kStages][KB][64 keys][64]
     uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + kStages * kKVBytes);
     uint64_t* q_full = bars;
@@ -128,13 +149,11 @@ paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     uint64_t* k_empty = k_full + kStages;         // [kStages]
     uint64_t* v_full = k_empty + kStages;         // [kStages]
     uint64_t* v_empty = v_full + kStages;         // [kStages]
-    uint64_t* s_full = v_empty + kStages;         // [2]
-    uint64_t* p_ready = s_full + 2;               // [2]
-    uint64_t* o_done = p_ready + 2;               // [2]
-    uint64_t* s_free = o_done + 2;                // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_free + 2);
+    uint64_t* s_full = v_empty + kStages;         // [kBufs]
+    uint64_t* p_ready = s_full + kBufs;           // [kBufs]
+    uint64_t* o_done = p_ready + kBufs;           // [kBufs]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + kBufs);
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int32_t* page_win = reinterpret_cast<int32_t*>(bars) + 256;     // [kPageWindow] block-table entries
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // tiles come longest first, and CTAs are handed out in the order of blockIdx.x: the kv heads of one tile are
@@ -151,21 +170,19 @@ paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
             mbar_init(&v_full[s], 1);
             mbar_init(&v_empty[s], 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kBufs; ++b) {
             mbar_init(&s_full[b], 1);
-            mbar_init(&p_ready[b], 4);
-            mbar_init(&s_free[b], 4);
+            mbar_init(&p_ready[b], kRowWarps);
             mbar_init(&o_done[b], 1);
         }
         mbar_fence_init();
         prefetch_tensormap(&tmap_q);
         prefetch_tensormap(&tmap_kv);
     }
-    // key/value stages start as zeros: pages that are skipped (beyond the request, or released by the
-    // window) leave their rows as they are, and those rows must hold finite numbers (their weights are 0)
-    for (int i = threadIdx.x; i < 2 * kStages * kKVBytes / 16; i += kThreads) reinterpret_cast<uint4*>(k_s)[i] = make_uint4(0, 0, 0, 0);
-    // so do the rows of Q that a tile of fewer than 128 rows leaves unwritten
-    for (int i = threadIdx.x; i < kQBytes / 16; i += kThreads) reinterpret_cast<uint4*>(q_s)[i] = make_uint4(0, 0, 0, 0);
+    // Where a tile of keys comes as several pages the stages start as zeros: pages that are skipped (beyond the request, or released by the window) leave
+    // their rows as they are, and those rows must hold finite numbers (their weights are 0).  (A tile out of one page always lands whole.)
+    if (p.page_size < BKV || kPagesMayBeSkipped)
+        for (int i = threadIdx.x; i < 2 * kStages * kKVBytes / 16; i += kThreads) reinterpret_cast<uint4*>(k_s)[i] = make_uint4(0, 0, 0, 0);
     fence_proxy_async();
     if (warp == 1) {
         tmem_alloc(tmem_slot, kTmemCols);
@@ -199,161 +216,152 @@ paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     const int n_iter = t_end - t_begin;
     forge::pdl_wait();
 
-    // the softmax rows keep a row's 64 scores in registers; the other warpgroup runs single threads and gives
-    // its registers up for that
+    // the softmax rows keep their scores in registers; the other warpgroup gives its registers up for that
+    const int rounds = __shfl_sync(0xffffffffu, n_iter, 0);
     if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsFew));
-    if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer
-        // The warp stages the request's block-table entries in shared memory, a window at a time (one coalesced
-        // read instead of a dependent global load per page); lane 0 then issues the copies.
+    if (warp == 0 || warp == kValueWarp) {
+        // ------------------------------------------------------------------ copies: keys (and the queries), values
+        const bool values = warp == kValueWarp;
         const int32_t* table = p.block_table + (size_t)s_req * p.max_pages;
-        const int ppt = BKV / p.page_size;                               // pages per key tile
-        const int iters_per_win = kPageWindow / ppt;
+        const int page_shift = 31 - __clz(p.page_size), ppt = BKV >> page_shift;       // (the page size divides 64); pages per key tile
         const uint32_t page_bytes = p.page_size * 128;
-        if (lane == 0) {
+        if (!values && lane == 0) {
             mbar_arrive_expect_tx(q_full, KB * tile_rows * 128);
             for (int kb = 0; kb < KB; ++kb) tma_load_3d(q_s + kb * kTileBytes, &tmap_q, q_full, kb * 64, kvh * G, qs0 + row0 / G);
         }
-        bool ok = true;
-        int st = 0, ph = 0;                                              // ring slot and its phase
-        for (int it0 = 0; it0 < n_iter && ok; it0 += iters_per_win) {
-            const int it1 = min(n_iter, it0 + iters_per_win);
-            const int first_page = (t_begin + it0) * ppt;
+        // one lane a page: its first row of the cache, or -1 where no row of the tile sees a key of it.  Asked for a tile ahead.
+        auto page_of = [&](int it) {
+            int page = -1;
+            const int tp = (t_begin + it) * BKV + (lane << page_shift), idx = tp >> page_shift;
+            if (lane < ppt && it < rounds && tp < kv_hi && tp + p.page_size > kv_lo && idx < p.max_pages) page = table[idx];
+            return page;
+        };
+        uint64_t* full = values ? v_full : k_full;
+        uint64_t* empty = values ? v_empty : k_empty;
+        uint8_t* ring = values ? v_s : k_s;
+        int st = 0, ph = 0, next_page = page_of(0);
+        for (int it = 0; it < rounds; ++it) {
+            int page = next_page;
+            next_page = page_of(it + 1);
+            if (page >= 0 && !FORGE_PAGE_OK(page)) page = -1;
+            const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0));
+            if (!warp_wait<true>(&empty[st], ph ^ 1, abort, p.status, values ? 9 : 1)) break;
+            if (lane == 0) mbar_arrive_expect_tx(&full[st], KB * n_valid * page_bytes);
             __syncwarp();
-            for (int i = lane; i < (it1 - it0) * ppt; i += 32)
-                page_win[i] = first_page + i < p.max_pages ? table[first_page + i] : -1;
-            __syncwarp();
-            if (lane == 0) {
-                for (int it = it0; it < it1 && ok; ++it) {
-                    const int t0 = (t_begin + it) * BKV;
-                    int rows[8], n_valid = 0;
-                    for (int i = 0; i < ppt; ++i) {
-                        const int tp = t0 + i * p.page_size, page = page_win[(it - it0) * ppt + i];
-                        const bool live = tp < kv_hi && tp + p.page_size > kv_lo && page >= 0 && FORGE_PAGE_OK(page);
-                        rows[i] = live ? (page * 2 * p.NKV + kvh) * p.page_size : -1;
-                        n_valid += live;
-                    }
-                    // keys first: Q K^T of a tile runs two tiles ahead of its P V
-                    if (!(ok = mbar_wait<true>(&k_empty[st], ph ^ 1, abort, p.status, 1))) break;
-                    mbar_arrive_expect_tx(&k_full[st], KB * n_valid * page_bytes);
-                    for (int i = 0; i < ppt; ++i)
-                        if (rows[i] >= 0)
-                            for (int kb = 0; kb < KB; ++kb)
-                                tma_load_2d(k_s + st * kKVBytes + kb * kKVBlock + i * page_bytes, &tmap_kv, &k_full[st], kb * 64, rows[i]);
-                    if (!(ok = mbar_wait<true>(&v_empty[st], ph ^ 1, abort, p.status, 9))) break;
-                    mbar_arrive_expect_tx(&v_full[st], KB * n_valid * page_bytes);
-                    for (int i = 0; i < ppt; ++i)
-                        if (rows[i] >= 0)
-                            for (int kb = 0; kb < KB; ++kb)
-                                tma_load_2d(v_s + st * kKVBytes + kb * kKVBlock + i * page_bytes, &tmap_kv, &v_full[st], kb * 64,
-                                            rows[i] + p.NKV * p.page_size);
-                    if (++st == kStages) { st = 0; ph ^= 1; }
-                }
+            if (page >= 0) {
+                const int row = ((page * 2 + (values ? 1 : 0)) * p.NKV + kvh) * p.page_size;
+                uint8_t* dst = ring + st * kKVBytes + lane * page_bytes;
+                if (ppt == 1) tma_load_3d(dst, &tmap_kv, &full[st], 0, row, 0);              // (a box of all blocks)
+                else
+                    for (int kb = 0; kb < KB; ++kb) tma_load_3d(dst + kb * kKVBlock, &tmap_kv, &full[st], 0, row, kb);
             }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (++st == kStages) { st = 0; ph ^= 1; }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------------ P V issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_pv = umma_idesc_bf16_f32_bmn(BQ, 64);        // one product per 64 columns of the head
-            const uint32_t p_addr = smem_u32(p_s), v_addr = smem_u32(v_s);
-            bool ok = true;
-            int vst = 0, vph = 0;
-            for (int it = 0; it < n_iter && ok; ++it) {
-                const int b = it & 1;
-                if (!(ok = mbar_wait<true>(&v_full[vst], vph, abort, p.status, 4))) break;
-                if (!(ok = mbar_wait<true>(&p_ready[b], (it >> 1) & 1, abort, p.status, 5))) break;
-                tc_fence_after_sync();
-                const uint32_t pa = p_addr + b * kTileBytes, va = v_addr + vst * kKVBytes;
+        // ------------------------------------------------------------------ P V
+        constexpr uint32_t idesc_pv = umma_idesc_bf16_f32_bmn(BQ, HD);
+        const uint32_t leader = elect_one(), t_at = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint64_t v_desc0 = umma_desc_mn_sw128(smem_u32(v_s), kKVBlock);
+        int vst = 0, vph = 0;
+        for (int it = 0; it < rounds; ++it) {
+            const int b = it % kBufs, bp = it / kBufs & 1;
+            if (!warp_wait<true>(&v_full[vst], vph, abort, p.status, 4)) break;
+            if (!warp_wait<true>(&p_ready[b], bp, abort, p.status, 5)) break;
+            tc_fence_after_sync();
+            const uint64_t v_desc = umma_desc_advance(v_desc0, vst * kKVBytes);
 #pragma unroll
-                for (int nb = 0; nb < KB; ++nb)
-#pragma unroll
-                    for (int k = 0; k < BKV / UMMA_K; ++k)
-                        umma_bf16(tmem_base + 2 * BKV + nb * 64, umma_desc_k_sw128(pa + k * 32),
-                                  umma_desc_mn_sw128(va + nb * kKVBlock + k * 2048, 0), idesc_pv, (it | k) != 0);
-                umma_commit(&o_done[b]);
-                umma_commit(&v_empty[vst]);
-                if (++vst == kStages) { vst = 0; vph ^= 1; }
-            }
+            for (int k = 0; k < BKV / UMMA_K; ++k)
+                umma_ts_by(leader, t_at + kTmemO, t_at + b * BKV + k * 8, umma_desc_advance(v_desc, k * 2048), idesc_pv, k > 0 ? 1 : (uint32_t)(it > 0));
+            umma_commit_by(leader, &o_done[b]);
+            umma_commit_by(leader, &v_empty[vst]);
+            if (++vst == kStages) { vst = 0; vph ^= 1; }
         }
     } else if (warp == kQkWarp) {
-        // ------------------------------------------------------------------ Q K^T issuer
-        // A thread issues one tcgen05 instruction or barrier probe every 50 to 100 clocks, so the two products
-        // have a thread each.  S has two buffers in TMEM, and the rows hold S of tile it in registers from
-        // the start of their work on it: its buffer takes the scores of tile it + 2 while they compute.
-        if (lane == 0) {
-            constexpr uint32_t idesc_qk = umma_idesc_bf16_f32(BQ, BKV);
-            const uint32_t q_addr = smem_u32(q_s), k_addr = smem_u32(k_s);
-            bool ok = mbar_wait<true>(q_full, 0, abort, p.status, 2);
-            int kst = 0, kph = 0;
-            for (int it = 0; it < n_iter && ok; ++it) {
-                const int b = it & 1;
-                if (!(ok = mbar_wait<true>(&k_full[kst], kph, abort, p.status, 3))) break;
-                if (it >= 2 && !(ok = mbar_wait<true>(&s_free[b], ((it - 2) >> 1) & 1, abort, p.status, 11))) break;
-                // P V of tile it - 2 has read its P buffer before these scores exist: the rows, who wait for the
-                // scores, then need no probe of their own before they overwrite that buffer (a probe costs them
-                // some 200 clocks of their dependent chain; this thread has the time)
-                if (it >= 2 && !(ok = mbar_wait<true>(&o_done[b], ((it - 2) >> 1) & 1, abort, p.status, 10))) break;
-                tc_fence_after_sync();
-                const uint32_t ka = k_addr + kst * kKVBytes;
+        // ------------------------------------------------------------------ Q K^T
+        constexpr uint32_t idesc_qk = umma_idesc_bf16_f32(BQ, BKV);
+        const uint32_t leader = elect_one(), t_at = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint64_t q_desc = umma_desc_k_sw128(smem_u32(q_s)), k_desc0 = umma_desc_k_sw128(smem_u32(k_s));
+        int kst = 0, kph = 0;
+        if (warp_wait<true>(q_full, 0, abort, p.status, 2))
+        for (int it = 0; it < rounds; ++it) {
+            const int b = it % kBufs, bp = it / kBufs & 1;
+            if (!warp_wait<true>(&k_full[kst], kph, abort, p.status, 3)) break;
+            // (the scores' buffer holds the weights of tile it - kBufs until its P V is done)
+            if (it >= kBufs && !warp_wait<true>(&o_done[b], bp ^ 1, abort, p.status, 10)) break;
+            tc_fence_after_sync();
+            const uint64_t k_desc = umma_desc_advance(k_desc0, kst * kKVBytes);
 #pragma unroll
-                for (int kb = 0; kb < KB; ++kb)
+            for (int kb = 0; kb < KB; ++kb)
 #pragma unroll
-                    for (int k = 0; k < 64 / UMMA_K; ++k)
-                        umma_bf16(tmem_base + b * BKV, umma_desc_k_sw128(q_addr + kb * kTileBytes + k * 32),
-                                  umma_desc_k_sw128(ka + kb * kKVBlock + k * 32), idesc_qk, (kb | k) != 0);
-                umma_commit(&s_full[b]);
-                umma_commit(&k_empty[kst]);
-                if (++kst == kStages) { kst = 0; kph ^= 1; }
-            }
+                for (int k = 0; k < 64 / UMMA_K; ++k)
+                    umma_bf16_by(leader, t_at + b * BKV, umma_desc_advance(q_desc, kb * kTileBytes + k * 32), umma_desc_advance(k_desc, kb * kKVBlock + k * 32),
+                                 idesc_qk, (kb | k) != 0);
+            umma_commit_by(leader, &s_full[b]);
+            umma_commit_by(leader, &k_empty[kst]);
+            if (++kst == kStages) { kst = 0; kph ^= 1; }
         }
     }
     } else {
-        // ------------------------------------------------------------------ softmax rows (warps 4..7)
+        // ------------------------------------------------------------------ softmax rows (warps 4..11)
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsMany));
-        const int quarter = warp & 3;                            // the quarter of TMEM's lanes that this warp may touch
+        const int half = (warp - 4) >> 2, quarter = warp & 3;    // the quarter of TMEM's lanes that this warp may touch
         const int r_local = quarter * 32 + lane;                 // row of the tile = TMEM lane
         const int r = row0 + r_local;
         const bool valid = r_local < rows_here;
         const int pos = ctx + r / G;
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-        const uint32_t t_out = t_lane + 2 * BKV;
+        const uint32_t t_out = t_lane + kTmemO;
         float m = -INFINITY, l = 0.f;
         bool ok = true;
-        for (int it = 0; it < n_iter && ok; ++it) {
-            const int j0 = (t_begin + it) * BKV, b = it & 1;
-            uint8_t* p_row = p_s + b * kTileBytes + r_local * 128;
-            if (!(ok = mbar_wait<true>(&s_full[b], (it >> 1) & 1, abort, p.status, 6))) break;
-            tc_fence_after_sync();
-            // the row's 64 scores stay in registers for both passes
-            uint32_t sv_lo[32], sv_hi[32];
-            tmem_ld_32x32b_x32(t_lane + b * BKV, sv_lo);
-            tmem_ld_32x32b_x32(t_lane + b * BKV + 32, sv_hi);
-            tmem_ld_wait();
-            tc_fence_before_sync();
+        // (a wait that ran out lets the loop go on without waiting: the two threads of a row have to meet in every round)
+        for (int it = 0; it < n_iter; ++it) {
+            const int j0 = (t_begin + it) * BKV + half * NK, b = it % kBufs, bp = it / kBufs & 1;
+            const uint32_t t_s = t_lane + b * BKV;
+            ok = ok && mbar_wait<true>(&s_full[b], bp, abort, p.status, 6);
             __syncwarp();
-            if (lane == 0) mbar_arrive(&s_free[b]);
+            tc_fence_after_sync();
+            uint32_t sv[NK];
+            tmem_ld_32x32b_x32(t_s + half * NK, sv);
+            tmem_ld_wait();
             // rows whose keys of this tile are all visible skip the per-key tests (all tiles but the ones on the
-            // diagonal or at the window's edge); masked scores become -inf here, once
-            const bool need_mask = !valid || j0 + BKV - 1 > pos || (p.window > 0 && j0 <= pos - p.window);
+            // diagonal or at the window's edge); masked scores become -inf here, once.  (A row that stands for no token may hold any number:
+            // nobody reads what comes of it.)
+            const bool need_mask = valid && (j0 + NK - 1 > pos || (p.window > 0 && j0 <= pos - p.window));
             if (need_mask) {
 #pragma unroll
-                for (int i = 0; i < BKV; ++i) {
+                for (int i = 0; i < NK; ++i) {
                     const int j = j0 + i;
-                    const bool vis = valid && j <= pos && (p.window <= 0 || j > pos - p.window);
-                    if (!vis) SV(i) = __float_as_uint(-INFINITY);
+                    if (!(j <= pos && (p.window <= 0 || j > pos - p.window))) sv[i] = __float_as_uint(-INFINITY);
                 }
             }
             // pass 1: the maximum of the raw scores (the scale is positive, so it commutes with the maximum),
             // in two independent chains of three-input maxima
             float a0 = -INFINITY, a1 = -INFINITY;
 #pragma unroll
-            for (int i = 0; i < BKV; i += 4) {
-                a0 = max3(a0, __uint_as_float(SV(i)), __uint_as_float(SV(i + 1)));
-                a1 = max3(a1, __uint_as_float(SV(i + 2)), __uint_as_float(SV(i + 3)));
+            for (int i = 0; i < NK; i += 4) {
+                a0 = max3(a0, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
+                a1 = max3(a1, __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]));
             }
-            const float mx_tile = fmaxf(a0, a1) * p.scale_log2;
+            float mx_tile = fmaxf(a0, a1) * p.scale_log2;
+            // Whether any of the two warps' rows has to move its reference; mostly none has, and the row's maximum is nobody's business.
+            // (Both have read their scores by then: either's weights may overwrite the other's.)
+            int moves;
+            __syncwarp();
+            tc_fence_before_sync();
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t"
+                "setp.gt.f32 p, %1, %2;\n\t"
+                "barrier.cta.red.or.pred.aligned q, %3, 64, p;\n\t"
+                "selp.s32 %0, 1, 0, q;\n\t}"
+                : "=r"(moves) : "f"(mx_tile), "f"(m + kRefSlack), "r"(1 + quarter) : "memory");
+            tc_fence_after_sync();
+            if (moves) {
+                meet[half][r_local] = mx_tile;
+                asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
+                mx_tile = fmaxf(mx_tile, meet[half ^ 1][r_local]);
+                asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
+            }
             // m is the reference of the row's exponents; -inf + slack is -inf, so the first visible key sets it
             const float m_new = mx_tile > m + kRefSlack ? mx_tile : m;
             const float alpha = m_new == m ? 1.0f : ex2_approx(m - m_new);
@@ -363,10 +371,11 @@ paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
             // and stores are warp-wide, so the decision is the warp's); P V of the previous tile must be
             // complete by then
             if (it > 0 && !__all_sync(0xffffffffu, alpha == 1.0f)) {
-                if (!(ok = mbar_wait<true>(&o_done[b ^ 1], ((it - 1) >> 1) & 1, abort, p.status, 7))) break;
+                ok = ok && mbar_wait<true>(&o_done[(it - 1) % kBufs], (it - 1) / kBufs & 1, abort, p.status, 7);
+                __syncwarp();
                 tc_fence_after_sync();
-#pragma unroll
-                for (int c = 0; c < HD; c += 32) {
+#pragma unroll 1
+                for (int c = half * (HD / 2); c < (half + 1) * (HD / 2); c += 32) {
                     uint32_t ov[32];
                     tmem_ld_32x32b_x32(t_out + c, ov);
                     tmem_ld_wait();
@@ -376,80 +385,90 @@ paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
                 }
                 tmem_st_wait();
             }
-            // (this P buffer was read by P V of the tile before the previous one: the thread that issued this
-            // tile's Q K^T waited for that)
-            // pass 2: weights (exp2 of -inf is 0), their sum, and P in the MMA's shared-memory layout
-            // (16-byte chunk ^ row % 8)
+            __syncwarp();                     // (the lanes may have parted over the mask; what follows is warp-wide)
+            // pass 2: weights (exp2 of -inf is 0), their sum, and P over the scores' columns
             const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), nref2 = pack_f32x2(-ref, -ref);
             uint64_t acc_a = pack_f32x2(0.f, 0.f), acc_b = acc_a;
+            uint32_t packed[16];
 #pragma unroll
-            for (int c = 0; c < BKV; c += 8) {
-                uint32_t packed[4];
-#pragma unroll
-                for (int i = 0; i < 8; i += 4) {
-                    float x0, x1, x2, x3;
-                    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(SV(c + i)), __uint_as_float(SV(c + i + 1))), scale2, nref2), x0, x1);
-                    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(SV(c + i + 2)), __uint_as_float(SV(c + i + 3))), scale2, nref2), x2, x3);
-                    const float p0 = ex2_approx(x0), p1 = ex2_approx(x1), p2 = ex2_approx(x2), p3 = ex2_approx(x3);
-                    acc_a = add_f32x2(acc_a, pack_f32x2(p0, p1));
-                    acc_b = add_f32x2(acc_b, pack_f32x2(p2, p3));
-                    __nv_bfloat162 h0 = __floats2bfloat162_rn(p0, p1), h1 = __floats2bfloat162_rn(p2, p3);
-                    packed[i >> 1] = *reinterpret_cast<uint32_t*>(&h0);
-                    packed[(i >> 1) + 1] = *reinterpret_cast<uint32_t*>(&h1);
-                }
-                *reinterpret_cast<uint4*>(p_row + (((c >> 3) ^ (r_local & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            for (int i = 0; i < NK; i += 4) {
+                float x0, x1, x2, x3;
+                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale2, nref2), x0, x1);
+                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3])), scale2, nref2), x2, x3);
+                const float p0 = ex2_approx(x0), p1 = ex2_approx(x1), p2 = ex2_approx(x2), p3 = ex2_approx(x3);
+                acc_a = add_f32x2(acc_a, pack_f32x2(p0, p1));
+                acc_b = add_f32x2(acc_b, pack_f32x2(p2, p3));
+                __nv_bfloat162 h0 = __floats2bfloat162_rn(p0, p1), h1 = __floats2bfloat162_rn(p2, p3);
+                packed[i >> 1] = *reinterpret_cast<uint32_t*>(&h0);
+                packed[(i >> 1) + 1] = *reinterpret_cast<uint32_t*>(&h1);
             }
+            tmem_st_32x32b_x16(t_s + half * 16, packed);
             float s0, s1, s2, s3;
             unpack_f32x2(acc_a, s0, s1);
             unpack_f32x2(acc_b, s2, s3);
             l = l * alpha + ((s0 + s1) + (s2 + s3));
-            // one arrival per warp: P is in shared memory for the tensor core to read (and O, if it was
-            // rescaled, is in TMEM)
+            // one arrival per warp: P is in TMEM for the tensor core to read (and O, if it was rescaled, too)
+            tmem_st_wait();
             tc_fence_before_sync();
-            fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_ready[b]);
         }
-        if (ok && n_iter > 0) ok = mbar_wait<true>(&o_done[(n_iter - 1) & 1], ((n_iter - 1) >> 1) & 1, abort, p.status, 8);
+        meet[half][r_local] = l;              // the row's sum of weights
+        asm volatile("barrier.cta.sync.aligned %0, 64;" ::"r"(1 + quarter) : "memory");
+        l = meet[0][r_local] + meet[1][r_local];
+        if (ok && n_iter > 0) ok = mbar_wait<true>(&o_done[(n_iter - 1) % kBufs], (n_iter - 1) / kBufs & 1, abort, p.status, 8);
         tc_fence_after_sync();
-        if (shares > 1) {
-            // one share of the tile's keys: the sums as they are, with the reference they were taken against
-            // (a share without a visible key, or one that gave up waiting, counts as nothing)
-            const bool have = __all_sync(0xffffffffu, ok) && n_iter > 0;
-            const size_t prow = ((size_t)slot * p.NKV + kvh) * BQ + r_local;
-            p.part_ml[prow * 2] = have ? m : -INFINITY;
-            p.part_ml[prow * 2 + 1] = have ? l : 0.f;
-            if (have) {
-                float* dst = p.part_o + prow * HD;
-#pragma unroll
-                for (int c = 0; c < HD; c += 32) {
-                    uint32_t ov[32];
-                    tmem_ld_32x32b_x32(t_out + c, ov);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(ov[i], ov[i + 1], ov[i + 2], ov[i + 3]);
-                }
-            }
-        } else if (ok && n_iter > 0) {
-            // every lane takes part in the TMEM loads (they are warp-wide instructions); only valid rows store
-            const float inv = l > 0.f ? 1.0f / l : 0.f;
-            __nv_bfloat16* dst = p.out + (size_t)(qs0 + r / G) * p.NH * HD + (size_t)(kvh * G + r % G) * HD;
-#pragma unroll
-            for (int c = 0; c < HD; c += 32) {
+        ok = __all_sync(0xffffffffu, ok);
+        const bool have = ok && n_iter > 0;
+        const size_t prow0 = ((size_t)slot * p.NKV + kvh) * BQ;
+        // one share of the tile's keys: the sums as they are, with the reference they were taken against
+        // (a share without a visible key, or one that gave up waiting, counts as nothing)
+        if (shares > 1 && half == 0) {
+            p.part_ml[(prow0 + r_local) * 2] = have ? m : -INFINITY;
+            p.part_ml[(prow0 + r_local) * 2 + 1] = have ? l : 0.f;
+        }
+        if (have) {
+            // 32 columns at a time go through 4 KB of shared memory of the warp's own (the queries and stages are done with), so that a store writes whole
+            // rows' pieces of 128 (64) bytes.  Every lane takes part; only valid rows store.
+            const float inv = shares > 1 ? 1.0f : l > 0.f ? 1.0f / l : 0.f;
+            uint8_t* stage = smem + (warp - 4) * 4096;
+            const long long own = shares > 1 ? (long long)(prow0 + r_local) * HD
+                                : valid ? (long long)(qs0 + r / G) * p.NH * HD + (long long)(kvh * G + r % G) * HD : -1;
+#pragma unroll 1
+            for (int c = half * (HD / 2); c < (half + 1) * (HD / 2); c += 32) {
                 uint32_t ov[32];
+                __syncwarp();
                 tmem_ld_32x32b_x32(t_out + c, ov);
                 tmem_ld_wait();
-                if (valid) {
+                if (shares > 1) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
+                    for (int j = 0; j < 8; ++j)
+                        *reinterpret_cast<uint4*>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(ov[4 * j], ov[4 * j + 1], ov[4 * j + 2], ov[4 * j + 3]);
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int row = i * 4 + (lane >> 3), j = lane & 7;
+                        const long long at = __shfl_sync(0xffffffffu, own, row);
+                        *reinterpret_cast<uint4*>(p.part_o + at + c + 4 * j) = *reinterpret_cast<const uint4*>(stage + row * 128 + ((j ^ (row & 7)) << 4));
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
                         uint32_t w[4];
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(ov[i + 2 * e]) * inv, __uint_as_float(ov[i + 2 * e + 1]) * inv);
+                            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(ov[8 * j + 2 * e]) * inv, __uint_as_float(ov[8 * j + 2 * e + 1]) * inv);
                             w[e] = *reinterpret_cast<uint32_t*>(&h);
                         }
-                        *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(w[0], w[1], w[2], w[3]);
+                        *reinterpret_cast<uint4*>(stage + lane * 64 + ((j ^ (lane >> 1 & 3)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int row = i * 8 + (lane >> 2), j = lane & 3;
+                        const long long at = __shfl_sync(0xffffffffu, own, row);
+                        const uint4 v = *reinterpret_cast<const uint4*>(stage + row * 64 + ((j ^ (row >> 1 & 3)) << 4));
+                        if (at >= 0) *reinterpret_cast<uint4*>(p.out + at + c + 8 * j) = v;
                     }
                 }
             }
@@ -533,7 +552,7 @@ extern "C" int forge_paged_attention_sm100(const void* q, const void* kv, void* 
     const char* err = nullptr;
     CUtensorMap tq, tkv;
     if (!bf16_q_map(q, T, NH, HD, BQ / G, G, &tq, &err)) return forge::fail(FORGE_ERR_UNSUPPORTED, "paged_attention_sm100: q: %s", err);
-    if (!bf16_tile_map(kv, num_pages * 2 * NKV * page_size, HD, page_size, &tkv, &err))
+    if (!bf16_kblock_map(kv, num_pages * 2 * NKV * page_size, HD, page_size, page_size == BKV ? KB : 1, &tkv, &err))
         return forge::fail(FORGE_ERR_UNSUPPORTED, "paged_attention_sm100: cache: %s", err);
     static forge::PerDeviceFlag configured_on;
     bool& configured = configured_on.current();
@@ -545,9 +564,9 @@ extern "C" int forge_paged_attention_sm100(const void* q, const void* kv, void* 
         cudaFuncAttributes attr;
         e = cudaFuncGetAttributes(&attr, paged_attention_sm100_kernel);
         if (e != cudaSuccess) return forge::fail(FORGE_ERR_LAUNCH, "paged_attention_sm100: %s", cudaGetErrorString(e));
-        if (attr.numRegs * 2 < kRegsFew + kRegsMany)
+        if (attr.numRegs * 3 < kRegsFew + 2 * kRegsMany)
             return forge::fail(FORGE_ERR_UNSUPPORTED, "paged_attention_sm100: built with %d registers per thread, needs %d",
-                               attr.numRegs, (kRegsFew + kRegsMany + 1) / 2);
+                               attr.numRegs, (kRegsFew + 2 * kRegsMany + 2) / 3);
         configured = true;
     }
     AttnTcParams p{(__nv_bfloat16*)out, block_table, tile_req, tile_row0, tile_cut, (float*)part_o, (float*)part_ml,
