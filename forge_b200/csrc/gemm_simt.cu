@@ -231,11 +231,11 @@ gemm_simt_few_kernel(const T* __restrict__ A, const T* __restrict__ W, const flo
 
 // ------------------------------------------------------------------------------------------------ many rows of A
 // More rows: tiles of BM x 64, a thread BM/16 x 4 elements (pairs of rows of A in one instruction), 16 channels a step through two
-// buffers in shared memory (both operands lie [channel][row]), the next step's numbers held in registers meanwhile.  Bound by the FMA
-// pipe.  Chunk sums are parked in shared memory.  Which tile height and how many CTAs share a
-// tile's sections is chosen on the host by the longest SM's work.
-// The 16 products of a 333-token prompt through those layers (117 GFLOP): 4.2 ms, 28 TFLOP/s, of 74 that the FMA pipe has; with 4 x 4
-// elements a thread and scalar loads, before, about 12 ms.
+// buffers in shared memory (both operands lie [channel][row]), the next step's numbers held in registers meanwhile.  Bound by shared
+// memory (three 16-byte loads a thread for 32 products).  Chunk sums are parked in shared memory.  Which tile height and how many CTAs share a
+// tile's sections is chosen on the host (see run).
+// The 16 products of a 333-token prompt through those layers (117 GFLOP): 4.0 ms, 29 TFLOP/s, of 74 that the FMA pipe has
+// (an eighth of which 333 rows lose in tiles of 128).
 constexpr int BN = 64, BK = 16, kTileThreads = 256;
 
 template <int BM> struct TileSmem {
@@ -442,17 +442,23 @@ int run(const T* A, const T* W, const float* bias, float* C, int M, int N, int K
         FORGE_FEW(1) FORGE_FEW(2) FORGE_FEW(4) FORGE_FEW(8) FORGE_FEW(16) FORGE_FEW(32)
 #undef FORGE_FEW
     }
-    // tile height and CTAs per tile: the least work of the busiest SM, in sections x rows; a tile of 64 rows reads a
-    // quarter more shared memory per product
-    const int sms = forge::sm_count();
+    // Tile height and CTAs per tile, by the time that their units take (a unit: a CTA's section of a tile, 40 us of 64 rows and 62 of 128 on an SM of its
+    // own and hardly less for two side by side).  Up to a third of the SMs every CTA has one to itself; from there on some SMs get two while others get
+    // none (a kernel's first CTAs go where the kernel ahead has left), as good as all at one CTA an SM; beyond two an SM they are dealt out as they
+    // finish, with half a unit of tail.  Clusters of three, and of other odd sizes, leave SMs out.  Fitted to 64 sizes of 40 to 512 rows: 0.8 % over
+    // the best choice on average, where the busiest SM's work alone (before) was 10 % over it: [2560 x 2048] at 333 rows 193 -> 124 us, [4096 x 4096] at 64
+    // 136 -> 84, [4096 x 14336] at 100 917 -> 472.
+    const double sms = forge::sm_count();
     int best_bm = 128, best_c = 1;
-    long long best = -1;
+    double best = -1.0;
     for (int bm = 64; bm <= 128; bm *= 2)
         for (int c = 1; c <= kMaxCluster && c <= sections; ++c) {
             const int rounds = (sections + c - 1) / c;
             if (c > 1 && rounds > 2) continue;                                    // parked sections beyond two do not fit beside a second CTA
-            const long long tiles = (long long)((M + bm - 1) / bm) * ((N + BN - 1) / BN);
-            const long long cost = ((tiles * c + sms - 1) / sms) * rounds * (bm == 64 ? 72 : 128) + c;
+            const double ctas = (double)((M + bm - 1) / bm) * ((N + BN - 1) / BN) * c;
+            const double share = ctas <= sms / 3 ? 1.0 : ctas <= 1.08 * sms ? 1.0 + (ctas - sms / 3) / (0.75 * sms) : ctas <= 2 * sms ? 2.0 : ctas / sms + 0.5;
+            const double packing = c <= 2 || ctas <= 1.3 * sms ? 1.0 : c == 3 ? 1.4 : (c & (c - 1)) ? 1.15 : 1.03;
+            const double cost = rounds * share * packing * (bm == 64 ? 40.0 : 62.0);
             if (best < 0 || cost < best) { best = cost; best_bm = bm; best_c = c; }
         }
     return best_bm == 64 ? launch_tile<64, T>(A, W, bias, C, M, N, K, accumulate, vec, best_c, stream)
