@@ -1,0 +1,38 @@
+"""The gated delta rule's preparation: the kernel of four channels a lane against the one of a channel a lane (which takes rows that do not begin on 16 bytes),
+bit for bit, over portions that begin, end and are cut anywhere in a warp's run of tokens, behind rings that are full and that are not."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("reqs", [[(0, 1), (5, 2), (0, 3), (1, 4), (2, 17), (100, 40), (0, 5)], [(0, 700)], [(3, 1), (64, 1), (0, 1)]])
+@pytest.mark.parametrize("N,M,V,taps", [(4, 2, 64, 4), (3, 3, 128, 3), (8, 1, 32, 2), (2, 1, 192, 4), (32, 16, 64, 4)])
+def test_both_kernels(reqs, N, M, V, taps):
+    from forge_b200 import kernels
+    K = 64
+    C = 2 * M * K + N * V
+    g = torch.Generator().manual_seed(N + V)
+    starts = [0]
+    for _, n in reqs:
+        starts.append(starts[-1] + n)
+    T, S = starts[-1], len(reqs)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(num_requests=S, num_tokens=T, q_start=i32(starts), slots=i32(list(range(S))[::-1]), tok_req=i32([s for s, (_, n) in enumerate(reqs) for _ in range(n)]),
+                            positions=i32([c + j for c, n in reqs for j in range(n)]))
+    width = (C + 2 * N + 3) // 4 * 4
+    p = torch.randn(T, width, generator=g).to(DEV)
+    conv = torch.randn(taps, C, generator=g).to(DEV)
+    rate, dt = torch.rand(N, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    state0 = torch.randn(S, (N * K * V + taps * C + 3) // 4 * 4, generator=g).to(DEV)
+    got = []
+    for col in (0, 1):
+        rows = torch.full((T, width + 4 * col), 7.0, device=DEV)
+        rows[:, col:col + width] = p
+        state = state0.clone()
+        got.append(kernels.gated_delta_prepare(rows, col, col + C, col + C + N, conv, rate, dt, batch, state, N, M, K, V) + (state,))
+    for a, b in zip(*got):
+        assert bool(torch.isfinite(a).all()) and torch.equal(a, b)
