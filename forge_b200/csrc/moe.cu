@@ -57,10 +57,11 @@ constexpr int kRouteThreads = 256;
 // FEW (bfloat16 inputs, up to FEW = 8 or 16 experts in no groups, rows of a multiple of 8 channels, all aligned to 16 bytes): a thread takes eight
 // channels against all experts, every load of theirs in flight together, and one warp with an expert a lane makes the scores and the choice.
 // (A warp an expert and one thread's choice out of shared memory: both are chains of memory latencies, 12 us for 8 tokens of
-// 4,096 channels, 5.7 us so.)
+// 4,096 channels, 5.7 us so.)  TB tokens a CTA: with many tokens it is the router's matrix, read again by every CTA, and the
+// butterflies that take the time (8 experts of 2,048 channels, 1,000 tokens: 9.9 us, with four tokens a CTA 5.1).
 constexpr int kFewExperts = 16;
 
-template <typename TA, int FEW>
+template <typename TA, int FEW, int TB = 1>
 __global__ void __launch_bounds__(kRouteThreads, FEW == 0 ? 6 : 0)          // (a warp an expert: six CTAs an SM where there are many tokens; else the compiler's choice)
 moe_route_kernel(const TA* __restrict__ x, const float* __restrict__ Wr, int32_t* __restrict__ idx, float* __restrict__ wts, int T,
                  int W, int E, int top, int softmax, int renorm, const float* __restrict__ corr, int groups, int keep, int group_top, float factor) {
@@ -71,14 +72,18 @@ moe_route_kernel(const TA* __restrict__ x, const float* __restrict__ Wr, int32_t
     float* s = sc;
     const TA* xr = x + (size_t)t * W;
     if constexpr (FEW > 0) {
-        __shared__ float parts[kRouteThreads / 32][FEW];
-        float a[FEW];
+        __shared__ float parts[TB][kRouteThreads / 32][FEW];
+        const int t0 = blockIdx.x * TB;
+        float a[TB][FEW];
 #pragma unroll
-        for (int e = 0; e < FEW; ++e) a[e] = 0.f;
+        for (int b = 0; b < TB; ++b)
+#pragma unroll
+            for (int e = 0; e < FEW; ++e) a[b][e] = 0.f;
         for (int c = threadIdx.x * 8; c < W; c += kRouteThreads * 8) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(xr + c);
+            uint4 raw[TB];
+#pragma unroll
+            for (int b = 0; b < TB; ++b) raw[b] = *reinterpret_cast<const uint4*>(x + (size_t)min(t0 + b, T - 1) * W + c);
             float4 w[8][2];
-            float xv[8];
 #pragma unroll
             for (int e0 = 0; e0 < FEW; e0 += 8) {
 #pragma unroll
@@ -87,35 +92,56 @@ moe_route_kernel(const TA* __restrict__ x, const float* __restrict__ Wr, int32_t
                     w[e][0] = r[0];
                     w[e][1] = r[1];
                 }
-                if (e0 == 0) {
-                    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+                for (int b = 0; b < TB; ++b) {
+                    float xv[8];
+                    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw[b]);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float2 f = __bfloat1622float2(p[i]);
                         xv[2 * i] = f.x;
                         xv[2 * i + 1] = f.y;
                     }
-                }
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    float v = a[e0 + e];
-                    v = fmaf(xv[0], w[e][0].x, v); v = fmaf(xv[1], w[e][0].y, v); v = fmaf(xv[2], w[e][0].z, v); v = fmaf(xv[3], w[e][0].w, v);
-                    v = fmaf(xv[4], w[e][1].x, v); v = fmaf(xv[5], w[e][1].y, v); v = fmaf(xv[6], w[e][1].z, v); v = fmaf(xv[7], w[e][1].w, v);
-                    a[e0 + e] = v;
+                    for (int e = 0; e < 8; ++e) {
+                        float v = a[b][e0 + e];
+                        v = fmaf(xv[0], w[e][0].x, v); v = fmaf(xv[1], w[e][0].y, v); v = fmaf(xv[2], w[e][0].z, v); v = fmaf(xv[3], w[e][0].w, v);
+                        v = fmaf(xv[4], w[e][1].x, v); v = fmaf(xv[5], w[e][1].y, v); v = fmaf(xv[6], w[e][1].z, v); v = fmaf(xv[7], w[e][1].w, v);
+                        a[b][e0 + e] = v;
+                    }
                 }
             }
         }
+        if constexpr (TB * FEW == 32) {
+            // 32 sums over the lanes, each in the order of warp_sum's butterfly: at every step a lane keeps the half of the numbers that its bit names
+            float v[32];
 #pragma unroll
-        for (int e = 0; e < FEW; ++e) {
-            a[e] = forge::warp_sum(a[e]);
-            if (lane == 0) parts[warp][e] = a[e];
+            for (int i = 0; i < 32; ++i) v[i] = a[i / FEW][i % FEW];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < o; ++i) {
+                    const bool upper = lane & o;
+                    const float other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + o], o);
+                    v[i] = (upper ? v[i + o] : v[i]) + other;
+                }
+            parts[lane / FEW][warp][lane % FEW] = v[0];
+        } else {
+#pragma unroll
+            for (int b = 0; b < TB; ++b)
+#pragma unroll
+                for (int e = 0; e < FEW; ++e) {
+                    a[b][e] = forge::warp_sum(a[b][e]);
+                    if (lane == 0) parts[b][warp][e] = a[b][e];
+                }
         }
         __syncthreads();
-        if (warp != 0) return;
+        const int t = t0 + warp;                              // a warp a token from here on
+        if (warp >= TB || t >= T) return;
         const bool mine = lane < E;
         float score = 0.f;
 #pragma unroll
-        for (int w = 0; w < kRouteThreads / 32; ++w) score += parts[w][min(lane, FEW - 1)];
+        for (int w = 0; w < kRouteThreads / 32; ++w) score += parts[warp][w][min(lane, FEW - 1)];
         if (softmax) {
             float m = mine ? score : -INFINITY;
 #pragma unroll
@@ -615,13 +641,14 @@ extern "C" int forge_moe_route(const void* x, int dtype, const float* Wr, int32_
     if (T == 0) return FORGE_OK;
     cudaError_t e = cudaSuccess;
     const size_t smem = sizeof(float) * (2 * E + (groups > 1 ? groups : 0));
-    // Few tokens wait for latencies, which the kernel of few experts hides; where there are more tokens than SMs its shorter rows (a row of 768 numbers is
-    // 96 of its 256 threads) cost more than that (300 tokens, 16 experts of 768: 6.1 us without it, 7.3 with it; 1,500 tokens, 4 of 1,024: 6.8
-    // and 9.1; 1,500 tokens, 8 of 4,096: 21.2 and 18.4).
-    const bool few_experts = E <= kFewExperts && groups <= 1 && (T <= forge::sm_count() || (E <= 8 && W >= 2048));
+    // Few tokens wait for latencies, which the kernel of few experts hides.  Where there are more tokens than SMs a CTA of one token costs more than that
+    // (300 tokens, 16 experts of 768: 6.1 us without it, 7.3 with it), of four less from two tokens an SM on, or where rows are long (8 experts: 300
+    // tokens of 768 4.3 us without it, 3.4 with it; 1,500 of 1,024 9.2 and 6.3, of 4,096 21.2 and 12.4; 200 of 512 3.4 and 3.6).
+    const bool few_experts = E <= kFewExperts && groups <= 1 && (T <= forge::sm_count() || (E <= 8 && (W >= 2048 || T > 2 * forge::sm_count())));
     if (dtype == FORGE_BF16 && few_experts && W % 8 == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0) {
-        auto few = E <= 8 ? moe_route_kernel<__nv_bfloat16, 8> : moe_route_kernel<__nv_bfloat16, 16>;
-        e = forge::launch(few, dim3(T), dim3(kRouteThreads), smem, stream, 1, (const __nv_bfloat16*)x, Wr, idx, wts, T, W, E, top, softmax, renorm, corr, 0, keep,
+        const bool many = E <= 8 && T > forge::sm_count();
+        auto few = many ? moe_route_kernel<__nv_bfloat16, 8, 4> : E <= 8 ? moe_route_kernel<__nv_bfloat16, 8> : moe_route_kernel<__nv_bfloat16, 16>;
+        e = forge::launch(few, dim3(many ? (T + 3) / 4 : T), dim3(kRouteThreads), smem, stream, 1, (const __nv_bfloat16*)x, Wr, idx, wts, T, W, E, top, softmax, renorm, corr, 0, keep,
                           group_top, factor);
         return forge::check_launch("moe_route", e);
     }
