@@ -1,4 +1,4 @@
-// The recurrences of recurrent_block.cu (and retention) over long portions, 32 tokens at a time (fp32 throughout), for heads of 64 key channels; which
+// The recurrences of recurrent_block.cu (and retention) over long portions, 32 tokens at a time (fp32 in and out), for heads of 64 key channels; which
 // steps take them is chunks_pay's choice, in the Python wrappers:
 //
 //     gated delta rule   S <- g_t S;   S <- S + k_t (b_t (v_t - S^T k_t))^T;   o_t = S^T q_t
@@ -14,11 +14,12 @@
 //     2  per (request, head, cols)  u = U - W S, the state before every chunk kept, S moved on        (fixed decay: S <- P_31 S + Z)
 //     3  per (chunk, head)          the outputs, from the kept states
 // The block scan they replace makes a chain of 900 instructions of every eight tokens with two to four warps an SM.  2,001 tokens in three portions, 32 heads:
-// 216 us with its gram matrices, 185 us here (solve 38, walk 103, outputs 44).  Fixed decay, 1,500 tokens in two portions, 64 heads: 252 us token by
+// 216 us with its gram matrices, 150 us here (solve 38, walk 74, outputs 38).  Fixed decay, 1,500 tokens in two portions, 64 heads: 252 us token by
 // token, 110 us here.  Every R is a
 // product of its decays (no quotients), so a decay of zero does no harm.  Scratch: W, U [chunks, N, 32, 64 | V] and the states
 // [chunks, N, 64, V], chunks = T / 32 + S.
 #include "common.cuh"
+#include "mma_sync.cuh"
 
 namespace {
 
@@ -193,130 +194,177 @@ chunk_update_kernel(const Chunks d) {
 }
 
 // ------------------------------------------------------------------------------------------------ 2: the walk
+// The small products of the walk on the tensor cores (m16n8k16): an fp32 number as the sum of three bfloat16 ones (its rounding, the rounding of what that
+// left, and of what that left: 2^-26 of it at most is missing), of the nine products of two such sums the six largest, each exact, fp32 sums.  The tensor
+// core cuts what an addend has below a sum's last place, so the large terms have a sum of their own over few steps; the state itself is moved on by
+// multiply-adds.  (A number that is not finite makes NaN of the sums that it takes part in.)
+struct Terms { uint32_t h, m, l; };                           // of two neighbouring numbers each
+__device__ __forceinline__ Terms split2(float x, float y) {
+    Terms t;
+    t.h = mma_sync::pack_bf16(x, y);
+    x -= __uint_as_float(t.h << 16);
+    y -= __uint_as_float(t.h & 0xffff0000u);
+    t.m = mma_sync::pack_bf16(x, y);
+    t.l = mma_sync::pack_bf16(x - __uint_as_float(t.m << 16), y - __uint_as_float(t.m & 0xffff0000u));
+    return t;
+}
+// main += the large term, rest += the others, of A (rows g and g + 8, steps 2t and 2t + 8 on) times B (steps 2t and 2t + 8 on, column g)
+__device__ __forceinline__ void mma_terms(float (&main)[4], float (&rest)[4], const Terms (&a)[4], const Terms (&b)[2]) {
+    const uint32_t ah[4] = {a[0].h, a[1].h, a[2].h, a[3].h}, am[4] = {a[0].m, a[1].m, a[2].m, a[3].m}, al[4] = {a[0].l, a[1].l, a[2].l, a[3].l};
+    mma_sync::mma_bf16(rest, al, b[0].h, b[1].h);
+    mma_sync::mma_bf16(main, ah, b[0].h, b[1].h);
+    mma_sync::mma_bf16(rest, ah, b[0].l, b[1].l);
+    mma_sync::mma_bf16(rest, am, b[0].m, b[1].m);
+    mma_sync::mma_bf16(rest, am, b[0].h, b[1].h);
+    mma_sync::mma_bf16(rest, ah, b[0].m, b[1].m);
+}
+// (the walk's: two chains of the others, as little as possible waits for the sum before)
+__device__ __forceinline__ void mma_terms(float (&main)[4], float (&rest)[2][4], const Terms (&a)[4], const Terms (&b)[2]) {
+    const uint32_t ah[4] = {a[0].h, a[1].h, a[2].h, a[3].h}, am[4] = {a[0].m, a[1].m, a[2].m, a[3].m}, al[4] = {a[0].l, a[1].l, a[2].l, a[3].l};
+    mma_sync::mma_bf16(rest[0], al, b[0].h, b[1].h);
+    mma_sync::mma_bf16(rest[1], am, b[0].h, b[1].h);
+    mma_sync::mma_bf16(main, ah, b[0].h, b[1].h);
+    mma_sync::mma_bf16(rest[0], ah, b[0].l, b[1].l);
+    mma_sync::mma_bf16(rest[1], ah, b[0].m, b[1].m);
+    mma_sync::mma_bf16(rest[0], am, b[0].m, b[1].m);
+}
+
 // DELTA: 16 columns of one head's S a CTA; the next chunk's W, K, U and decays are on their way while the present one is worked on.  A chunk is
-// two small products, one after the other: u = U - W S (32 x 16 numbers over 64 channels) and S + K^T u (64 x 16 over 32 tokens).  What
-// bounds them is how often shared memory is asked, so a thread has 4 x 4 numbers of a product and the warps share the sum: eight channels a
-// warp, eight tokens two warps, the parts added up out of shared memory (a whole sum of 1 x 4 numbers a thread asked twice as often, and three
-// portions of 2,001 tokens in all, 32 heads, took 146 us; 103 us so).
-constexpr int kWalkThreads = 256, kPartLd = kColsB + 4;
-constexpr int kStageB = 2 * CH * K + CH * kColsB + CH;        // floats of a chunk's W, K, U, decays
-constexpr int kPartB = 8 * CH * kPartLd;                      // eight parts of u or four of S
-static_assert(kPartB == 4 * K * kPartLd, "both fill it");
-constexpr size_t kWalkSmem = sizeof(float) * (2 * kStageB + kPartB + K * kColsB + CH * kColsB + CH + 4);
+// two small products, one after the other: u = U - W S (32 x 16 numbers over 64 channels, of which four warps take half and four the other half; those
+// ask for the next chunk while the first finish u) and S <- P S + K^T u (64 x 16 over 32 tokens; a warp keeps its 16 x 8 numbers of S in registers).  As fp32 multiply-adds, 4 x 4 numbers a thread and the sums shared by the warps, shared memory was asked
+// six times as often and a chunk had four meetings instead of three: three portions of 2,001 tokens in all, 32 heads, 104 us; 92 us so, and 74 us with the
+// longest portion's CTAs first (what is left: the two products' splits and meetings, 32 times one after the other).
+constexpr int kWalkThreads = 256, LDW = CH + 4, LDC = kColsB + 4;
+constexpr int kStageB = K * LDW + CH * LD + CH * LDC + CH;    // floats of a chunk's W, K, U, decays
+constexpr size_t kWalkSmem = sizeof(float) * (2 * kStageB + K * LDC + 2 * CH * LDC);
+
+// The request that is the rank-th longest (of up to 32; of more they stay in their order): the kernel ends with the longest walk, whose CTAs come first
+// and so each to an SM of its own.  Every lane gets it.
+__device__ __forceinline__ int longest(const Chunks& d, int rank, int lane) {
+    if (d.S > 32) return rank;
+    const int n = lane < d.S ? d.q_start[lane + 1] - d.q_start[lane] : -1;
+    int before = 0;
+    for (int i = 0; i < d.S; ++i) {
+        const int other = __shfl_sync(0xffffffffu, n, i);
+        before += other > n || (other == n && i < lane);
+    }
+    return __ffs(__ballot_sync(0xffffffffu, lane < d.S && before == rank)) - 1;
+}
 
 __global__ void __launch_bounds__(kWalkThreads, 3)
 chunk_walk_kernel(const Chunks d) {
     extern __shared__ __align__(16) float sm[];
-    float* part = sm + 2 * kStageB;                           // [8][32][16 + 4] or [4][64][16 + 4]
-    float* S = part + kPartB;                                 // [64][16]
-    float* us = S + K * kColsB;                               // [32][16]: u_t times the decays behind it
-    float* wt = us + CH * kColsB;                             // [32]: the decays behind a token, then the chunk's whole decay
+    float* S = sm + 2 * kStageB;                              // [64][16 + 4]
+    float* us = S + K * LDC;                                  // [32][16 + 4]: u_t times the decays behind it
+    float* part = us + CH * LDC;                              // [32][16 + 4]: W S over the second half of the channels
     forge::pdl_launch_dependents();
     forge::pdl_wait();
-    const int s = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * kColsB, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, tq = lane & 3;
+    const int cols = d.V / kColsB, head = blockIdx.x / cols % d.N, c0 = blockIdx.x % cols * kColsB, s = longest(d, blockIdx.x / (cols * d.N), lane);
     const int t_lo = d.q_start[s], t_hi = d.q_start[s + 1];
     if (t_lo >= t_hi) return;
     const int chunks = (t_hi - t_lo + CH - 1) / CH, at0 = first_chunk(d.q_start, s);
     const float* k = d.k + (size_t)head / (d.N / d.M) * K;
+    constexpr int kFetch = kWalkThreads / 2;                  // threads that copy: the second half of the CTA
     auto fetch = [&](int i) {
+        const int tid = (int)threadIdx.x - kFetch;
         if (i < chunks) {
             float* w = sm + (i & 1) * kStageB;
             const int t0 = t_lo + i * CH, n = min(CH, t_hi - t0);
             const size_t at = ((size_t)(at0 + i) * d.N + head) * CH;
 #pragma unroll
-            for (int h = 0; h < CH * K / 4; h += kWalkThreads) {
+            for (int h = 0; h < CH * K / 4; h += kFetch) {
                 const int e = h + tid, r = e / (K / 4), c = e % (K / 4) * 4;
-                stage16(w + e * 4, d.w + at * K + e * 4, true);
-                stage16(w + CH * K + e * 4, k + (size_t)(r < n ? t0 + r : t0) * d.ld_k + c, r < n);
+                stage16(w + e / (CH / 4) * LDW + e % (CH / 4) * 4, d.w + at * K + e * 4, true);                  // [channel][token]
+                stage16(w + K * LDW + r * LD + c, k + (size_t)(r < n ? t0 + r : t0) * d.ld_k + c, r < n);        // [token][channel]
             }
-            if (tid < CH * kColsB / 4) stage16(w + 2 * CH * K + tid * 4, d.u + (at + tid / 4) * d.V + c0 + tid % 4 * 4, true);
-            else if (tid < CH * kColsB / 4 + CH) {
-                const int t = tid - CH * kColsB / 4;
-                float* dst = w + 2 * CH * K + CH * kColsB + t;
+            float* u = w + K * LDW + CH * LD;
+            stage16(u + tid / 4 * LDC + tid % 4 * 4, d.u + (at + tid / 4) * d.V + c0 + tid % 4 * 4, true);
+            if (tid < CH) {
+                const int t = tid;
+                float* dst = u + CH * LDC + t;
                 if (t < n) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(d.g + (size_t)(t0 + t) * d.N + head) : "memory");
                 else *dst = 1.0f;
             }
         }
         stages_commit();
     };
-    fetch(0);
-    // four numbers of S stay with a thread: row tid / 4, columns tid % 4 * 4 ..
-    const int row = tid / 4, col = tid % 4 * 4;
-    float* S_g = d.state + (size_t)d.slots[s] * d.stride + (size_t)head * K * d.V + (size_t)row * d.V + c0 + col;
-    float4 own = *reinterpret_cast<const float4*>(S_g);
-    *reinterpret_cast<float4*>(S + row * kColsB + col) = own;
-    const int tg = lane / 4 * 4, cg = lane % 4 * 4;           // a thread's 4 x 4 numbers: tokens tg .. (or rows) and columns cg ..
+    static_assert(kFetch == CH * kColsB / 4, "a piece of U a thread");
+    if (warp >= 4) fetch(0);
+    // a warp's part of S: rows row0 + gr (and 8 further on), columns col0 + 2 tq and the next
+    const int row0 = (warp >> 1) * 16 + gr, col0 = (warp & 1) * 8 + 2 * tq;
+    float* S_g = d.state + (size_t)d.slots[s] * d.stride + (size_t)head * K * d.V + (size_t)row0 * d.V + c0 + col0;
+    float2 own0 = *reinterpret_cast<const float2*>(S_g), own1 = *reinterpret_cast<const float2*>(S_g + 8 * d.V);
+    *reinterpret_cast<float2*>(S + row0 * LDC + col0) = own0;
+    *reinterpret_cast<float2*>(S + (row0 + 8) * LDC + col0) = own1;
     for (int i = 0; i < chunks; ++i) {
-        fetch(i + 1);
-        stages_wait<1>();
-        __syncthreads();                                      // chunk i is here and S stands
+        stages_wait<0>();
+        __syncthreads();                                      // chunk i is here, S stands, and nobody is at chunk i - 1 any more
         const float* w = sm + (i & 1) * kStageB;
-        const float* ks = w + CH * K;
-        if (tid < CH) {                                       // the decays behind token t, and the chunk's
-            float x = w[2 * CH * K + CH * kColsB + tid];      // becomes g_t .. g_31
+        const float* ks = w + K * LDW;
+        const float* U = ks + CH * LD;
+        const int m0 = (warp & 1) * 16 + gr, n0 = (warp >> 1 & 1) * 8, c = n0 + 2 * tq;
+        float main[4] = {0.f, 0.f, 0.f, 0.f}, rest[2][4] = {};
 #pragma unroll
-            for (int o = 1; o < CH; o <<= 1) {
-                const float y = __shfl_down_sync(0xffffffffu, x, o);
-                if (tid + o < CH) x *= y;
-            }
-            const float next = __shfl_down_sync(0xffffffffu, x, 1);
-            wt[tid] = tid + 1 < CH ? next : 1.0f;
-            if (tid == 0) wt[CH] = x;
+        for (int kk = 0; kk < K / 2; kk += 16) {
+            const int from = (warp >> 2) * (K / 2) + kk + 2 * tq;
+            const float* a = w + from * LDW + m0;
+            const float* b = S + from * LDC + n0 + gr;
+            const Terms at[4] = {split2(a[0], a[LDW]), split2(a[8], a[LDW + 8]), split2(a[8 * LDW], a[9 * LDW]), split2(a[8 * LDW + 8], a[9 * LDW + 8])};
+            const Terms bt[2] = {split2(b[0], b[LDC]), split2(b[8 * LDC], b[9 * LDC])};
+            mma_terms(main, rest, at, bt);
         }
-        *reinterpret_cast<float4*>(d.s + (((size_t)(at0 + i) * d.N + head) * K + row) * d.V + c0 + col) = own;
-        float a[4][4];
-        auto product = [&](const float* l, int ld_l, const float* r) {      // eight steps of a (+)= l[k][4] r[k][4]
+        // the decays behind token `lane`, and the chunk's (lane 0's)
+        float x = U[CH * LDC + lane];                         // becomes g_lane .. g_31
 #pragma unroll
-            for (int x = 0; x < 4; ++x) a[x][0] = a[x][1] = a[x][2] = a[x][3] = 0.f;
+        for (int o = 1; o < CH; o <<= 1) {
+            const float y = __shfl_down_sync(0xffffffffu, x, o);
+            if (lane + o < CH) x *= y;
+        }
+        const float p = __shfl_sync(0xffffffffu, x, 0), next = __shfl_down_sync(0xffffffffu, x, 1), behind = lane + 1 < CH ? next : 1.0f;
+        if (warp >= 4) {
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-                const float4 x = *reinterpret_cast<const float4*>(l + kk * ld_l), y = *reinterpret_cast<const float4*>(r + kk * kColsB);
-                const float xv[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    a[e][0] = fmaf(xv[e], y.x, a[e][0]);
-                    a[e][1] = fmaf(xv[e], y.y, a[e][1]);
-                    a[e][2] = fmaf(xv[e], y.z, a[e][2]);
-                    a[e][3] = fmaf(xv[e], y.w, a[e][3]);
-                }
-            }
-        };
-        auto leave = [&](float* dst) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) *reinterpret_cast<float4*>(dst + e * kPartLd) = make_float4(a[e][0], a[e][1], a[e][2], a[e][3]);
-        };
-        product(w + warp * 8 * CH + tg, CH, S + warp * 8 * kColsB + cg);
-        leave(part + (warp * CH + tg) * kPartLd + cg);
-        __syncthreads();
-        {
-            const int t = tid / 8, c = tid % 8 * 2;
-            float2 u = *reinterpret_cast<const float2*>(w + 2 * CH * K + t * kColsB + c);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const float2 x = *reinterpret_cast<const float2*>(part + (q * CH + t) * kPartLd + c);
-                u.x -= x.x;
-                u.y -= x.y;
-            }
-            const float r = wt[t];
-            *reinterpret_cast<float2*>(us + t * kColsB + c) = make_float2(u.x * r, u.y * r);
-            *reinterpret_cast<float2*>(d.u + (((size_t)(at0 + i) * d.N + head) * CH + t) * d.V + c0 + c) = u;
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float2*>(part + (m0 + 8 * h) * LDC + c) =
+                    make_float2(main[2 * h] + (rest[0][2 * h] + rest[1][2 * h]), main[2 * h + 1] + (rest[0][2 * h + 1] + rest[1][2 * h + 1]));
         }
         __syncthreads();
-        const int half = (warp & 1) * 32, t8 = (warp >> 1) * 8;             // rows half + tg .., tokens t8 .. t8 + 7
-        product(ks + t8 * K + half + tg, K, us + t8 * kColsB + cg);
-        leave(part + ((warp >> 1) * K + half + tg) * kPartLd + cg);
-        __syncthreads();
-        const float p = wt[CH];
-        own.x *= p; own.y *= p; own.z *= p; own.w *= p;
+        if (warp < 4) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float4 x = *reinterpret_cast<const float4*>(part + (q * K + row) * kPartLd + col);
-            own.x += x.x; own.y += x.y; own.z += x.z; own.w += x.w;
+            for (int h = 0; h < 2; ++h) {
+                const int t = m0 + 8 * h;
+                float2 u = *reinterpret_cast<const float2*>(U + t * LDC + c);
+                const float2 half = *reinterpret_cast<const float2*>(part + t * LDC + c);
+                u.x -= (main[2 * h] + (rest[0][2 * h] + rest[1][2 * h])) + half.x;
+                u.y -= (main[2 * h + 1] + (rest[0][2 * h + 1] + rest[1][2 * h + 1])) + half.y;
+                const float r = __shfl_sync(0xffffffffu, behind, t);
+                *reinterpret_cast<float2*>(us + t * LDC + c) = make_float2(u.x * r, u.y * r);
+                *reinterpret_cast<float2*>(d.u + (((size_t)(at0 + i) * d.N + head) * CH + t) * d.V + c0 + c) = u;
+            }
+        } else {
+            fetch(i + 1);
         }
-        *reinterpret_cast<float4*>(S + row * kColsB + col) = own;
-        // (chunk i's buffer was last read before the last barrier, and part, us and wt are not written before the next one)
+        float* kept = d.s + (((size_t)(at0 + i) * d.N + head) * K + row0) * d.V + c0 + col0;
+        *reinterpret_cast<float2*>(kept) = own0;
+        *reinterpret_cast<float2*>(kept + 8 * d.V) = own1;
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 4; ++e) main[e] = rest[0][e] = rest[1][e] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < CH; kk += 16) {
+            const float* a = ks + (kk + 2 * tq) * LD + row0;
+            const float* b = us + (kk + 2 * tq) * LDC + (warp & 1) * 8 + gr;
+            const Terms at[4] = {split2(a[0], a[LD]), split2(a[8], a[LD + 8]), split2(a[8 * LD], a[9 * LD]), split2(a[8 * LD + 8], a[9 * LD + 8])};
+            const Terms bt[2] = {split2(b[0], b[LDC]), split2(b[8 * LDC], b[9 * LDC])};
+            mma_terms(main, rest, at, bt);
+        }
+        own0.x = fmaf(p, own0.x, main[0] + (rest[0][0] + rest[1][0])); own0.y = fmaf(p, own0.y, main[1] + (rest[0][1] + rest[1][1]));
+        own1.x = fmaf(p, own1.x, main[2] + (rest[0][2] + rest[1][2])); own1.y = fmaf(p, own1.y, main[3] + (rest[0][3] + rest[1][3]));
+        *reinterpret_cast<float2*>(S + row0 * LDC + col0) = own0;
+        *reinterpret_cast<float2*>(S + (row0 + 8) * LDC + col0) = own1;
     }
-    *reinterpret_cast<float4*>(S_g) = own;
+    *reinterpret_cast<float2*>(S_g) = own0;
+    *reinterpret_cast<float2*>(S_g + 8 * d.V) = own1;
 }
 
 // Fixed decay: four neighbouring numbers of the state a thread; where Z of a chunk lay the state before it stays.
@@ -356,19 +404,28 @@ chunk_sum_kernel(const Chunks d) {
 }
 
 // ------------------------------------------------------------------------------------------------ 3: the outputs
-// A CTA has 64 of a head's value columns, a thread eight tokens x four columns (bound by shared memory: a wider tile reads less of it).
-constexpr int kOutThreads = 64, TJ = CH * VB / 4 / kOutThreads;
+// A CTA has 64 of a head's value columns and makes three products on the tensor cores (terms as in the walk): q k^T (32 x 32, under the triangle of decays),
+// q S (32 x 64 over 64 channels) and the triangle times u (over 32 tokens).  As fp32 multiply-adds, eight tokens x four columns a thread, shared memory was
+// asked for 12 bytes a product: 2,001 tokens of 32 heads 44.5 us, 37.7 us so (q, k, u, S in and the outputs out: 10 us at full bandwidth; the rest is
+// splits and a CTA's two waits).
+constexpr int kOutThreads = 128, LDV = VB + 4, LDM = CH + 4;
+constexpr size_t kOutSmem = sizeof(float) * (2 * CH * LD + K * LDV + CH * LDV + CH * LDM);
+
 template <bool DELTA>
-__global__ void __launch_bounds__(kOutThreads)
+__global__ void __launch_bounds__(kOutThreads, 4)
 chunk_output_kernel(const Chunks d) {
-    __shared__ __align__(16) float qs[CH * LD], S[K * VB], us[CH * VB], Mx[CH][CH + 4];
+    extern __shared__ __align__(16) float sm[];
     __shared__ float R[CH][CH + 1], gs[CH], P[CH];
-    float* ks = S;                                            // the keys until the products stand, then the state
-    static_assert(CH * LD <= K * VB, "the keys fit where the state will lie");
+    float* qs = sm;                                           // [32][64 + 4]
+    float* ks = qs + CH * LD;                                 // [32][64 + 4]
+    float* S = ks + CH * LD;                                  // [64][64 + 4]: the state before the chunk
+    float* us = S + K * LDV;                                  // [32][64 + 4]
+    float* Mx = us + CH * LDV;                                // [32][32 + 4]: the triangle
     forge::pdl_launch_dependents();
     forge::pdl_wait();
     int t0;
     const int chunk = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * VB, n = chunk_tokens(d, chunk, t0), tid = threadIdx.x;
+    const int warp = tid >> 5, lane = tid & 31, gr = lane >> 2, tq = lane & 3;
     if (n <= 0) return;
     const int hk = head / (d.N / d.M);
     stage_rows<kOutThreads>(qs, d.q + (size_t)t0 * d.ld_q + hk * K, d.ld_q, n);
@@ -376,9 +433,11 @@ chunk_output_kernel(const Chunks d) {
     stages_commit();
     const float* u = DELTA ? d.u + ((size_t)chunk * d.N + head) * CH * d.V + v0 : d.v + (size_t)t0 * d.ld_v + (size_t)head * d.V + v0;
     const int ld_u = DELTA ? d.V : d.ld_v;
+    const float* kept = d.s + ((size_t)chunk * d.N + head) * K * d.V + v0;
+    for (int i = tid; i < K * VB / 4; i += kOutThreads) stage16(S + i / (VB / 4) * LDV + i % (VB / 4) * 4, kept + (size_t)(i / (VB / 4)) * d.V + i % (VB / 4) * 4, true);
     for (int i = tid; i < CH * VB / 4; i += kOutThreads) {
         const int r = i / (VB / 4), c = i % (VB / 4) * 4;
-        stage16(us + r * VB + c, r < n ? u + (size_t)r * ld_u + c : u, r < n);
+        stage16(us + r * LDV + c, r < n ? u + (size_t)r * ld_u + c : u, r < n);
     }
     stages_commit();
     if (tid < CH) gs[tid] = tid >= n ? 1.0f : DELTA ? d.g[(size_t)(t0 + tid) * d.N + head] : d.g[head];
@@ -391,71 +450,119 @@ chunk_output_kernel(const Chunks d) {
     stages_wait<1>();
     __syncthreads();
     {
-        const int j = tid >> 1, i0 = tid & 1;
-        float acc[CH / 2];
+        // rows m0 .. m0 + 15 of the triangle, columns n0 .. n0 + 15 (above the diagonal: zeros, whatever the keys there)
+        const int m0 = (warp & 1) * 16, n0 = (warp >> 1) * 16;
+        float main[2][4] = {}, rest[2][4] = {};
+        if (n0 <= m0) {
 #pragma unroll
-        for (int m = 0; m < CH / 2; ++m) acc[m] = 0.f;
-#pragma unroll 4
-        for (int c = 0; c < K; c += 4) {
-            const float4 qj = *reinterpret_cast<const float4*>(qs + j * LD + c);
+            for (int kk = 0; kk < K; kk += 16) {
+                const float* a = qs + (m0 + gr) * LD + kk + 2 * tq;
+                auto pair = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return split2(v.x, v.y); };
+                const Terms at[4] = {pair(a), pair(a + 8 * LD), pair(a + 8), pair(a + 8 * LD + 8)};
 #pragma unroll
-            for (int m = 0; m < CH / 2; ++m) acc[m] = dot4(qj, *reinterpret_cast<const float4*>(ks + (i0 + 2 * m) * LD + c), acc[m]);
+                for (int h = 0; h < 2; ++h) {
+                    const float* b = ks + (n0 + 8 * h + gr) * LD + kk + 2 * tq;
+                    const Terms bt[2] = {pair(b), pair(b + 8)};
+                    mma_terms(main[h], rest[h], at, bt);
+                }
+            }
         }
 #pragma unroll
-        for (int m = 0; m < CH / 2; ++m) Mx[j][i0 + 2 * m] = R[j][i0 + 2 * m] * acc[m];
-    }
-    __syncthreads();                                          // the keys have been read
-    const float* kept = d.s + ((size_t)chunk * d.N + head) * K * d.V + v0;
-    for (int i = tid; i < K * VB / 4; i += kOutThreads) stage16(S + i * 4, kept + (size_t)(i / (VB / 4)) * d.V + i % (VB / 4) * 4, true);
-    stages_commit();
-    const int j0 = tid / 16 * TJ, c = tid % 16 * 4;
-    float acc[TJ][4];
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int a = 0; a < TJ; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.f;
+            for (int e = 0; e < 4; ++e) {
+                const int j = m0 + gr + (e >> 1) * 8, i = n0 + 8 * h + 2 * tq + (e & 1);
+                Mx[j * LDM + i] = i <= j ? R[j][i] * (main[h][e] + rest[h][e]) : 0.f;
+            }
+    }
     stages_wait<0>();
     __syncthreads();
-#pragma unroll 2
-    for (int kk = 0; kk < K; kk += 4) {
-        float qv[TJ][4];
+    bool odd = false;                                         // numbers among the u that are none: a later token's must not meet the triangle's zeros
+    for (int i = tid; i < CH * VB; i += kOutThreads) odd |= !isfinite(us[i / VB * LDV + i % VB]);
+    odd = __syncthreads_or(odd);
+    // a warp's 16 columns of all tokens: 16 x 8 tiles [m][h]
+    const int c0 = warp * 16;
+    float main[2][2][4] = {}, rest[2][2][4] = {}, o[2][2][4];
 #pragma unroll
-        for (int a = 0; a < TJ; ++a) *reinterpret_cast<float4*>(qv[a]) = *reinterpret_cast<const float4*>(qs + (j0 + a) * LD + kk);
+    for (int kk = 0; kk < K; kk += 16) {
+        Terms bt[2][2];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float4 x = *reinterpret_cast<const float4*>(S + (kk + e) * VB + c);
+        for (int h = 0; h < 2; ++h) {
+            const float* b = S + (kk + 2 * tq) * LDV + c0 + 8 * h + gr;
+            bt[h][0] = split2(b[0], b[LDV]);
+            bt[h][1] = split2(b[8 * LDV], b[9 * LDV]);
+        }
 #pragma unroll
-            for (int a = 0; a < TJ; ++a) {
-                acc[a][0] = fmaf(qv[a][e], x.x, acc[a][0]);
-                acc[a][1] = fmaf(qv[a][e], x.y, acc[a][1]);
-                acc[a][2] = fmaf(qv[a][e], x.z, acc[a][2]);
-                acc[a][3] = fmaf(qv[a][e], x.w, acc[a][3]);
-            }
+        for (int m = 0; m < 2; ++m) {
+            const float* a = qs + (16 * m + gr) * LD + kk + 2 * tq;
+            auto pair = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return split2(v.x, v.y); };
+            const Terms at[4] = {pair(a), pair(a + 8 * LD), pair(a + 8), pair(a + 8 * LD + 8)};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) mma_terms(main[m][h], rest[m][h], at, bt[h]);
         }
     }
 #pragma unroll
-    for (int a = 0; a < TJ; ++a)
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] *= P[j0 + a];
-    for (int i = 0; i < j0 + TJ; i += 4) {                     // (the triangle's zeros take part up to the block on the diagonal)
-        float mv[TJ][4];
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int a = 0; a < TJ; ++a) *reinterpret_cast<float4*>(mv[a]) = *reinterpret_cast<const float4*>(&Mx[j0 + a][i]);
+            for (int e = 0; e < 4; ++e) {
+                o[m][h][e] = (main[m][h][e] + rest[m][h][e]) * P[16 * m + gr + (e >> 1) * 8];
+                main[m][h][e] = rest[m][h][e] = 0.f;
+            }
+    if (!odd) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float4 x = *reinterpret_cast<const float4*>(us + (i + e) * VB + c);
+        for (int kk = 0; kk < CH; kk += 16) {
+            Terms bt[2][2];
 #pragma unroll
-            for (int a = 0; a < TJ; ++a) {
-                if (i + e > j0 + a) continue;                 // a later token takes no part, whatever its numbers
-                acc[a][0] = fmaf(mv[a][e], x.x, acc[a][0]);
-                acc[a][1] = fmaf(mv[a][e], x.y, acc[a][1]);
-                acc[a][2] = fmaf(mv[a][e], x.z, acc[a][2]);
-                acc[a][3] = fmaf(mv[a][e], x.w, acc[a][3]);
+            for (int h = 0; h < 2; ++h) {
+                const float* b = us + (kk + 2 * tq) * LDV + c0 + 8 * h + gr;
+                bt[h][0] = split2(b[0], b[LDV]);
+                bt[h][1] = split2(b[8 * LDV], b[9 * LDV]);
+            }
+#pragma unroll
+            for (int m = kk / 16; m < 2; ++m) {                           // (the first 16 tokens see none of the others)
+                const float* a = Mx + (16 * m + gr) * LDM + kk + 2 * tq;
+                auto pair = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return split2(v.x, v.y); };
+                const Terms at[4] = {pair(a), pair(a + 8 * LDM), pair(a + 8), pair(a + 8 * LDM + 8)};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) mma_terms(main[m][h], rest[m][h], at, bt[h]);
             }
         }
+    } else {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j = 16 * m + gr + (e >> 1) * 8, c = c0 + 8 * h + 2 * tq + (e & 1);
+                    for (int i = 0; i <= j; ++i) main[m][h][e] = fmaf(Mx[j * LDM + i], us[i * LDV + c], main[m][h][e]);
+                }
     }
 #pragma unroll
-    for (int a = 0; a < TJ; ++a)
-        if (j0 + a < n)
-            *reinterpret_cast<float4*>(d.out + (size_t)(t0 + j0 + a) * d.N * d.V + (size_t)head * d.V + v0 + c) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int j = 16 * m + gr + 8 * r;
+            if (j >= n) continue;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float2*>(d.out + (size_t)(t0 + j) * d.N * d.V + (size_t)head * d.V + v0 + c0 + 8 * h + 2 * tq) =
+                    make_float2(o[m][h][2 * r] + (main[m][h][2 * r] + rest[m][h][2 * r]), o[m][h][2 * r + 1] + (main[m][h][2 * r + 1] + rest[m][h][2 * r + 1]));
+        }
+}
+
+template <bool DELTA>
+cudaError_t launch_output(const Chunks& d, unsigned chunks, cudaStream_t stream) {
+    static forge::PerDeviceFlag flag;
+    bool& done = flag.current();
+    if (!done) {
+        const cudaError_t e = cudaFuncSetAttribute(chunk_output_kernel<DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOutSmem);
+        if (e != cudaSuccess) return e;
+        done = true;
+    }
+    return forge::launch(chunk_output_kernel<DELTA>, dim3(chunks, d.N, d.V / VB), dim3(kOutThreads), kOutSmem, stream, 1, d);
 }
 
 bool aligned(const float* p, long long ld) { return ((uintptr_t)p & 15) == 0 && ld % 4 == 0; }
@@ -492,8 +599,8 @@ extern "C" int forge_gated_delta_chunks(const float* q, int ld_q, const float* k
     }
     const unsigned chunks = T / CH + S;
     cudaError_t e = forge::launch(chunk_solve_kernel, dim3(chunks, N), dim3(kThreads), 0, stream, 1, d);
-    if (e == cudaSuccess) e = forge::launch(chunk_walk_kernel, dim3(S, N, V / kColsB), dim3(kWalkThreads), kWalkSmem, stream, 1, d);
-    if (e == cudaSuccess) e = forge::launch(chunk_output_kernel<true>, dim3(chunks, N, V / VB), dim3(kOutThreads), 0, stream, 1, d);
+    if (e == cudaSuccess) e = forge::launch(chunk_walk_kernel, dim3((unsigned)S * N * (V / kColsB)), dim3(kWalkThreads), kWalkSmem, stream, 1, d);
+    if (e == cudaSuccess) e = launch_output<true>(d, chunks, stream);
     return forge::check_launch("gated_delta_chunks", e);
 }
 
@@ -507,6 +614,6 @@ extern "C" int forge_decay_chunks(const float* q, int ld_q, const float* k, int 
     const unsigned chunks = T / CH + S;
     cudaError_t e = forge::launch(chunk_update_kernel, dim3(chunks, N, V / VB), dim3(kThreads), 0, stream, 1, d);
     if (e == cudaSuccess) e = forge::launch(chunk_sum_kernel, dim3(S, N, (K * V / 4 + kThreads - 1) / kThreads), dim3(kThreads), 0, stream, 1, d);
-    if (e == cudaSuccess) e = forge::launch(chunk_output_kernel<false>, dim3(chunks, N, V / VB), dim3(kOutThreads), 0, stream, 1, d);
+    if (e == cudaSuccess) e = launch_output<false>(d, chunks, stream);
     return forge::check_launch("decay_chunks", e);
 }
