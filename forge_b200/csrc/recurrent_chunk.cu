@@ -14,7 +14,7 @@
 //     2  per (request, head, cols)  u = U - W S, the state before every chunk kept, S moved on        (fixed decay: S <- P_31 S + Z)
 //     3  per (chunk, head)          the outputs, from the kept states
 // The block scan they replace makes a chain of 900 instructions of every eight tokens with two to four warps an SM.  2,001 tokens in three portions, 32 heads:
-// 216 us with its gram matrices, 150 us here (solve 38, walk 74, outputs 38).  Fixed decay, 1,500 tokens in two portions, 64 heads: 252 us token by
+// 216 us with its gram matrices, 140 us here (solve 29, walk 73, outputs 38).  Fixed decay, 1,500 tokens in two portions, 64 heads: 252 us token by
 // token, 110 us here.  Every R is a
 // product of its decays (no quotients), so a decay of zero does no harm.  Scratch: W, U [chunks, N, 32, 64 | V] and the states
 // [chunks, N, 64, V], chunks = T / 32 + S.
@@ -69,10 +69,6 @@ __device__ __forceinline__ void stage_rows(float* dst, const float* src, int ld,
     }
 }
 
-__device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
-    return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, acc))));
-}
-
 // r[j][i] = g_{i+1} .. g_j for i <= j (zero above): thread j of the first 32 makes row j.
 __device__ __forceinline__ void decay_triangle(float (*r)[CH + 1], const float* g) {
     if (threadIdx.x < CH) {
@@ -85,8 +81,60 @@ __device__ __forceinline__ void decay_triangle(float (*r)[CH + 1], const float* 
     }
 }
 
+// The products of chunks on the tensor cores (m16n8k16): an fp32 number as the sum of three bfloat16 ones (its rounding, the rounding of what that
+// left, and of what that left: 2^-26 of it at most is missing), of the nine products of two such sums the six largest, each exact, fp32 sums.  The tensor
+// core cuts what an addend has below a sum's last place, so the large terms have a sum of their own over few steps; the state itself is moved on by
+// multiply-adds.  (A number that is not finite makes NaN of the sums that it takes part in.)
+struct Terms { uint32_t h, m, l; };                           // of two neighbouring numbers each
+__device__ __forceinline__ Terms split2(float x, float y) {
+    Terms t;
+    t.h = mma_sync::pack_bf16(x, y);
+    x -= __uint_as_float(t.h << 16);
+    y -= __uint_as_float(t.h & 0xffff0000u);
+    t.m = mma_sync::pack_bf16(x, y);
+    t.l = mma_sync::pack_bf16(x - __uint_as_float(t.m << 16), y - __uint_as_float(t.m & 0xffff0000u));
+    return t;
+}
+// main += the large term, rest += the others, of A (rows g and g + 8, steps 2t and 2t + 8 on) times B (steps 2t and 2t + 8 on, column g)
+__device__ __forceinline__ void mma_terms(float (&main)[4], float (&rest)[4], const Terms (&a)[4], const Terms (&b)[2]) {
+    const uint32_t ah[4] = {a[0].h, a[1].h, a[2].h, a[3].h}, am[4] = {a[0].m, a[1].m, a[2].m, a[3].m}, al[4] = {a[0].l, a[1].l, a[2].l, a[3].l};
+    mma_sync::mma_bf16(rest, al, b[0].h, b[1].h);
+    mma_sync::mma_bf16(main, ah, b[0].h, b[1].h);
+    mma_sync::mma_bf16(rest, ah, b[0].l, b[1].l);
+    mma_sync::mma_bf16(rest, am, b[0].m, b[1].m);
+    mma_sync::mma_bf16(rest, am, b[0].h, b[1].h);
+    mma_sync::mma_bf16(rest, ah, b[0].m, b[1].m);
+}
+// (the walk's: two chains of the others, as little as possible waits for the sum before)
+__device__ __forceinline__ void mma_terms(float (&main)[4], float (&rest)[2][4], const Terms (&a)[4], const Terms (&b)[2]) {
+    const uint32_t ah[4] = {a[0].h, a[1].h, a[2].h, a[3].h}, am[4] = {a[0].m, a[1].m, a[2].m, a[3].m}, al[4] = {a[0].l, a[1].l, a[2].l, a[3].l};
+    mma_sync::mma_bf16(rest[0], al, b[0].h, b[1].h);
+    mma_sync::mma_bf16(rest[1], am, b[0].h, b[1].h);
+    mma_sync::mma_bf16(main, ah, b[0].h, b[1].h);
+    mma_sync::mma_bf16(rest[0], ah, b[0].l, b[1].l);
+    mma_sync::mma_bf16(rest[1], ah, b[0].m, b[1].m);
+    mma_sync::mma_bf16(rest[0], am, b[0].m, b[1].m);
+}
+
+// main + rest = A B^T, 16 x 16 over 64: rows gr (and 8 further on) of A and of B at rows of LD, two 16 x 8 tiles
+__device__ __forceinline__ void square16(float (&main)[2][4], float (&rest)[2][4], const float* a, const float* b, int gr, int tq) {
+    auto pair = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return split2(v.x, v.y); };
+    a += gr * LD + 2 * tq;
+    b += gr * LD + 2 * tq;
+#pragma unroll
+    for (int kk = 0; kk < K; kk += 16) {
+        const Terms at[4] = {pair(a + kk), pair(a + 8 * LD + kk), pair(a + kk + 8), pair(a + 8 * LD + kk + 8)};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const Terms bt[2] = {pair(b + 8 * h * LD + kk), pair(b + 8 * h * LD + kk + 8)};
+            mma_terms(main[h], rest[h], at, bt);
+        }
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ 1: before the walk
-// DELTA: thread c solves the triangle for column c of [W | U].
+// DELTA: thread c solves the triangle for column c of [W | U].  The triangle itself, k k^T, is three 16 x 16 products on the tensor cores: as fp32 dot
+// products its operands were two thirds of the shared-memory reads that bound the kernel (2,001 tokens, 32 heads: 38.8 us, 28.7 so).
 __global__ void __launch_bounds__(kThreads)
 chunk_solve_kernel(const Chunks d) {
     __shared__ __align__(16) float ks[CH * LD], A[CH][CH + 4];
@@ -111,18 +159,19 @@ chunk_solve_kernel(const Chunks d) {
     stages_wait<0>();
     __syncthreads();
     {
-        const int j = tid >> 2, i0 = tid & 3;                 // entries (j, i0 + 4 m): a warp's rows lie in different banks
-        float acc[CH / 4];
+        // rows m0 .. m0 + 15, columns n0 .. n0 + 15 of k k^T under the diagonal, kept transposed: what row i does to the rows below
+        const int warp = tid >> 5, gr = (tid & 31) >> 2, tq = tid & 3, m0 = (warp & 1) * 16, n0 = (warp >> 1) * 16;
+        if (n0 <= m0) {
+            float main[2][4] = {}, rest[2][4] = {};
+            square16(main, rest, ks + m0 * LD, ks + n0 * LD, gr, tq);
 #pragma unroll
-        for (int m = 0; m < CH / 4; ++m) acc[m] = 0.f;
-#pragma unroll 4
-        for (int c = 0; c < K; c += 4) {
-            const float4 kj = *reinterpret_cast<const float4*>(ks + j * LD + c);
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int m = 0; m < CH / 4; ++m) acc[m] = dot4(kj, *reinterpret_cast<const float4*>(ks + (i0 + 4 * m) * LD + c), acc[m]);
+                for (int e = 0; e < 4; ++e) {
+                    const int j = m0 + gr + (e >> 1) * 8, i = n0 + 8 * h + 2 * tq + (e & 1);
+                    A[i][j] = bs[j] * R[j][i] * (main[h][e] + rest[h][e]);
+                }
         }
-#pragma unroll
-        for (int m = 0; m < CH / 4; ++m) A[i0 + 4 * m][j] = bs[j] * R[j][i0 + 4 * m] * acc[m];        // transposed: what row i does to the rows below
     }
     __syncthreads();
     for (int c = tid; c < K + d.V; c += kThreads) {
@@ -194,41 +243,6 @@ chunk_update_kernel(const Chunks d) {
 }
 
 // ------------------------------------------------------------------------------------------------ 2: the walk
-// The small products of the walk on the tensor cores (m16n8k16): an fp32 number as the sum of three bfloat16 ones (its rounding, the rounding of what that
-// left, and of what that left: 2^-26 of it at most is missing), of the nine products of two such sums the six largest, each exact, fp32 sums.  The tensor
-// core cuts what an addend has below a sum's last place, so the large terms have a sum of their own over few steps; the state itself is moved on by
-// multiply-adds.  (A number that is not finite makes NaN of the sums that it takes part in.)
-struct Terms { uint32_t h, m, l; };                           // of two neighbouring numbers each
-__device__ __forceinline__ Terms split2(float x, float y) {
-    Terms t;
-    t.h = mma_sync::pack_bf16(x, y);
-    x -= __uint_as_float(t.h << 16);
-    y -= __uint_as_float(t.h & 0xffff0000u);
-    t.m = mma_sync::pack_bf16(x, y);
-    t.l = mma_sync::pack_bf16(x - __uint_as_float(t.m << 16), y - __uint_as_float(t.m & 0xffff0000u));
-    return t;
-}
-// main += the large term, rest += the others, of A (rows g and g + 8, steps 2t and 2t + 8 on) times B (steps 2t and 2t + 8 on, column g)
-__device__ __forceinline__ void mma_terms(float (&main)[4], float (&rest)[4], const Terms (&a)[4], const Terms (&b)[2]) {
-    const uint32_t ah[4] = {a[0].h, a[1].h, a[2].h, a[3].h}, am[4] = {a[0].m, a[1].m, a[2].m, a[3].m}, al[4] = {a[0].l, a[1].l, a[2].l, a[3].l};
-    mma_sync::mma_bf16(rest, al, b[0].h, b[1].h);
-    mma_sync::mma_bf16(main, ah, b[0].h, b[1].h);
-    mma_sync::mma_bf16(rest, ah, b[0].l, b[1].l);
-    mma_sync::mma_bf16(rest, am, b[0].m, b[1].m);
-    mma_sync::mma_bf16(rest, am, b[0].h, b[1].h);
-    mma_sync::mma_bf16(rest, ah, b[0].m, b[1].m);
-}
-// (the walk's: two chains of the others, as little as possible waits for the sum before)
-__device__ __forceinline__ void mma_terms(float (&main)[4], float (&rest)[2][4], const Terms (&a)[4], const Terms (&b)[2]) {
-    const uint32_t ah[4] = {a[0].h, a[1].h, a[2].h, a[3].h}, am[4] = {a[0].m, a[1].m, a[2].m, a[3].m}, al[4] = {a[0].l, a[1].l, a[2].l, a[3].l};
-    mma_sync::mma_bf16(rest[0], al, b[0].h, b[1].h);
-    mma_sync::mma_bf16(rest[1], am, b[0].h, b[1].h);
-    mma_sync::mma_bf16(main, ah, b[0].h, b[1].h);
-    mma_sync::mma_bf16(rest[0], ah, b[0].l, b[1].l);
-    mma_sync::mma_bf16(rest[1], ah, b[0].m, b[1].m);
-    mma_sync::mma_bf16(rest[0], am, b[0].m, b[1].m);
-}
-
 // DELTA: 16 columns of one head's S a CTA; the next chunk's W, K, U and decays are on their way while the present one is worked on.  A chunk is
 // two small products, one after the other: u = U - W S (32 x 16 numbers over 64 channels, of which four warps take half and four the other half; those
 // ask for the next chunk while the first finish u) and S <- P S + K^T u (64 x 16 over 32 tokens; a warp keeps its 16 x 8 numbers of S in registers).  As fp32 multiply-adds, 4 x 4 numbers a thread and the sums shared by the warps, shared memory was asked
@@ -453,20 +467,7 @@ chunk_output_kernel(const Chunks d) {
         // rows m0 .. m0 + 15 of the triangle, columns n0 .. n0 + 15 (above the diagonal: zeros, whatever the keys there)
         const int m0 = (warp & 1) * 16, n0 = (warp >> 1) * 16;
         float main[2][4] = {}, rest[2][4] = {};
-        if (n0 <= m0) {
-#pragma unroll
-            for (int kk = 0; kk < K; kk += 16) {
-                const float* a = qs + (m0 + gr) * LD + kk + 2 * tq;
-                auto pair = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return split2(v.x, v.y); };
-                const Terms at[4] = {pair(a), pair(a + 8 * LD), pair(a + 8), pair(a + 8 * LD + 8)};
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float* b = ks + (n0 + 8 * h + gr) * LD + kk + 2 * tq;
-                    const Terms bt[2] = {pair(b), pair(b + 8)};
-                    mma_terms(main[h], rest[h], at, bt);
-                }
-            }
-        }
+        if (n0 <= m0) square16(main, rest, qs + m0 * LD, ks + n0 * LD, gr, tq);
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
