@@ -15,8 +15,7 @@
 //     3  per (chunk, head)          the outputs, from the kept states
 // The block scan they replace makes a chain of 900 instructions of every eight tokens with two to four warps an SM.  2,001 tokens in three portions, 32 heads:
 // 216 us with its gram matrices, 140 us here (solve 29, walk 73, outputs 38).  Fixed decay, 1,500 tokens in two portions, 64 heads: 252 us token by
-// token, 110 us here.  Every R is a
-// product of its decays (no quotients), so a decay of zero does no harm.  Scratch: W, U [chunks, N, 32, 64 | V] and the states
+// token, 110 us here before the outputs went to the tensor cores.  Every R is a product of its decays (no quotients), so a decay of zero does no harm.  Scratch: W, U [chunks, N, 32, 64 | V] and the states
 // [chunks, N, 64, V], chunks = T / 32 + S.
 #include "common.cuh"
 #include "mma_sync.cuh"

@@ -1358,6 +1358,7 @@ def chunks_pay(kind, lens, N, V):
                    portions of 400 of 64 heads 96 and 131
       lightning    scan 6 + 0.1 longest, chunks 13 + 1.2 W: 400 tokens of 32 heads 51 and 29, four portions of 400 of 64 heads of 128 256 and 288
       retention    scan the larger of 4 + 0.168 longest and 1.6 W, chunks 13 + 1.15 W: 200 tokens of 64 heads 45 and 29, 64 tokens of 32 heads 14 and 25
+    (The delta rule's chunks take 0.75 of these times since their products are on the tensor cores; the line stays where they are faster for certain.)
     Below some work a step waits for the host, which two kernels more keep longer: hence the least work, or the longest portion, of the last line."""
     longest = max(lens)
     W, filled = (n * N * V / 64000.0 for n in (sum(lens), sum(-(-n // CHUNK_TOKENS) for n in lens) * CHUNK_TOKENS))
