@@ -330,7 +330,9 @@ head_finish_kernel(const float* __restrict__ o, const float* __restrict__ weight
 // Retention for a step in which every request brings one token: a CTA per (request, head) asks for its state first, rotates q and k meanwhile,
 // and norms, gates and stores the head itself.  A row of the state is V / 4 packs of four value channels; thread t holds pack t % CG (CG = V / 4)
 // of the rows t / CG, t / CG + RG, ...; the RG partial sums of an output are added in their order.  Bound by the state's way in and out (64 requests,
-// 64 heads of 64 x 64: 134 MB; the scan of portions with the rotation before and the norm behind it 57 us, 33 us so, 4.1 TB/s).
+// 64 heads of 64 x 64: 134 MB; the scan of portions with the rotation before and the norm behind it 57 us, 33 us so, 4.1 TB/s; what lies on its way decides, so
+// the packs wait in shared memory: in registers, beside the angles' slow path, three CTAs an SM were left (one with 16 packs a thread), now six: 24.4 us, 5.5 TB/s;
+// eight with 32 registers a thread 28.9).
 constexpr int kRetThreads = 256, kRetHeld = 16;
 bool retention_token_fits(int K, int V) {
     const int cg = V / 4;
@@ -338,24 +340,26 @@ bool retention_token_fits(int K, int V) {
 }
 
 template <int HELD, typename TA>
-__global__ void __launch_bounds__(kRetThreads)
+__global__ void __launch_bounds__(kRetThreads, HELD <= 4 ? 6 : HELD <= 8 ? 5 : 3)
 retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const int32_t* __restrict__ positions, const float* __restrict__ freq, int rot_dims,
                        float k_scale, const float* __restrict__ decay, float* __restrict__ state, long long state_stride, const int32_t* __restrict__ q_start,
                        const int32_t* __restrict__ slots, const float* __restrict__ weight, float eps, TA* __restrict__ out, long long out_ld, int N, int K, int V) {
     __shared__ float qs[256], ks[256], red[8];
     __shared__ __align__(16) float4 part[kRetThreads];
+    extern __shared__ __align__(16) float4 stage[];           // [HELD][kRetThreads], each read by the thread that asked for it
     forge::pdl_launch_dependents();
     forge::pdl_wait();
     const int s = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, t = q_start[s];
     const int CG = V / 4, RG = kRetThreads / CG, rg = tid / CG, cp = tid % CG;
     const bool live = rg < RG;
     float4* S = reinterpret_cast<float4*>(state + (size_t)slots[s] * state_stride + (size_t)head * K * V);
-    float4 held[HELD];
 #pragma unroll
     for (int m = 0; m < HELD; ++m) {
         const int row = rg + m * RG;
-        held[m] = live && row < K ? S[(size_t)row * CG + cp] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live && row < K)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(stage + m * kRetThreads + tid)), "l"(S + (size_t)row * CG + cp) : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
     const float dec = decay[head];
     float4 vv = make_float4(0.f, 0.f, 0.f, 0.f), gate = vv, w = vv;
     if (live) {
@@ -384,6 +388,7 @@ retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const
         qs[i] = qp[i];
         ks[i] = kp[i] * k_scale;
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -391,7 +396,7 @@ retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const
         const int row = rg + m * RG;
         if (!live || row >= K) continue;
         const float kk = ks[row], qq = qs[row];
-        float4 x = held[m];
+        float4 x = stage[m * kRetThreads + tid];
         x.x = fmaf(dec, x.x, kk * vv.x); x.y = fmaf(dec, x.y, kk * vv.y); x.z = fmaf(dec, x.z, kk * vv.z); x.w = fmaf(dec, x.w, kk * vv.w);
         S[(size_t)row * CG + cp] = x;
         acc.x = fmaf(qq, x.x, acc.x); acc.y = fmaf(qq, x.y, acc.y); acc.z = fmaf(qq, x.z, acc.z); acc.w = fmaf(qq, x.w, acc.w);
@@ -419,6 +424,19 @@ retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const
     dst[1] = forge::from_float<TA>(o.y * inv * w.y * (gate.y * sigmoidf(gate.y)));
     dst[2] = forge::from_float<TA>(o.z * inv * w.z * (gate.z * sigmoidf(gate.z)));
     dst[3] = forge::from_float<TA>(o.w * inv * w.w * (gate.w * sigmoidf(gate.w)));
+}
+
+template <int HELD, typename TA, typename... Args>
+cudaError_t retention_token_launch(dim3 grid, cudaStream_t stream, Args... args) {
+    constexpr int kBytes = HELD * kRetThreads * (int)sizeof(float4);
+    static forge::PerDeviceFlag flag;
+    bool& done = flag.current();
+    if (!done) {
+        const cudaError_t e = cudaFuncSetAttribute(retention_token_kernel<HELD, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+        if (e != cudaSuccess) return e;
+        done = true;
+    }
+    return forge::launch(retention_token_kernel<HELD, TA>, grid, dim3(kRetThreads), kBytes, stream, 1, args...);
 }
 
 // The same for heads of 32, 64 or 128 channels and aligned rows: K / 4 neighbouring lanes a head with four channels each, so that a warp has 4, 2
@@ -775,8 +793,8 @@ extern "C" int forge_retention_token(const float* q, int ld_q, const float* k, i
     if (S == 0) return FORGE_OK;
     const int rg = kRetThreads / (V / 4), held = (K + rg - 1) / rg;
     cudaError_t e = cudaSuccess;
-#define FORGE_RET(HELD) FORGE_DISPATCH_DTYPE(dtype, TT, e = forge::launch(retention_token_kernel<HELD, TT>, dim3(S, N), dim3(kRetThreads), 0, stream, 1, ScanInput{q, ld_q}, \
-        ScanInput{k, ld_k}, ScanInput{v, ld_v}, ScanInput{g, ld_g}, positions, freq, rot_dims, k_scale, decay, state, state_stride, q_start, slots, weight, eps, (TT*)out, out_ld, N, K, V))
+#define FORGE_RET(HELD) FORGE_DISPATCH_DTYPE(dtype, TT, (e = retention_token_launch<HELD, TT>(dim3(S, N), stream, ScanInput{q, ld_q}, ScanInput{k, ld_k}, ScanInput{v, ld_v}, \
+        ScanInput{g, ld_g}, positions, freq, rot_dims, k_scale, decay, state, state_stride, q_start, slots, weight, eps, (TT*)out, out_ld, N, K, V)))
     if (held <= 4) FORGE_RET(4); else if (held <= 8) FORGE_RET(8); else FORGE_RET(kRetHeld);
 #undef FORGE_RET
     return forge::check_launch("retention_token", e);
