@@ -199,11 +199,11 @@ __global__ void __launch_bounds__(128)
 delta_prepare_vec_kernel(const DeltaPrepare d, int run) {
     const int lane = threadIdx.x & 31, first = (blockIdx.x * 4 + (threadIdx.x >> 5)) * run, last = min(first + run, d.T);
     const int C = d.cv.channels, qk = 2 * d.M * d.K, c0 = blockIdx.y * 128, c = c0 + lane * 4;
+    forge::pdl_wait();                                                    // (the filter too may come from the kernel ahead)
+    if (first >= d.T) return;
     float4 w[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[j] = j < d.cv.taps ? *reinterpret_cast<const float4*>(d.cv.w + (size_t)j * C + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    forge::pdl_wait();
-    if (first >= d.T) return;
     const float* x = d.p.p + c;
     const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 x1 = none, x2 = none, x3 = none;

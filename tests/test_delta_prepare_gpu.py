@@ -36,3 +36,29 @@ def test_both_kernels(reqs, N, M, V, taps):
         got.append(kernels.gated_delta_prepare(rows, col, col + C, col + C + N, conv, rate, dt, batch, state, N, M, K, V) + (state,))
     for a, b in zip(*got):
         assert bool(torch.isfinite(a).all()) and torch.equal(a, b)
+
+
+def test_the_filter_may_come_from_the_kernel_ahead():
+    """The filter is looked up in a table, another one each time into the same buffer, by a kernel launched right before the preparation: none of the
+    buffer's old numbers may enter."""
+    from forge_b200 import kernels
+    N, M, K, V, taps, T = 64, 32, 64, 64, 4, 40
+    C = 2 * M * K + N * V
+    g = torch.Generator().manual_seed(5)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(num_requests=1, num_tokens=T, q_start=i32([0, T]), slots=i32([0]), tok_req=i32([0] * T), positions=i32(list(range(T))))
+    p = torch.randn(T, C + 2 * N, generator=g).to(DEV)
+    rate, dt = torch.rand(N, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV)
+    state = torch.zeros(1, N * K * V + taps * C, device=DEV)
+    tables = [torch.randn(1024, C, generator=g).to(DEV) for _ in range(3)]
+    ids = torch.arange(1023, -1, -1, dtype=torch.int32, device=DEV)
+    prepare = lambda conv: kernels.gated_delta_prepare(p, 0, C, C + N, conv, rate, dt, batch, state, N, M, K, V)[0]
+    wants = [prepare(t.flip(0)[-taps:].contiguous()) for t in tables]
+    torch.cuda.synchronize()
+    got = []
+    for i in range(12):
+        rows = kernels.embedding(ids, tables[i % 3])
+        got.append(prepare(rows[-taps:]))                     # (the rows that the kernel ahead writes last)
+        del rows                                              # its buffer is the next round's
+    for i, y in enumerate(got):
+        assert torch.equal(y, wants[i % 3]), i
