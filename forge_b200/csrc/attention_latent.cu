@@ -83,15 +83,15 @@ latent_expand_kernel(const float* __restrict__ q, long long ld, const int32_t* _
                      __nv_bfloat16* __restrict__ c_out, __nv_bfloat16* __restrict__ kr_out) {
     __shared__ float2 turn[64];                                 // (cos, sin) of the token's position, R <= 128
     forge::pdl_launch_dependents();
+    forge::pdl_wait();
     if ((int)blockIdx.x < T) {
         const int t = blockIdx.x;
-        if ((int)threadIdx.x < (R >> 1)) {                      // (positions and frequencies were there before the step's first kernel)
+        if ((int)threadIdx.x < (R >> 1)) {
             float sn, cs;
             sincosf((float)positions[t] * freq[threadIdx.x], &sn, &cs);
             turn[threadIdx.x] = make_float2(cs * amp, sn * amp);
         }
         __syncthreads();
-        forge::pdl_wait();
         const int width = D + R, pieces = width >> 3;           // (D and R are multiples of 16)
         const float* src = q + (size_t)t * ld;
         __nv_bfloat16* dst = q_out + (size_t)t * H * width;
@@ -139,7 +139,6 @@ latent_expand_kernel(const float* __restrict__ q, long long ld, const int32_t* _
         }
         return;
     }
-    forge::pdl_wait();
     const int lane = threadIdx.x & 31, n = ((int)blockIdx.x - T) * (kExpandThreads / 32) + (threadIdx.x >> 5);
     if (n >= rows) return;
     int lo = 0, hi = S - 1;                                     // the last request that begins at or before row n

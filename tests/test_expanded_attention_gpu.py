@@ -78,3 +78,27 @@ def test_rows_behind_a_request_are_never_seen():
     kv[70:] = float("nan")
     kr[70:] = float("nan")
     assert torch.equal(kernels.expanded_attention(q, kv, kr, starts, batch, H, D, R, E, 0.1)[:70], whole)
+
+
+def test_positions_may_come_from_the_kernel_ahead():
+    """The tokens' positions are written by a kernel launched right before, other ones each time into the same buffer: none of the old ones may enter."""
+    from forge_b200 import kernels
+    H, C, D, R, ps, T = 2, 64, 64, 32, 64, 64
+    batch, table, n_pages, g = _batch([(0, T)], ps, C + R, seed=2)
+    cache, group = torch.zeros(n_pages, ps * (C + R), dtype=torch.bfloat16, device=DEV), SimpleNamespace(block_table=table.to(DEV))
+    q, freq = torch.randn(T, H * (D + R), generator=g).to(DEV), (10000.0 ** (-2.0 * torch.arange(R // 2) / R)).to(DEV)
+    places = [torch.randint(0, 20000, (T,), generator=g) for _ in range(3)]
+    rows = [torch.nn.functional.one_hot(p, 20000).float().to(DEV) for p in places]
+
+    def expand(positions):
+        batch.positions = positions
+        return kernels.latent_expand(q, cache, group, batch, H, C, D, R, ps, freq)[0]
+
+    wants = [expand(p.to(torch.int32).to(DEV)) for p in places]
+    torch.cuda.synchronize()
+    got = []
+    for i in range(12):
+        got.append(expand(kernels.argmax(rows[i % 3])))
+        batch.positions = None                                # its buffer is the next round's
+    for i, y in enumerate(got):
+        assert torch.equal(y, wants[i % 3]), i
