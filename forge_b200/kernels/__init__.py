@@ -966,10 +966,11 @@ def headmix_plan(batch, TQ, device):
 
 
 def _tokens_before(batch):
-    """How many tokens each of the step's requests had in the cache before it."""
+    """How many tokens each of the step's requests had in the cache before it (a request that brings none: 0)."""
     before = getattr(batch, "host_context_before", None)
-    if not before:                     # (a batch that was not laid out by the engine)
-        before = batch.host_context_before = batch.positions[torch.tensor(batch.host_q_start[:-1], device=batch.positions.device)].tolist()
+    if not before:                     # (a batch that was not laid out by the engine: the position of a request's first token)
+        qs, positions = batch.host_q_start, batch.positions.tolist()
+        before = batch.host_context_before = [positions[a] if a < b else 0 for a, b in zip(qs, qs[1:])]
     return before
 
 
