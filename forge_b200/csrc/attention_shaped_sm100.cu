@@ -35,11 +35,6 @@ constexpr int kThreads = 384, kRowWarps = 8, NK = BKV / 2;      // four warps th
 // two CTAs an SM: 65,536 / (2 x 384) registers a thread, dealt out anew between the three warpgroups
 constexpr int kLaunchRegs = 80, kRegsFew = 48, kRegsMany = 96;
 static_assert(kRegsFew + 2 * kRegsMany <= 3 * kLaunchRegs, "the warpgroups cannot hold more registers than the CTA was given");
-#if FORGE_CHECKS
-constexpr bool kPagesMayBeSkipped = true;                      // (a checks build skips a page id that is none)
-#else
-constexpr bool kPagesMayBeSkipped = false;
-#endif
 constexpr int kQBlock = BQ * 128, kBlock = BKV * 128;          // bytes of 64 channels of the queries / of a tile of keys
 constexpr int kMaxStages = 3, kBarBytes = 256, kSmemLimit = 227 * 1024 - 1024;      // (1 KB of it is the rows' meeting place)
 constexpr int kSmemTwo = (228 * 1024 - 2 * 2048) / 2;          // of two CTAs an SM (1 KB of each is the system's, 1 KB the meeting place)
@@ -155,6 +150,17 @@ __device__ __forceinline__ u64 pair2(uint32_t lo, uint32_t hi) {
 __device__ __forceinline__ float low2(u64 v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float high2(u64 v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
+// Boxes of a tile that bring nothing (behind the window, beyond the request, or without a page in the table) count as zeros: what the slot held before may
+// be no number, which a weight of 0 would not silence.  (Out of line: the copies' loop has no instruction to spare.)
+__device__ __noinline__ void clear_boxes(uint8_t* tile, int blocks, uint32_t missing, uint32_t box_bytes) {
+    for (; missing != 0; missing &= missing - 1)
+        for (int b = 0; b < blocks; ++b)
+            for (uint32_t at = (threadIdx.x & 31) * 16; at < box_bytes; at += 512)
+                *reinterpret_cast<uint4*>(tile + b * kBlock + (__ffs(missing) - 1) * box_bytes + at) = make_uint4(0, 0, 0, 0);
+    fence_proxy_async();
+    __syncwarp();
+}
+
 template <bool SHAPED, int PER_SM>
 __global__ void __launch_bounds__(kThreads, PER_SM)
 shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -209,13 +215,6 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         prefetch_tensormap(&tmap_k);
         prefetch_tensormap(&tmap_v);
     }
-    // Where a tile of keys comes as several pages the stages start as zeros: pages that are skipped (behind the window, beyond the request) leave their
-    // rows as they are, and those rows must hold finite numbers (their weights are 0).  (A tile out of one page always lands whole.)
-    if (p.box_rows < BKV || kPagesMayBeSkipped) {
-        uint4* z = reinterpret_cast<uint4*>(k_s);
-        const int n = (int)(reinterpret_cast<uint8_t*>(q_full) - k_s) / 16;
-        for (int i = threadIdx.x; i < n; i += kThreads) z[i] = make_uint4(0, 0, 0, 0);
-    }
     fence_proxy_async();
     if (warp == 1) {
         tmem_alloc(tmem_slot, p.tmem_cols);
@@ -261,6 +260,7 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             return page;
         };
         const uint32_t box_bytes = p.box_rows * 128;
+        const uint32_t all_boxes = (1u << ppt) - 1;
         int st = 0, ph = 0, next_page = -1;
         if (warp == 0) {
             if (lane == 0) {
@@ -275,9 +275,11 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 int page = next_page;
                 next_page = page_of(it + 1);
                 if (page >= 0 && !packed && !FORGE_PAGE_OK(page)) page = -1;
-                const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0)), row = packed ? row0 + j0 : row0 + (j0 & page_mask);
+                const uint32_t live = __ballot_sync(0xffffffffu, page >= 0);
+                const int row = packed ? row0 + j0 : row0 + (j0 & page_mask);
                 if (!warp_wait<true>(&k_empty[st], ph ^ 1, abort, p.status, 1)) break;
-                if (lane == 0) mbar_arrive_expect_tx(&k_full[st], p.key_blocks * n_valid * box_bytes);
+                if (live != all_boxes) clear_boxes(k_s + st * p.key_blocks * kBlock, p.key_blocks, all_boxes & ~live, box_bytes);
+                if (lane == 0) mbar_arrive_expect_tx(&k_full[st], p.key_blocks * __popc(live) * box_bytes);
                 __syncwarp();
                 if (page >= 0) {
                     uint8_t* dst = k_s + st * p.key_blocks * kBlock + lane * box_bytes;
@@ -299,12 +301,14 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 int page = next_page;
                 next_page = page_of(it + 1);
                 if (page >= 0 && !packed && !FORGE_PAGE_OK(page)) page = -1;
-                const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0)), row = packed ? row0 + j0 : row0 + (j0 & page_mask);
+                const uint32_t live = __ballot_sync(0xffffffffu, page >= 0);
+                const int row = packed ? row0 + j0 : row0 + (j0 & page_mask);
                 const bool last = j0 + BKV - 1 > pos_last;                // rows behind the last token: cleared below
                 uint64_t* landed = last ? tail : &v_full[st];
                 uint8_t* vd = v_s + st * p.value_blocks * kBlock;
                 if (!warp_wait<true>(&v_empty[st], ph ^ 1, abort, p.status, 2)) break;
-                if (lane == 0) mbar_arrive_expect_tx(landed, p.value_blocks * n_valid * box_bytes);
+                if (live != all_boxes) clear_boxes(vd, p.value_blocks, all_boxes & ~live, box_bytes);
+                if (lane == 0) mbar_arrive_expect_tx(landed, p.value_blocks * __popc(live) * box_bytes);
                 __syncwarp();
                 if (page >= 0)
                     for (int b = 0; b < p.value_blocks; b += p.v_boxed)

@@ -40,11 +40,6 @@ using namespace sm100;
 
 constexpr int HD = FORGE_ATT_HD, BQ = 128, BKV = 64, UMMA_K = 16;
 static_assert(HD == 64 || HD == 128, "head size 64 or 128");
-#if FORGE_CHECKS
-constexpr bool kPagesMayBeSkipped = true;         // (a checks build skips a page id that is none)
-#else
-constexpr bool kPagesMayBeSkipped = false;
-#endif
 constexpr int KB = HD / 64;                       // 64-wide blocks of the head: Q, K and V tiles are KB swizzled blocks
 constexpr int kThreads = 384;                     // warps 0-3: keys, P V, Q K^T, values; warps 4-11: the softmax rows
 constexpr int kQkWarp = 2, kValueWarp = 3, kRowWarps = 8, NK = BKV / 2;  // NK: a thread's keys of a tile
@@ -179,10 +174,6 @@ paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
         prefetch_tensormap(&tmap_q);
         prefetch_tensormap(&tmap_kv);
     }
-    // Where a tile of keys comes as several pages the stages start as zeros: pages that are skipped (beyond the request, or released by the window) leave
-    // their rows as they are, and those rows must hold finite numbers (their weights are 0).  (A tile out of one page always lands whole.)
-    if (p.page_size < BKV || kPagesMayBeSkipped)
-        for (int i = threadIdx.x; i < 2 * kStages * kKVBytes / 16; i += kThreads) reinterpret_cast<uint4*>(k_s)[i] = make_uint4(0, 0, 0, 0);
     fence_proxy_async();
     if (warp == 1) {
         tmem_alloc(tmem_slot, kTmemCols);
@@ -245,9 +236,20 @@ paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
             int page = next_page;
             next_page = page_of(it + 1);
             if (page >= 0 && !FORGE_PAGE_OK(page)) page = -1;
-            const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0));
+            const uint32_t live = __ballot_sync(0xffffffffu, page >= 0);
             if (!warp_wait<true>(&empty[st], ph ^ 1, abort, p.status, values ? 9 : 1)) break;
-            if (lane == 0) mbar_arrive_expect_tx(&full[st], KB * n_valid * page_bytes);
+            // Pages that bring nothing (beyond the request, released by the window, or none in the table) count as zeros: what the slot held before may
+            // be no number, which a weight of 0 would not silence
+            if (__popc(live) < ppt) {
+                for (int i = 0; i < ppt; ++i)
+                    if (!(live >> i & 1))
+                        for (int kb = 0; kb < KB; ++kb)
+                            for (uint32_t at = lane * 16; at < page_bytes; at += 512)
+                                *reinterpret_cast<uint4*>(ring + st * kKVBytes + kb * kKVBlock + i * page_bytes + at) = make_uint4(0, 0, 0, 0);
+                fence_proxy_async();
+                __syncwarp();
+            }
+            if (lane == 0) mbar_arrive_expect_tx(&full[st], KB * __popc(live) * page_bytes);
             __syncwarp();
             if (page >= 0) {
                 const int row = ((page * 2 + (values ? 1 : 0)) * p.NKV + kvh) * p.page_size;
