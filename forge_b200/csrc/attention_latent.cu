@@ -91,8 +91,7 @@ latent_expand_kernel(const float* __restrict__ q, long long ld, const int32_t* _
             sincosf((float)positions[t] * freq[threadIdx.x], &sn, &cs);
             turn[threadIdx.x] = make_float2(cs * amp, sn * amp);
         }
-        __syncthreads();
-        const int width = D + R, pieces = width >> 3;           // (D and R are multiples of 16)
+        const int width = D + R, plain = D >> 3, turned = R >> 3;
         const float* src = q + (size_t)t * ld;
         __nv_bfloat16* dst = q_out + (size_t)t * H * width;
         const bool vec = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
@@ -105,37 +104,47 @@ latent_expand_kernel(const float* __restrict__ q, long long ld, const int32_t* _
                 for (int i = 0; i < 4; ++i) v[i] = p[i];
             }
         };
-        for (int i = threadIdx.x; i < H * pieces; i += kExpandThreads) {
-            const int h = i / pieces, c = (i - h * pieces) << 3;
-            const float* s = src + (size_t)h * width + c;
+        auto store8 = [&](size_t at, const float* v) {
+            *reinterpret_cast<uint4*>(dst + at) =
+                make_uint4(mma_sync::pack_bf16(v[0], v[1]), mma_sync::pack_bf16(v[2], v[3]), mma_sync::pack_bf16(v[4], v[5]), mma_sync::pack_bf16(v[6], v[7]));
+        };
+        for (int i = threadIdx.x; i < H * plain; i += kExpandThreads) {          // (first, so that nobody waits for the angles)
+            const int h = i / plain;
+            const size_t at = (size_t)h * width + ((i - h * plain) << 3);
+            float v[8];
+            load4(src + at, v);
+            load4(src + at + 4, v + 4);
+            store8(at, v);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < H * turned; i += kExpandThreads) {
+            const int h = i / turned, r = (i - h * turned) << 3, half = R >> 1;
+            const size_t at = (size_t)h * width + D + r;
+            const float* s = src + at;
             float v[8];
             load4(s, v);
             load4(s + 4, v + 4);
-            if (c >= D) {
-                const int r = c - D, half = R >> 1;
-                if (!halves) {
+            if (!halves) {
 #pragma unroll
-                    for (int e = 0; e < 8; e += 2) {
-                        const float2 w = turn[(r + e) >> 1];
-                        const float a = v[e], b = v[e + 1];
-                        v[e] = a * w.x - b * w.y;
-                        v[e + 1] = b * w.x + a * w.y;
-                    }
-                } else {                                        // (R a multiple of 16: a piece of eight lies in one half)
-                    const bool first = r < half;
-                    const float* other = first ? s + half : s - half;
-                    float o[8];
-                    load4(other, o);
-                    load4(other + 4, o + 4);
+                for (int e = 0; e < 8; e += 2) {
+                    const float2 w = turn[(r + e) >> 1];
+                    const float a = v[e], b = v[e + 1];
+                    v[e] = a * w.x - b * w.y;
+                    v[e + 1] = b * w.x + a * w.y;
+                }
+            } else {                                            // (R a multiple of 16: a piece of eight lies in one half)
+                const bool first = r < half;
+                const float* other = first ? s + half : s - half;
+                float o[8];
+                load4(other, o);
+                load4(other + 4, o + 4);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float2 w = turn[first ? r + e : r + e - half];
-                        v[e] = first ? v[e] * w.x - o[e] * w.y : v[e] * w.x + o[e] * w.y;
-                    }
+                for (int e = 0; e < 8; ++e) {
+                    const float2 w = turn[first ? r + e : r + e - half];
+                    v[e] = first ? v[e] * w.x - o[e] * w.y : v[e] * w.x + o[e] * w.y;
                 }
             }
-            *reinterpret_cast<uint4*>(dst + (size_t)h * width + c) =
-                make_uint4(mma_sync::pack_bf16(v[0], v[1]), mma_sync::pack_bf16(v[2], v[3]), mma_sync::pack_bf16(v[4], v[5]), mma_sync::pack_bf16(v[6], v[7]));
+            store8(at, v);
         }
         return;
     }
