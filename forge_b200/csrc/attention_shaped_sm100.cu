@@ -45,7 +45,7 @@ struct ShapedParams {
     __nv_bfloat16* out;               // row t at out + t * out_ld, head h's values from h * E on (u == null)
     float* u;                         // fp32 [T, H, M, E], normalised (two maps)
     long long out_ld;
-    const __nv_bfloat16* q;           // (q_tmem) [T, H, D]
+    const __nv_bfloat16* q;           // (q_tmem or packed) [T, H, q_channels]
     const int32_t* block_table;
     const int4* tiles;                // (first token, tokens, request, the first token's position)
     const float *r1, *r2, *sink;
@@ -55,6 +55,7 @@ struct ShapedParams {
     int k_boxed, v_boxed;             // blocks that one copy of a tile of keys (values) brings: all, where a page holds a whole tile, else one
     int latent;                       // the value blocks are key blocks too
     const int32_t* row_start;         // (packed keys and values) a request's first row, else null
+    const __nv_bfloat16 *kv, *kr;     // (packed) [rows, H, D + E] and [rows, q_channels - D]
     int q_tmem;                       // ... and the query channels that meet them are in TMEM, not in shared memory
     int stages, page_size, box_rows, max_pages, window, chunk, vec_out;
     float scale, softcap, out_scale;
@@ -161,10 +162,58 @@ __device__ __noinline__ void clear_boxes(uint8_t* tile, int blocks, uint32_t mis
     __syncwarp();
 }
 
+// (Packed keys and values.)  A weight of 0 does not silence a number that is none: one among the values of a token reaches the tokens before it in its
+// tile, up to 127 of them.  A row with such a result therefore looks whether a later token of its tile has such a value in these 32 columns, and if so adds
+// its outputs up again over the keys that it sees, a thread on its own: time only where there is such a number.
+__device__ __noinline__ void without_later_tokens(const ShapedParams& p, uint32_t columns, int head, int tok, int row0, int pos, int pos_last, float mult,
+                                                  float ref, float inv) {
+    const int R = p.q_channels - p.D, width = p.D + p.E;
+    const size_t ld = (size_t)p.H * width;
+    const __nv_bfloat16* q = p.q + ((size_t)tok * p.H + head) * p.q_channels;
+    const __nv_bfloat16* kv = p.kv + row0 * ld + (size_t)head * width;
+    const __nv_bfloat16* kr = p.kr + (size_t)row0 * R;
+    auto low = [](uint32_t w) { return __uint_as_float(w << 16); };
+    auto high = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
+    auto dot = [&](const __nv_bfloat16* a, const __nv_bfloat16* b, int n, float sum) {
+        for (int i = 0; i < n; i += 8) {
+            const uint4 x = *reinterpret_cast<const uint4*>(a + i), y = *reinterpret_cast<const uint4*>(b + i);
+            sum = fmaf(low(x.x), low(y.x), sum); sum = fmaf(high(x.x), high(y.x), sum); sum = fmaf(low(x.y), low(y.y), sum); sum = fmaf(high(x.y), high(y.y), sum);
+            sum = fmaf(low(x.z), low(y.z), sum); sum = fmaf(high(x.z), high(y.z), sum); sum = fmaf(low(x.w), low(y.w), sum); sum = fmaf(high(x.w), high(y.w), sum);
+        }
+        return sum;
+    };
+    for (; columns != 0; columns &= columns - 1) {
+        const int c = (__ffs(columns) - 1) * 32;
+        bool none = false;
+        for (int j = pos + 1; j <= pos_last && !none; ++j)
+            for (int i = 0; i < 32; i += 2) {
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(kv + j * ld + p.D + c + i);
+                none |= !isfinite(low(w)) || !isfinite(high(w));
+            }
+        if (!none) continue;
+        float acc[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+        for (int j = 0; j <= pos; ++j) {
+            const float s = dot(q + p.D, kr + (size_t)j * R, R, dot(q, kv + j * ld, p.D, 0.f)), x = ex2(fmaf(s, mult, -ref));
+            const uint32_t* v = reinterpret_cast<const uint32_t*>(kv + j * ld + p.D + c);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const uint32_t w = v[i];
+                acc[2 * i] = fmaf(x, low(w), acc[2 * i]);
+                acc[2 * i + 1] = fmaf(x, high(w), acc[2 * i + 1]);
+            }
+        }
+        uint32_t* dst = reinterpret_cast<uint32_t*>(p.out + (size_t)tok * p.out_ld + (size_t)head * p.E + c);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) dst[i] = pack_bf16(acc[2 * i] * inv, acc[2 * i + 1] * inv);
+    }
+}
+
 template <bool SHAPED, int PER_SM>
 __global__ void __launch_bounds__(kThreads, PER_SM)
 shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                              const __grid_constant__ CUtensorMap tmap_v, const ShapedParams p) {
+                              const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ ShapedParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ float meet[2][BQ];                                   // [half]: what a row's two threads tell each other
     const int tile = blockIdx.x / p.inner;
@@ -565,6 +614,7 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             uint8_t* stage = smem + (warp - 4) * 4096;
             const long long own = !valid ? -1 : v0 + (p.u != nullptr ? (((long long)tok * p.H + head) * p.M + mp) * p.E : (long long)tok * p.out_ld + (long long)head * p.E);
             const int share = p.VC / 2;
+            uint32_t odd = 0;                            // the 32 columns (a bit each) among whose results are numbers that are none
             for (int c = half * share; c < (half + 1) * share; c += 32) {
                 uint32_t ov[32];
                 __syncwarp();
@@ -572,6 +622,12 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * inv);
+                if (!SHAPED && p.row_start != nullptr) {
+                    float z = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) z = fmaf(__uint_as_float(ov[i]), 0.f, z);
+                    if (z != 0.f) odd |= 1u << (c >> 5);
+                }
                 if (p.u != nullptr) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
@@ -608,6 +664,10 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                         }
                     }
                 }
+            }
+            if (!SHAPED && p.row_start != nullptr) {     // (a sum of weights that is none: a key or a query is, and the result what it has to be)
+                __syncwarp();
+                if (odd != 0 && valid && isfinite(l)) without_later_tokens(p, odd, head, tok, p.row_start[req], pos, pos_last, sl2, m == -INFINITY ? 0.f : m, inv);
             }
         }
     }
@@ -779,6 +839,7 @@ extern "C" int forge_expanded_attention_sm100(const void* q, const void* kv, con
     p.sink = sink;
     p.H = H; p.heads = 1; p.inner = H; p.M = 1; p.D = D; p.E = E; p.VC = E;
     p.q_channels = D + R; p.key_blocks = (D + R + 63) / 64; p.value_blocks = E / 64; p.latent = 0;
+    p.q = (const __nv_bfloat16*)q; p.kv = (const __nv_bfloat16*)kv; p.kr = (const __nv_bfloat16*)kr;
     p.k_boxed = 1; p.v_boxed = boxed;
     p.page_size = BKV; p.max_pages = 1;
     p.vec_out = ((uintptr_t)out & 15) == 0 && out_ld % 8 == 0; p.scale = scale; p.out_scale = 1.0f; p.status = status;

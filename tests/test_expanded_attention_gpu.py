@@ -102,3 +102,35 @@ def test_positions_may_come_from_the_kernel_ahead():
         batch.positions = None                                # its buffer is the next round's
     for i, y in enumerate(got):
         assert torch.equal(y, wants[i % 3]), i
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+def test_a_value_that_is_none_reaches_no_token_before_its_own(bad):
+    """Values of one channel in the middle of a tile of 128 tokens, at its edges and at the end: the tokens before them keep their results, those from
+    there on have none in that channel, and all else is as it was bit for bit."""
+    from forge_b200 import kernels
+    H, D, R, E, reqs = 3, 64, 32, 128, [(90, 300), (0, 40)]
+    batch, _, _, g = _batch(reqs, 64, 64, seed=3)
+    q = torch.randn(340, H * (D + R), generator=g).to(torch.bfloat16)
+    kv, kr = torch.randn(430, H * (D + E), generator=g).to(torch.bfloat16), torch.randn(430, R, generator=g).to(torch.bfloat16)
+    starts = torch.tensor([0, 390], dtype=torch.int32, device=DEV)
+    run = lambda kv: kernels.expanded_attention(q.to(DEV), kv.to(DEV), kr.to(DEV), starts, batch, H, D, R, E, 0.1).double().cpu().view(340, H, E)
+    whole = run(kv)
+    spots = [(90 + 17, 0, 5), (90 + 127, 1, 40), (90 + 128, 1, 100), (90 + 299, 2, 127), (390 + 39, 0, 64)]          # (row, head, channel)
+    for row, h, e in spots:
+        kv[row, h * (D + E) + D + e] = bad
+    got = run(kv)
+    kernels.check_kernel_status(DEV)
+    want, again = whole.clone(), torch.zeros(340, H, E, dtype=torch.bool)
+    for row, h, e in spots:
+        t = row - 90 if row < 390 else 300 + row - 390
+        end = 300 if row < 390 else 340
+        want[t:end, h, e] = math.nan
+        first = t - t % 128 if row < 390 else 300
+        again[first:t, h, e // 32 * 32:e // 32 * 32 + 32] = True          # (added up anew: the same number but for the sums' order)
+    assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+    fine = torch.isfinite(want)
+    assert torch.equal(got[fine & ~again], want[fine & ~again])
+    # (two roundings of sums that differ by some 2^-16 of the weights' two terms: neighbouring bfloat16 numbers at most, 2^-7 of the smaller one apart)
+    off, size = (got - whole).abs()[fine & again], whole.abs()[fine & again]
+    assert bool((off <= 2.0 ** -7 * size + 1e-5).all()) and float((off > 0).double().mean()) < 0.05, float((off - 2.0 ** -7 * size).max())
