@@ -11,7 +11,8 @@
 // and what waits for S is little: the triangle of the u_j is solved for both of its right-hand sides ahead, U from b_j v_j and W from
 // b_j P_j k_j, so that u = U - W S.  Three kernels, of which only the second walks a request's chunks one after the other:
 //     1  per (chunk, head)          W and U                          (fixed decay: Z = sum_i R_i,31 k_i v_i^T, all a chunk does to the state)
-//     2  per (request, head, cols)  u = U - W S, the state before every chunk kept, S moved on        (fixed decay: S <- P_31 S + Z)
+//     2  per (request, head, cols)  u = U - W S (left where the outputs will be), the state before every chunk kept, S moved on
+//                                   (fixed decay: S <- P_31 S + Z)
 //     3  per (chunk, head)          the outputs, from the kept states
 // The block scan they replace makes a chain of 900 instructions of every eight tokens with two to four warps an SM.  2,001 tokens in three portions, 32 heads:
 // 216 us with its gram matrices, 140 us here (solve 29, walk 73, outputs 38).  Fixed decay, 1,500 tokens in two portions, 64 heads: 252 us token by
@@ -83,7 +84,8 @@ __device__ __forceinline__ void decay_triangle(float (*r)[CH + 1], const float* 
 // The products of chunks on the tensor cores (m16n8k16): an fp32 number as the sum of three bfloat16 ones (its rounding, the rounding of what that
 // left, and of what that left: 2^-26 of it at most is missing), of the nine products of two such sums the six largest, each exact, fp32 sums.  The tensor
 // core cuts what an addend has below a sum's last place, so the large terms have a sum of their own over few steps; the state itself is moved on by
-// multiply-adds.  (A number that is not finite makes NaN of the sums that it takes part in.)
+// multiply-adds.  A number that is not finite, or that rounds to a bfloat16 infinity, makes NaN of the sums that it takes part in: a sum that is not finite
+// is therefore made again by multiply-adds (made_again; in the walk, whose loop has neither a register nor a branch to spare, all of it: walk_again).
 struct Terms { uint32_t h, m, l; };                           // of two neighbouring numbers each
 __device__ __forceinline__ Terms split2(float x, float y) {
     Terms t;
@@ -115,8 +117,21 @@ __device__ __forceinline__ void mma_terms(float (&main)[4], float (&rest)[2][4],
     mma_sync::mma_bf16(rest[0], am, b[0].m, b[1].m);
 }
 
-// main + rest = A B^T, 16 x 16 over 64: rows gr (and 8 further on) of A and of B at rows of LD, two 16 x 8 tiles
-__device__ __forceinline__ void square16(float (&main)[2][4], float (&rest)[2][4], const float* a, const float* b, int gr, int tq) {
+// Whether a number among four is not finite, as one number that is then NaN, else zero.
+__device__ __forceinline__ float odd4(const float (&x)[4]) { return fmaf(x[0], 0.f, x[1] * 0.f) + fmaf(x[2], 0.f, x[3] * 0.f); }
+// A sum of the tensor cores, or if it is not finite the multiply-adds of a[i * lda] b[i * ldb], i < n, that it stands for.
+__device__ __forceinline__ float made_again(float sum, const float* a, int lda, const float* b, int ldb, int n) {
+    if (isfinite(sum)) return sum;
+    sum = 0.f;
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) sum = fmaf(a[i * lda], b[i * ldb], sum);
+    return sum;
+}
+
+// A B^T, 16 x 16 over 64: rows gr (and 8 further on) of A and of B at rows of LD, two 16 x 8 tiles
+__device__ __forceinline__ void square16(float (&main)[2][4], const float* a, const float* b, int gr, int tq) {
+    float rest[2][4] = {};
+    const float *a0 = a + gr * LD, *b0 = b + 2 * tq * LD;
     auto pair = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return split2(v.x, v.y); };
     a += gr * LD + 2 * tq;
     b += gr * LD + 2 * tq;
@@ -128,6 +143,16 @@ __device__ __forceinline__ void square16(float (&main)[2][4], float (&rest)[2][4
             const Terms bt[2] = {pair(b + 8 * h * LD + kk), pair(b + 8 * h * LD + kk + 8)};
             mma_terms(main[h], rest[h], at, bt);
         }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) main[h][e] += rest[h][e];
+    if (odd4(main[0]) + odd4(main[1]) != 0.f) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) main[h][e] = made_again(main[h][e], a0 + (e >> 1) * 8 * LD, 1, b0 + (8 * h + (e & 1)) * LD, 1, K);
     }
 }
 
@@ -161,14 +186,14 @@ chunk_solve_kernel(const Chunks d) {
         // rows m0 .. m0 + 15, columns n0 .. n0 + 15 of k k^T under the diagonal, kept transposed: what row i does to the rows below
         const int warp = tid >> 5, gr = (tid & 31) >> 2, tq = tid & 3, m0 = (warp & 1) * 16, n0 = (warp >> 1) * 16;
         if (n0 <= m0) {
-            float main[2][4] = {}, rest[2][4] = {};
-            square16(main, rest, ks + m0 * LD, ks + n0 * LD, gr, tq);
+            float main[2][4] = {};
+            square16(main, ks + m0 * LD, ks + n0 * LD, gr, tq);
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int j = m0 + gr + (e >> 1) * 8, i = n0 + 8 * h + 2 * tq + (e & 1);
-                    A[i][j] = bs[j] * R[j][i] * (main[h][e] + rest[h][e]);
+                    A[i][j] = bs[j] * R[j][i] * main[h][e];
                 }
         }
     }
@@ -264,8 +289,42 @@ __device__ __forceinline__ int longest(const Chunks& d, int rank, int lane) {
     return __ffs(__ballot_sync(0xffffffffu, lane < d.S && before == rank)) - 1;
 }
 
+// A CTA's whole walk by multiply-adds, where a sum of the tensor cores was not finite: all that the walk read is still there.  (A function of its own: its
+// numbers would take registers from the loop that has none to spare.)
+__device__ __noinline__ void walk_again(const Chunks& d, float* sm, int s, int head, int c0) {
+    const int tid = threadIdx.x, t_lo = d.q_start[s], t_hi = d.q_start[s + 1];
+    float *S = sm, *us = S + K * kColsB;                                     // [64][16], [32][16]: u times the decays behind it
+    float* S_g = d.state + (size_t)d.slots[s] * d.stride + (size_t)head * K * d.V + c0;
+    for (int i = tid; i < K * kColsB; i += kWalkThreads) S[i] = S_g[(size_t)(i / kColsB) * d.V + i % kColsB];
+    size_t at = (size_t)first_chunk(d.q_start, s) * d.N + head;
+    for (int t0 = t_lo; t0 < t_hi; t0 += CH, at += d.N) {
+        const int n = min(CH, t_hi - t0);
+        __syncthreads();
+        for (int i = tid; i < K * kColsB; i += kWalkThreads) d.s[(at * K + i / kColsB) * d.V + c0 + i % kColsB] = S[i];
+        for (int i = tid; i < n * kColsB; i += kWalkThreads) {
+            const int t = i / kColsB, c = i % kColsB;
+            float w = 0.f, behind = 1.f;
+            for (int k = 0; k < K; ++k) w = fmaf(d.w[(at * K + k) * CH + t], S[k * kColsB + c], w);
+            for (int j = n - 1; j > t; --j) behind *= d.g[(size_t)(t0 + j) * d.N + head];
+            const float u = d.u[(at * CH + t) * d.V + c0 + c] - w;
+            d.out[((size_t)(t0 + t) * d.N + head) * d.V + c0 + c] = u;
+            us[i] = u * behind;
+        }
+        __syncthreads();
+        float p = 1.f;
+        for (int j = n - 1; j >= 0; --j) p *= d.g[(size_t)(t0 + j) * d.N + head];
+        for (int i = tid; i < K * kColsB; i += kWalkThreads) {
+            float z = 0.f;
+            for (int t = 0; t < n; ++t) z = fmaf(d.k[(size_t)(t0 + t) * d.ld_k + head / (d.N / d.M) * K + i / kColsB], us[t * kColsB + i % kColsB], z);
+            S[i] = fmaf(p, S[i], z);
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < K * kColsB; i += kWalkThreads) S_g[(size_t)(i / kColsB) * d.V + i % kColsB] = S[i];
+}
+
 __global__ void __launch_bounds__(kWalkThreads, 3)
-chunk_walk_kernel(const Chunks d) {
+chunk_walk_kernel(const __grid_constant__ Chunks d) {
     extern __shared__ __align__(16) float sm[];
     float* S = sm + 2 * kStageB;                              // [64][16 + 4]
     float* us = S + K * LDC;                                  // [32][16 + 4]: u_t times the decays behind it
@@ -310,6 +369,9 @@ chunk_walk_kernel(const Chunks d) {
     float2 own0 = *reinterpret_cast<const float2*>(S_g), own1 = *reinterpret_cast<const float2*>(S_g + 8 * d.V);
     *reinterpret_cast<float2*>(S + row0 * LDC + col0) = own0;
     *reinterpret_cast<float2*>(S + (row0 + 8) * LDC + col0) = own1;
+    // (u goes to where the outputs will be: U stays, should the walk have to be made again)
+    float* u_at = d.out + ((size_t)(t_lo + (warp & 1) * 16 + gr) * d.N + head) * d.V + c0 + (warp >> 1 & 1) * 8 + 2 * tq;
+    float odd = 0.f;                                          // NaN once a sum of a second product (and so of a first one) is not finite
     for (int i = 0; i < chunks; ++i) {
         stages_wait<0>();
         __syncthreads();                                      // chunk i is here, S stands, and nobody is at chunk i - 1 any more
@@ -352,8 +414,9 @@ chunk_walk_kernel(const Chunks d) {
                 u.y -= (main[2 * h + 1] + (rest[0][2 * h + 1] + rest[1][2 * h + 1])) + half.y;
                 const float r = __shfl_sync(0xffffffffu, behind, t);
                 *reinterpret_cast<float2*>(us + t * LDC + c) = make_float2(u.x * r, u.y * r);
-                *reinterpret_cast<float2*>(d.u + (((size_t)(at0 + i) * d.N + head) * CH + t) * d.V + c0 + c) = u;
+                if (t < t_hi - t_lo - i * CH) *reinterpret_cast<float2*>(u_at + (size_t)8 * h * d.N * d.V) = u;
             }
+            u_at += (size_t)CH * d.N * d.V;
         } else {
             fetch(i + 1);
         }
@@ -371,10 +434,17 @@ chunk_walk_kernel(const Chunks d) {
             const Terms bt[2] = {split2(b[0], b[LDC]), split2(b[8 * LDC], b[9 * LDC])};
             mma_terms(main, rest, at, bt);
         }
-        own0.x = fmaf(p, own0.x, main[0] + (rest[0][0] + rest[1][0])); own0.y = fmaf(p, own0.y, main[1] + (rest[0][1] + rest[1][1]));
-        own1.x = fmaf(p, own1.x, main[2] + (rest[0][2] + rest[1][2])); own1.y = fmaf(p, own1.y, main[3] + (rest[0][3] + rest[1][3]));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) main[e] += rest[0][e] + rest[1][e];
+        odd += odd4(main);
+        own0.x = fmaf(p, own0.x, main[0]); own0.y = fmaf(p, own0.y, main[1]);
+        own1.x = fmaf(p, own1.x, main[2]); own1.y = fmaf(p, own1.y, main[3]);
         *reinterpret_cast<float2*>(S + row0 * LDC + col0) = own0;
         *reinterpret_cast<float2*>(S + (row0 + 8) * LDC + col0) = own1;
+    }
+    if (__syncthreads_or(odd != 0.f)) {
+        walk_again(d, sm, s, head, c0);
+        return;
     }
     *reinterpret_cast<float2*>(S_g) = own0;
     *reinterpret_cast<float2*>(S_g + 8 * d.V) = own1;
@@ -444,8 +514,9 @@ chunk_output_kernel(const Chunks d) {
     stage_rows<kOutThreads>(qs, d.q + (size_t)t0 * d.ld_q + hk * K, d.ld_q, n);
     stage_rows<kOutThreads>(ks, d.k + (size_t)t0 * d.ld_k + hk * K, d.ld_k, n);
     stages_commit();
-    const float* u = DELTA ? d.u + ((size_t)chunk * d.N + head) * CH * d.V + v0 : d.v + (size_t)t0 * d.ld_v + (size_t)head * d.V + v0;
-    const int ld_u = DELTA ? d.V : d.ld_v;
+    // (DELTA: the walk left u where this CTA's outputs will be)
+    const float* u = (DELTA ? d.out + (size_t)t0 * d.N * d.V : d.v + (size_t)t0 * d.ld_v) + (size_t)head * d.V + v0;
+    const int ld_u = DELTA ? d.N * d.V : d.ld_v;
     const float* kept = d.s + ((size_t)chunk * d.N + head) * K * d.V + v0;
     for (int i = tid; i < K * VB / 4; i += kOutThreads) stage16(S + i / (VB / 4) * LDV + i % (VB / 4) * 4, kept + (size_t)(i / (VB / 4)) * d.V + i % (VB / 4) * 4, true);
     for (int i = tid; i < CH * VB / 4; i += kOutThreads) {
@@ -465,21 +536,18 @@ chunk_output_kernel(const Chunks d) {
     {
         // rows m0 .. m0 + 15 of the triangle, columns n0 .. n0 + 15 (above the diagonal: zeros, whatever the keys there)
         const int m0 = (warp & 1) * 16, n0 = (warp >> 1) * 16;
-        float main[2][4] = {}, rest[2][4] = {};
-        if (n0 <= m0) square16(main, rest, qs + m0 * LD, ks + n0 * LD, gr, tq);
+        float main[2][4] = {};
+        if (n0 <= m0) square16(main, qs + m0 * LD, ks + n0 * LD, gr, tq);
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int j = m0 + gr + (e >> 1) * 8, i = n0 + 8 * h + 2 * tq + (e & 1);
-                Mx[j * LDM + i] = i <= j ? R[j][i] * (main[h][e] + rest[h][e]) : 0.f;
+                Mx[j * LDM + i] = i <= j ? R[j][i] * main[h][e] : 0.f;
             }
     }
     stages_wait<0>();
     __syncthreads();
-    bool odd = false;                                         // numbers among the u that are none: a later token's must not meet the triangle's zeros
-    for (int i = tid; i < CH * VB; i += kOutThreads) odd |= !isfinite(us[i / VB * LDV + i % VB]);
-    odd = __syncthreads_or(odd);
     // a warp's 16 columns of all tokens: 16 x 8 tiles [m][h]
     const int c0 = warp * 16;
     float main[2][2][4] = {}, rest[2][2][4] = {}, o[2][2][4];
@@ -501,44 +569,60 @@ chunk_output_kernel(const Chunks d) {
             for (int h = 0; h < 2; ++h) mma_terms(main[m][h], rest[m][h], at, bt[h]);
         }
     }
+    float odd = 0.f;
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                o[m][h][e] = (main[m][h][e] + rest[m][h][e]) * P[16 * m + gr + (e >> 1) * 8];
+                o[m][h][e] = main[m][h][e] + rest[m][h][e];
                 main[m][h][e] = rest[m][h][e] = 0.f;
             }
-    if (!odd) {
-#pragma unroll
-        for (int kk = 0; kk < CH; kk += 16) {
-            Terms bt[2][2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float* b = us + (kk + 2 * tq) * LDV + c0 + 8 * h + gr;
-                bt[h][0] = split2(b[0], b[LDV]);
-                bt[h][1] = split2(b[8 * LDV], b[9 * LDV]);
-            }
-#pragma unroll
-            for (int m = kk / 16; m < 2; ++m) {                           // (the first 16 tokens see none of the others)
-                const float* a = Mx + (16 * m + gr) * LDM + kk + 2 * tq;
-                auto pair = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return split2(v.x, v.y); };
-                const Terms at[4] = {pair(a), pair(a + 8 * LDM), pair(a + 8), pair(a + 8 * LDM + 8)};
-#pragma unroll
-                for (int h = 0; h < 2; ++h) mma_terms(main[m][h], rest[m][h], at, bt[h]);
-            }
+            odd += odd4(o[m][h]);
         }
-    } else {
+    if (odd != 0.f) {
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+        for (int i = 0; i < 16; ++i) {
+            float& x = o[i >> 3][i >> 2 & 1][i & 3];
+            x = made_again(x, qs + (16 * (i >> 3) + gr + (i >> 1 & 1) * 8) * LD, 1, S + c0 + 8 * (i >> 2 & 1) + 2 * tq + (i & 1), LDV, K);
+        }
+    }
+    __syncwarp();                                             // (the lanes may have parted over a sum that was made again)
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+    for (int kk = 0; kk < CH; kk += 16) {
+        Terms bt[2][2];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int j = 16 * m + gr + (e >> 1) * 8, c = c0 + 8 * h + 2 * tq + (e & 1);
-                    for (int i = 0; i <= j; ++i) main[m][h][e] = fmaf(Mx[j * LDM + i], us[i * LDV + c], main[m][h][e]);
-                }
+        for (int h = 0; h < 2; ++h) {
+            const float* b = us + (kk + 2 * tq) * LDV + c0 + 8 * h + gr;
+            bt[h][0] = split2(b[0], b[LDV]);
+            bt[h][1] = split2(b[8 * LDV], b[9 * LDV]);
+        }
+#pragma unroll
+        for (int m = kk / 16; m < 2; ++m) {                               // (the first 16 tokens see none of the others)
+            const float* a = Mx + (16 * m + gr) * LDM + kk + 2 * tq;
+            auto pair = [](const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return split2(v.x, v.y); };
+            const Terms at[4] = {pair(a), pair(a + 8 * LDM), pair(a + 8), pair(a + 8 * LDM + 8)};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) mma_terms(main[m][h], rest[m][h], at, bt[h]);
+        }
+    }
+    odd = 0.f;
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) main[m][h][e] += rest[m][h][e];
+            odd += odd4(main[m][h]);
+        }
+    if (odd != 0.f) {                                         // (a later token's number that is none has met the triangle's zeros: only up to the own token now)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int j = 16 * (i >> 3) + gr + (i >> 1 & 1) * 8;
+            float& x = main[i >> 3][i >> 2 & 1][i & 3];
+            x = made_again(x, Mx + j * LDM, 1, us + c0 + 8 * (i >> 2 & 1) + 2 * tq + (i & 1), LDV, j + 1);
+        }
     }
 #pragma unroll
     for (int m = 0; m < 2; ++m)
@@ -549,7 +633,7 @@ chunk_output_kernel(const Chunks d) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
                 *reinterpret_cast<float2*>(d.out + (size_t)(t0 + j) * d.N * d.V + (size_t)head * d.V + v0 + c0 + 8 * h + 2 * tq) =
-                    make_float2(o[m][h][2 * r] + (main[m][h][2 * r] + rest[m][h][2 * r]), o[m][h][2 * r + 1] + (main[m][h][2 * r + 1] + rest[m][h][2 * r + 1]));
+                    make_float2(__fmul_rn(o[m][h][2 * r], P[j]) + main[m][h][2 * r], __fmul_rn(o[m][h][2 * r + 1], P[j]) + main[m][h][2 * r + 1]);
         }
 }
 
