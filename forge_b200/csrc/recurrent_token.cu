@@ -98,7 +98,8 @@ __device__ __forceinline__ void convolve_tile(const DeltaPrepare& d, const float
         for (int k = 0; k < kPrepTokens; ++k) {
             float a = 0.f;
 #pragma unroll
-            for (int j = TP - 1; j >= 0; --j) a = fmaf(w[j], v[TP - 1 + k - j], a);
+            for (int j = TP - 1; j >= 0; --j)
+                if (j < d.cv.taps) a = fmaf(w[j], v[TP - 1 + k - j], a);      // (a tap that the filter has not meets no input, not even one that is none)
             y[k] = siluf(a);
         }
         return;
@@ -183,14 +184,14 @@ delta_prepare_kernel(const DeltaPrepare d, int tiles) {
 // The same for q and k heads of 64 channels where everything is aligned to 16 bytes: a lane has four neighbouring channels (a warp two heads), walks down
 // `run` tokens with the taps' inputs in registers and asks for the next four tokens' at a time.  Every number is the other kernel's, bit for bit (the squares
 // of a head are added in the order of its butterfly).  Bound by memory: 2,001 tokens of 4,096 channels, 66 MB, 40.0 us with a channel a lane, 21.6 us so; 381 tokens of 6,144 channels 17.2 and 7.7.
-__device__ __forceinline__ float4 taps_of(const float4 (&w)[4], const float4& x0, const float4& x1, const float4& x2, const float4& x3, int pos) {
+__device__ __forceinline__ float4 taps_of(const float4 (&w)[4], const float4& x0, const float4& x1, const float4& x2, const float4& x3, int reach) {
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     auto add = [&](const float4& u, const float4& v) {
         a.x = fmaf(u.x, v.x, a.x); a.y = fmaf(u.y, v.y, a.y); a.z = fmaf(u.z, v.z, a.z); a.w = fmaf(u.w, v.w, a.w);
     };
-    if (pos >= 3) add(w[3], x3);                                          // (nothing before the sequence's start, not even a weight that is none)
-    if (pos >= 2) add(w[2], x2);
-    if (pos >= 1) add(w[1], x1);
+    if (reach >= 3) add(w[3], x3);                                        // (reach: the tokens before this one that the sequence and the filter have)
+    if (reach >= 2) add(w[2], x2);
+    if (reach >= 1) add(w[1], x1);
     add(w[0], x0);
     return make_float4(siluf(a.x), siluf(a.y), siluf(a.z), siluf(a.w));
 }
@@ -231,7 +232,7 @@ delta_prepare_vec_kernel(const DeltaPrepare d, int run) {
                 x2 = before(2);
                 x3 = before(3);
             }
-            float4 y = taps_of(w, in[i], x1, x2, x3, pos);
+            float4 y = taps_of(w, in[i], x1, x2, x3, min(pos, d.cv.taps - 1));
             x3 = x2;
             x2 = x1;
             x1 = in[i];

@@ -62,3 +62,24 @@ def test_the_filter_may_come_from_the_kernel_ahead():
         del rows                                              # its buffer is the next round's
     for i, y in enumerate(got):
         assert torch.equal(y, wants[i % 3]), i
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("col", [0, 1])
+def test_a_number_that_is_none_reaches_as_far_as_the_filter(taps, col):
+    """A NaN among the inputs of one token reaches that token and the taps - 1 tokens behind it, in both kernels, wherever it lies in a warp's run."""
+    from forge_b200 import kernels
+    N, M, K, V, T = 2, 1, 64, 64, 40
+    C = 2 * M * K + N * V
+    g = torch.Generator().manual_seed(taps)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(num_requests=1, num_tokens=T, q_start=i32([0, T]), slots=i32([0]), tok_req=i32([0] * T), positions=i32(list(range(T))))
+    rate, dt, conv = torch.rand(N, generator=g).to(DEV), torch.randn(N, generator=g).to(DEV), torch.randn(taps, C, generator=g).to(DEV)
+    for at in (0, 5, 14, 15, 16, 39):
+        p = torch.randn(T, C + 2 * N + 4 * col, generator=g)
+        p[at, col:col + C] = float("nan")
+        state = torch.zeros(1, (N * K * V + taps * C + 3) // 4 * 4, device=DEV)
+        qkv = kernels.gated_delta_prepare(p.to(DEV), col, col + C, col + C + N, conv, rate, dt, batch, state, N, M, K, V)[0].cpu()
+        none = torch.zeros(T, dtype=torch.bool)
+        none[at:at + taps] = True
+        assert bool(torch.isnan(qkv[none]).all()) and bool(torch.isfinite(qkv[~none]).all()), at
