@@ -467,6 +467,7 @@ class StepWorkspace:
     def reserve(self, nbytes):
         nbytes = -(-int(nbytes) // self.ALIGN) * self.ALIGN
         if nbytes > self.capacity:
+            self._whole, self.buf, self.typed, self.capacity = None, None, {}, 0     # (given back first: never both at a time)
             whole = torch.empty(nbytes + self.ALIGN, dtype=torch.uint8, device=self.device)
             whole[nbytes:].fill_(self.CANARY_BYTE)              # canary words behind the buffer: nothing ever writes them
             self._whole, self.buf = whole, whole[:nbytes]
@@ -1664,7 +1665,21 @@ def latent_attention(q, cache, group_batch, batch, H, C, R, page_size, scale, wi
     return out
 
 
-EXPANDED_SCRATCH = 1 << 30          # bytes of keys and values that a layer may spell out
+EXPANDED_SCRATCH = 1 << 30          # bytes that a layer may take to spell keys and values out: those, the packed rows and the rounded queries
+ASK_FROM = 64 << 20                 # bytes of scratch from which on the device is asked whether it has them
+
+
+def _scratch_fits(nbytes, device):
+    """Whether a step can take nbytes more of scratch that it could do without: out of the open workspace, or, where that has to grow (by an eighth more than
+    the step needs; its old buffer is given back first), out of what is left on the device."""
+    ws = _active_workspace[0]
+    if ws is not None and ws.hold == 0 and device == ws.device:
+        if ws.offset + ws.back + nbytes <= ws.capacity:
+            return True
+        nbytes = max(nbytes, (ws.offset + ws.back + nbytes) * 9 // 8 - ws.capacity)
+    if nbytes < ASK_FROM or device.type != "cuda":
+        return True
+    return nbytes <= torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
 
 
 def latent_expand_supports(H, D, R, E, C, dtype, scale):
@@ -1680,7 +1695,8 @@ def latent_expand_pays(batch, H, D, R, E, C):
     queries against a tile of keys holds its CTA for 0.8 + C / 230 (absorbed; a CTA a chunk of 256 values) or 0.9 + (D + R + E) / 450, the attention lasts
     as long as its longest row of tiles or the SMs' share of all, the product runs at 0.7 and the per-head ones at 0.13 PFLOP/s.  Measured
     (device, a layer of 32 heads of 128, 4,096 wide): 24 tokens 78 -> 61, 1,600 tokens 522 -> 272, 24 behind 1,000 cached 111 -> 94, four requests of 25 behind
-    1,000 133 -> 134; many cached rows that few tokens see, as in a step of mostly single tokens, stay absorbed."""
+    1,000 133 -> 134; many cached rows that few tokens see, as in a step of mostly single tokens, stay absorbed.  So does a step whose scratch is more than
+    EXPANDED_SCRATCH or than the device has left (a runner's cache may leave little): the other form needs none that grows with the rows."""
     key = ("expand", H, D, R, E, C)
     pays = batch.attention_plan.get(key)
     if pays is None:
@@ -1688,7 +1704,8 @@ def latent_expand_pays(batch, H, D, R, E, C):
         if _brings_portions(batch):
             qs, before = batch.host_q_start, _tokens_before(batch)
             rows = before[-1] + qs[-1] + sum(before[:-1])
-            if 2 * rows * H * (D + E) <= EXPANDED_SCRATCH:
+            scratch = 2 * (rows * (H * (D + E) + C + R) + batch.num_tokens * H * (D + R))
+            if scratch <= EXPANDED_SCRATCH:
                 def tiles(TQ):                                  # (of keys: the longest row of tiles, all)
                     longest = total = 0
                     for c, a, b in zip(before, qs, qs[1:]):
@@ -1701,7 +1718,7 @@ def latent_expand_pays(batch, H, D, R, E, C):
                 far_x, work_x = tiles(128)
                 absorbed = max(far, work * max(1, C // 256) / sms) * (0.8 + C / 230) + 2 * H * T * C * (D + E) / 130e6 + 10
                 expanded = max(far_x, work_x * H / sms) * (0.9 + (D + R + E) / 450) + 2 * H * rows * C * (D + E) / 700e6 + 12
-                pays = expanded < absorbed
+                pays = expanded < absorbed and _scratch_fits(scratch, batch.positions.device)
         batch.attention_plan[key] = pays
     return pays
 

@@ -33,3 +33,45 @@ def test_requests_that_bring_nothing_have_nothing_before():
     assert kernels._tokens_before(SimpleNamespace(num_requests=2, host_q_start=[0, 0, 1], positions=torch.tensor([4], dtype=torch.int32))) == [0, 4]
     # the tiles of a step with such requests: (first token, tokens, request, first position), furthest first
     assert kernels.shaped_plan(batch, 2, torch.device("cpu")).tolist() == [[4, 1, 2, 32], [2, 2, 2, 30], [0, 2, 0, 7]]
+
+
+def test_a_step_stays_absorbed_where_its_scratch_does_not_fit(monkeypatch):
+    """What the device has left decides where the open workspace has to grow; a step that fits into it asks nobody."""
+    monkeypatch.setattr(kernels, "_sm_count", lambda device: 148)
+    device, asked = torch.device("cuda", 0), []
+    left = lambda n: monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: asked.append(d) or (n, 180 << 30))
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda d: 3 << 20)
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda d: 1 << 20)
+    ws = SimpleNamespace(hold=0, device=device, offset=20 << 20, back=0, capacity=30 << 20)
+    monkeypatch.setattr(kernels, "_active_workspace", [ws])
+
+    def pays(tokens=8000):
+        batch = SimpleNamespace(num_requests=1, num_tokens=tokens, host_q_start=[0, tokens], host_context_before=[0], attention_plan={},
+                                positions=SimpleNamespace(device=device))
+        return kernels.latent_expand_pays(batch, 32, 128, 64, 128, 512)
+
+    need = 2 * (8000 * (32 * 256 + 576) + 8000 * 32 * 192)
+    grown = (need + ws.offset) * 9 // 8 - ws.capacity
+    left(grown - (2 << 20))
+    assert pays() and len(asked) == 1
+    left(grown - (2 << 20) - 1)
+    assert not pays()
+    asked.clear()
+    ws.capacity = ws.offset + need
+    left(0)
+    assert pays() and pays(1600) and not asked                # the workspace holds it
+    ws.capacity = 0
+    assert pays(1000) and not asked                           # little enough not to ask
+    monkeypatch.setattr(kernels, "_active_workspace", [None])
+    assert not pays() and asked == [device]
+
+
+def test_a_workspace_that_grows_gives_its_buffer_back_first(monkeypatch):
+    ws = kernels.StepWorkspace("cpu")
+    ws.reserve(1000)
+    with ws.step():
+        kernels.new_tensor((500,), torch.float32, ws.device)
+        kernels.new_tensor((500,), torch.float32, ws.device)
+        take, seen = torch.empty, []
+        monkeypatch.setattr(torch, "empty", lambda *a, **k: seen.append((ws.buf, ws.typed)) or take(*a, **k))
+    assert seen == [(None, {})] and ws.capacity >= 4000 and ws.canary_intact()
