@@ -332,34 +332,43 @@ head_finish_kernel(const float* __restrict__ o, const float* __restrict__ weight
 // of the rows t / CG, t / CG + RG, ...; the RG partial sums of an output are added in their order.  Bound by the state's way in and out (64 requests,
 // 64 heads of 64 x 64: 134 MB; the scan of portions with the rotation before and the norm behind it 57 us, 33 us so, 4.1 TB/s; what lies on its way decides, so
 // the packs wait in shared memory: in registers, beside the angles' slow path, three CTAs an SM were left (one with 16 packs a thread), now six: 24.4 us, 5.5 TB/s;
-// eight with 32 registers a thread 28.9).
+// eight with 32 registers a thread 28.9).  Where all CTAs are at work at once even so, the way through shared memory only costs: there the packs wait in
+// registers (STAGED false; see retention_in_registers).  Same bits.
 constexpr int kRetThreads = 256, kRetHeld = 16;
 bool retention_token_fits(int K, int V) {
     const int cg = V / 4;
     return V % 4 == 0 && V > 0 && cg <= 64 && K > 0 && K <= 256 && (K + kRetThreads / cg - 1) / (kRetThreads / cg) <= kRetHeld;
 }
 
-template <int HELD, typename TA>
-__global__ void __launch_bounds__(kRetThreads, HELD <= 4 ? 6 : HELD <= 8 ? 5 : 3)
+// Measured, us a step in a chain of them, registers and shared memory: heads of 64 x 64, 256 CTAs (4 requests of 64 heads) 3.9 and 4.6, 128 3.8 and 3.6,
+// 512 6.6 and 5.2; of 64 x 128, 256 CTAs 4.4 and 5.7, 64 4.1 and 3.7, 512 8.2 and 7.6; of 128 x 128, 128 CTAs 4.7 and 6.6, 256 8.3 and 7.4.  So: registers
+// as long as all CTAs are resident (three an SM, two, one), but not where each has an SM of its own and holds few packs.
+bool retention_in_registers(int ctas, int held, int sms) { return held <= 8 ? ctas > sms && ctas <= (held <= 4 ? 3 : 2) * sms : ctas <= sms; }
+
+template <int HELD, bool STAGED, typename TA>
+__global__ void __launch_bounds__(kRetThreads, STAGED ? (HELD <= 4 ? 6 : HELD <= 8 ? 5 : 3) : (HELD <= 4 ? 3 : HELD <= 8 ? 2 : 1))
 retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const int32_t* __restrict__ positions, const float* __restrict__ freq, int rot_dims,
                        float k_scale, const float* __restrict__ decay, float* __restrict__ state, long long state_stride, const int32_t* __restrict__ q_start,
                        const int32_t* __restrict__ slots, const float* __restrict__ weight, float eps, TA* __restrict__ out, long long out_ld, int N, int K, int V) {
     __shared__ float qs[256], ks[256], red[8];
     __shared__ __align__(16) float4 part[kRetThreads];
-    extern __shared__ __align__(16) float4 stage[];           // [HELD][kRetThreads], each read by the thread that asked for it
+    extern __shared__ __align__(16) float4 stage[];           // (STAGED) [HELD][kRetThreads], each read by the thread that asked for it
     forge::pdl_launch_dependents();
     forge::pdl_wait();
     const int s = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, t = q_start[s];
     const int CG = V / 4, RG = kRetThreads / CG, rg = tid / CG, cp = tid % CG;
     const bool live = rg < RG;
     float4* S = reinterpret_cast<float4*>(state + (size_t)slots[s] * state_stride + (size_t)head * K * V);
+    float4 held[STAGED ? 1 : HELD];
 #pragma unroll
     for (int m = 0; m < HELD; ++m) {
         const int row = rg + m * RG;
-        if (live && row < K)
+        if constexpr (!STAGED)
+            held[m] = live && row < K ? S[(size_t)row * CG + cp] : make_float4(0.f, 0.f, 0.f, 0.f);
+        else if (live && row < K)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(stage + m * kRetThreads + tid)), "l"(S + (size_t)row * CG + cp) : "memory");
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (STAGED) asm volatile("cp.async.commit_group;" ::: "memory");
     const float dec = decay[head];
     float4 vv = make_float4(0.f, 0.f, 0.f, 0.f), gate = vv, w = vv;
     if (live) {
@@ -388,7 +397,7 @@ retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const
         qs[i] = qp[i];
         ks[i] = kp[i] * k_scale;
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (STAGED) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -396,7 +405,7 @@ retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const
         const int row = rg + m * RG;
         if (!live || row >= K) continue;
         const float kk = ks[row], qq = qs[row];
-        float4 x = stage[m * kRetThreads + tid];
+        float4 x = STAGED ? stage[m * kRetThreads + tid] : held[STAGED ? 0 : m];
         x.x = fmaf(dec, x.x, kk * vv.x); x.y = fmaf(dec, x.y, kk * vv.y); x.z = fmaf(dec, x.z, kk * vv.z); x.w = fmaf(dec, x.w, kk * vv.w);
         S[(size_t)row * CG + cp] = x;
         acc.x = fmaf(qq, x.x, acc.x); acc.y = fmaf(qq, x.y, acc.y); acc.z = fmaf(qq, x.z, acc.z); acc.w = fmaf(qq, x.w, acc.w);
@@ -428,15 +437,17 @@ retention_token_kernel(ScanInput q, ScanInput k, ScanInput v, ScanInput g, const
 
 template <int HELD, typename TA, typename... Args>
 cudaError_t retention_token_launch(dim3 grid, cudaStream_t stream, Args... args) {
+    if (retention_in_registers((int)grid.x * (int)grid.y, HELD, forge::sm_count()))
+        return forge::launch(retention_token_kernel<HELD, false, TA>, grid, dim3(kRetThreads), 0, stream, 1, args...);
     constexpr int kBytes = HELD * kRetThreads * (int)sizeof(float4);
     static forge::PerDeviceFlag flag;
     bool& done = flag.current();
     if (!done) {
-        const cudaError_t e = cudaFuncSetAttribute(retention_token_kernel<HELD, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+        const cudaError_t e = cudaFuncSetAttribute(retention_token_kernel<HELD, true, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
         if (e != cudaSuccess) return e;
         done = true;
     }
-    return forge::launch(retention_token_kernel<HELD, TA>, grid, dim3(kRetThreads), kBytes, stream, 1, args...);
+    return forge::launch(retention_token_kernel<HELD, true, TA>, grid, dim3(kRetThreads), kBytes, stream, 1, args...);
 }
 
 // The same for heads of 32, 64 or 128 channels and aligned rows: K / 4 neighbouring lanes a head with four channels each, so that a warp has 4, 2
