@@ -643,10 +643,13 @@ extern "C" int forge_moe_route(const void* x, int dtype, const float* Wr, int32_
     const size_t smem = sizeof(float) * (2 * E + (groups > 1 ? groups : 0));
     // Few tokens wait for latencies, which the kernel of few experts hides.  Where there are more tokens than SMs a CTA of one token costs more than that
     // (300 tokens, 16 experts of 768: 6.1 us without it, 7.3 with it), of four less from two tokens an SM on, or where rows are long (8 experts: 300
-    // tokens of 768 4.3 us without it, 3.4 with it; 1,500 of 1,024 9.2 and 6.3, of 4,096 21.2 and 12.4; 200 of 512 3.4 and 3.6).
+    // tokens of 768 4.3 us without it, 3.4 with it; 1,500 of 1,024 9.2 and 6.3, of 4,096 21.2 and 12.4; 200 of 512 3.4 and 3.6).  Between two and
+    // three tokens an SM the CTAs of one token are all at work at once, and where a CTA of four walks long rows they are done first (400 tokens of 7,168: 8.6 us
+    // and 9.5, of 4,096 6.0 and 6.4; of 2,048 4.3 both; 600 of 7,168 16.0 and 9.8, 296 of 7,168 8.7 and 7.9).
     const bool few_experts = E <= kFewExperts && groups <= 1 && (T <= forge::sm_count() || (E <= 8 && (W >= 2048 || T > 2 * forge::sm_count())));
     if (dtype == FORGE_BF16 && few_experts && W % 8 == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0) {
-        const bool many = E <= 8 && T > forge::sm_count();
+        const int sms = forge::sm_count();
+        const bool many = E <= 8 && T > sms && !(W > 2048 && T > 2 * sms && T <= 3 * sms);
         auto few = many ? moe_route_kernel<__nv_bfloat16, 8, 4> : E <= 8 ? moe_route_kernel<__nv_bfloat16, 8> : moe_route_kernel<__nv_bfloat16, 16>;
         e = forge::launch(few, dim3(many ? (T + 3) / 4 : T), dim3(kRouteThreads), smem, stream, 1, (const __nv_bfloat16*)x, Wr, idx, wts, T, W, E, top, softmax, renorm, corr, 0, keep,
                           group_top, factor);
