@@ -1980,12 +1980,13 @@ def attention_plan(batch, group, device, only_below=None):
 
 TC_MIN_SHARE = 8     # key tiles (of 64 keys) that a share of a tile's keys holds at least
 TC_MAX_SHARES = 32
+TC_LONG_SHARE = 28    # ... and from how many on two shares on an SM are done before one twice as long alone
 
 
 def attention_plan_tc(batch, group, device, n_kv_heads=1, head_dim=64, window=0, shares=None):
     """Tiles of (128 // group) whole tokens, that is up to 128 rows, for the requests that bring at least TC_MIN_ROWS
     rows, heaviest (most keys) first.  When the step has at most half as many (tile, kv head) pairs as the GPU has
-    places for the kernel's CTAs, the keys of the long tiles are cut into shares, in proportion to their length, so that the places
+    places for the kernel's CTAs (two an SM), the keys of the long tiles are cut into shares, in proportion to their length, so that the places
     are taken (a short portion on a long context); ``shares`` forces a number for every tile (tests)."""
     key = ("tc", group, n_kv_heads, head_dim, window, shares)
     plan = batch.attention_plan.get(key)
@@ -2002,22 +2003,28 @@ def attention_plan_tc(batch, group, device, n_kv_heads=1, head_dim=64, window=0,
             kv_hi = ctx + (min(rows, r0 + tile_rows) - 1) // group + 1
             kv_lo = max(0, ctx + r0 // group - window + 1) if window else 0
             tiles.append((-(-kv_hi // KV_TILE) - kv_lo // KV_TILE, s, r0))
-    places = _sm_count(device) * (2 if head_dim <= 64 else 1)
     total = max(1, sum(t[0] for t in tiles) * n_kv_heads)
 
-    def worth(n, scale):        # n / (total / places): how many places this tile's keys are worth
-        return max(1, min(n // TC_MIN_SHARE, n * places * scale // (10 * total), TC_MAX_SHARES))
-    if shares is not None:
-        cut = [max(1, min(int(shares), t[0], TC_MAX_SHARES)) for t in tiles]
-    else:
-        cut = [1] * len(tiles)
+    def cut_for(places):
+        def worth(n, scale):        # n / (total / places): how many places this tile's keys are worth
+            return max(1, min(n // TC_MIN_SHARE, n * places * scale // (10 * total), TC_MAX_SHARES))
         # (with more than half of the places taken already there is nothing to gain that pays for the second kernel)
         for scale in range(10, 4, -1) if 2 * len(tiles) * n_kv_heads <= places else ():
             # short tiles count as one whole place each: shrink the others' worth until all fit
             trial = [worth(t[0], scale) for t in tiles]
             if sum(trial) * n_kv_heads <= places:
-                cut = trial
-                break
+                return trial
+        return [1] * len(tiles)
+    sms = _sm_count(device)
+    if shares is not None:
+        cut = [max(1, min(int(shares), t[0], TC_MAX_SHARES)) for t in tiles]
+    else:
+        # Two CTAs share an SM.  With heads of 128 a share runs faster on an SM of its own: where one share an SM takes all SMs and is short, more
+        # and shorter ones do not pay for their sums on the way (us, 32/8 heads of 128, one and two shares an SM: 64 tokens behind 8,000 31.6 and 35.6, 24 behind
+        # 30,000 50 and 52; else 128 behind 8,000 44 and 38, 100 behind 30,000 112 and 83, 300 behind 16,000 211 and 118).
+        cut = cut_for(sms) if head_dim > 64 else None
+        if cut is None or sum(cut) * n_kv_heads < 0.95 * sms or max(t[0] / z for t, z in zip(tiles, cut)) >= TC_LONG_SHARE:
+            cut = cut_for(2 * sms)
     entries, merges, slots = [], [], 0
     for (n, s, r0), z in zip(tiles, cut):
         if z > 1:

@@ -66,7 +66,7 @@ def test_a_whole_prompt_is_left_alone(on_cpu):
                                                ([(5000, 64), (0, 70)], 4, 2, 64)])
 def test_short_portions_on_long_contexts_are_cut_to_fill_the_places(on_cpu, reqs, group, nkv, hd):
     plan = plan_of(reqs, group, nkv, hd)
-    places = 148 * (2 if hd <= 64 else 1)
+    places = 148 * 2                                    # two CTAs share an SM with either size of head
     assert plan["num_merge"] > 0
     assert plan["num_tiles"] * nkv <= places, "the shares must not need a second wave of CTAs"
     uncut = plan_of(reqs, group, nkv, hd, shares=1)
@@ -90,8 +90,15 @@ def test_short_contexts_are_not_cut(on_cpu):
 
 
 def test_more_than_half_of_the_places_taken_is_left_alone(on_cpu):
-    plan = plan_of([(20000, 512)], 7, 4, 128)          # 29 tiles x 4 kv heads = 116 of 148 places
-    assert plan["num_merge"] == 0 and plan["num_tiles"] == 29
+    plan = plan_of([(20000, 1024)], 7, 4, 128)         # 57 tiles x 4 kv heads = 228 of 296 places
+    assert plan["num_merge"] == 0 and plan["num_tiles"] == 57
+
+
+def test_heads_of_128_share_an_sm_where_that_shortens_long_shares(on_cpu):
+    # 116 of 296 places: two shares a tile; and (8000, 64): 18 shares of 14 key tiles on SMs of their own rather than 30 of eight
+    assert plan_of([(20000, 512)], 7, 4, 128)["num_tiles"] == 58
+    assert plan_of([(8000, 64)], 4, 8, 128)["num_tiles"] == 18
+    assert plan_of([(8000, 128)], 4, 8, 128)["num_tiles"] == 36 and plan_of([(30000, 100)], 4, 8, 128)["num_tiles"] == 36
 
 
 @pytest.mark.parametrize("shares", [2, 5, 32, 100])
