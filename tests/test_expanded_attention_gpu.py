@@ -44,7 +44,9 @@ def test_expanded(H, C, D, R, E, ps, halves, col):
     turned = torch.cat([u * cs - v * sn, v * cs + u * sn], -1) if halves else torch.stack([u * cs - v * sn, v * cs + u * sn], -1).flatten(-2)
     ref = torch.cat([q[..., :D], turned], -1)
     got = qr.double().cpu().view(T, H, W)
-    assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all())
+    pair = 1.5 * (u.abs() + v.abs())
+    pair = torch.cat([pair, pair], -1) if halves else torch.stack([pair, pair], -1).flatten(-2)
+    assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-6 * torch.cat([torch.zeros_like(q[..., :D]), pair], -1)).all())
     # attention, over keys and values of any values
     kv = torch.randn(len(want), H * (D + E), generator=g).to(torch.bfloat16)
     wide = torch.full((T, H * E + 6), 3.0, dtype=torch.bfloat16, device=DEV)
