@@ -3,7 +3,7 @@
 // up to 128 rows of queries over tiles of 64 keys with a two-term softmax weight:
 //
 //   S = Q K^T      tcgen05.mma M=128 N=64 per 16 channels, Q (all its channels) and the key blocks in shared memory, S in TMEM (two buffers)
-//   softmax        128 threads, one row each, 64 scores in registers, fp32; a weight becomes two bfloat16 numbers, its rounding and
+//   softmax        256 threads, two a row with 32 of its scores each in registers, fp32; a weight becomes two bfloat16 numbers, its rounding and
 //                  what the rounding left over (16 bits of mantissa, as in the mma.sync kernels), written to TMEM over the scores it came from
 //   O += P V       tcgen05.mma M=128 N=VC with P from TMEM, once for the rest and once for the rounding, V MN-major as the cache has it
 //

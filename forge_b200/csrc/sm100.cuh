@@ -189,7 +189,7 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
 }
 // The descriptor of the same kind of tile `bytes` further on in shared memory (a multiple of 16; the start
 // address field holds address >> 4 and shared memory ends below 2^18, so the sum never leaves the field).  One
-// thread issues every MMA of a CTA and, being alone in its warp, runs an instruction every few cycles: building
+// lane issues every MMA of a kind, its warp walking the loop with it at an instruction every few cycles: building
 // a descriptor from scratch for each MMA costs more than a small MMA takes, adding to a base does not.
 __device__ __forceinline__ uint64_t umma_desc_advance(uint64_t desc, uint32_t bytes) {
     const uint32_t lo = static_cast<uint32_t>(desc) + (bytes >> 4);

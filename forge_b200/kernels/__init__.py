@@ -1352,16 +1352,20 @@ def chunk_scratch_bytes(T, requests, N, K, V, delta):
 
 
 def chunks_pay(kind, lens, N, V):
-    """Whether the chunked kernels are the faster ones for portions of ``lens`` tokens (measured from 64 to 1,600 tokens of 1 to 16 requests, 4 to 64
-    heads of 64, 128 and 192 value channels, both forms; times in microseconds, W thousands of (token, head of 64 value channels), tokens of the chunked
-    form filled up to whole chunks).  The scans are a chain of the longest portion's tokens or blocks, the chunked form shortens the chain and costs
-    more for every token: the longer one portion is against the step's whole work, the more it gives.
-      delta        scan 7 + 0.117 longest, chunks 16 + 0.04 longest and 0.9 more for W: 800 tokens of 32 heads 104 and 76, 300 tokens 46 and 43, two
-                   portions of 400 of 64 heads 96 and 131
-      lightning    scan 6 + 0.1 longest, chunks 13 + 1.2 W: 400 tokens of 32 heads 51 and 29, four portions of 400 of 64 heads of 128 256 and 288
-      retention    scan the larger of 4 + 0.168 longest and 1.6 W, chunks 13 + 1.15 W: 200 tokens of 64 heads 45 and 29, 64 tokens of 32 heads 14 and 25
-    (The delta rule's chunks take 0.75 of these times since their products are on the tensor cores; the line stays where they are faster for certain.)
-    Below some work a step waits for the host, which two kernels more keep longer: hence the least work, or the longest portion, of the last line."""
+    """Whether the chunked kernels are the faster ones for portions of ``lens`` tokens.  The scans are a chain of the longest portion's tokens or blocks, the
+    chunked form shortens the chain and costs more for every token: the longer one portion is against the step's whole work, the more it gives.  The lines
+    follow from estimates in microseconds, W thousands of (token, head of 64 value channels), tokens of the chunked form filled up to whole chunks, fitted to
+    the chunked kernels as they were before their products went to the tensor cores:
+      delta        scan 7 + 0.117 longest, chunks 16 + 0.04 longest and 0.9 more for W
+      lightning    scan 6 + 0.1 longest, chunks 13 + 1.2 W
+      retention    scan the larger of 4 + 0.168 longest and 1.6 W, chunks 13 + 1.15 W
+    The present kernels, scan and chunks, a step on the device by itself:
+      delta        800 tokens of 32 heads 110 and 70, 300 tokens 52 and 42 (goes by the scan), two portions of 400 of 64 heads 103 and 116
+      lightning    400 tokens of 32 heads 58 and 32, four portions of 400 of 64 heads of 128 271 and 282, of 700 of 64 heads of 64 312 and 247 (by the scan)
+      retention    200 tokens of 64 heads 52 and 32, 64 tokens of 32 heads 22 and 25
+    Over 200 steps of each kind (32 to 1,600 tokens in 1 to 8 portions, 8 to 64 heads of 64 and 128) the lines took chunks in 30, 86 and 99 and never where the
+    scan was the faster one; in 56, 84 and 81 they left chunks that were faster by themselves.  Below some work a step waits for the host, which two kernels more
+    keep longer: hence the least work, or the longest portion, of the last line."""
     longest = max(lens)
     W, filled = (n * N * V / 64000.0 for n in (sum(lens), sum(-(-n // CHUNK_TOKENS) for n in lens) * CHUNK_TOKENS))
     if kind == "delta":
@@ -1693,9 +1697,12 @@ def latent_expand_pays(batch, H, D, R, E, C):
     step sees, then D + R and E channels a score and an output) than with the matrices moved to the query and the output (C + R and C
     channels, and two per-head products over the step's tokens).  Estimated once per step and set of sizes, in microseconds: a tile of
     queries against a tile of keys holds its CTA for 0.8 + C / 230 (absorbed; a CTA a chunk of 256 values) or 0.9 + (D + R + E) / 450, the attention lasts
-    as long as its longest row of tiles or the SMs' share of all, the product runs at 0.7 and the per-head ones at 0.13 PFLOP/s.  Measured
-    (device, a layer of 32 heads of 128, 4,096 wide): 24 tokens 78 -> 61, 1,600 tokens 522 -> 272, 24 behind 1,000 cached 111 -> 94, four requests of 25 behind
-    1,000 133 -> 134; many cached rows that few tokens see, as in a step of mostly single tokens, stay absorbed.  So does a step whose scratch is more than
+    as long as its longest row of tiles or the SMs' share of all, the product runs at 0.7 and the per-head ones at 0.13 PFLOP/s: fitted to both attention
+    kernels as they were when one thread had a row.  Measured with the present ones (device, a layer of 32 heads of 128, 4,096 wide): 24 tokens 88 -> 67,
+    1,600 tokens 476 -> 249, 24 behind 1,000 cached 116 -> 91, four requests of 25 behind 1,000 136 -> 149, eight of 50 behind 500 181 -> 167 (stays
+    absorbed).  Over 230 steps (8 to 1,600 tokens of 1 to 17 requests behind 0 to 8,000, heads of 64 and 128) the estimate never spelled out where that was more
+    than 2 % slower; 30 steps it left absorbed though spelling out was faster, most of them of few tokens behind few.  Many cached rows that few tokens see, as
+    in a step of mostly single tokens, stay absorbed (eight tokens behind 4,000 each beside a portion of 100: 214 and 542).  So does a step whose scratch is more than
     EXPANDED_SCRATCH or than the device has left (a runner's cache may leave little): the other form needs none that grows with the rows."""
     key = ("expand", H, D, R, E, C)
     pays = batch.attention_plan.get(key)

@@ -7,7 +7,8 @@ import torch
 from forge_b200 import kernels
 
 # (cached, new) of the step's requests, width of a head, and what the rule says.  Spelling out was measured to be the faster form wherever it says so, and
-# the slower one with 64 single tokens behind 2,000; two single tokens are no portion, and 70,000 rows are more than the scratch may hold.
+# the slower one with 8 single tokens behind 4,000 and with 16 behind 1,000, of which the steps here have more; two single tokens are no portion, and
+# 70,000 rows are more than the scratch may hold.
 STEPS = [([(0, 1600)], 128, True), ([(700, 512), (0, 1024)], 128, True), ([(1000, 24)], 128, True), ([(0, 400)], 64, True), ([(1000, 100)], 64, True),
          ([(4000, 8)], 128, True), ([(4000, 1)] * 40 + [(0, 24)], 128, False), ([(2000, 1)] * 64 + [(0, 8)], 64, False),
          ([(0, 1), (0, 1)], 128, False), ([(30000, 40000)], 128, False)]
