@@ -1683,7 +1683,8 @@ def _scratch_fits(nbytes, device):
         nbytes = max(nbytes, (ws.offset + ws.back + nbytes) * 9 // 8 - ws.capacity)
     if nbytes < ASK_FROM or device.type != "cuda":
         return True
-    return nbytes <= torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+    free = torch.cuda.mem_get_info(device)[0]
+    return nbytes <= free or nbytes <= free + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
 
 
 def latent_expand_supports(H, D, R, E, C, dtype, scale):
@@ -1725,7 +1726,8 @@ def latent_expand_pays(batch, H, D, R, E, C):
                 far_x, work_x = tiles(128)
                 absorbed = max(far, work * max(1, C // 256) / sms) * (0.8 + C / 230) + 2 * H * T * C * (D + E) / 130e6 + 10
                 expanded = max(far_x, work_x * H / sms) * (0.9 + (D + R + E) / 450) + 2 * H * rows * C * (D + E) / 700e6 + 12
-                pays = expanded < absorbed and _scratch_fits(scratch, batch.positions.device)
+                # (the other form takes 2 C + R numbers for every token and head: no more than that is there in any case)
+                pays = expanded < absorbed and (scratch <= 2 * T * H * (2 * C + R) or _scratch_fits(scratch, batch.positions.device))
         batch.attention_plan[key] = pays
     return pays
 

@@ -47,25 +47,26 @@ def test_a_step_stays_absorbed_where_its_scratch_does_not_fit(monkeypatch):
     ws = SimpleNamespace(hold=0, device=device, offset=20 << 20, back=0, capacity=30 << 20)
     monkeypatch.setattr(kernels, "_active_workspace", [ws])
 
-    def pays(tokens=8000):
-        batch = SimpleNamespace(num_requests=1, num_tokens=tokens, host_q_start=[0, tokens], host_context_before=[0], attention_plan={},
+    def pays(cached, tokens):
+        batch = SimpleNamespace(num_requests=1, num_tokens=tokens, host_q_start=[0, tokens], host_context_before=[cached], attention_plan={},
                                 positions=SimpleNamespace(device=device))
         return kernels.latent_expand_pays(batch, 32, 128, 64, 128, 512)
 
-    need = 2 * (8000 * (32 * 256 + 576) + 8000 * 32 * 192)
+    need = 2 * (20100 * (32 * 256 + 576) + 100 * 32 * 192)
     grown = (need + ws.offset) * 9 // 8 - ws.capacity
     left(grown - (2 << 20))
-    assert pays() and len(asked) == 1
+    assert pays(20000, 100) and len(asked) == 1
     left(grown - (2 << 20) - 1)
-    assert not pays()
+    assert not pays(20000, 100)
     asked.clear()
     ws.capacity = ws.offset + need
     left(0)
-    assert pays() and pays(1600) and not asked                # the workspace holds it
+    assert pays(20000, 100) and not asked                     # the workspace holds it
     ws.capacity = 0
-    assert pays(1000) and not asked                           # little enough not to ask
+    assert pays(1000, 100) and not asked                      # little enough not to ask
+    assert pays(0, 8000) and not asked                        # the other form would take more
     monkeypatch.setattr(kernels, "_active_workspace", [None])
-    assert not pays() and asked == [device]
+    assert not pays(20000, 100) and asked == [device]
 
 
 def test_a_workspace_that_grows_gives_its_buffer_back_first(monkeypatch):
