@@ -11,7 +11,7 @@
 // and what waits for S is little: the triangle of the u_j is solved for both of its right-hand sides ahead, U from b_j v_j and W from
 // b_j P_j k_j, so that u = U - W S.  Three kernels, of which only the second walks a request's chunks one after the other:
 //     1  per (chunk, head)          W and U                          (fixed decay: Z = sum_i R_i,31 k_i v_i^T, all a chunk does to the state)
-//     2  per (request, head, cols)  u = U - W S (left where the outputs will be), the state before every chunk kept, S moved on
+//     2  per (request, head, cols)  u = U - W S, the state before every chunk kept, S moved on
 //                                   (fixed decay: S <- P_31 S + Z)
 //     3  per (chunk, head)          the outputs, from the kept states
 // The block scan they replace makes a chain of 900 instructions of every eight tokens with two to four warps an SM.  2,001 tokens in three portions, 32 heads:
@@ -289,38 +289,39 @@ __device__ __forceinline__ int longest(const Chunks& d, int rank, int lane) {
     return __ffs(__ballot_sync(0xffffffffu, lane < d.S && before == rank)) - 1;
 }
 
-// A CTA's whole walk by multiply-adds, where a sum of the tensor cores was not finite: all that the walk read is still there.  (A function of its own: its
-// numbers would take registers from the loop that has none to spare.)
+// A CTA's whole walk once more, token by token with multiply-adds, where a sum of the tensor cores was not finite: from the inputs (u has taken U's place),
+// the u of every token and the states before the chunks.  A thread has four rows of one column.  (A function of its own: its numbers would take registers
+// from the loop that has none to spare.)
 __device__ __noinline__ void walk_again(const Chunks& d, float* sm, int s, int head, int c0) {
-    const int tid = threadIdx.x, t_lo = d.q_start[s], t_hi = d.q_start[s + 1];
-    float *S = sm, *us = S + K * kColsB;                                     // [64][16], [32][16]: u times the decays behind it
-    float* S_g = d.state + (size_t)d.slots[s] * d.stride + (size_t)head * K * d.V + c0;
-    for (int i = tid; i < K * kColsB; i += kWalkThreads) S[i] = S_g[(size_t)(i / kColsB) * d.V + i % kColsB];
-    size_t at = (size_t)first_chunk(d.q_start, s) * d.N + head;
-    for (int t0 = t_lo; t0 < t_hi; t0 += CH, at += d.N) {
-        const int n = min(CH, t_hi - t0);
-        __syncthreads();
-        for (int i = tid; i < K * kColsB; i += kWalkThreads) d.s[(at * K + i / kColsB) * d.V + c0 + i % kColsB] = S[i];
-        for (int i = tid; i < n * kColsB; i += kWalkThreads) {
-            const int t = i / kColsB, c = i % kColsB;
-            float w = 0.f, behind = 1.f;
-            for (int k = 0; k < K; ++k) w = fmaf(d.w[(at * K + k) * CH + t], S[k * kColsB + c], w);
-            for (int j = n - 1; j > t; --j) behind *= d.g[(size_t)(t0 + j) * d.N + head];
-            const float u = d.u[(at * CH + t) * d.V + c0 + c] - w;
-            d.out[((size_t)(t0 + t) * d.N + head) * d.V + c0 + c] = u;
-            us[i] = u * behind;
+    constexpr int kGroups = kWalkThreads / kColsB, kRows = K / kGroups;
+    const int c = threadIdx.x % kColsB, rg = threadIdx.x / kColsB, t_lo = d.q_start[s], t_hi = d.q_start[s + 1];
+    float* S_g = d.state + (size_t)d.slots[s] * d.stride + ((size_t)head * K + rg * kRows) * d.V + c0 + c;
+    float S[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) S[i] = S_g[(size_t)i * d.V];
+    for (int t = t_lo; t < t_hi; ++t) {
+        const size_t at = (size_t)(first_chunk(d.q_start, s) + (t - t_lo) / CH) * d.N + head;
+        const float* k = d.k + (size_t)t * d.ld_k + head / (d.N / d.M) * K + rg * kRows;
+        const float g = d.g[(size_t)t * d.N + head];
+        float part = 0.f;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            if ((t - t_lo) % CH == 0) d.s[(at * K + rg * kRows + i) * d.V + c0 + c] = S[i];
+            S[i] *= g;
+            part = fmaf(S[i], k[i], part);
         }
+        float* parts = sm + (t & 1) * kWalkThreads;           // (a meeting a token: the other half is still read by who is behind)
+        parts[threadIdx.x] = part;
         __syncthreads();
-        float p = 1.f;
-        for (int j = n - 1; j >= 0; --j) p *= d.g[(size_t)(t0 + j) * d.N + head];
-        for (int i = tid; i < K * kColsB; i += kWalkThreads) {
-            float z = 0.f;
-            for (int t = 0; t < n; ++t) z = fmaf(d.k[(size_t)(t0 + t) * d.ld_k + head / (d.N / d.M) * K + i / kColsB], us[t * kColsB + i % kColsB], z);
-            S[i] = fmaf(p, S[i], z);
-        }
+        float sum = 0.f;
+        for (int r = 0; r < kGroups; ++r) sum += parts[r * kColsB + c];
+        const float u = d.beta[(size_t)t * d.N + head] * (d.v[(size_t)t * d.ld_v + (size_t)head * d.V + c0 + c] - sum);
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) S[i] = fmaf(k[i], u, S[i]);
+        if (rg == 0) d.u[(at * CH + (t - t_lo) % CH) * d.V + c0 + c] = u;
     }
-    __syncthreads();
-    for (int i = tid; i < K * kColsB; i += kWalkThreads) S_g[(size_t)(i / kColsB) * d.V + i % kColsB] = S[i];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) S_g[(size_t)i * d.V] = S[i];
 }
 
 __global__ void __launch_bounds__(kWalkThreads, 3)
@@ -369,8 +370,6 @@ chunk_walk_kernel(const __grid_constant__ Chunks d) {
     float2 own0 = *reinterpret_cast<const float2*>(S_g), own1 = *reinterpret_cast<const float2*>(S_g + 8 * d.V);
     *reinterpret_cast<float2*>(S + row0 * LDC + col0) = own0;
     *reinterpret_cast<float2*>(S + (row0 + 8) * LDC + col0) = own1;
-    // (u goes to where the outputs will be: U stays, should the walk have to be made again)
-    float* u_at = d.out + ((size_t)(t_lo + (warp & 1) * 16 + gr) * d.N + head) * d.V + c0 + (warp >> 1 & 1) * 8 + 2 * tq;
     float odd = 0.f;                                          // NaN once a sum of a second product (and so of a first one) is not finite
     for (int i = 0; i < chunks; ++i) {
         stages_wait<0>();
@@ -414,9 +413,8 @@ chunk_walk_kernel(const __grid_constant__ Chunks d) {
                 u.y -= (main[2 * h + 1] + (rest[0][2 * h + 1] + rest[1][2 * h + 1])) + half.y;
                 const float r = __shfl_sync(0xffffffffu, behind, t);
                 *reinterpret_cast<float2*>(us + t * LDC + c) = make_float2(u.x * r, u.y * r);
-                if (t < t_hi - t_lo - i * CH) *reinterpret_cast<float2*>(u_at + (size_t)8 * h * d.N * d.V) = u;
+                *reinterpret_cast<float2*>(d.u + (((size_t)(at0 + i) * d.N + head) * CH + t) * d.V + c0 + c) = u;
             }
-            u_at += (size_t)CH * d.N * d.V;
         } else {
             fetch(i + 1);
         }
@@ -514,9 +512,8 @@ chunk_output_kernel(const Chunks d) {
     stage_rows<kOutThreads>(qs, d.q + (size_t)t0 * d.ld_q + hk * K, d.ld_q, n);
     stage_rows<kOutThreads>(ks, d.k + (size_t)t0 * d.ld_k + hk * K, d.ld_k, n);
     stages_commit();
-    // (DELTA: the walk left u where this CTA's outputs will be)
-    const float* u = (DELTA ? d.out + (size_t)t0 * d.N * d.V : d.v + (size_t)t0 * d.ld_v) + (size_t)head * d.V + v0;
-    const int ld_u = DELTA ? d.N * d.V : d.ld_v;
+    const float* u = DELTA ? d.u + ((size_t)chunk * d.N + head) * CH * d.V + v0 : d.v + (size_t)t0 * d.ld_v + (size_t)head * d.V + v0;
+    const int ld_u = DELTA ? d.V : d.ld_v;
     const float* kept = d.s + ((size_t)chunk * d.N + head) * K * d.V + v0;
     for (int i = tid; i < K * VB / 4; i += kOutThreads) stage16(S + i / (VB / 4) * LDV + i % (VB / 4) * 4, kept + (size_t)(i / (VB / 4)) * d.V + i % (VB / 4) * 4, true);
     for (int i = tid; i < CH * VB / 4; i += kOutThreads) {
