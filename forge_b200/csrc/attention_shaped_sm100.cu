@@ -151,17 +151,6 @@ __device__ __forceinline__ u64 pair2(uint32_t lo, uint32_t hi) {
 __device__ __forceinline__ float low2(u64 v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float high2(u64 v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
-// Boxes of a tile that bring nothing (behind the window, beyond the request, or without a page in the table) count as zeros: what the slot held before may
-// be no number, which a weight of 0 would not silence.  (Out of line: the copies' loop has no instruction to spare.)
-__device__ __noinline__ void clear_boxes(uint8_t* tile, int blocks, uint32_t missing, uint32_t box_bytes) {
-    for (; missing != 0; missing &= missing - 1)
-        for (int b = 0; b < blocks; ++b)
-            for (uint32_t at = (threadIdx.x & 31) * 16; at < box_bytes; at += 512)
-                *reinterpret_cast<uint4*>(tile + b * kBlock + (__ffs(missing) - 1) * box_bytes + at) = make_uint4(0, 0, 0, 0);
-    fence_proxy_async();
-    __syncwarp();
-}
-
 // (Packed keys and values.)  A weight of 0 does not silence a number that is none: one among the values of a token reaches the tokens before it in its
 // tile, up to 127 of them.  A row with such a result therefore looks whether a later token of its tile has such a value in these 32 columns, and if so adds
 // its outputs up again over the keys that it sees, a thread on its own: time only where there is such a number.
@@ -298,7 +287,8 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
         const int head_blocks = packed ? group * ((p.D + p.E) / 64) : 0, row0 = packed ? p.row_start[req] : group * p.page_size;
         const int rounds = __shfl_sync(0xffffffffu, n_iter, 0);
         // one lane a box of rows: its page, or -1 where no token of the tile sees a key.  Asked for a tile ahead: a trip to the table takes longer than
-        // the products of a small tile
+        // the products of a small tile.  A box without a page (behind the window, beyond the request, or none in the table) is copied all the same, from before
+        // the cache's first page: the copy fills zeros in.  What the slot held before may be no number, which a weight of 0 would not silence
         auto page_of = [&](int it) {
             int page = -1;
             if (lane < ppt && it < rounds) {
@@ -309,7 +299,6 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
             return page;
         };
         const uint32_t box_bytes = p.box_rows * 128;
-        const uint32_t all_boxes = (1u << ppt) - 1;
         int st = 0, ph = 0, next_page = -1;
         if (warp == 0) {
             if (lane == 0) {
@@ -324,13 +313,11 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 int page = next_page;
                 next_page = page_of(it + 1);
                 if (page >= 0 && !packed && !FORGE_PAGE_OK(page)) page = -1;
-                const uint32_t live = __ballot_sync(0xffffffffu, page >= 0);
                 const int row = packed ? row0 + j0 : row0 + (j0 & page_mask);
                 if (!warp_wait<true>(&k_empty[st], ph ^ 1, abort, p.status, 1)) break;
-                if (live != all_boxes) clear_boxes(k_s + st * p.key_blocks * kBlock, p.key_blocks, all_boxes & ~live, box_bytes);
-                if (lane == 0) mbar_arrive_expect_tx(&k_full[st], p.key_blocks * __popc(live) * box_bytes);
+                if (lane == 0) mbar_arrive_expect_tx(&k_full[st], p.key_blocks * kBlock);
                 __syncwarp();
-                if (page >= 0) {
+                if (lane < ppt) {
                     uint8_t* dst = k_s + st * p.key_blocks * kBlock + lane * box_bytes;
                     for (int b = 0; b < others; b += p.v_boxed)
                         tma_load_4d(dst + b * kBlock, &tmap_v, &k_full[st], 0, row, head_blocks + (b < skip ? b : b + p.value_blocks), page);
@@ -350,16 +337,14 @@ shaped_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const 
                 int page = next_page;
                 next_page = page_of(it + 1);
                 if (page >= 0 && !packed && !FORGE_PAGE_OK(page)) page = -1;
-                const uint32_t live = __ballot_sync(0xffffffffu, page >= 0);
                 const int row = packed ? row0 + j0 : row0 + (j0 & page_mask);
                 const bool last = j0 + BKV - 1 > pos_last;                // rows behind the last token: cleared below
                 uint64_t* landed = last ? tail : &v_full[st];
                 uint8_t* vd = v_s + st * p.value_blocks * kBlock;
                 if (!warp_wait<true>(&v_empty[st], ph ^ 1, abort, p.status, 2)) break;
-                if (live != all_boxes) clear_boxes(vd, p.value_blocks, all_boxes & ~live, box_bytes);
-                if (lane == 0) mbar_arrive_expect_tx(landed, p.value_blocks * __popc(live) * box_bytes);
+                if (lane == 0) mbar_arrive_expect_tx(landed, p.value_blocks * kBlock);
                 __syncwarp();
-                if (page >= 0)
+                if (lane < ppt)
                     for (int b = 0; b < p.value_blocks; b += p.v_boxed)
                         tma_load_4d(vd + b * kBlock + lane * box_bytes, &tmap_v, landed, 0, row, block0 + b, page);
                 if (last) {

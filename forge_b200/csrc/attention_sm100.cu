@@ -236,22 +236,12 @@ paged_attention_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
             int page = next_page;
             next_page = page_of(it + 1);
             if (page >= 0 && !FORGE_PAGE_OK(page)) page = -1;
-            const uint32_t live = __ballot_sync(0xffffffffu, page >= 0);
             if (!warp_wait<true>(&empty[st], ph ^ 1, abort, p.status, values ? 9 : 1)) break;
-            // Pages that bring nothing (beyond the request, released by the window, or none in the table) count as zeros: what the slot held before may
-            // be no number, which a weight of 0 would not silence
-            if (__popc(live) < ppt) {
-                for (int i = 0; i < ppt; ++i)
-                    if (!(live >> i & 1))
-                        for (int kb = 0; kb < KB; ++kb)
-                            for (uint32_t at = lane * 16; at < page_bytes; at += 512)
-                                *reinterpret_cast<uint4*>(ring + st * kKVBytes + kb * kKVBlock + i * page_bytes + at) = make_uint4(0, 0, 0, 0);
-                fence_proxy_async();
-                __syncwarp();
-            }
-            if (lane == 0) mbar_arrive_expect_tx(&full[st], KB * __popc(live) * page_bytes);
+            if (lane == 0) mbar_arrive_expect_tx(&full[st], kKVBytes);
             __syncwarp();
-            if (page >= 0) {
+            // A page that brings nothing (beyond the request, released by the window, or none in the table) is copied all the same, from rows before the
+            // cache's first: the copy fills zeros in.  What the slot held before may be no number, which a weight of 0 would not silence.
+            if (lane < ppt) {
                 const int row = ((page * 2 + (values ? 1 : 0)) * p.NKV + kvh) * p.page_size;
                 uint8_t* dst = ring + st * kKVBytes + lane * page_bytes;
                 if (ppt == 1) tma_load_3d(dst, &tmap_kv, &full[st], 0, row, 0);              // (a box of all blocks)
