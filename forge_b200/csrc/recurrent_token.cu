@@ -94,14 +94,19 @@ __device__ __forceinline__ void convolve_tile(const DeltaPrepare& d, const float
         }
 #pragma unroll
         for (int j = 0; j < TP; ++j) w[j] = j < d.cv.taps ? __ldg(d.cv.w + (size_t)j * d.cv.channels + c) : 0.f;
+        // (a tap that the filter has not meets no input, not even one that is none)
+        auto sums = [&](bool whole) {
 #pragma unroll
-        for (int k = 0; k < kPrepTokens; ++k) {
-            float a = 0.f;
+            for (int k = 0; k < kPrepTokens; ++k) {
+                float a = 0.f;
 #pragma unroll
-            for (int j = TP - 1; j >= 0; --j)
-                if (j < d.cv.taps) a = fmaf(w[j], v[TP - 1 + k - j], a);      // (a tap that the filter has not meets no input, not even one that is none)
-            y[k] = siluf(a);
-        }
+                for (int j = TP - 1; j >= 0; --j)
+                    if (whole || j < d.cv.taps) a = fmaf(w[j], v[TP - 1 + k - j], a);
+                y[k] = siluf(a);
+            }
+        };
+        if (d.cv.taps == TP) sums(true);
+        else sums(false);
         return;
     }
     for (int k = 0; k < kPrepTokens; ++k) {
